@@ -74,8 +74,8 @@ def parse():
     ap.add_argument("--extras-steps", type=int, default=400, help="batched section: steps per variant")
     ap.add_argument("--learned-runs", type=int, default=40, help="learned section: teacher runs")
     ap.add_argument("--learned-steps", type=int, default=1000, help="learned section: timed steps")
-    ap.add_argument("--path", choices=["fused", "slab", "hs", "dropin", "default", "all"], default="default",
-                    help="default = per-call loop (per-kernel timing) + Simulation.run (hs path); "
+    ap.add_argument("--path", choices=["fused", "slab", "hs", "ahead", "dropin", "default", "all"], default="default",
+                    help="default = per-call loop (per-kernel timing) + Simulation.run (ahead path); hs = E and H+S launches; "
                          "slab = run over the per-update kernels; fused = the opt-in fused step")
     return ap.parse_args()
 
@@ -165,7 +165,9 @@ def algorithmic_bytes(N: int, face_cells: int, elem: int, poynting: bool):
     # run()'s H+S kernel: H read (one copy) and written (the other), E read, S written;
     # psi_H read / written
     hs = N * 12 * elem + face_cells * 4 * elem
-    return {"k_bulk_e": e, "k_bulk_h": h, "k_bulk_s": s, "k_bulk_hs": hs}, step
+    # the same launch with the next step's E in it: dt/eps read and E written too, psi_E read / written
+    ahead = N * 18 * elem + face_cells * 8 * elem
+    return {"k_bulk_e": e, "k_bulk_h": h, "k_bulk_s": s, "k_tile_h": hs, "k_tile_h (E ahead)": ahead}, step
 
 
 # FP64 DFT monitor of the c2 ringdown (the north star's "FP64 DFT monitor at 5 interior points"):
@@ -325,8 +327,9 @@ def time_dropin(sim, lib, wave_dev, ind, K, W, poynting, world):
 
 
 def time_run(sim, lib, wave_dev, ind, K, W, world, mode, monitor=None):
-    """K steps in one fdtd_run call bracketed by CUDA events. mode: 'hs' (E in place, H and S
-    in one launch), 'fused' (one kernel per step) or None (the per-update kernels); monitor: a
+    """K steps in one fdtd_run call bracketed by CUDA events. mode: 'ahead' (H, S and the next
+    step's E in one launch), 'hs' (E in place, H and S in one launch), 'fused' (one kernel per
+    step) or None (the per-update kernels); monitor: a
     DftMonitor sampled after every timed step (inside the timed region)."""
     import torch
     from opencl_fdtd_gb300 import _lib
@@ -335,6 +338,7 @@ def time_run(sim, lib, wave_dev, ind, K, W, world, mode, monitor=None):
         sim._ensure_scratch(mode)
     bufs = sim._buffers()
     sim._attach_scratch(mode)
+    sim._set_ahead(mode == "ahead")
     st = ctypes.c_void_p(stream.cuda_stream)
     idx = (ctypes.c_int64 * 1)(ind)
     esz = wave_dev.element_size()
@@ -361,16 +365,17 @@ def time_run(sim, lib, wave_dev, ind, K, W, world, mode, monitor=None):
     return e0.elapsed_time(e1)
 
 
-def run_kernel_ms(sim, lib, wave_dev, ind, steps):
-    """Mean launch times of the H+S path's two kernels: one more fdtd_run with the plan's
-    timing events on (CUDA events on the launching stream around update_E and the H+S kernel
-    of up to 64 sampled steps)."""
+def run_kernel_ms(sim, lib, wave_dev, ind, steps, mode):
+    """Mean launch times of an H path's kernels: one more fdtd_run with the plan's timing events on
+    (CUDA events on the launching stream around update_E and the H launch of up to 64 sampled
+    steps). On the 'ahead' path update_E runs in the first step only."""
     import torch
     from opencl_fdtd_gb300 import _lib
     stream = sim.queue
-    sim._ensure_scratch("hs")
+    sim._ensure_scratch(mode)
     bufs = sim._buffers()
-    sim._attach_scratch("hs")
+    sim._attach_scratch(mode)
+    sim._set_ahead(mode == "ahead")
     idx = (ctypes.c_int64 * 1)(ind)
     src = _lib.FdtdPointSources(1, 0, ctypes.addressof(idx), wave_dev.data_ptr())
     _lib.check(lib.fdtd_plan_tune(sim._plan, _lib.FDTD_TUNE_TIMING, 1))
@@ -382,7 +387,9 @@ def run_kernel_ms(sim, lib, wave_dev, ind, steps):
     ms = (ctypes.c_double * 2)()
     n = ctypes.c_int32()
     _lib.check(lib.fdtd_run_kernel_ms(sim._plan, ms, ctypes.byref(n)))
-    return {"k_bulk_e": ms[0], "k_bulk_hs": ms[1]}, n.value
+    if mode == "ahead":
+        return {"k_tile_h (E ahead)": ms[1]}, n.value
+    return {"k_bulk_e": ms[0], "k_tile_h": ms[1]}, n.value
 
 
 def c2_parity(wl, steps: int):
@@ -519,9 +526,12 @@ def main():
     if args.path in ("dropin", "default", "all"):
         res["dropin"] = time_dropin(sim, lib, wave_dev, ind, K, W, poynting, world)
     mon = sim.dft_monitor(monitor_points(wl), monitor_omegas(), record=False) if wl["name"] == "c2" else None
-    if args.path in ("hs", "default", "all") and poynting:
-        res["hs"] = time_run(sim, lib, wave_dev, ind, K, W, world, "hs", monitor=mon)
-        hs_per = run_kernel_ms(sim, lib, wave_dev, ind, min(W + K, 640))
+    if args.path in ("ahead", "default", "all"):
+        res["ahead"] = time_run(sim, lib, wave_dev, ind, K, W, world, "ahead", monitor=mon)
+        hs_per = {"ahead": run_kernel_ms(sim, lib, wave_dev, ind, min(W + K, 640), "ahead")}
+    if args.path in ("hs", "all") and poynting:
+        res["hs"] = time_run(sim, lib, wave_dev, ind, K, W, world, "hs", monitor=mon if args.path == "hs" else None)
+        hs_per = {"hs": run_kernel_ms(sim, lib, wave_dev, ind, min(W + K, 640), "hs"), **(hs_per if args.path == "all" else {})}
     if args.path in ("slab", "all"):
         res["slab"] = time_run(sim, lib, wave_dev, ind, K, W, world, None)
         sim.tune(slab=0)
@@ -553,7 +563,7 @@ def main():
                          "mean_launch_ms": round(per[dom], 5),
                          "per_kernel_ms": {k: round(v, 5) for k, v in per.items()}}}
     compulsory = N * (18 if poynting else 15) * elem + fc * 8 * elem
-    for name in ("fused", "slab", "hs"):
+    for name in ("fused", "slab", "hs", "ahead"):
         if name not in res:
             continue
         total = allmax(res[name])
@@ -561,15 +571,16 @@ def main():
         ach = step_bytes / (ms * 1e-3) / 1e9
         nslab = (wl["shape"][0] + sim.slab_planes() - 1) // sim.slab_planes()
         # per step: the path's kernels (the workload's one point source is added inside k_step
-        # on the fused path and inside the E kernel on the hs path) and the DFT monitor sample
-        # when the monitor is timed (on the hs path by one block of the H+S launch unless the
-        # plan's hs_dft is off)
-        launches = {"fused": K, "hs": 2 * K,
+        # on the fused path and inside the kernel that updates E on the hs and ahead paths) and the
+        # DFT monitor sample when the monitor is timed (on the hs and ahead paths by one block of
+        # the H launch unless the plan's hs_dft is off)
+        launches = {"fused": K, "hs": 2 * K, "ahead": K + 1,
                     "slab": K * ((3 if poynting else 2) * nslab + (3 if poynting else 1) + 1)}[name]
-        if mon is not None and ((name == "hs" and not sim.tuning("hs_dft"))
+        if mon is not None and ((name in ("hs", "ahead") and not sim.tuning("hs_dft"))
                                 or (name == "fused" and args.path == "fused")):
             launches += K
-        kname = {"fused": "k_step", "hs": "step (k_bulk_e + k_bulk_hs)",
+        kname = {"fused": "k_step", "hs": "step (k_bulk_e + k_tile_h)",
+                 "ahead": "k_tile_h (E ahead): one launch per step",
                  "slab": "step (k_bulk_e/h/s over L2 slabs)"}[name]
         out_paths[name] = {
             "ms_per_step": ms, "value": world * N * K / (total * 1e-3) / 1e6, "gpu_launches": launches,
@@ -582,18 +593,20 @@ def main():
                          "compulsory_bytes_per_step": compulsory,
                          "compulsory_frac": round(compulsory / (ms * 1e-3) / 1e9 / peak, 4),
                          "mean_step_ms": round(ms, 5)}}
-    if "hs" in out_paths:
-        per, nsamp = hs_per
+    for name in ("hs", "ahead"):
+        if name not in out_paths:
+            continue
+        per, nsamp = hs_per[name]
         dom = max(per, key=lambda k: per[k])
         ach = per_launch[dom] / (per[dom] * 1e-3) / 1e9
-        out_paths["hs"]["kernel_roofline"] = {
+        out_paths[name]["kernel_roofline"] = {
             "bound": "hbm", "kernel": dom, "achieved": round(ach, 1), "peak": peak, "unit": "GB/s",
             "frac": round(ach / peak, 4), "peak_source": peak_kind, "traffic": traffic.get(dom),
             "algorithmic_bytes_per_launch": per_launch[dom], "mean_launch_ms": round(per[dom], 5),
             "per_kernel_ms": {k: round(v, 5) for k, v in per.items()}, "sampled_launches": nsamp,
             "per_kernel_frac": {k: round(per_launch[k] / (v * 1e-3) / 1e9 / peak, 4)
                                 for k, v in per.items()}}
-    cands = [n for n in ("fused", "slab", "hs") if n in out_paths]
+    cands = [n for n in ("fused", "slab", "hs", "ahead") if n in out_paths]
     head = min(cands, key=lambda n: out_paths[n]["ms_per_step"]) if cands else "dropin"
     hp = out_paths[head]
     step_gbs = step_bytes / (hp["ms_per_step"] * 1e-3) / 1e9
@@ -601,7 +614,7 @@ def main():
     launch = ({"hs_xchunk": sim.tuning("hs_xchunk_used"), "pdl": sim.tuning("pdl"),
                "dft_in_hs_launch": sim.tuning("hs_dft"), "e_xchunk": sim.tuning("xchunk"),
                "e_form": sim.tuning("e_form")}
-              if head == "hs" else None)
+              if head in ("hs", "ahead") else None)
 
     e2e = None
     if not args.no_e2e:
@@ -609,7 +622,8 @@ def main():
         e2e_mon = (sim.dft_monitor(monitor_points(wl), monitor_omegas(), record=False)
                    if wl["name"] == "c2" else None)
         e2e = run_e2e(sim, wl, args.e2e_steps, world, run_api=(head != "dropin"),
-                      path={"fused": "fused", "hs": "hs", "slab": "plain"}.get(head, "auto"), monitor=e2e_mon)
+                      path={"fused": "fused", "hs": "hs", "slab": "plain", "ahead": "ahead"}.get(head, "auto"),
+                      monitor=e2e_mon)
 
     mon_out = None
     if mon is not None and mon.samples:
@@ -636,7 +650,8 @@ def main():
             "data": "synthetic (seeded L3 cavity geometry and source)",
             "config": workload_config(wl, fc, elem, poynting),
             "path": {"fused": "Simulation.run(path='fused'): one fused E+source+H+S kernel per step",
-                                "hs": "Simulation.run: E in place, point source, H+S in one launch (H ping-pong)",
+                                "ahead": "Simulation.run: H, S and the next step's E in one launch (E and H ping-pong)",
+                                "hs": "Simulation.run(path='hs'): E in place, point source, H+S in one launch (H ping-pong)",
                                 "slab": "Simulation.run(path='plain'): E, point source, H, S update kernels",
                                 "dropin": "per-call update_E / source add / update_H / update_S"}[head],
             "parallelism": "replicas" if world > 1 else "single GPU",

@@ -97,11 +97,12 @@ typedef struct FdtdBuffers {
     void *ce, *cm;
     /* Optional second copies for fdtd_run (same sizes as E, H, psi_e, psi_h). With H2 and every
      * psi_h2 set (E2 NULL), steps run update_E in place and H and S in one launch that reads
-     * one copy of H and writes the other (z rows of at most 224 cells; longer rows, Bloch
-     * boundaries or overlapping CPML faces use the per-update kernels). With E2, H2 and every psi_e2 / psi_h2 set, each step
-     * is one launch of the one-pass kernel, which reads one copy of everything and writes the
-     * other. At the end the result is always back in E, H, psi_e, psi_h. When NULL, fdtd_run
-     * uses the per-update kernels. Results are identical either way. */
+     * one copy of H and writes the other (Poynting on, z rows of at most 224 cells). With E2, H2 and
+     * every psi_e2 / psi_h2 set, each step is one launch: with FDTD_TUNE_HS_AHEAD the H and S launch
+     * that also makes the next step's E (float32, no learned boundary), else the one-pass kernel;
+     * both read one copy of everything and write the other. Bloch boundaries and overlapping CPML
+     * faces take the per-update kernels. At the end the result is always back in E, H, psi_e,
+     * psi_h. When NULL, fdtd_run uses the per-update kernels. Results are identical either way. */
     void *E2, *H2;
     void *psi_e2[6][2], *psi_h2[6][2];
 } FdtdBuffers;
@@ -120,7 +121,8 @@ int fdtd_plan_create(const FdtdDesc *desc, FdtdPlan **out);
 int fdtd_plan_destroy(FdtdPlan *plan);
 
 /* Tuning keys of fdtd_plan_tune. Any values give the same results.
- *   XCHUNK        consecutive x planes one thread of the update kernels advances (default 8)
+ *   XCHUNK        consecutive x planes one thread of the update kernels advances (default 8, fewer
+ *                 on grids too small to fill the GPU with that many)
  *   SLAB          x planes per L2-resident slab of fdtd_run's per-update schedule
  *                 (default 0 = whole grid)
  *   FUSED_ROWS    own y rows of a tile of the one-pass step (default 0: the most that fit a
@@ -135,16 +137,20 @@ int fdtd_plan_destroy(FdtdPlan *plan);
  *   FUSED_SHAPE   block shape of the one-pass step: 1 large (up to 1024 threads, one block per
  *                 SM), 2 small (up to 512 threads, two blocks per SM; float32 only), 0
  *                 (default) small when its tiles hold at least 3 own rows
- *   HS_XCHUNK     x planes one block of the H+S kernel of fdtd_run marches; 0 (default): chosen
- *                 per launch among 14..24 so that the grid best fills whole waves of resident
- *                 blocks (18 on the 395x345x73 grid of a 152-SM GPU)
- *   HS_PREFETCH   1: the H+S kernel loads the next plane ahead (one block per SM); 0: not
- *                 (two blocks per SM, the default)
+ *   HS_XCHUNK     x planes one block of the H kernel of fdtd_run marches; 0 (default): chosen per
+ *                 launch so that the grid best fills whole waves of resident blocks, among 14..24
+ *                 (18 on the 395x345x73 grid of a 152-SM GPU) and with the next step's E, or where
+ *                 those make no wave, among 1..12
+ *   HS_PREFETCH   accepted, without effect: the H kernel always issues the next plane's loads before
+ *                 the barrier of the current one
  *   HS_REVERSE    1 (default): the H+S kernel takes its x chunks in descending order, so that it
- *                 starts on the planes update_E wrote last (still in L2); 0: ascending
+ *                 starts on the planes update_E wrote last (still in L2); 0: ascending (with HS_AHEAD
+ *                 the order alternates from step to step and this picks the first)
+ *   HS_AHEAD      1: with second copies of E and H, the H launch of every step but the last also
+ *                 makes the next step's E; 0 (default): those copies select the one-pass step
  *   HS_DFT        1 (default): on the H+S path the step's DFT monitor sample is taken by one extra
  *                 block of the H+S launch; 0: by the monitor kernel on a side stream beside it
- *   PDL           1 (default): on the H+S path the E and H+S kernels are launched with
+ *   PDL           1 (default): the E and H kernels of fdtd_run are launched with
  *                 programmatic stream serialization (each may be scheduled while the kernel
  *                 before it finishes, and waits for it before touching memory); 0: plain stream
  *                 order
@@ -169,6 +175,7 @@ int fdtd_plan_destroy(FdtdPlan *plan);
 #define FDTD_TUNE_HS_DFT 13
 #define FDTD_TUNE_PDL 14
 #define FDTD_TUNE_E_FORM 15
+#define FDTD_TUNE_HS_AHEAD 16
 /* Read-only keys of fdtd_plan_get: the path of the last fdtd_run (FDTD_PATH_*), the tiling
  * of its last one-pass launch (own rows per tile, x chunk, stages, threads per block, shape)
  * and the x chunk of its last H+S launch. */
@@ -181,7 +188,7 @@ int fdtd_plan_destroy(FdtdPlan *plan);
 #define FDTD_GET_HS_XCHUNK_USED 106
 #define FDTD_PATH_NONE 0
 #define FDTD_PATH_PER_UPDATE 1     /* update_E, sources, update_H, update_S launches */
-#define FDTD_PATH_HS 2             /* update_E in place, sources, H and S in one launch */
+#define FDTD_PATH_HS 2             /* H and S in one launch, after update_E or (HS_AHEAD) with the next step's E */
 #define FDTD_PATH_ONEPASS 3        /* E, sources, H and S of a step in one launch */
 int fdtd_plan_tune(FdtdPlan *plan, int32_t key, int32_t value);
 /* Current value of a tuning key. */
@@ -273,19 +280,20 @@ int fdtd_count_nonfinite(FdtdPlan *plan, const FdtdBuffers *buf, uint32_t *count
 /* Run nsteps canonical steps (fdtd.py:162-175: E, F, point sources, H, G, S) on the stream
  * with no host round trip. src and mon may be NULL; mon is sampled after every step and its
  * step / series_row advance by nsteps. With the second copies of FdtdBuffers set (and no
- * Bloch boundaries, at most 8 sources, no overlapping CPML faces) each step is two launches
- * (H2 and psi_h2: update_E in place, then H and S) or one (E2, H2 and every psi copy: the
- * one-pass step); oS is then written on the last step only. The path taken is read back with
- * fdtd_plan_get(FDTD_GET_LAST_RUN_PATH). On the H+S path the E kernel adds up to 8 point
- * sources itself (without a learned boundary), the monitor sample of each step is taken by
- * one extra block of the H+S launch (FDTD_TUNE_HS_DFT; 0: by the monitor kernel on a stream of
- * the plan beside the H+S launch, joined back into `stream` before the call returns), and the
- * two kernels use programmatic dependent launch (FDTD_TUNE_PDL). */
+ * Bloch boundaries, no overlapping CPML faces) a step is two launches (H2 and psi_h2: update_E in
+ * place, then H and S) or one (E2, H2 and every psi copy: FDTD_TUNE_HS_AHEAD, or the one-pass step
+ * with at most 8 sources); oS is then written on the last step only. The path taken is read back
+ * with fdtd_plan_get(FDTD_GET_LAST_RUN_PATH). The kernel that updates E adds up to 8 point sources
+ * itself (without a learned boundary); on the H path the monitor sample of each step is taken by
+ * one extra block of the H launch (FDTD_TUNE_HS_DFT; 0: by the monitor kernel on a stream of the
+ * plan beside the H launch, joined back into `stream` before the call returns). The E and H kernels
+ * of a run use programmatic dependent launch (FDTD_TUNE_PDL). */
 int fdtd_run(FdtdPlan *plan, const FdtdBuffers *buf, void *stream, int32_t nsteps,
              const FdtdPointSources *src, FdtdDftMonitor *mon);
 
 /* Mean launch time in ms over the sampled steps of the last fdtd_run made with FDTD_TUNE_TIMING
- * on: update_E (ms[0]) and the H+S kernel (ms[1]) on the H+S path, the step kernel (ms[0]; ms[1]
+ * on: update_E (ms[0]; with HS_AHEAD the first step's, averaged over all samples) and the H kernel
+ * (ms[1]) on the H path, the step kernel (ms[0]; ms[1]
  * = 0) on the one-pass path; and the number of samples (0 if none). Profiling aid; no
  * counterpart in the reference. */
 int fdtd_run_kernel_ms(const FdtdPlan *plan, double ms[2], int32_t *samples);

@@ -74,11 +74,14 @@ bool faces_disjoint(const FdtdPlan *p)
 template <typename R>
 YeeK<R> make_yee(const FdtdPlan *p, bool etype, bool imag, R *P, const R *Q, const R *Rp,
                  const R *mat, const R *coef, R *oS, void *const psi[6][2],
-                 const void *const inv_tab[3])
+                 const void *const inv_tab[3], R *W = nullptr, void *const (*psi_w)[2] = nullptr)
 {
+    // W, psi_w: where the bulk kernels write the field and its psi (in place when NULL)
+    if (!psi_w) psi_w = psi;
     YeeK<R> k;
     std::memset(&k, 0, sizeof(k));
     k.P = P;
+    k.W = W ? W : P;
     k.Q = Q;
     k.Rp = Rp;
     k.mat = mat;
@@ -113,14 +116,15 @@ YeeK<R> make_yee(const FdtdPlan *p, bool etype, bool imag, R *P, const R *Q, con
         fk.psi_v = (R *)psi[f][1];
         AxisK<R> &ak = k.ax[pd.axis];
         const uint32_t sa = pd.axis == 0 ? p->sx : pd.axis == 1 ? p->sy : p->sz;
-        if (pd.polarity == 0) {
-            ak.Tn = pd.thickness;
-            ak.n0 = fk.p0; ak.n1 = fk.p1; ak.n2 = fk.p2;
-            ak.nu = fk.psi_u; ak.nv = fk.psi_v;
-        } else if ((uint32_t)pd.thickness <= sa) {
-            ak.Tp = pd.thickness;
-            ak.p0 = fk.p0; ak.p1 = fk.p1; ak.p2 = fk.p2;
-            ak.pu = fk.psi_u; ak.pv = fk.psi_v;
+        if (pd.polarity == 1 && (uint32_t)pd.thickness > sa) continue;
+        if (pd.polarity == 0) ak.Tn = pd.thickness;
+        else ak.Tp = pd.thickness;
+        ak.f.tab[pd.polarity][0] = fk.p0;
+        ak.f.tab[pd.polarity][1] = fk.p1;
+        ak.f.tab[pd.polarity][2] = fk.p2;
+        for (int c = 0; c < 2; ++c) {
+            ak.f.A[pd.polarity][c] = (const R *)psi[f][c];
+            ak.f.B[pd.polarity][c] = (R *)psi_w[f][c];
         }
     }
     k.bloch_mask = 0;
@@ -140,35 +144,42 @@ YeeK<R> make_yee(const FdtdPlan *p, bool etype, bool imag, R *P, const R *Q, con
     return k;
 }
 
+// The point sources of step t as arguments of a kernel that adds them itself (at most YEE_SRC).
+template <typename R, typename K>
+void kernel_sources(const FdtdPlan *p, K &k, const FdtdPointSources *src, int t)
+{
+    k.nsrc = src->n;
+    k.src_t = t;
+    k.src_stride = src->n;
+    k.src_values = (const R *)src->values;
+    for (int s = 0; s < src->n; ++s) {
+        const uint64_t ind = (uint64_t)src->index[s], cell = ind % p->N;
+        k.src_c[s] = (int32_t)(ind / p->N);
+        k.src_x[s] = (uint32_t)(cell / p->syz);
+        k.src_j[s] = (uint32_t)(cell % p->syz);
+        k.src_col[s] = s;
+    }
+}
+
 // With `src` (E only, all planes): the bulk kernel adds the step's point sources itself after
 // the update, when there are at most YEE_SRC of them; *added tells the caller.
 template <typename R>
 int run_update_e(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, bool imag,
                  uint32_t xbeg = 0, uint32_t xend = 0xffffffffu,
                  const FdtdPointSources *src = nullptr, int t = 0, bool *added = nullptr,
-                 bool pdl = false)
+                 bool pdl = false, void *W = nullptr, void *const (*psi_w)[2] = nullptr)
 {
     R *P = (R *)(imag ? b->F : b->E);
     const R *Q = (const R *)(imag ? b->G : b->H);
     const R *Rp = p->d.n_bloch ? (const R *)(imag ? b->H : b->G) : nullptr;
     void *const(*psi)[2] = imag ? b->psi_f : b->psi_e;
     YeeK<R> k = make_yee<R>(p, true, imag, P, Q, Rp, (const R *)b->eps, (const R *)b->ce, nullptr,
-                            psi, b->inv_dh);
+                            psi, b->inv_dh, (R *)W, psi_w);
     k.xbeg = xbeg;
     k.xend = xend < p->sx ? xend : p->sx;
     if (added) *added = false;
     if (src && added && !imag && k.bulk && src->n > 0 && src->n <= YEE_SRC && k.xbeg == 0 && k.xend == p->sx) {
-        k.nsrc = src->n;
-        k.src_t = t;
-        k.src_stride = src->n;
-        k.src_values = (const R *)src->values;
-        for (int s = 0; s < src->n; ++s) {
-            const uint64_t ind = (uint64_t)src->index[s], cell = ind % p->N;
-            k.src_c[s] = (int32_t)(ind / p->N);
-            k.src_x[s] = (uint32_t)(cell / p->syz);
-            k.src_j[s] = (uint32_t)(cell % p->syz);
-            k.src_col[s] = s;
-        }
+        kernel_sources<R>(p, k, src, t);
         *added = true;
     }
     return check_cuda(launch_yee_e<R>(k, st, pdl), imag ? "update_F launch" : "update_E launch");
@@ -176,7 +187,8 @@ int run_update_e(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, bool imag,
 
 template <typename R>
 int run_update_h(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, bool imag,
-                 uint32_t xbeg = 0, uint32_t xend = 0xffffffffu)
+                 uint32_t xbeg = 0, uint32_t xend = 0xffffffffu, bool pdl = false, void *W = nullptr,
+                 void *const (*psi_w)[2] = nullptr)
 {
     R *P = (R *)(imag ? b->G : b->H);
     const R *Q = (const R *)(imag ? b->F : b->E);
@@ -185,10 +197,10 @@ int run_update_h(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, bool imag,
     const bool poynt = p->d.do_poynting && !imag;
     YeeK<R> k = make_yee<R>(p, false, imag, P, Q, Rp, p->d.has_mu ? (const R *)b->mu : nullptr,
                             p->d.has_mu ? (const R *)b->cm : nullptr,
-                            poynt ? (R *)b->oS : nullptr, psi, b->inv_de);
+                            poynt ? (R *)b->oS : nullptr, psi, b->inv_de, (R *)W, psi_w);
     k.xbeg = xbeg;
     k.xend = xend < p->sx ? xend : p->sx;
-    return check_cuda(launch_yee_h<R>(k, p->d.has_mu != 0, poynt, st),
+    return check_cuda(launch_yee_h<R>(k, p->d.has_mu != 0, poynt, st, pdl),
                       imag ? "update_G launch" : "update_H launch");
 }
 
@@ -387,36 +399,83 @@ static int side_stream(FdtdPlan *p)
     return check_cuda(cudaEventCreateWithFlags(&p->ev_join, cudaEventDisableTiming), "join event");
 }
 
-// x chunk of the H+S kernel when none is set: among 14..24 planes, the one whose grid (plus
-// the extra blocks) best fills whole waves of resident blocks, two per SM; the smallest such
-// chunk on a tie. On the 395x345x73 grid (69 row blocks, 152 SMs) it is 18: 1518 blocks, 4.99
-// waves, which ran 2% faster per step than 16 planes (5.67 waves).
-static uint32_t hs_auto_xchunk(const FdtdPlan *p, uint32_t nrowblk, uint32_t extra)
+// Tiles and x chunk of an H launch. A tile is own rows by own columns (a z row in nseg equal
+// segments) of a block whose threads also evaluate one halo row and one halo column: of the splits the
+// one with the most own cells, in segments of at least 37 cells where the row is that long (shorter runs waste memory sectors).
+// The x chunk (unless set) makes the launch's whole waves of resident blocks, two per SM, as full as
+// it can: for the form with the next step's E among 1..12 planes by the time the waves take, which is
+// a block's planes and the one it evaluates ahead of them (a step of 200^3 cells: 0.153 ms at 9 planes,
+// 0.166 at 20; of 64^3: 0.0138 at 3, 0.0166 at 4); for the other, where that makes a wave at all, among
+// 14..24 by the share of whole waves (on the 395x345x73 grid 18: 1518 blocks, 4.99 waves, 2% faster
+// per step than 16).
+template <typename R>
+static void hs_layout(const FdtdPlan *p, HSK<R> &k, const HSForm &f, uint32_t extra)
 {
-    int nsm = 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess || nsm <= 0)
-        nsm = 1;
-    const double slots = 2.0 * nsm;
-    uint32_t best = 16;
-    double best_eff = -1.0;
-    for (uint32_t xc = 14; xc <= 24; ++xc) {
-        const double waves = (double)(nrowblk * ((p->sx + xc - 1u) / xc) + extra) / slots;
-        const double eff = waves / std::ceil(waves);
-        if (eff > best_eff + 1e-12) {
-            best_eff = eff;
-            best = xc;
+    const bool ahead = f.ahead;
+    const uint32_t threads = (uint32_t)hs_threads(f.ahead, f.mu, f.dxmode);
+    uint64_t best = 0;
+    for (uint32_t n = (p->sz + threads / 2u - 2u) / (threads / 2u - 1u); n <= p->sz; ++n) {
+        const uint32_t len = (p->sz + n - 1u) / n;
+        if (best && len < 37u) break;
+        uint32_t r = threads / (len + 1u) - 1u;                  // at least one own row
+        if (r > p->sy) r = p->sy;
+        const uint32_t nseg = (p->sz + len - 1u) / len, tiles = nseg * ((p->sy + r - 1u) / r);
+        const uint64_t share = ((uint64_t)p->syz << 20) / ((uint64_t)tiles * threads);
+        if (share > best) {
+            best = share;
+            k.rows = r;
+            k.seglen = len;
+            k.nseg = nseg;
+            k.ntile = tiles;
         }
     }
-    return best;
+    int nsm = 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, p->device) != cudaSuccess || nsm <= 0) nsm = 1;
+    const double slots = 2.0 * nsm;
+    // chunks of 14 planes and more only where they make a wave
+    const bool shorter = ahead || (double)((uint64_t)k.ntile * ((p->sx + 13u) / 14u)) < slots;
+    k.xchunk = p->hs_xchunk;
+    double best_eff = -1.0;
+    for (uint32_t xc = shorter ? 1u : 14u; !p->hs_xchunk && xc <= (shorter ? 12u : 24u); ++xc) {
+        const double waves = (double)((uint64_t)k.ntile * ((p->sx + xc - 1u) / xc) + extra) / slots;
+        const double eff = shorter ? 1.0 / (std::ceil(waves) * (xc + 1u)) : waves / std::ceil(waves);
+        if (eff > best_eff * (1.0 + 1e-12)) {
+            best_eff = eff;
+            k.xchunk = xc;
+        }
+    }
+    if (k.xchunk > p->sx) k.xchunk = p->sx;
+    k.nchunk = (p->sx + k.xchunk - 1u) / k.xchunk;
 }
 
-// Multi-step path with the H+S kernel: update_E in place, point sources, then H and S in one
-// launch that reads H (and the H-side psi) from one copy and writes the other; the copies
-// swap every step and the state is brought home after an odd number of steps.
+// Copies one field and its psi arrays (the ones of `bytes` per face) from src to dst.
+static int copy_state(const FdtdPlan *p, void *dst, const void *src, void *const dpsi[6][2], void *const spsi[6][2],
+                      cudaStream_t st)
+{
+    int rc = check_cuda(cudaMemcpyAsync(dst, src, 3 * (size_t)p->N * p->elem, cudaMemcpyDeviceToDevice, st), "copy field");
+    for (int f = 0; !rc && f < p->d.n_pml; ++f) {
+        const FdtdPmlDesc &pd = p->d.pml[f];
+        const uint32_t sa = pd.axis == 0 ? p->sx : pd.axis == 1 ? p->sy : p->sz;
+        if (pd.polarity == 1 && (uint32_t)pd.thickness > sa) continue;   // a face that never applies
+        const size_t pb = (size_t)(p->N / sa) * (size_t)pd.thickness * p->elem;
+        for (int c = 0; !rc && c < 2 && pb; ++c)
+            rc = check_cuda(cudaMemcpyAsync(dpsi[f][c], spsi[f][c], pb, cudaMemcpyDeviceToDevice, st), "copy psi");
+    }
+    return rc;
+}
+
+// Multi-step path with the H kernel (hs_fused.cu), which reads H (and the H-side psi) from one copy
+// and writes the other. Without `ahead` a step is update_E in place, then H and S in one launch.
+// With `ahead` (E has a second copy too) the H launch of every step but the last also makes the
+// next step's E, so that a call is one update_E, nsteps - 1 launches for a whole step each, and the
+// last step's H (and S). The copies swap as they are written; where the count of swaps is odd the
+// launch that can go either way (the first E, or the last H without Poynting) makes it even, and
+// otherwise the state is copied home at the end.
 template <typename R>
 int run_hs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
-           const FdtdPointSources *src, const FdtdDftMonitor *mon)
+           const FdtdPointSources *src, const FdtdDftMonitor *mon, bool ahead)
 {
+    int rc;
     HSK<R> k;
     std::memset(&k, 0, sizeof(k));
     k.sx = p->sx;
@@ -427,18 +486,19 @@ int run_hs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
     k.dt = (R)p->d.dt;
     k.inv_d = (R)(1.0 / p->d.dx);
     k.sf = (R)((double)k.dt * 0.125);
-    for (int r = 0; r < 3; ++r) k.inv_de[r] = p->d.uniform ? nullptr : (const R *)b->inv_de[r];
-    const int dxmode = !p->d.uniform ? 2 : ((R)(1.0 / p->d.dx) == R(1) ? 0 : 1);
-    k.cm = p->d.has_mu ? (const R *)b->cm : nullptr;
-    k.S = (R *)b->S;
-    k.oS = (R *)b->oS;
-    k.dsz = FastDiv::make(p->sz);
-    k.rows = (uint32_t)HS_THREADS / p->sz - 1u;
-    k.reverse = p->hs_reverse;
-    k.nrowblk = (k.sy + k.rows - 1u) / k.rows;
-    k.xchunk = p->hs_xchunk ? p->hs_xchunk : hs_auto_xchunk(p, k.nrowblk, mon && p->hs_dft ? 1u : 0u);
-    k.nchunk = (k.sx + k.xchunk - 1u) / k.xchunk;
-    p->hs_xchunk_used = (int32_t)k.xchunk;
+    for (int r = 0; r < 3; ++r) {
+        k.inv_de[r] = p->d.uniform ? nullptr : (const R *)b->inv_de[r];
+        k.inv_dh[r] = p->d.uniform ? nullptr : (const R *)b->inv_dh[r];
+    }
+    HSForm form;
+    form.dxmode = !p->d.uniform ? 2 : ((R)(1.0 / p->d.dx) == R(1) ? 0 : 1);
+    form.mu = p->d.has_mu != 0;
+    form.poynting = p->d.do_poynting != 0;
+    form.ahead = ahead;
+    k.cm = form.mu ? (const R *)b->cm : nullptr;
+    k.ce = (const R *)b->ce;
+    k.S = form.poynting ? (R *)b->S : nullptr;
+    k.oS = form.poynting ? (R *)b->oS : nullptr;
     int fidx[3][2] = {{-1, -1}, {-1, -1}, {-1, -1}};
     for (int f = 0; f < p->d.n_pml; ++f) {
         const FdtdPmlDesc &pd = p->d.pml[f];
@@ -447,80 +507,110 @@ int run_hs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
         HSAxis<R> &a = k.ax[pd.axis];
         if (pd.polarity == 0) a.Tn = pd.thickness;
         else a.Tp = pd.thickness;
-        for (int c = 0; c < 3; ++c) a.tab[pd.polarity][c] = (const R *)p->tab[f][3 + c];
+        for (int c = 0; c < 3; ++c) {
+            a.e.tab[pd.polarity][c] = (const R *)p->tab[f][c];
+            a.h.tab[pd.polarity][c] = (const R *)p->tab[f][3 + c];
+        }
         fidx[pd.axis][pd.polarity] = f;
     }
+    void *const E[2] = {b->E, b->E2}, *const H[2] = {b->H, b->H2};
+    void *const(*const psi_e[2])[2] = {b->psi_e, b->psi_e2};
+    void *const(*const psi_h[2])[2] = {b->psi_h, b->psi_h2};
     FdtdBuffers bb = *b;
-    void *H[2] = {b->H, b->H2};
-    int rc;
     KernelTimer timer(p, nsteps, st);
     if ((rc = timer.init())) return rc;
-    // the step's DFT sample: in the H+S launch (one extra block) or on the side stream beside it
+    // the step's DFT sample: in the H launch (one extra block) or on the side stream beside it
     const bool dft_in = mon && p->hs_dft;
     const bool dft_side = mon && !p->hs_dft;
     const bool pdl = p->pdl != 0;
     if (dft_side && (rc = side_stream(p))) return rc;
+    form.ahead = ahead && nsteps > 1;
+    hs_layout<R>(p, k, form, dft_in ? 1u : 0u);
+    int ce = 0, ch = 0;                      // the copies that hold E and H
     for (int t = 0; t < nsteps; ++t) {
-        const int a = t & 1, o = a ^ 1;
-        bb.H = H[a];
-        // the previous step's DFT sample has read E
+        bb.H = H[ch];
+        // the previous step's DFT sample has read the E that is written next
         if (dft_side && t > 0 && (rc = check_cuda(cudaStreamWaitEvent(st, p->ev_join, 0), "join wait"))) return rc;
-        if ((rc = lbc_before_e(p, b, H[a], st))) return rc;
         if ((rc = timer.mark(t, 0))) return rc;
-        // without a learned boundary (whose E fix-up comes before the sources) the E kernel
-        // adds the point sources itself
-        bool added = false;
-        if ((rc = run_update_e<R>(p, &bb, st, false, 0, 0xffffffffu, p->lbc_mask ? nullptr : src, t, &added, pdl))) return rc;
+        if (t == 0 || !ahead) {
+            // without a learned boundary (whose E fix-up comes before the sources) the E kernel
+            // adds the point sources itself
+            const bool away = ahead && ((nsteps - 1) & 1);
+            bool added = false;
+            if ((rc = lbc_before_e(p, b, H[ch], st))) return rc;
+            if ((rc = run_update_e<R>(p, &bb, st, false, 0, 0xffffffffu, p->lbc_mask ? nullptr : src, t, &added, pdl,
+                                      away ? E[1] : nullptr, away ? psi_e[1] : nullptr))) return rc;
+            if (away) ce = 1;
+            if ((rc = lbc_after_e(p, b, H[ch], st))) return rc;
+            bb.E = E[ce];
+            if (!added && src && src->n > 0 && (rc = run_point_sources<R>(p, &bb, st, src, t))) return rc;
+        }
         if ((rc = timer.mark(t, 1))) return rc;
-        if ((rc = lbc_after_e(p, b, H[a], st))) return rc;
-        if (!added && src && src->n > 0 && (rc = run_point_sources<R>(p, &bb, st, src, t))) return rc;
-        // the H+S launch leaves E unchanged, so the step's DFT sample of E is taken by its last
-        // block, or (hs_dft off) runs on the side stream beside it and the next step's E update
-        // waits for it (above)
+        // the H launch leaves this step's E unchanged, so the step's DFT sample is taken by its last
+        // block, or (hs_dft off) runs on the side stream beside it and the next write of E waits for
+        // it (above)
         k.dft_on = dft_in ? 1 : 0;
-        if (dft_in) k.dft = dft_args<R>(p, b->E, mon, t);
+        if (dft_in) k.dft = dft_args<R>(p, E[ce], mon, t);
         if (dft_side) {
             if ((rc = check_cuda(cudaEventRecord(p->ev_fork, st), "fork event"))) return rc;
             if ((rc = check_cuda(cudaStreamWaitEvent(p->side, p->ev_fork, 0), "side stream wait"))) return rc;
-            if ((rc = run_dft<R>(p, b->E, p->side, mon, t))) return rc;
+            if ((rc = run_dft<R>(p, E[ce], p->side, mon, t))) return rc;
             if ((rc = check_cuda(cudaEventRecord(p->ev_join, p->side), "join event"))) return rc;
         }
-        k.E = (const R *)b->E;
-        k.HA = (const R *)H[a];
-        k.HB = (R *)H[o];
-        for (int r = 0; r < 3; ++r)
-            for (int side = 0; side < 2; ++side) {
-                const int f = fidx[r][side];
-                if (f < 0) continue;
-                void *const *pa = a ? b->psi_h2[f] : b->psi_h[f];
-                void *const *po = o ? b->psi_h2[f] : b->psi_h[f];
-                for (int c = 0; c < 2; ++c) {
-                    k.ax[r].A[side][c] = (const R *)pa[c];
-                    k.ax[r].B[side][c] = (R *)po[c];
-                }
-            }
-        k.write_oS = t == nsteps - 1;
+        const bool last = t == nsteps - 1;
+        form.ahead = ahead && !last;
         if ((rc = timer.mark(t, 2))) return rc;
-        if ((rc = check_cuda(launch_hs<R>(k, p->d.has_mu != 0, dxmode, p->hs_prefetch != 0, pdl, st), "H+S launch"))) return rc;
+        if (!form.poynting && !form.ahead) {
+            // the last H: nothing but H is wanted of it, in place or into the home copy
+            bb.E = E[ce];
+            bb.H = H[ch];
+            for (int f = 0; f < p->d.n_pml; ++f)
+                for (int c = 0; c < 2; ++c) bb.psi_h[f][c] = psi_h[ch][f][c];
+            if ((rc = run_update_h<R>(p, &bb, st, false, 0, 0xffffffffu, pdl, H[0], psi_h[0]))) return rc;
+            if (dft_in && (rc = run_dft<R>(p, E[ce], st, mon, t))) return rc;
+            ch = 0;
+        } else {
+            k.E = (const R *)E[ce];
+            k.EB = (R *)E[ce ^ 1];
+            k.HA = (const R *)H[ch];
+            k.HB = (R *)H[ch ^ 1];
+            for (int r = 0; r < 3; ++r)
+                for (int side = 0; side < 2; ++side) {
+                    const int f = fidx[r][side];
+                    if (f < 0) continue;
+                    for (int c = 0; c < 2; ++c) {
+                        k.ax[r].h.A[side][c] = (const R *)psi_h[ch][f][c];
+                        k.ax[r].h.B[side][c] = (R *)psi_h[ch ^ 1][f][c];
+                        k.ax[r].e.A[side][c] = (const R *)psi_e[ce][f][c];
+                        k.ax[r].e.B[side][c] = (R *)psi_e[ce ^ 1][f][c];
+                    }
+                }
+            if (ahead && last && t > 0) hs_layout<R>(p, k, form, dft_in ? 1u : 0u);
+            p->hs_xchunk_used = (int32_t)k.xchunk;
+            k.write_oS = last;
+            // with E in the launch, odd steps run the other way, so that each starts on the planes the
+            // one before it touched last (still in L2)
+            k.reverse = ahead ? (t & 1) ^ p->hs_reverse : p->hs_reverse;
+            k.nsrc = 0;
+            const bool in_kernel = form.ahead && src && src->n > 0 && src->n <= YEE_SRC;
+            if (in_kernel) kernel_sources<R>(p, k, src, t + 1);
+            if ((rc = check_cuda(launch_hs<R>(k, form, pdl, st), "H+S launch"))) return rc;
+            ch ^= 1;
+            if (form.ahead) {
+                ce ^= 1;
+                bb.E = E[ce];
+                if (!in_kernel && src && src->n > 0 && (rc = run_point_sources<R>(p, &bb, st, src, t + 1))) return rc;
+            }
+        }
         if ((rc = timer.mark(t, 3))) return rc;
-        if ((rc = lbc_after_h(p, b, H[o], st))) return rc;
+        if ((rc = lbc_after_h(p, b, H[ch], st))) return rc;
     }
     // the caller's stream sees the last DFT sample
     if (dft_side && nsteps > 0 && (rc = check_cuda(cudaStreamWaitEvent(st, p->ev_join, 0), "join wait"))) return rc;
     if ((rc = timer.finish())) return rc;
-    if (nsteps & 1) {
-        const size_t fb = 3 * (size_t)p->N * p->elem;
-        rc = check_cuda(cudaMemcpyAsync(b->H, b->H2, fb, cudaMemcpyDeviceToDevice, st), "copy H");
-        for (int f = 0; !rc && f < p->d.n_pml; ++f) {
-            const FdtdPmlDesc &pd = p->d.pml[f];
-            const size_t cells = (size_t)p->N / (pd.axis == 0 ? p->sx : pd.axis == 1 ? p->sy : p->sz);
-            const size_t pb = cells * (size_t)pd.thickness * p->elem;
-            for (int c = 0; !rc && c < 2 && pb; ++c)
-                rc = check_cuda(cudaMemcpyAsync(b->psi_h[f][c], b->psi_h2[f][c], pb, cudaMemcpyDeviceToDevice, st), "copy psi_h");
-        }
-        if (rc) return rc;
-    }
-    return FDTD_OK;
+    if (ce) rc = copy_state(p, b->E, b->E2, b->psi_e, b->psi_e2, st);
+    if (!rc && ch) rc = copy_state(p, b->H, b->H2, b->psi_h, b->psi_h2, st);
+    return rc;
 }
 
 // Per-update kernels over x slabs small enough to stay resident in L2: E on slab s, then H
@@ -535,18 +625,19 @@ int run_slabs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
     const uint32_t sx = p->sx;
     // the learned boundary's E corrections must land before any H update reads them: whole grid
     const uint32_t W = p->slab && !p->lbc_mask ? p->slab : sx;
-    const bool bloch = p->d.n_bloch != 0, poynt = p->d.do_poynting != 0;
+    const bool bloch = p->d.n_bloch != 0, poynt = p->d.do_poynting != 0, pdl = p->pdl != 0;
     int rc;
     if (W >= sx) {
         // one slab: the plain whole-grid sequence
         for (int t = 0; t < nsteps; ++t) {
+            bool added = false;
             if ((rc = lbc_before_e(p, b, b->H, st))) return rc;
-            if ((rc = run_update_e<R>(p, b, st, false))) return rc;
-            if (bloch && (rc = run_update_e<R>(p, b, st, true))) return rc;
+            if ((rc = run_update_e<R>(p, b, st, false, 0, 0xffffffffu, p->lbc_mask ? nullptr : src, t, &added, pdl))) return rc;
+            if (bloch && (rc = run_update_e<R>(p, b, st, true, 0, 0xffffffffu, nullptr, 0, nullptr, pdl))) return rc;
             if ((rc = lbc_after_e(p, b, b->H, st))) return rc;
-            if (src && src->n > 0 && (rc = run_point_sources<R>(p, b, st, src, t))) return rc;
-            if ((rc = run_update_h<R>(p, b, st, false))) return rc;
-            if (bloch && (rc = run_update_h<R>(p, b, st, true))) return rc;
+            if (!added && src && src->n > 0 && (rc = run_point_sources<R>(p, b, st, src, t))) return rc;
+            if ((rc = run_update_h<R>(p, b, st, false, 0, 0xffffffffu, pdl))) return rc;
+            if (bloch && (rc = run_update_h<R>(p, b, st, true, 0, 0xffffffffu, pdl))) return rc;
             if ((rc = lbc_after_h(p, b, b->H, st))) return rc;
             if (poynt && (rc = run_update_s<R>(p, b, st))) return rc;
             if (mon && (rc = run_dft<R>(p, b->E, st, mon, t))) return rc;
@@ -880,15 +971,26 @@ bool fused_eligible(const FdtdPlan *p, const FdtdBuffers *b, const FdtdPointSour
     return step_layout<float>(p, k, shape, threads, smem);
 }
 
-// The H+S path: Poynting on, no Bloch boundaries, CPML faces of one axis disjoint, dt/eps
-// (and dt/mu) caches and the H scratch copies present, and a z row that fits a block.
-bool hs_eligible(const FdtdPlan *p, const FdtdBuffers *b)
+// The H path: no Bloch boundaries, CPML faces of one axis disjoint, dt/eps (and dt/mu) caches and
+// the second copies of H present, and a form of the kernel: with the next step's E (second copies of E
+// too, float32, no learned boundary), or else Poynting on and z rows of at most 224 cells.
+bool hs_eligible(const FdtdPlan *p, const FdtdBuffers *b, bool ahead)
 {
-    if (!p->d.do_poynting || p->d.n_bloch || !faces_disjoint(p)) return false;
-    if (!b->ce || (p->d.has_mu && !b->cm) || !b->H2 || !b->S || !b->oS) return false;
-    if (2 * p->sz > (uint32_t)HS_THREADS) return false;   // at least one own row plus the halo row
+    if (p->d.n_bloch || !faces_disjoint(p)) return false;
+    if (!b->ce || (p->d.has_mu && !b->cm) || !b->H2) return false;
+    if (p->d.do_poynting && (!b->S || !b->oS)) return false;
+    HSForm f;
+    f.mu = p->d.has_mu != 0;
+    f.poynting = p->d.do_poynting != 0;
+    f.dxmode = 0;
+    f.ahead = ahead;
+    if (!ahead && 2 * p->sz > 448) return false;
+    if (!(p->d.dtype == FDTD_F64 ? hs_form_exists<double>(f) : hs_form_exists<float>(f))) return false;
+    if (ahead && (!b->E2 || p->lbc_mask)) return false;
     for (int f = 0; f < p->d.n_pml; ++f)
-        if (p->d.pml[f].thickness > 0 && (!b->psi_h2[f][0] || !b->psi_h2[f][1])) return false;
+        if (p->d.pml[f].thickness > 0 &&
+            (!b->psi_h2[f][0] || !b->psi_h2[f][1] || (ahead && (!b->psi_e2[f][0] || !b->psi_e2[f][1]))))
+            return false;
     return true;
 }
 
@@ -925,7 +1027,7 @@ int fdtd_plan_create(const FdtdDesc *desc, FdtdPlan **out)
     p->syz = p->sy * p->sz;
     p->N = (uint64_t)p->sx * p->syz;
     p->elem = desc->dtype == FDTD_F64 ? 8 : 4;
-    p->xchunk = 8;
+    p->xchunk = 0;
     // Whole-grid launches measured fastest on GB300 for the 395x345x73 workload (0.33 ms per
     // step against 0.43-0.86 ms for 48- to 8-plane slabs), so slabs are opt-in.
     p->slab = 0;
@@ -942,6 +1044,7 @@ int fdtd_plan_create(const FdtdDesc *desc, FdtdPlan **out)
     p->eform = 1;
     p->hs_xchunk_used = 0;
     p->hs_dft = 1;
+    p->hs_ahead = 0;
     p->pdl = 1;
     p->timing = 0;
     p->kernel_ms[0] = p->kernel_ms[1] = 0.0;
@@ -1061,6 +1164,10 @@ int fdtd_plan_tune(FdtdPlan *p, int32_t key, int32_t value)
         if (value != 0 && value != 1) return fail(FDTD_ERR_INVALID, "pdl must be 0 or 1");
         p->pdl = value;
         return FDTD_OK;
+    case FDTD_TUNE_HS_AHEAD:
+        if (value != 0 && value != 1) return fail(FDTD_ERR_INVALID, "hs_ahead must be 0 or 1");
+        p->hs_ahead = value;
+        return FDTD_OK;
     case FDTD_TUNE_E_FORM:
         if (value != 0 && value != 1) return fail(FDTD_ERR_INVALID, "e_form must be 0 or 1");
         p->eform = value;
@@ -1074,7 +1181,7 @@ int fdtd_plan_get(const FdtdPlan *p, int32_t key, int32_t *value)
 {
     if (!p || !value) return fail(FDTD_ERR_INVALID, "plan or value is NULL");
     switch (key) {
-    case FDTD_TUNE_XCHUNK: *value = p->xchunk; return FDTD_OK;
+    case FDTD_TUNE_XCHUNK: *value = p->xchunk ? p->xchunk : 8; return FDTD_OK;
     case FDTD_TUNE_SLAB: *value = (int32_t)p->slab; return FDTD_OK;
     case FDTD_TUNE_FUSED_ROWS: *value = (int32_t)p->fused_rows; return FDTD_OK;
     case FDTD_TUNE_FUSED_XCHUNK: *value = (int32_t)p->fused_xchunk; return FDTD_OK;
@@ -1094,6 +1201,7 @@ int fdtd_plan_get(const FdtdPlan *p, int32_t key, int32_t *value)
     case FDTD_TUNE_HS_DFT: *value = p->hs_dft; return FDTD_OK;
     case FDTD_TUNE_PDL: *value = p->pdl; return FDTD_OK;
     case FDTD_TUNE_E_FORM: *value = p->eform; return FDTD_OK;
+    case FDTD_TUNE_HS_AHEAD: *value = p->hs_ahead; return FDTD_OK;
     case FDTD_TUNE_TIMING: *value = p->timing; return FDTD_OK;
     default: return fail(FDTD_ERR_INVALID, "unknown tuning key");
     }
@@ -1334,15 +1442,16 @@ int fdtd_run(FdtdPlan *p, const FdtdBuffers *b, void *stream, int32_t nsteps,
             return fail(FDTD_ERR_INVALID, "fdtd_run: point source index out of range");
     if ((rc = check_monitor(p, mon))) return rc;
     const bool f64 = p->d.dtype == FDTD_F64;
-    if (!b->E2 && hs_eligible(p, b)) {
+    const bool ahead = p->hs_ahead && hs_eligible(p, b, true);
+    if (ahead || (!b->E2 && hs_eligible(p, b, false))) {
         if ((rc = check_run_buffers(p, b))) return rc;
         cudaStream_t st = (cudaStream_t)stream;
         p->last_run_path = FDTD_PATH_HS;
-        rc = f64 ? run_hs<double>(p, b, st, nsteps, src, mon) : run_hs<float>(p, b, st, nsteps, src, mon);
+        rc = f64 ? run_hs<double>(p, b, st, nsteps, src, mon, ahead) : run_hs<float>(p, b, st, nsteps, src, mon, ahead);
         if (!rc && mon) { mon->step += nsteps; mon->series_row += nsteps; }
         return rc;
     }
-    if (!p->lbc_mask && fused_eligible(p, b, src)) {
+    if (!p->lbc_mask && !p->hs_ahead && fused_eligible(p, b, src)) {
         if ((rc = check_psi(p, b->psi_e, "fdtd_run")) || (rc = check_psi(p, b->psi_h, "fdtd_run")))
             return rc;
         cudaStream_t st = (cudaStream_t)stream;

@@ -12,7 +12,7 @@ struct FdtdPlan {
     uint64_t N;
     size_t elem;                // bytes per element of the plan's dtype
     int device;                 // device that was current at creation
-    int32_t xchunk;             // x planes a bulk-kernel thread marches
+    int32_t xchunk;             // x planes a bulk-kernel thread marches (0: automatic)
     int32_t eform;              // form of the bulk E kernel (FDTD_TUNE_E_FORM)
     uint32_t slab;              // x planes per L2-resident slab in fdtd_run (0: whole grid)
     uint32_t fused_rows;        // own rows of a one-pass step tile (0: the most that fit)
@@ -23,11 +23,12 @@ struct FdtdPlan {
     int32_t last_run_path;      // FDTD_PATH_* of the last fdtd_run
     int32_t step_cfg[5];        // last one-pass launch: rows, xchunk, stages, threads, shape
     uint32_t hs_xchunk;         // x planes one block of the H+S kernel marches
-    int32_t hs_prefetch;        // H+S kernel issues the next plane's loads early
+    int32_t hs_prefetch;        // accepted, without effect
     int32_t hs_reverse;         // H+S kernel takes its x chunks in descending order
     int32_t hs_xchunk_used;     // x chunk of the last H+S launch (hs_xchunk or the automatic one)
+    int32_t hs_ahead;           // H path: with second copies of E, make the next step's E in the H launch
     int32_t hs_dft;             // H+S path: the DFT sample in the H+S launch, not a side stream
-    int32_t pdl;                // H+S path: programmatic dependent launches of E and H+S
+    int32_t pdl;                // fdtd_run: programmatic dependent launches of E and H
     int32_t timing;             // fdtd_run's H+S path records per-kernel CUDA events
     int32_t *status = nullptr;  // device word: bits of bounded waits inside kernels that ran out
     // side stream of fdtd_run's H+S path when hs_dft is off: the step's DFT monitor sample runs

@@ -1,77 +1,42 @@
-// H update and Poynting vector in one pass (the multi-step path of fdtd_run).
+// The H kernel of fdtd_run: the H update of a step and, in the same launch, its Poynting vector
+// and the E update of the next step.
 //
-// The drop-in update_H writes the six Poynting products oS (24 B per cell) and update_S reads
-// them back with their minus neighbours (36 B per cell). Here the H update reads H from one
-// buffer and writes it to another (ping-pong, with the H-side CPML arrays), so every value it
-// reads is read-only for the whole launch; S is then formed in the same launch:
-//   * a block owns whole z rows [y0, y0 + rows) and marches a chunk of x planes; it also
-//     evaluates the row y0 - 1, owned by another block, without writing it (its inputs are
-//     read-only, so the values are the owner's); after each plane's H update the products go
-//     to shared memory;
-//   * S at (x, y, z) takes the products of its own cell, of z-1 (same row), of y-1 (the row
-//     before, in the block) and of x-1 (the thread's previous plane, kept in registers).
-// With update_E in place this gives a step of 96 B per cell plus 32 B per CPML face-cell,
-// the algorithmic figure of the two-pass accounting (84 + 12). Per-cell arithmetic and its
-// order are those of update_H and update_S (compiled with --fmad=false), so fields and S are
-// bit-identical to the per-call loop. Bloch boundaries are handled by the per-update path.
+// Per-update kernels move every field once per update: E and H are read twice per step, and the
+// six Poynting products go through memory (update_h.cl:142-155, update_s.cl:21-36). Here H is read
+// from one buffer and written to another (ping-pong, with the H-side CPML arrays), so every value
+// this launch reads is read-only, and a cell that a neighbour's result needs can be evaluated again:
+//   * S at (x, y, z) takes the products of its own cell and of x-1, y-1 and z-1; the next E update
+//     takes H_new at exactly the same four cells. One halo feeds both: the plane before the chunk,
+//     a row and a column before the tile.
+//   * with the next step's E in the launch (AHEAD; E ping-pongs too), a step reads E, H and dt/eps
+//     once and writes E, H and S once: 72 B per cell in float32, 32 B per absorbing cell of a face,
+//     against 96 B for update_E and H+S in two launches. Without it (the last step of a call, and
+//     steps whose E needs a learned boundary's fix-up first) the launch leaves E alone.
+//
+// What bounds it: a step of the 395x345x73 grid with six 8-cell faces takes 0.189 ms (update_E and
+// H+S in two launches: 0.231), 813 MB at 4.3 TB/s; without faces 0.150 ms. Plain copies of the same
+// nine read and nine written streams take 0.115-0.139 ms there, so what is left is instruction issue:
+// about 290 instructions per warp and plane, 60 of them arithmetic, and the absorbing columns' code
+// on top (0.204 ms before the tile's face columns were given threads of their own). 200^3 cells:
+// 0.153 ms (0.244 in two or three launches); 300^3: 0.444 (0.736).
+//
+// Measured and left out (0.150 / 0.204 ms without and with faces at the time): strips of rows per
+// thread with shuffles and no barrier (0.151 / 0.211: 4 warps per scheduler, every instruction of the
+// face code exposed), a separate copy of the march for warps without faces (spills: 0.175 / 0.370),
+// code per face side (spills: 0.172 / 0.258), staging by per-thread asynchronous copies (0.215).
+//
+// Per-cell arithmetic and its order are those of update_H, update_S and update_E (compiled with
+// --fmad=false), so fields and S are bit-identical to the per-call loop.
 #include "yee_common.cuh"
 #include "yee_device.cuh"
 #include "hs_fused.h"
 
 namespace fdtd {
 
-// CPML face of one axis for a cell: depth ir (-1 outside) and side (0 = 'n', 1 = 'p').
-// Thickness and psi pointers are read from the launch parameters on use; the coefficients of
-// a thread's y and z faces, fixed for its march, are loaded once into registers (cy, cz),
-// those of the x face on use.
-struct HSF {
-    int ir, side;
-};
-
+// Everything one H evaluation at (x, y, z) reads besides E at the cell.
 template <typename R>
-__device__ __forceinline__ HSF hs_face(const HSAxis<R> &a, uint32_t s, uint32_t c)
-{
-    HSF f;
-    f.ir = -1;
-    f.side = 0;
-    if (c < (uint32_t)a.Tn) {
-        f.ir = (int)c;
-    } else if (a.Tp && c >= s - (uint32_t)a.Tp) {
-        f.ir = (int)(s - 1u - c);
-        f.side = 1;
-    }
-    return f;
-}
-
-template <typename R>
-__device__ __forceinline__ uint32_t hs_T(const HSAxis<R> &a, const HSF &f)
-{
-    return (uint32_t)(f.side ? a.Tp : a.Tn);
-}
-
-template <typename R>
-__device__ __forceinline__ const R *hs_tab(const HSAxis<R> &a, const HSF &f, int c)
-{
-    return f.side ? a.tab[1][c] : a.tab[0][c];
-}
-
-template <typename R>
-__device__ __forceinline__ const R *hs_A(const HSAxis<R> &a, const HSF &f, int c)
-{
-    return f.side ? a.A[1][c] : a.A[0][c];
-}
-
-template <typename R>
-__device__ __forceinline__ R *hs_B(const HSAxis<R> &a, const HSF &f, int c)
-{
-    return f.side ? a.B[1][c] : a.B[0][c];
-}
-
-// Everything one H evaluation at (x, y, z) reads.
-template <typename R>
-struct HSLoad {
-    R ex, ey, ez;                 // E at the cell
-    R ey1, ez1;                   // E_y, E_z at x+1 (wrapped)
+struct HLoads {
+    R ex1, ey1, ez1;              // E at x+1 (wrapped): the next plane's own
     R rxy, rzy;                   // E_x, E_z at y+1 (wrapped)
     R rxz, ryz;                   // E_x, E_y at z+1 (wrapped)
     R hx, hy, hz;                 // old H at the cell
@@ -79,254 +44,369 @@ struct HSLoad {
     R xu, xv, yu, yv, zu, zv;     // old psi_H of the faces the cell is in
 };
 
-template <typename R, bool MU>
-__device__ __forceinline__ void hs_load(const HSK<R> &k, uint32_t x, uint32_t i, uint32_t dpy,
-                                        uint32_t dpz, const HSF &fx, const HSF &fy,
-                                        const HSF &fz, uint32_t y, uint32_t z, HSLoad<R> &v)
+// psi index of a cell at plane x in the face of axis AX it is in
+template <int AX>
+__device__ __forceinline__ uint32_t psi_at(const FaceAt &f, uint32_t Tn, uint32_t Tp, uint32_t x, uint32_t y, uint32_t z,
+                                           uint32_t sy, uint32_t sz)
 {
-    const uint64_t N = k.N;
-    const uint32_t sx = k.sx, syz = k.syz;
-    const R *Ex = k.E, *Ey = k.E + N, *Ez = k.E + 2 * N;
-    const uint32_t i1 = (x + 1u < sx) ? i + syz : i - (sx - 1u) * syz;
-    const uint32_t ipy = i + dpy, ipz = i + dpz;   // 32-bit wrap arithmetic
-    v.ex = ldg(Ex + i); v.ey = ldg(Ey + i); v.ez = ldg(Ez + i);
-    v.ey1 = ldg(Ey + i1); v.ez1 = ldg(Ez + i1);
-    v.rxy = ldg(Ex + ipy); v.rzy = ldg(Ez + ipy);
-    v.rxz = ldg(Ex + ipz); v.ryz = ldg(Ey + ipz);
-    v.hx = ldg(k.HA + i); v.hy = ldg(k.HA + N + i); v.hz = ldg(k.HA + 2 * N + i);
-    v.cx = v.cy = v.cz = R(0);
-    if (MU) { v.cx = ldg(k.cm + i); v.cy = ldg(k.cm + N + i); v.cz = ldg(k.cm + 2 * N + i); }
-    v.xu = v.xv = v.yu = v.yv = v.zu = v.zv = R(0);
-    if (fx.ir >= 0) {
-        const uint32_t ip = psi_index<0>((uint32_t)fx.ir, hs_T(k.ax[0], fx), x, y, z, k.sy, k.sz);
-        v.xu = ldg(hs_A(k.ax[0], fx, 0) + ip); v.xv = ldg(hs_A(k.ax[0], fx, 1) + ip);
-    }
-    if (fy.ir >= 0) {
-        const uint32_t ip = psi_index<1>((uint32_t)fy.ir, hs_T(k.ax[1], fy), x, y, z, k.sy, k.sz);
-        v.yu = ldg(hs_A(k.ax[1], fy, 0) + ip); v.yv = ldg(hs_A(k.ax[1], fy, 1) + ip);
-    }
-    if (fz.ir >= 0) {
-        const uint32_t ip = psi_index<2>((uint32_t)fz.ir, hs_T(k.ax[2], fz), x, y, z, k.sy, k.sz);
-        v.zu = ldg(hs_A(k.ax[2], fz, 0) + ip); v.zv = ldg(hs_A(k.ax[2], fz, 1) + ip);
-    }
+    return psi_index<AX>((uint32_t)f.ir, f.side ? Tp : Tn, x, y, z, sy, sz);
 }
 
-// H_new and the six products from loaded values (update_h.cl:36-43, 63-70, 80-155).
-// wr: write H_new and the advanced psi to the B buffers.
-template <typename R, int DX, bool MU>
-__device__ __forceinline__ void hs_math(const HSK<R> &k, uint32_t x, uint32_t y, uint32_t z,
-                                        uint32_t i, const HSF &fx, const HSF &fy,
-                                        const HSF &fz, const HSLoad<R> &v, bool wr, R *os,
-                                        const R *cy, const R *cz)
+// A block marches a chunk of x planes with a tile of the (y, z) plane, one cell per thread: a row
+// and a column of halo cells (owned by other tiles, evaluated from the same read-only inputs,
+// never written) before its own rows and columns. After each plane's H update the values that
+// neighbours need (products, H_new) go to shared memory in slots that alternate by plane, so one
+// barrier per plane suffices; x - 1 values stay in registers. The next plane's loads are issued
+// before the barrier. The columns inside the z faces take the block's last threads, so that few warps
+// hold absorbing cells; the others skip the CPML code.
+template <typename R, int DX, bool MU, bool AHEAD>
+__global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const __grid_constant__ HSK<R> k)
 {
-    R d_xy = v.rxy - v.ex;
-    R d_xz = v.rxz - v.ex;
-    R d_yx = v.ey1 - v.ey;
-    R d_yz = v.ryz - v.ey;
-    R d_zx = v.ez1 - v.ez;
-    R d_zy = v.rzy - v.ez;
-    if (DX != 0) {
-        R ix = k.inv_d, iy = k.inv_d, iz = k.inv_d;
-        if (DX == 2) { ix = ldg(k.inv_de[0] + x); iy = ldg(k.inv_de[1] + y); iz = ldg(k.inv_de[2] + z); }
-        d_xy = d_xy * iy; d_xz = d_xz * iz; d_yx = d_yx * ix;
-        d_yz = d_yz * iz; d_zx = d_zx * ix; d_zy = d_zy * iy;
-    }
-    R px = R(0), py = R(0), pz = R(0);
-    if (fx.ir >= 0) {
-        const HSAxis<R> &a = k.ax[0];
-        R su, sv;
-        face_update<R, false, 0>(ldg(hs_tab(a, fx, 0) + fx.ir), ldg(hs_tab(a, fx, 1) + fx.ir),
-                                  ldg(hs_tab(a, fx, 2) + fx.ir), v.xu, v.xv, su, sv,
-                                  d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-        if (wr) {
-            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, hs_T(a, fx), x, y, z, k.sy, k.sz);
-            hs_B(a, fx, 0)[ip] = su;
-            hs_B(a, fx, 1)[ip] = sv;
-        }
-    }
-    if (fy.ir >= 0) {
-        const HSAxis<R> &a = k.ax[1];
-        R su, sv;
-        face_update<R, false, 1>(cy[0], cy[1], cy[2], v.yu, v.yv, su, sv,
-                                  d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-        if (wr) {
-            const uint32_t ip = psi_index<1>((uint32_t)fy.ir, hs_T(a, fy), x, y, z, k.sy, k.sz);
-            hs_B(a, fy, 0)[ip] = su;
-            hs_B(a, fy, 1)[ip] = sv;
-        }
-    }
-    if (fz.ir >= 0) {
-        const HSAxis<R> &a = k.ax[2];
-        R su, sv;
-        face_update<R, false, 2>(cz[0], cz[1], cz[2], v.zu, v.zv, su, sv,
-                                  d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-        if (wr) {
-            const uint32_t ip = psi_index<2>((uint32_t)fz.ir, hs_T(a, fz), x, y, z, k.sy, k.sz);
-            hs_B(a, fz, 0)[ip] = su;
-            hs_B(a, fz, 1)[ip] = sv;
-        }
-    }
-    R hx, hy, hz;
-    if (MU) {
-        hx = v.hx - v.cx * ((d_zy - d_yz) - px);
-        hy = v.hy - v.cy * ((d_xz - d_zx) - py);
-        hz = v.hz - v.cz * ((d_yx - d_xy) - pz);
-    } else {
-        hx = v.hx - k.dt * ((d_zy - d_yz) - px);
-        hy = v.hy - k.dt * ((d_xz - d_zx) - py);
-        hz = v.hz - k.dt * ((d_yx - d_xy) - pz);
-    }
-    if (wr) {
-        const uint64_t N = k.N;
-        k.HB[i] = hx;
-        k.HB[N + i] = hy;
-        k.HB[2 * N + i] = hz;
-    }
-    const R ahx = hx + v.hx, ahy = hy + v.hy, ahz = hz + v.hz;
-    os[0] = (v.ey1 + v.ey) * ahz;
-    os[3] = (-(v.ez1 + v.ez)) * ahy;
-    os[1] = (v.rzy + v.ez) * ahx;
-    os[4] = (-(v.rxy + v.ex)) * ahz;
-    os[2] = (v.rxz + v.ex) * ahy;
-    os[5] = (-(v.ryz + v.ey)) * ahx;
-}
-
-// S at the cell of thread t from the products of one plane in shared memory (six planes of
-// HS_THREADS values: xy, yz, zx, xz, yx, zy) and the thread's x-1 products (update_s.cl:33-36);
-// the x-1 products become this plane's.
-template <typename R>
-__device__ __forceinline__ void hs_s(const HSK<R> &k, const R *q, uint32_t t, uint32_t z,
-                                     uint32_t i, R &prev_yx, R &prev_zx)
-{
-    const uint64_t N = k.N;
-    const uint32_t sz = k.sz;
-    const uint32_t tz = z ? t - 1u : t + sz - 1u;  // z-1, wrapped within the row
-    const R a_xy = q[t], a_yz = q[HS_THREADS + t], a_zx = q[2 * HS_THREADS + t];
-    const R a_xz = q[3 * HS_THREADS + t], a_yx = q[4 * HS_THREADS + t], a_zy = q[5 * HS_THREADS + t];
-    const R xy_y = q[t - sz], zy_y = q[5 * HS_THREADS + t - sz];
-    const R xz_z = q[3 * HS_THREADS + tz], yz_z = q[HS_THREADS + tz];
-    k.S[i] = (((a_xy + a_xz) + xy_y) + xz_z) * k.sf;
-    k.S[N + i] = (((a_yz + a_yx) + yz_z) + prev_yx) * k.sf;
-    k.S[2 * N + i] = (((a_zx + a_zy) + prev_zx) + zy_y) * k.sf;
-    prev_yx = a_yx;
-    prev_zx = a_zx;
-}
-
-// Thread t of a block works on window row w = t / sz (cell z = t % sz): row 0 is the halo row
-// y0 - 1 (wrapped), whose products only feed S of row y0; rows 1..rows are the block's own
-// rows y0 .. y0 + rows - 1. Every thread evaluates exactly one cell per plane, so a barrier
-// waits for no extra work. The products go to shared memory slots that alternate by plane,
-// which is what lets one barrier per plane suffice.
-// PF: issue the next plane's loads before the current plane's arithmetic (one block per SM
-// with room for both sets of registers); otherwise (two blocks per SM) they are issued after
-// the products are stored, so that the last plane's are in flight during the barrier and the
-// S assembly.
-// The grid is one-dimensional: block b takes row block b % nrowblk and x chunk b / nrowblk (row
-// blocks fastest). With dft_on one more block (the last) takes the step's DFT monitor sample
-// of E, which this launch leaves unchanged; a single block keeps a grid that fills whole
-// waves of resident blocks doing so.
-template <typename R, int DX, bool MU, bool PF>
-__global__ void __launch_bounds__(HS_THREADS, PF ? 1 : 2) k_bulk_hs(const HSK<R> k)
-{
-    __shared__ R sS[2][6][HS_THREADS];
+    // values exchanged: products xy, zy (to y + 1), xz, yz (to z + 1); H_new x, y, z
+    constexpr int XY = 0, ZY = 1, XZ = 2, YZ = 3, HX = 4, HY = 5, HZ = 6, NV = AHEAD ? 7 : 4;
+    constexpr uint32_t HS_THREADS = (uint32_t)hs_threads(AHEAD, MU, DX);
+    __shared__ R sV[2][NV][HS_THREADS];
+    __shared__ R sC[AHEAD ? 6 : 3][HS_THREADS];   // z-face coefficients of each thread: H, then E
     grid_dependency_sync();
     const uint32_t t = threadIdx.x;
-    const uint32_t chunk = blockIdx.x / k.nrowblk;
-    if (chunk >= k.nchunk) {
+    const uint32_t chunk0 = blockIdx.x / k.ntile;
+    if (chunk0 >= k.nchunk) {
+        // the step's DFT sample: E is not written by this launch
         const int nq = k.dft.npoint * (k.dft.nfreq > 0 ? k.dft.nfreq : 1);
-        for (int q = (int)t; q < nq; q += HS_THREADS) dft_sample(k.dft, q);
+        for (int q = (int)t; q < nq; q += (int)HS_THREADS) dft_sample(k.dft, q);
         return;
     }
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
     const uint64_t N = k.N;
-    const uint32_t y0 = (blockIdx.x - chunk * k.nrowblk) * k.rows;
-    const uint32_t nrow = min(k.rows, sy - y0);
-    const bool act = t < (nrow + 1u) * sz;
-    const uint32_t w = act ? k.dsz.div(t) : 0u;
-    const uint32_t z = act ? t - w * sz : 0u;
-    const uint32_t y = w ? y0 + w - 1u : (y0 ? y0 - 1u : sy - 1u);
-    const bool own = act && w > 0;
+    const uint32_t tile = blockIdx.x - chunk0 * k.ntile;
+    const uint32_t yt = tile / k.nseg, seg = tile - yt * k.nseg;
+    const uint32_t y0 = yt * k.rows, z0 = seg * k.seglen;
+    const uint32_t nrow = min(k.rows, sy - y0), len = min(k.seglen, sz - z0), ext = k.seglen + 1u;
+    // columns 0 (the halo, z0 - 1) .. len of the tile: a leading and a trailing run lies in the z
+    // faces, [ca, cb) between them does not
+    const uint32_t Tn = (uint32_t)k.ax[2].Tn, Tp = (uint32_t)k.ax[2].Tp;
+    uint32_t ca = 0u, cb = len + 1u;
+    if (Tn + Tp) {
+        const uint32_t halo = z0 ? z0 - 1u : sz - 1u, past = z0 + len;
+        if (z0 < Tn) ca = min(Tn - z0, len) + 1u;
+        else if (z0 >= sz - Tp && halo >= sz - Tp) ca = len + 1u;
+        else if (halo < Tn || halo >= sz - Tp) ca = 1u;
+        if (past > sz - Tp && ca <= len) cb = len + 1u - min(past - (sz - Tp), len + 1u - ca);
+    }
+    const uint32_t nin = cb - ca, nface = len + 1u - nin, ins = nin * (nrow + 1u);
+    uint32_t w, c;
+    if (t < ins) {
+        w = t / nin;
+        c = ca + t - w * nin;
+    } else {
+        const uint32_t u = t - ins;
+        w = nface ? u / nface : nrow + 1u;
+        c = u - w * nface;
+        c = c < ca ? c : c + nin;
+    }
+    const bool act = w <= nrow && c <= len;
+    const bool own = act && w > 0u && c > 0u;
+    // The thread's place in the exchange. Threads beyond the tile share the last place, which no cell
+    // has when there are such threads and nobody reads (stores under a condition made the compiler spill).
+    const uint32_t p = act ? w * ext + c : HS_THREADS - 1u;
+    const uint32_t y = act ? (w ? y0 + w - 1u : (y0 ? y0 - 1u : sy - 1u)) : y0;
+    const uint32_t z = act ? (c ? z0 + c - 1u : (z0 ? z0 - 1u : sz - 1u)) : z0;
     const uint32_t j = y * sz + z;
-    // chunks in descending x order start where the preceding update_E (ascending) finished, on
-    // planes still in L2
-    const uint32_t xa = (k.reverse ? k.nchunk - 1u - chunk : chunk) * k.xchunk;
+    const uint32_t chunk = k.reverse ? k.nchunk - 1u - chunk0 : chunk0;
+    const uint32_t xa = chunk * k.xchunk;
     const uint32_t xb = min(xa + k.xchunk, sx);
     // plus neighbours (common.cl:82-84) in 32-bit wrap arithmetic
     const uint32_t dpy = (y + 1u < sy) ? sz : 0u - (sy - 1u) * sz;
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
-    const HSF fy = hs_face<R>(k.ax[1], sy, y);
-    const HSF fz = hs_face<R>(k.ax[2], sz, z);
-    // CPML coefficients of the thread's y and z faces, fixed for the march
-    R cy[3] = {R(0), R(0), R(0)}, cz[3] = {R(0), R(0), R(0)};
-    if (fy.ir >= 0)
-        for (int c = 0; c < 3; ++c) cy[c] = ldg(hs_tab(k.ax[1], fy, c) + fy.ir);
-    if (fz.ir >= 0)
-        for (int c = 0; c < 3; ++c) cz[c] = ldg(hs_tab(k.ax[2], fz, c) + fz.ir);
-
-    R prev_yx = R(0), prev_zx = R(0);
-    if (own) {
-        // products yx, zx of plane xa - 1 (the x-1 neighbour of the chunk's first S)
-        const uint32_t xp = xa ? xa - 1u : sx - 1u;
-        const uint32_t ip = xp * syz + j;
-        const HSF fx = hs_face<R>(k.ax[0], sx, xp);
-        HSLoad<R> v;
-        hs_load<R, MU>(k, xp, ip, dpy, dpz, fx, fy, fz, y, z, v);
-        R os[6];
-        hs_math<R, DX, MU>(k, xp, y, z, ip, fx, fy, fz, v, false, os, cy, cz);
-        prev_yx = os[4];
-        prev_zx = os[2];
-    }
-    HSLoad<R> cur;
-    uint32_t i = xa * syz + j;
-    if (act) hs_load<R, MU>(k, xa, i, dpy, dpz, hs_face<R>(k.ax[0], sx, xa), fy, fz, y, z, cur);
-    for (uint32_t x = xa; x < xb; ++x, i += syz) {
-        const HSF fx = hs_face<R>(k.ax[0], sx, x);
-        const int slot = (int)(x & 1u);
-        HSLoad<R> nxt;
-        if (act) {
-            if (PF && x + 1u < xb) hs_load<R, MU>(k, x + 1u, i + syz, dpy, dpz, hs_face<R>(k.ax[0], sx, x + 1u), fy, fz, y, z, nxt);
-            R os[6];
-            hs_math<R, DX, MU>(k, x, y, z, i, fx, fy, fz, cur, own, os, cy, cz);
+    FaceAt fy = face_at(k.ax[1].Tn, k.ax[1].Tp, sy, y), fz = face_at(k.ax[2].Tn, k.ax[2].Tp, sz, z);
+    if (!act) fy.ir = fz.ir = -1;
+    const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
+    if (fz.ir >= 0) {
 #pragma unroll
-            for (int c = 0; c < 6; ++c) sS[slot][c][t] = os[c];
-            if (own && k.write_oS) {
-#pragma unroll
-                for (int c = 0; c < 6; ++c) k.oS[(uint64_t)c * N + i] = os[c];
-            }
-            // the next plane's loads fly during the barrier and the S assembly
-            if (!PF && x + 1u < xb)
-                hs_load<R, MU>(k, x + 1u, i + syz, dpy, dpz, hs_face<R>(k.ax[0], sx, x + 1u), fy, fz, y, z, cur);
+        for (int q = 0; q < 3; ++q) {
+            sC[q][t] = face_tab(k.ax[2].h, fz, q);
+            if (AHEAD) sC[3 + q][t] = face_tab(k.ax[2].e, fz, q);
         }
+    }
+    R iy = k.inv_d, iz = k.inv_d, iyh = k.inv_d, izh = k.inv_d;
+    if (DX == 2) {
+        iy = ldg(k.inv_de[1] + y);
+        iz = ldg(k.inv_de[2] + z);
+        if (AHEAD) { iyh = ldg(k.inv_dh[1] + y); izh = ldg(k.inv_dh[2] + z); }
+    }
+    bool srcs = false;                                           // a point source of the next step in the tile
+    if (AHEAD) {
+        for (int s = 0; s < k.nsrc; ++s) srcs |= own && k.src_j[s] == j;
+        srcs = __any_sync(0xffffffffu, srcs) != 0;
+    }
+    const R *const E0 = k.E, *const E1 = k.E + N, *const E2 = k.E + 2 * N;
+    const R *const H0 = k.HA, *const H1 = k.HA + N, *const H2 = k.HA + 2 * N;
+
+    const bool xf = xa < (uint32_t)k.ax[0].Tn + 1u || (k.ax[0].Tp && (xa == 0u || xb > sx - (uint32_t)k.ax[0].Tp));
+    auto load = [&](uint32_t x, uint32_t i, uint32_t i1, HLoads<R> &v) {
+        const uint32_t ipy = i + dpy, ipz = i + dpz;             // 32-bit wrap arithmetic
+        v.ex1 = ldg(E0 + i1); v.ey1 = ldg(E1 + i1); v.ez1 = ldg(E2 + i1);
+        v.rxy = ldg(E0 + ipy); v.rzy = ldg(E2 + ipy);
+        v.rxz = ldg(E0 + ipz); v.ryz = ldg(E1 + ipz);
+        v.hx = ldg(H0 + i); v.hy = ldg(H1 + i); v.hz = ldg(H2 + i);
+        if (MU) { v.cx = ldg(k.cm + i); v.cy = ldg(k.cm + N + i); v.cz = ldg(k.cm + 2 * N + i); }
+        if (wf && fz.ir >= 0) {
+            const uint32_t ip = psi_at<2>(fz, k.ax[2].Tn, k.ax[2].Tp, x, y, z, sy, sz);
+            v.zu = ldg(face_A(k.ax[2].h, fz, 0) + ip); v.zv = ldg(face_A(k.ax[2].h, fz, 1) + ip);
+        }
+        if (wf && fy.ir >= 0) {
+            const uint32_t ip = psi_at<1>(fy, k.ax[1].Tn, k.ax[1].Tp, x, y, z, sy, sz);
+            v.yu = ldg(face_A(k.ax[1].h, fy, 0) + ip); v.yv = ldg(face_A(k.ax[1].h, fy, 1) + ip);
+        }
+        FaceAt fx;
+        fx.ir = -1;
+        fx.side = 0;
+        if (xf) fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
+        if (fx.ir >= 0) {
+            const uint32_t ip = (uint32_t)fx.ir * syz + j;
+            v.xu = ldg(face_A(k.ax[0].h, fx, 0) + ip); v.xv = ldg(face_A(k.ax[0].h, fx, 1) + ip);
+        }
+    };
+
+    // The march evaluates plane xa - 1 first, without writing: its products and H_new are the x - 1
+    // neighbours of the chunk's first plane.
+    uint32_t x = xa ? xa - 1u : sx - 1u;
+    uint32_t i = x * syz + j;
+    R ex = ldg(E0 + i), ey = ldg(E1 + i), ez = ldg(E2 + i);
+    R p_yx = R(0), p_zx = R(0), p_hy = R(0), p_hz = R(0);
+    HLoads<R> v;
+    uint32_t i1 = xa * syz + j;
+    load(x, i, i1, v);
+    const uint32_t nv = xb - xa + 1u;
+    for (uint32_t n = 0; n < nv; ++n) {
+        const bool wr = own && n > 0u;
+        FaceAt fx;
+        fx.ir = -1;
+        fx.side = 0;
+        if (xf) fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
+        // what the E update after the barrier reads
+        R c0, c1, c2, exu, exv, eyu, eyv, ezu, ezv;
+        if (AHEAD) {
+            c0 = ldg(k.ce + i); c1 = ldg(k.ce + N + i); c2 = ldg(k.ce + 2 * N + i);
+            if (wf && fz.ir >= 0) {
+                const uint32_t ip = psi_at<2>(fz, k.ax[2].Tn, k.ax[2].Tp, x, y, z, sy, sz);
+                ezu = ldg(face_A(k.ax[2].e, fz, 0) + ip); ezv = ldg(face_A(k.ax[2].e, fz, 1) + ip);
+            }
+            if (wf && fy.ir >= 0) {
+                const uint32_t ip = psi_at<1>(fy, k.ax[1].Tn, k.ax[1].Tp, x, y, z, sy, sz);
+                eyu = ldg(face_A(k.ax[1].e, fy, 0) + ip); eyv = ldg(face_A(k.ax[1].e, fy, 1) + ip);
+            }
+            if (fx.ir >= 0) {
+                const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                exu = ldg(face_A(k.ax[0].e, fx, 0) + ip); exv = ldg(face_A(k.ax[0].e, fx, 1) + ip);
+            }
+        }
+        // ---- H (update_h.cl): forward differences (36-43)
+        R d_xy = v.rxy - ex;
+        R d_xz = v.rxz - ex;
+        R d_yx = v.ey1 - ey;
+        R d_yz = v.ryz - ey;
+        R d_zx = v.ez1 - ez;
+        R d_zy = v.rzy - ez;
+        if (DX != 0) {
+            const R ix = DX == 2 ? ldg(k.inv_de[0] + x) : k.inv_d;
+            d_xy = d_xy * iy; d_xz = d_xz * iz; d_yx = d_yx * ix;
+            d_yz = d_yz * iz; d_zx = d_zx * ix; d_zy = d_zy * iy;
+        }
+        // CPML (80-116): at most one face per axis
+        R px = R(0), py = R(0), pz = R(0);
+        if (fx.ir >= 0) {
+            R su, sv;
+            face_update<R, false, 0>(face_tab(k.ax[0].h, fx, 0), face_tab(k.ax[0].h, fx, 1), face_tab(k.ax[0].h, fx, 2),
+                                     v.xu, v.xv, su, sv, d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+            if (wr) {
+                const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                face_B(k.ax[0].h, fx, 0)[ip] = su;
+                face_B(k.ax[0].h, fx, 1)[ip] = sv;
+            }
+        }
+        if (wf && fy.ir >= 0) {
+            R su, sv;
+            face_update<R, false, 1>(face_tab(k.ax[1].h, fy, 0), face_tab(k.ax[1].h, fy, 1), face_tab(k.ax[1].h, fy, 2),
+                                     v.yu, v.yv, su, sv, d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+            if (wr) {
+                const uint32_t ip = psi_at<1>(fy, k.ax[1].Tn, k.ax[1].Tp, x, y, z, sy, sz);
+                face_B(k.ax[1].h, fy, 0)[ip] = su;
+                face_B(k.ax[1].h, fy, 1)[ip] = sv;
+            }
+        }
+        if (wf && fz.ir >= 0) {
+            R su, sv;
+            face_update<R, false, 2>(sC[0][t], sC[1][t], sC[2][t], v.zu, v.zv, su, sv, d_xy, d_xz, d_yx, d_yz, d_zx, d_zy,
+                                     px, py, pz);
+            if (wr) {
+                const uint32_t ip = psi_at<2>(fz, k.ax[2].Tn, k.ax[2].Tp, x, y, z, sy, sz);
+                face_B(k.ax[2].h, fz, 0)[ip] = su;
+                face_B(k.ax[2].h, fz, 1)[ip] = sv;
+            }
+        }
+        // 129-131
+        const R hx = v.hx - (MU ? v.cx : k.dt) * ((d_zy - d_yz) - px);
+        const R hy = v.hy - (MU ? v.cy : k.dt) * ((d_xz - d_zx) - py);
+        const R hz = v.hz - (MU ? v.cz : k.dt) * ((d_yx - d_xy) - pz);
+        R(*const sv)[HS_THREADS] = sV[n & 1u];
+        R s0, s1, s2, o_yx, o_zx;                                // S from the cell's own and the x - 1 products
+        // products (63-70, 135-155)
+        const R ahx = hx + v.hx, ahy = hy + v.hy, ahz = hz + v.hz;
+        const R o_xy = (v.ey1 + ey) * ahz;
+        const R o_xz = (-(v.ez1 + ez)) * ahy;
+        const R o_yz = (v.rzy + ez) * ahx;
+        o_yx = (-(v.rxy + ex)) * ahz;
+        o_zx = (v.rxz + ex) * ahy;
+        const R o_zy = (-(v.ryz + ey)) * ahx;
+        sv[XY][p] = o_xy;
+        sv[ZY][p] = o_zy;
+        sv[XZ][p] = o_xz;
+        sv[YZ][p] = o_yz;
+        s0 = o_xy + o_xz;
+        s1 = o_yz + o_yx;
+        s2 = (o_zx + o_zy) + p_zx;
+        if (!AHEAD && wr && k.write_oS) {
+            k.oS[i] = o_xy;
+            (k.oS + N)[i] = o_yz;
+            (k.oS + 2 * N)[i] = o_zx;
+            (k.oS + 3 * N)[i] = o_xz;
+            (k.oS + 4 * N)[i] = o_yx;
+            (k.oS + 5 * N)[i] = o_zy;
+        }
+        if (AHEAD) {
+            sv[HX][p] = hx;
+            sv[HY][p] = hy;
+            sv[HZ][p] = hz;
+        }
+        const R ox = ex, oy = ey, oz = ez;                       // E at the cell, for its update
+        ex = v.ex1;
+        ey = v.ey1;
+        ez = v.ez1;
+        // the next plane's loads fly during the barrier and what follows it
+        const uint32_t xn = n ? x + 1u : xa;
+        const uint32_t in = i1;
+        i1 = xn + 1u == sx ? j : in + syz;
+        if (n + 1u < nv) load(xn, in, i1, v);
         __syncthreads();
-        if (own) hs_s<R>(k, sS[slot][0], t, z, i, prev_yx, prev_zx);
-        if (PF && act) cur = nxt;
+        if (wr) {
+            k.HB[i] = hx;
+            (k.HB + N)[i] = hy;
+            (k.HB + 2 * N)[i] = hz;
+            if (k.S) {
+                // S (update_s.cl:33-36)
+                k.S[i] = ((s0 + sv[XY][p - ext]) + sv[XZ][p - 1u]) * k.sf;
+                (k.S + N)[i] = ((s1 + sv[YZ][p - 1u]) + p_yx) * k.sf;
+                (k.S + 2 * N)[i] = (s2 + sv[ZY][p - ext]) * k.sf;
+            }
+            if (AHEAD) {
+                // ---- the next step's E (update_e.cl): backward differences (39-46)
+                R e_xy = hx - sv[HX][p - ext];
+                R e_xz = hx - sv[HX][p - 1u];
+                R e_yx = hy - p_hy;
+                R e_yz = hy - sv[HY][p - 1u];
+                R e_zx = hz - p_hz;
+                R e_zy = hz - sv[HZ][p - ext];
+                if (DX != 0) {
+                    const R ix = DX == 2 ? ldg(k.inv_dh[0] + x) : k.inv_d;
+                    e_xy = e_xy * iyh; e_xz = e_xz * izh; e_yx = e_yx * ix;
+                    e_yz = e_yz * izh; e_zx = e_zx * ix; e_zy = e_zy * iyh;
+                }
+                // CPML (64-100)
+                R qx = R(0), qy = R(0), qz = R(0);
+                if (fx.ir >= 0) {
+                    R su, sw;
+                    face_update<R, true, 0>(face_tab(k.ax[0].e, fx, 0), face_tab(k.ax[0].e, fx, 1), face_tab(k.ax[0].e, fx, 2),
+                                            exu, exv, su, sw, e_xy, e_xz, e_yx, e_yz, e_zx, e_zy, qx, qy, qz);
+                    const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                    face_B(k.ax[0].e, fx, 0)[ip] = su;
+                    face_B(k.ax[0].e, fx, 1)[ip] = sw;
+                }
+                if (wf && fy.ir >= 0) {
+                    R su, sw;
+                    face_update<R, true, 1>(face_tab(k.ax[1].e, fy, 0), face_tab(k.ax[1].e, fy, 1), face_tab(k.ax[1].e, fy, 2),
+                                            eyu, eyv, su, sw, e_xy, e_xz, e_yx, e_yz, e_zx, e_zy, qx, qy, qz);
+                    const uint32_t ip = psi_at<1>(fy, k.ax[1].Tn, k.ax[1].Tp, x, y, z, sy, sz);
+                    face_B(k.ax[1].e, fy, 0)[ip] = su;
+                    face_B(k.ax[1].e, fy, 1)[ip] = sw;
+                }
+                if (wf && fz.ir >= 0) {
+                    R su, sw;
+                    face_update<R, true, 2>(sC[3][t], sC[4][t], sC[5][t], ezu, ezv, su, sw, e_xy, e_xz, e_yx, e_yz, e_zx,
+                                            e_zy, qx, qy, qz);
+                    const uint32_t ip = psi_at<2>(fz, k.ax[2].Tn, k.ax[2].Tp, x, y, z, sy, sz);
+                    face_B(k.ax[2].e, fz, 0)[ip] = su;
+                    face_B(k.ax[2].e, fz, 1)[ip] = sw;
+                }
+                // 105-107
+                R nx = ox + c0 * ((e_zy - e_yz) + qx);
+                R ny = oy + c1 * ((e_xz - e_zx) + qy);
+                R nz = oz + c2 * ((e_yx - e_xy) + qz);
+                if (srcs) {
+                    // point sources in list order (fdtd.py:168-169)
+                    for (int s = 0; s < k.nsrc; ++s) {
+                        if (k.src_x[s] != x || k.src_j[s] != j) continue;
+                        const R val = k.src_values[(int64_t)k.src_t * k.src_stride + k.src_col[s]];
+                        if (k.src_c[s] == 0) nx = nx + val;
+                        else if (k.src_c[s] == 1) ny = ny + val;
+                        else nz = nz + val;
+                    }
+                }
+                k.EB[i] = nx;
+                (k.EB + N)[i] = ny;
+                (k.EB + 2 * N)[i] = nz;
+            }
+        }
+        p_yx = o_yx;
+        p_zx = o_zx;
+        if (AHEAD) {
+            p_hy = hy;
+            p_hz = hz;
+        }
+        x = xn;
+        i = in;
     }
 }
 
-template <typename R, int DX, bool PF>
-static cudaError_t launch_hs_dx(const HSK<R> &k, bool mu, dim3 g, bool pdl, cudaStream_t st)
+// Double precision is bound by its arithmetic units, for which evaluating the halo again costs more
+// than the memory passes saved: only the form without the next step's E exists there. With the next
+// step's E, Poynting may be off (S NULL: the products are formed and S is not written).
+template <typename R, int DX, bool MU>
+static void (*hs_kernel_mu(const HSForm &f))(HSK<R>)
 {
-    if (mu) return launch_dependent(k_bulk_hs<R, DX, true, PF>, g, HS_THREADS, st, pdl, k);
-    return launch_dependent(k_bulk_hs<R, DX, false, PF>, g, HS_THREADS, st, pdl, k);
+    if constexpr (sizeof(R) == 4)
+        if (f.ahead) return k_tile_h<R, DX, MU, true>;
+    return f.poynting && !f.ahead ? k_tile_h<R, DX, MU, false> : nullptr;
 }
 
-template <typename R, bool PF>
-static cudaError_t launch_hs_pf(const HSK<R> &k, bool mu, int dxmode, dim3 g, bool pdl, cudaStream_t st)
+template <typename R, int DX>
+static void (*hs_kernel_dx(const HSForm &f))(HSK<R>)
 {
-    if (dxmode == 0) return launch_hs_dx<R, 0, PF>(k, mu, g, pdl, st);
-    if (dxmode == 1) return launch_hs_dx<R, 1, PF>(k, mu, g, pdl, st);
-    return launch_hs_dx<R, 2, PF>(k, mu, g, pdl, st);
+    return f.mu ? hs_kernel_mu<R, DX, true>(f) : hs_kernel_mu<R, DX, false>(f);
 }
 
 template <typename R>
-cudaError_t launch_hs(const HSK<R> &k, bool mu, int dxmode, bool prefetch, bool pdl, cudaStream_t st)
+static void (*hs_kernel(const HSForm &f))(HSK<R>)
 {
-    const dim3 g(k.nrowblk * k.nchunk + (k.dft_on ? 1u : 0u), 1, 1);
-    if (prefetch) return launch_hs_pf<R, true>(k, mu, dxmode, g, pdl, st);
-    return launch_hs_pf<R, false>(k, mu, dxmode, g, pdl, st);
+    return f.dxmode == 0 ? hs_kernel_dx<R, 0>(f) : f.dxmode == 1 ? hs_kernel_dx<R, 1>(f) : hs_kernel_dx<R, 2>(f);
 }
 
-template cudaError_t launch_hs<float>(const HSK<float> &, bool, int, bool, bool, cudaStream_t);
-template cudaError_t launch_hs<double>(const HSK<double> &, bool, int, bool, bool, cudaStream_t);
+template <typename R>
+bool hs_form_exists(const HSForm &f)
+{
+    return hs_kernel<R>(f) != nullptr;
+}
+
+template <typename R>
+cudaError_t launch_hs(const HSK<R> &k, const HSForm &f, bool pdl, cudaStream_t st)
+{
+    const dim3 g(k.ntile * k.nchunk + (k.dft_on ? 1u : 0u), 1, 1);
+    return launch_dependent(hs_kernel<R>(f), g, (unsigned)hs_threads(f.ahead, f.mu, f.dxmode), st, pdl, k);
+}
+
+template bool hs_form_exists<float>(const HSForm &);
+template bool hs_form_exists<double>(const HSForm &);
+template cudaError_t launch_hs<float>(const HSK<float> &, const HSForm &, bool, cudaStream_t);
+template cudaError_t launch_hs<double>(const HSK<double> &, const HSForm &, bool, cudaStream_t);
 
 }  // namespace fdtd

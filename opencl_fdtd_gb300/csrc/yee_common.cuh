@@ -47,19 +47,19 @@ __device__ __forceinline__ void grid_dependency_sync()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launches kern<<<g, block, 0, st>>>(arg), with programmatic stream serialization when pdl.
+// Launches kern<<<g, block, smem, st>>>(arg), with programmatic stream serialization when pdl.
 template <typename K>
 inline cudaError_t launch_dependent(void (*kern)(K), dim3 g, unsigned block, cudaStream_t st,
-                                    bool pdl, const K &arg)
+                                    bool pdl, const K &arg, size_t smem = 0)
 {
     if (!pdl) {
-        kern<<<g, block, 0, st>>>(arg);
+        kern<<<g, block, smem, st>>>(arg);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = g;
     cfg.blockDim = dim3(block, 1, 1);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -69,15 +69,24 @@ inline cudaError_t launch_dependent(void (*kern)(K), dim3 g, unsigned block, cud
     return cudaLaunchKernelEx(&cfg, kern, arg);
 }
 
-// CPML faces of one axis as the bulk kernels see them: the low ('n') face covers
-// c < Tn, the high ('p') face c >= s - Tp (Tp = 0 when the face never applies). Faces of one
-// axis never overlap in a bulk launch (the plan falls back to the generic kernels then), so
-// every cell sees at most one face per axis and the order of faces cannot change a result.
+// The CPML faces of one axis for one update: coefficient tables [n/p][p0,p1,p2], the auxiliary
+// arrays read (A) and written (B), [n/p][u/v]; A and B are the same arrays when the update runs in
+// place.
+template <typename R>
+struct FacePsi {
+    const R *tab[2][3];
+    const R *A[2][2];
+    R *B[2][2];
+};
+
+// Faces of one axis as the bulk kernels see them: the low ('n') face covers c < Tn, the high ('p')
+// face c >= s - Tp (Tp = 0 when the face never applies). Faces of one axis never overlap in a bulk
+// launch (the plan falls back to the generic kernels then), so every cell sees at most one face
+// per axis and the order of faces cannot change a result.
 template <typename R>
 struct AxisK {
     int32_t Tn, Tp;
-    const R *n0, *n1, *n2, *p0, *p1, *p2;
-    R *nu, *nv, *pu, *pv;
+    FacePsi<R> f;
 };
 
 // One CPML face as one update kernel sees it (E tables for E-type kernels, H tables for
@@ -99,7 +108,8 @@ constexpr int YEE_SRC = 8;       // point sources the bulk E kernel can add itse
 
 template <typename R>
 struct YeeK {
-    R *P;
+    R *P;                       // the updated field; the bulk kernels read it here
+    R *W;                       // and write it here (P itself in place)
     const R *Q;
     const R *Rp;
     const R *mat;
@@ -115,7 +125,8 @@ struct YeeK {
     FaceK<R> face[6];
     AxisK<R> ax[3];
     FastDiv dsz;
-    int32_t xchunk, bulk;
+    uint32_t xchunk;            // x planes a bulk-kernel thread marches (0: chosen by the launcher)
+    int32_t bulk;               // 1: the bulk kernels apply
     uint32_t xbeg, xend;        // planes [xbeg, xend) this launch updates
     // point sources the bulk E kernel adds after the update, in list order (fdtd.py:168-169):
     // E[c][x, j] += src_values[src_t * src_stride + src_col] for each of nsrc sources
@@ -133,7 +144,7 @@ struct SK {
     uint64_t N;
     R sf;
     FastDiv dsz;
-    int32_t xchunk, _pad;
+    uint32_t xchunk;
     uint32_t xbeg, xend;        // planes [xbeg, xend) this launch updates
 };
 

@@ -1,4 +1,4 @@
-// Device helpers shared by the per-update kernels (yee_kernels.cu) and the H+S kernel
+// Device helpers shared by the per-update kernels (yee_kernels.cu) and the H kernel of fdtd_run
 // (hs_fused.cu): read-only loads, CPML depth lookup and the per-face CPML arithmetic.
 #pragma once
 
@@ -51,66 +51,90 @@ __device__ __forceinline__ uint32_t psi_index(uint32_t ir, uint32_t T, uint32_t 
     return (x * sy + y) * T + ir;
 }
 
-// Per-thread view of one axis's CPML faces for a coordinate that stays fixed during the march
-// (y or z): depth index, thickness and coefficients, or ir < 0 outside both faces.
-template <typename R>
-struct FixedFace {
-    int ir;
-    uint32_t T;
-    R p0, p1, p2;
-    R *pu, *pv;
+// CPML face of one axis for a coordinate: depth ir (-1 outside) and side (0 = 'n', 1 = 'p').
+struct FaceAt {
+    int ir, side;
 };
 
-template <typename R, bool ETYPE>
-__device__ __forceinline__ FixedFace<R> fixed_face(const AxisK<R> &a, uint32_t s, uint32_t c)
+__device__ __forceinline__ FaceAt face_at(int Tn, int Tp, uint32_t s, uint32_t c)
 {
-    FixedFace<R> f;
+    FaceAt f;
     f.ir = -1;
-    f.T = 0;
-    f.p0 = f.p1 = f.p2 = R(0);
-    f.pu = f.pv = nullptr;
-    if (c < (uint32_t)a.Tn) {
+    f.side = 0;
+    if (c < (uint32_t)Tn) {
         f.ir = (int)c;
-        f.T = (uint32_t)a.Tn;
-        f.p0 = ldg(a.n0 + c); f.p1 = ldg(a.n1 + c); f.p2 = ldg(a.n2 + c);
-        f.pu = a.nu;
-        f.pv = a.nv;
-    } else if (a.Tp && c >= s - (uint32_t)a.Tp) {
-        const uint32_t ir = s - 1u - c;
-        f.ir = (int)ir;
-        f.T = (uint32_t)a.Tp;
-        f.p0 = ldg(a.p0 + ir); f.p1 = ldg(a.p1 + ir); f.p2 = ldg(a.p2 + ir);
-        f.pu = a.pu;
-        f.pv = a.pv;
+    } else if (Tp && c >= s - (uint32_t)Tp) {
+        f.ir = (int)(s - 1u - c);
+        f.side = 1;
     }
     return f;
 }
 
-// x-face of plane x (uniform across the block): depth, thickness and psi arrays
+// coefficient c (p0, p1, p2) at the face's depth; psi arrays read and written
 template <typename R>
-struct XFace {
-    int ir;
-    uint32_t T;
-    const R *t0, *t1, *t2;
-    R *pu, *pv;
-};
+__device__ __forceinline__ R face_tab(const FacePsi<R> &a, const FaceAt &f, int c)
+{
+    return ldg((f.side ? a.tab[1][c] : a.tab[0][c]) + f.ir);
+}
 
 template <typename R>
-__device__ __forceinline__ XFace<R> x_face(const AxisK<R> &a, uint32_t sx, uint32_t x)
+__device__ __forceinline__ const R *face_A(const FacePsi<R> &a, const FaceAt &f, int c)
 {
-    XFace<R> f;
+    return f.side ? a.A[1][c] : a.A[0][c];
+}
+
+template <typename R>
+__device__ __forceinline__ R *face_B(const FacePsi<R> &a, const FaceAt &f, int c)
+{
+    return f.side ? a.B[1][c] : a.B[0][c];
+}
+
+// Per-thread view of one axis's CPML faces for a coordinate that stays fixed during the march
+// (y or z): depth index (ir < 0 outside both faces), thickness, coefficients and psi arrays. AWAY:
+// psi is written to other arrays than it is read from.
+template <typename R, bool AWAY>
+struct FixedFace {
+    int ir;
+    uint32_t T;
+    R p0, p1, p2;
+    R *pu, *pv;                 // written, and read unless AWAY
+    const R *ru, *rv;
+
+    __device__ __forceinline__ R u(uint32_t i) const { return AWAY ? ru[i] : pu[i]; }
+    __device__ __forceinline__ R v(uint32_t i) const { return AWAY ? rv[i] : pv[i]; }
+};
+
+template <typename R, bool AWAY>
+__device__ __forceinline__ FixedFace<R, AWAY> fixed_face(const AxisK<R> &a, uint32_t s, uint32_t c, bool act)
+{
+    FixedFace<R, AWAY> f;
     f.ir = -1;
     f.T = 0;
-    f.t0 = f.t1 = f.t2 = nullptr;
+    f.p0 = f.p1 = f.p2 = R(0);
     f.pu = f.pv = nullptr;
-    if (x < (uint32_t)a.Tn) {
-        f.ir = (int)x; f.T = (uint32_t)a.Tn;
-        f.t0 = a.n0; f.t1 = a.n1; f.t2 = a.n2; f.pu = a.nu; f.pv = a.nv;
-    } else if (a.Tp && x >= sx - (uint32_t)a.Tp) {
-        f.ir = (int)(sx - 1u - x); f.T = (uint32_t)a.Tp;
-        f.t0 = a.p0; f.t1 = a.p1; f.t2 = a.p2; f.pu = a.pu; f.pv = a.pv;
+    f.ru = f.rv = nullptr;
+    const FaceAt at = face_at(a.Tn, a.Tp, s, c);
+    if (act && at.ir >= 0) {
+        f.ir = at.ir;
+        f.T = (uint32_t)(at.side ? a.Tp : a.Tn);
+        f.p0 = face_tab(a.f, at, 0);
+        f.p1 = face_tab(a.f, at, 1);
+        f.p2 = face_tab(a.f, at, 2);
+        f.pu = face_B(a.f, at, 0);
+        f.pv = face_B(a.f, at, 1);
+        if (AWAY) {
+            f.ru = face_A(a.f, at, 0);
+            f.rv = face_A(a.f, at, 1);
+        }
     }
     return f;
+}
+
+// True when an x face covers a plane of [xa, xb): what a block asks once, before its march.
+template <typename R>
+__device__ __forceinline__ bool x_faces(const AxisK<R> &a, uint32_t sx, uint32_t xa, uint32_t xb)
+{
+    return xa < (uint32_t)a.Tn || (a.Tp && xb > sx - (uint32_t)a.Tp);
 }
 
 }  // namespace fdtd

@@ -253,18 +253,21 @@ struct EForm {
     static constexpr int min_blocks = FORM == 0 ? EMINB : 4;
 };
 
-template <typename R, int DX, bool BLOCH, int FORM>
+template <typename R, int DX, bool BLOCH, int FORM, bool AWAY>
 __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(const YeeK<R> k)
 {
     constexpr bool PF = EForm<FORM>::prefetch;
     grid_dependency_sync();
     const uint32_t j = blockIdx.x * EBLOCK + threadIdx.x;
-    if (j >= k.syz) return;
+    const bool act = j < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
     const uint32_t y = k.dsz.div(j);
     const uint32_t z = j - y * sz;
-    const uint32_t xa = k.xbeg + blockIdx.y * (uint32_t)k.xchunk;
-    const uint32_t xb = min(xa + (uint32_t)k.xchunk, k.xend);
+    const FixedFace<R, AWAY> fy = fixed_face<R, AWAY>(k.ax[1], sy, y, act);
+    const FixedFace<R, AWAY> fz = fixed_face<R, AWAY>(k.ax[2], sz, z, act);
+    if (!act) return;
+    const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
+    const uint32_t xb = min(xa + k.xchunk, k.xend);
     const uint64_t N = k.N;
     const R *__restrict__ Qx = k.Q;
     const R *__restrict__ Qy = k.Q + N;
@@ -272,23 +275,25 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
     const R *__restrict__ Cx = k.coef;
     const R *__restrict__ Cy = k.coef + N;
     const R *__restrict__ Cz = k.coef + 2 * N;
+    // W may be P itself: a thread reads its own cells of P only, each before it writes it
     R *__restrict__ Px = k.P;
     R *__restrict__ Py = k.P + N;
     R *__restrict__ Pz = k.P + 2 * N;
+    R *__restrict__ Wx = AWAY ? k.W : k.P;
+    R *__restrict__ Wy = AWAY ? k.W + N : Py;
+    R *__restrict__ Wz = AWAY ? k.W + 2 * N : Pz;
     // y/z minus neighbours with periodic wrap (common.cl:75-81), fixed for the thread
     const uint32_t dmy = y ? 0u - sz : (sy - 1u) * sz;
     const uint32_t dmz = z ? 0xffffffffu : sz - 1u;
     const bool by = BLOCH && (k.bloch_mask & 2) && y == 0;
     const bool bz = BLOCH && (k.bloch_mask & 4) && z == 0;
-    const FixedFace<R> fy = fixed_face<R, true>(k.ax[1], sy, y);
-    const FixedFace<R> fz = fixed_face<R, true>(k.ax[2], sz, z);
     R iy = k.inv_d, iz = k.inv_d;
     if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
     // a point source in this block's cells and planes (block-uniform)
     bool srcs = false;
     for (int s = 0; s < k.nsrc; ++s)
         srcs |= k.src_j[s] / (uint32_t)EBLOCK == blockIdx.x &&
-                (k.src_x[s] - k.xbeg) / (uint32_t)k.xchunk == blockIdx.y;
+                (k.src_x[s] - k.xbeg) / k.xchunk == blockIdx.y;
 
     auto load = [&](uint32_t x, uint32_t i) {
         ELoad<R> v;
@@ -303,18 +308,18 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
         v.ex = Px[i]; v.ey = Py[i]; v.ez = Pz[i];
         v.cx = ldg(Cx + i); v.cy = ldg(Cy + i); v.cz = ldg(Cz + i);
         v.xu = v.xv = v.yu = v.yv = v.zu = v.zv = R(0);
-        const XFace<R> fx = x_face<R>(k.ax[0], sx, x);
+        const FaceAt fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
         if (fx.ir >= 0) {
-            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, fx.T, x, y, z, sy, sz);
-            v.xu = fx.pu[ip]; v.xv = fx.pv[ip];
+            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, 0u, x, y, z, sy, sz);
+            v.xu = face_A(k.ax[0].f, fx, 0)[ip]; v.xv = face_A(k.ax[0].f, fx, 1)[ip];
         }
         if (fy.ir >= 0) {
             const uint32_t ip = psi_index<1>((uint32_t)fy.ir, fy.T, x, y, z, sy, sz);
-            v.yu = fy.pu[ip]; v.yv = fy.pv[ip];
+            v.yu = fy.u(ip); v.yv = fy.v(ip);
         }
         if (fz.ir >= 0) {
             const uint32_t ip = psi_index<2>((uint32_t)fz.ir, fz.T, x, y, z, sy, sz);
-            v.zu = fz.pu[ip]; v.zv = fz.pv[ip];
+            v.zu = fz.u(ip); v.zv = fz.v(ip);
         }
         return v;
     };
@@ -353,13 +358,13 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
         }
         // CPML (update_e.cl:64-100): at most one face per axis
         R px = R(0), py = R(0), pz = R(0);
-        const XFace<R> fx = x_face<R>(k.ax[0], sx, x);
+        const FaceAt fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
         if (fx.ir >= 0) {
             R su, sv;
-            face_update<R, true, 0>(ldg(fx.t0 + fx.ir), ldg(fx.t1 + fx.ir), ldg(fx.t2 + fx.ir),
+            face_update<R, true, 0>(face_tab(k.ax[0].f, fx, 0), face_tab(k.ax[0].f, fx, 1), face_tab(k.ax[0].f, fx, 2),
                                     cur.xu, cur.xv, su, sv, d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, fx.T, x, y, z, sy, sz);
-            fx.pu[ip] = su; fx.pv[ip] = sv;
+            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, 0u, x, y, z, sy, sz);
+            face_B(k.ax[0].f, fx, 0)[ip] = su; face_B(k.ax[0].f, fx, 1)[ip] = sv;
         }
         if (fy.ir >= 0) {
             R su, sv;
@@ -389,9 +394,9 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
                 else ez = ez + val;
             }
         }
-        Px[i] = ex;
-        Py[i] = ey;
-        Pz[i] = ez;
+        (AWAY ? Wx : Px)[i] = ex;
+        (AWAY ? Wy : Py)[i] = ey;
+        (AWAY ? Wz : Pz)[i] = ez;
         hy_m = cur.hy;
         hz_m = cur.hz;
         if (PF) cur = nxt;
@@ -410,31 +415,46 @@ struct HLoad {
     R xu, xv, yu, yv, zu, zv;     // psi of the faces the cell is in
 };
 
-template <typename R, int DX, bool MU, bool POYNT, bool BLOCH>
-__global__ void __launch_bounds__(BLOCK, 3) k_bulk_h(const YeeK<R> k)
+// Forms of the bulk H kernel, as those of E: with the next plane loaded one iteration ahead at three
+// blocks per SM (80 registers); with dt/mu or Bloch partners, whose values would spill there, with each
+// plane loaded when it is updated, at four (64 registers).
+constexpr bool h_prefetch(bool mu, bool bloch) { return !mu && !bloch; }
+constexpr int h_min_blocks(bool mu, bool bloch) { return h_prefetch(mu, bloch) ? 3 : 4; }
+
+template <typename R, int DX, bool MU, bool POYNT, bool BLOCH, bool AWAY>
+__global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH)) k_bulk_h(const YeeK<R> k)
 {
+    constexpr bool PF = h_prefetch(MU, BLOCH);
+    grid_dependency_sync();
     const uint32_t j = blockIdx.x * BLOCK + threadIdx.x;
-    if (j >= k.syz) return;
+    const bool act = j < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
     const uint32_t y = k.dsz.div(j);
     const uint32_t z = j - y * sz;
-    const uint32_t xa = k.xbeg + blockIdx.y * (uint32_t)k.xchunk;
-    const uint32_t xb = min(xa + (uint32_t)k.xchunk, k.xend);
+    const FixedFace<R, AWAY> fy = fixed_face<R, AWAY>(k.ax[1], sy, y, act);
+    const FixedFace<R, AWAY> fz = fixed_face<R, AWAY>(k.ax[2], sz, z, act);
+    const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
+    if (!act) return;
+    const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
+    const uint32_t xb = min(xa + k.xchunk, k.xend);
+    const bool xf = x_faces(k.ax[0], sx, xa, xb);
     const uint64_t N = k.N;
     const R *__restrict__ Qx = k.Q;
     const R *__restrict__ Qy = k.Q + N;
     const R *__restrict__ Qz = k.Q + 2 * N;
-    R *__restrict__ Px = k.P;
-    R *__restrict__ Py = k.P + N;
-    R *__restrict__ Pz = k.P + 2 * N;
+    // W may be P itself: a thread reads its own cells of P only, each before it writes it
+    const R *__restrict__ Px = k.P;
+    const R *__restrict__ Py = k.P + N;
+    const R *__restrict__ Pz = k.P + 2 * N;
+    R *__restrict__ Wx = k.W;
+    R *__restrict__ Wy = k.W + N;
+    R *__restrict__ Wz = k.W + 2 * N;
     // y/z plus neighbours with periodic wrap (common.cl:82-84), fixed for the thread
     const uint32_t dpy = (y + 1u < sy) ? sz : 0u - (sy - 1u) * sz;
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
     const bool bx = BLOCH && (k.bloch_mask & 1) != 0;
     const bool by = BLOCH && (k.bloch_mask & 2) && y + 1u == sy;
     const bool bz = BLOCH && (k.bloch_mask & 4) && z + 1u == sz;
-    const FixedFace<R> fy = fixed_face<R, false>(k.ax[1], sy, y);
-    const FixedFace<R> fz = fixed_face<R, false>(k.ax[2], sz, z);
     R iy = k.inv_d, iz = k.inv_d;
     if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
     const R dt = k.dt;
@@ -455,28 +475,34 @@ __global__ void __launch_bounds__(BLOCK, 3) k_bulk_h(const YeeK<R> k)
         v.cx = v.cy = v.cz = R(0);
         if (MU) { v.cx = ldg(k.coef + i); v.cy = ldg(k.coef + N + i); v.cz = ldg(k.coef + 2 * N + i); }
         v.xu = v.xv = v.yu = v.yv = v.zu = v.zv = R(0);
-        const XFace<R> fx = x_face<R>(k.ax[0], sx, x);
-        if (fx.ir >= 0) {
-            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, fx.T, x, y, z, sy, sz);
-            v.xu = fx.pu[ip]; v.xv = fx.pv[ip];
+        if (xf) {
+            const FaceAt fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
+            if (fx.ir >= 0) {
+                const uint32_t ip = psi_index<0>((uint32_t)fx.ir, 0u, x, y, z, sy, sz);
+                v.xu = face_A(k.ax[0].f, fx, 0)[ip]; v.xv = face_A(k.ax[0].f, fx, 1)[ip];
+            }
         }
-        if (fy.ir >= 0) {
-            const uint32_t ip = psi_index<1>((uint32_t)fy.ir, fy.T, x, y, z, sy, sz);
-            v.yu = fy.pu[ip]; v.yv = fy.pv[ip];
-        }
-        if (fz.ir >= 0) {
-            const uint32_t ip = psi_index<2>((uint32_t)fz.ir, fz.T, x, y, z, sy, sz);
-            v.zu = fz.pu[ip]; v.zv = fz.pv[ip];
+        if (wf) {
+            if (fy.ir >= 0) {
+                const uint32_t ip = psi_index<1>((uint32_t)fy.ir, fy.T, x, y, z, sy, sz);
+                v.yu = fy.u(ip); v.yv = fy.v(ip);
+            }
+            if (fz.ir >= 0) {
+                const uint32_t ip = psi_index<2>((uint32_t)fz.ir, fz.T, x, y, z, sy, sz);
+                v.zu = fz.u(ip); v.zv = fz.v(ip);
+            }
         }
         return v;
     };
 
     uint32_t i = xa * syz + j;
     R ex = ldg(Qx + i), ey = ldg(Qy + i), ez = ldg(Qz + i);
-    HLoad<R> cur = load(xa, i);
+    HLoad<R> cur;
+    if (PF) cur = load(xa, i);
     for (uint32_t x = xa; x < xb; ++x, i += syz) {
         HLoad<R> nxt;
-        if (x + 1u < xb) nxt = load(x + 1u, i + syz);
+        if (!PF) cur = load(x, i);
+        else if (x + 1u < xb) nxt = load(x + 1u, i + syz);
         R n_yx = cur.ey1, n_zx = cur.ez1, n_xy = cur.rxy, n_zy = cur.rzy, n_xz = cur.rxz, n_yz = cur.ryz;
         if (bx && x + 1u == sx) { n_yx = n_yx * k.br[0] + cur.byx * k.bi[0]; n_zx = n_zx * k.br[0] + cur.bzx * k.bi[0]; }
         if (by) { n_xy = n_xy * k.br[1] + cur.bxy * k.bi[1]; n_zy = n_zy * k.br[1] + cur.bzy * k.bi[1]; }
@@ -495,27 +521,31 @@ __global__ void __launch_bounds__(BLOCK, 3) k_bulk_h(const YeeK<R> k)
         }
         // CPML (update_h.cl:80-116): at most one face per axis
         R px = R(0), py = R(0), pz = R(0);
-        const XFace<R> fx = x_face<R>(k.ax[0], sx, x);
-        if (fx.ir >= 0) {
-            R su, sv;
-            face_update<R, false, 0>(ldg(fx.t0 + fx.ir), ldg(fx.t1 + fx.ir), ldg(fx.t2 + fx.ir),
-                                     cur.xu, cur.xv, su, sv, d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-            const uint32_t ip = psi_index<0>((uint32_t)fx.ir, fx.T, x, y, z, sy, sz);
-            fx.pu[ip] = su; fx.pv[ip] = sv;
+        if (xf) {
+            const FaceAt fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
+            if (fx.ir >= 0) {
+                R su, sv;
+                face_update<R, false, 0>(face_tab(k.ax[0].f, fx, 0), face_tab(k.ax[0].f, fx, 1), face_tab(k.ax[0].f, fx, 2),
+                                        cur.xu, cur.xv, su, sv, d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = psi_index<0>((uint32_t)fx.ir, 0u, x, y, z, sy, sz);
+                face_B(k.ax[0].f, fx, 0)[ip] = su; face_B(k.ax[0].f, fx, 1)[ip] = sv;
+            }
         }
-        if (fy.ir >= 0) {
-            R su, sv;
-            face_update<R, false, 1>(fy.p0, fy.p1, fy.p2, cur.yu, cur.yv, su, sv,
-                                     d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-            const uint32_t ip = psi_index<1>((uint32_t)fy.ir, fy.T, x, y, z, sy, sz);
-            fy.pu[ip] = su; fy.pv[ip] = sv;
-        }
-        if (fz.ir >= 0) {
-            R su, sv;
-            face_update<R, false, 2>(fz.p0, fz.p1, fz.p2, cur.zu, cur.zv, su, sv,
-                                     d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-            const uint32_t ip = psi_index<2>((uint32_t)fz.ir, fz.T, x, y, z, sy, sz);
-            fz.pu[ip] = su; fz.pv[ip] = sv;
+        if (wf) {
+            if (fy.ir >= 0) {
+                R su, sv;
+                face_update<R, false, 1>(fy.p0, fy.p1, fy.p2, cur.yu, cur.yv, su, sv,
+                                        d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = psi_index<1>((uint32_t)fy.ir, fy.T, x, y, z, sy, sz);
+                fy.pu[ip] = su; fy.pv[ip] = sv;
+            }
+            if (fz.ir >= 0) {
+                R su, sv;
+                face_update<R, false, 2>(fz.p0, fz.p1, fz.p2, cur.zu, cur.zv, su, sv,
+                                        d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = psi_index<2>((uint32_t)fz.ir, fz.T, x, y, z, sy, sz);
+                fz.pu[ip] = su; fz.pv[ip] = sv;
+            }
         }
         R hx, hy, hz;
         if (MU) {
@@ -528,9 +558,9 @@ __global__ void __launch_bounds__(BLOCK, 3) k_bulk_h(const YeeK<R> k)
             hy = cur.hy - dt * ((d_xz - d_zx) - py);
             hz = cur.hz - dt * ((d_yx - d_xy) - pz);
         }
-        Px[i] = hx;
-        Py[i] = hy;
-        Pz[i] = hz;
+        Wx[i] = hx;
+        Wy[i] = hy;
+        Wz[i] = hz;
         if (POYNT) {
             // E averaged in space with the plain wrapped neighbours, H in time
             // (update_h.cl:63-70, 135-137); planes xy, yz, zx, xz, yx, zy (update_h.cl:142-154)
@@ -546,7 +576,7 @@ __global__ void __launch_bounds__(BLOCK, 3) k_bulk_h(const YeeK<R> k)
         ex = cur.ex1;
         ey = cur.ey1;
         ez = cur.ez1;
-        cur = nxt;
+        if (PF) cur = nxt;
     }
 }
 
@@ -565,8 +595,8 @@ __global__ void __launch_bounds__(BLOCK) k_bulk_s(const SK<R> k)
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
     const uint32_t y = k.dsz.div(j);
     const uint32_t z = j - y * sz;
-    const uint32_t xa = k.xbeg + blockIdx.y * (uint32_t)k.xchunk;
-    const uint32_t xb = min(xa + (uint32_t)k.xchunk, k.xend);
+    const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
+    const uint32_t xb = min(xa + k.xchunk, k.xend);
     const uint64_t N = k.N;
     const R *__restrict__ oxy = k.oS;
     const R *__restrict__ oyz = k.oS + N;
@@ -647,9 +677,27 @@ __global__ void k_point_sources(const PointK<R> k)
 }
 
 // ---- launchers ------------------------------------------------------------------------------
-static inline dim3 bulk_grid(uint32_t syz, uint32_t nx, int xchunk, uint32_t block = BLOCK)
+static uint32_t sm_count()
 {
-    return dim3((syz + block - 1) / block, (nx + (uint32_t)xchunk - 1) / (uint32_t)xchunk, 1);
+    static int n[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1u;
+    if (!n[dev] && cudaDeviceGetAttribute(&n[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n[dev] = 1;
+    return (uint32_t)n[dev];
+}
+
+// x planes a thread of a bulk kernel marches when none is set (xchunk 0): 8, or on grids too small to
+// fill the GPU that way the most that still gives every SM its resident blocks (1 at least), since
+// such a launch takes as long as one thread's march.
+template <typename K>
+static dim3 bulk_grid(K &k, uint32_t block, uint32_t resident)
+{
+    const uint32_t nj = (k.syz + block - 1) / block, nx = k.xend - k.xbeg;
+    if (!k.xchunk) {
+        const uint64_t slots = (uint64_t)sm_count() * resident, all = (uint64_t)nj * nx;
+        k.xchunk = all >= 8u * slots ? 8u : (uint32_t)(all / slots > 1u ? all / slots : 1u);
+    }
+    return dim3(nj, (nx + k.xchunk - 1) / k.xchunk, 1);
 }
 
 static inline dim3 plane_grid(uint32_t syz, uint32_t nx)
@@ -657,58 +705,59 @@ static inline dim3 plane_grid(uint32_t syz, uint32_t nx)
     return dim3((syz + BLOCK - 1) / BLOCK, nx, 1);
 }
 
+// away: the result goes to other arrays (the first step of fdtd_run's E-ahead path; no Bloch there)
 template <typename R, bool BLOCH, int DX>
-static void (*bulk_e_form(int form))(YeeK<R>)
+static void (*bulk_e_form(int form, bool away))(YeeK<R>)
 {
-    if (form == 1) return k_bulk_e<R, DX, BLOCH, 1>;
-    return k_bulk_e<R, DX, BLOCH, 0>;
+    if (!BLOCH && away) return k_bulk_e<R, DX, false, 1, true>;
+    if (form == 1) return k_bulk_e<R, DX, BLOCH, 1, false>;
+    return k_bulk_e<R, DX, BLOCH, 0, false>;
 }
 
 template <typename R, bool BLOCH>
-static void (*bulk_e_kernel(int dxmode, int form))(YeeK<R>)
+static void (*bulk_e_kernel(int dxmode, int form, bool away))(YeeK<R>)
 {
-    if (dxmode == 0) return bulk_e_form<R, BLOCH, 0>(form);
-    if (dxmode == 1) return bulk_e_form<R, BLOCH, 1>(form);
-    return bulk_e_form<R, BLOCH, 2>(form);
+    if (dxmode == 0) return bulk_e_form<R, BLOCH, 0>(form, away);
+    if (dxmode == 1) return bulk_e_form<R, BLOCH, 1>(form, away);
+    return bulk_e_form<R, BLOCH, 2>(form, away);
 }
 
 template <typename R>
-cudaError_t launch_yee_e(const YeeK<R> &k, cudaStream_t st, bool pdl)
+cudaError_t launch_yee_e(const YeeK<R> &kk, cudaStream_t st, bool pdl)
 {
+    YeeK<R> k = kk;
     if (k.xend <= k.xbeg) return cudaSuccess;
     if (!k.bulk) {
         k_generic_e<R><<<plane_grid(k.syz, k.xend - k.xbeg), BLOCK, 0, st>>>(k);
         return cudaGetLastError();
     }
-    const dim3 g = bulk_grid(k.syz, k.xend - k.xbeg, k.xchunk, EBLOCK);
+    const dim3 g = bulk_grid(k, EBLOCK, 4u);
     const int f = k.eform;
-    return launch_dependent(k.bloch_mask ? bulk_e_kernel<R, true>(k.dxmode, f) : bulk_e_kernel<R, false>(k.dxmode, f),
+    const bool away = k.W != k.P;
+    return launch_dependent(k.bloch_mask ? bulk_e_kernel<R, true>(k.dxmode, f, away) : bulk_e_kernel<R, false>(k.dxmode, f, away),
                             g, EBLOCK, st, pdl, k);
 }
 
+// away: as above (the last step of that path; no Poynting or Bloch there)
 template <typename R, int DX, bool BLOCH>
-static void bulk_h(const YeeK<R> &k, bool mu, bool poynting, cudaStream_t st)
+static void (*bulk_h_kernel(bool mu, bool poynting, bool away))(YeeK<R>)
 {
-    const dim3 g = bulk_grid(k.syz, k.xend - k.xbeg, k.xchunk);
-    if (mu) {
-        if (poynting) k_bulk_h<R, DX, true, true, BLOCH><<<g, BLOCK, 0, st>>>(k);
-        else k_bulk_h<R, DX, true, false, BLOCH><<<g, BLOCK, 0, st>>>(k);
-    } else {
-        if (poynting) k_bulk_h<R, DX, false, true, BLOCH><<<g, BLOCK, 0, st>>>(k);
-        else k_bulk_h<R, DX, false, false, BLOCH><<<g, BLOCK, 0, st>>>(k);
-    }
+    if (away) return mu ? k_bulk_h<R, DX, true, false, false, true> : k_bulk_h<R, DX, false, false, false, true>;
+    if (mu) return poynting ? k_bulk_h<R, DX, true, true, BLOCH, false> : k_bulk_h<R, DX, true, false, BLOCH, false>;
+    return poynting ? k_bulk_h<R, DX, false, true, BLOCH, false> : k_bulk_h<R, DX, false, false, BLOCH, false>;
 }
 
-template <typename R, int DX>
-static void bulk_h_dispatch(const YeeK<R> &k, bool mu, bool poynting, cudaStream_t st)
+template <typename R, bool BLOCH>
+static void (*bulk_h_kernel(int dxmode, bool mu, bool poynting, bool away))(YeeK<R>)
 {
-    if (k.bloch_mask) bulk_h<R, DX, true>(k, mu, poynting, st);
-    else bulk_h<R, DX, false>(k, mu, poynting, st);
+    return dxmode == 0 ? bulk_h_kernel<R, 0, BLOCH>(mu, poynting, away) : dxmode == 1 ? bulk_h_kernel<R, 1, BLOCH>(mu, poynting, away)
+                                                                                 : bulk_h_kernel<R, 2, BLOCH>(mu, poynting, away);
 }
 
 template <typename R>
-cudaError_t launch_yee_h(const YeeK<R> &k, bool mu, bool poynting, cudaStream_t st)
+cudaError_t launch_yee_h(const YeeK<R> &kk, bool mu, bool poynting, cudaStream_t st, bool pdl)
 {
+    YeeK<R> k = kk;
     if (k.xend <= k.xbeg) return cudaSuccess;
     if (!k.bulk) {
         const dim3 g = plane_grid(k.syz, k.xend - k.xbeg);
@@ -721,17 +770,19 @@ cudaError_t launch_yee_h(const YeeK<R> &k, bool mu, bool poynting, cudaStream_t 
         }
         return cudaGetLastError();
     }
-    if (k.dxmode == 0) bulk_h_dispatch<R, 0>(k, mu, poynting, st);
-    else if (k.dxmode == 1) bulk_h_dispatch<R, 1>(k, mu, poynting, st);
-    else bulk_h_dispatch<R, 2>(k, mu, poynting, st);
-    return cudaGetLastError();
+    const bool away = k.W != k.P;
+    const dim3 g = bulk_grid(k, BLOCK, (uint32_t)h_min_blocks(mu, k.bloch_mask != 0));
+    return launch_dependent(k.bloch_mask ? bulk_h_kernel<R, true>(k.dxmode, mu, poynting, away) : bulk_h_kernel<R, false>(k.dxmode, mu, poynting, away),
+                            g, BLOCK, st, pdl, k);
 }
 
 template <typename R>
-cudaError_t launch_poynting(const SK<R> &k, cudaStream_t st)
+cudaError_t launch_poynting(const SK<R> &kk, cudaStream_t st)
 {
+    SK<R> k = kk;
     if (k.xend <= k.xbeg) return cudaSuccess;
-    k_bulk_s<R><<<bulk_grid(k.syz, k.xend - k.xbeg, k.xchunk), BLOCK, 0, st>>>(k);
+    const dim3 g = bulk_grid(k, BLOCK, 5u);
+    k_bulk_s<R><<<g, BLOCK, 0, st>>>(k);
     return cudaGetLastError();
 }
 
@@ -764,7 +815,7 @@ cudaError_t launch_point_sources(const PointK<R> &k, cudaStream_t st)
 
 #define FDTD_INSTANTIATE(R)                                                              \
     template cudaError_t launch_yee_e<R>(const YeeK<R> &, cudaStream_t, bool);         \
-    template cudaError_t launch_yee_h<R>(const YeeK<R> &, bool, bool, cudaStream_t);   \
+    template cudaError_t launch_yee_h<R>(const YeeK<R> &, bool, bool, cudaStream_t, bool); \
     template cudaError_t launch_poynting<R>(const SK<R> &, cudaStream_t);              \
     template cudaError_t launch_prepare<R>(const PrepK<R> &, cudaStream_t);            \
     template cudaError_t launch_fieldsrc<R>(const JK<R> &, cudaStream_t);              \

@@ -203,6 +203,7 @@ class Simulation:
         self._buf_key = None
         self._buf = _lib.FdtdBuffers()
         self._scratch = None
+        self._ahead = False
         self.steps_run = 0
 
         self.update_E = self._create_operation(self._lib.fdtd_update_e)
@@ -410,7 +411,7 @@ class Simulation:
         b.H2 = H2.data_ptr()
         for f, (u, v) in enumerate(ph2):
             b.psi_h2[f][0], b.psi_h2[f][1] = u.data_ptr(), v.data_ptr()
-        if mode == "fused":
+        if mode in ("fused", "ahead"):
             b.E2 = E2.data_ptr()
             for f, (u, v) in enumerate(pe2):
                 b.psi_e2[f][0], b.psi_e2[f][1] = u.data_ptr(), v.data_ptr()
@@ -422,7 +423,7 @@ class Simulation:
         if H2 is None:
             H2 = torch.empty_like(self.H)
             ph2 = [(torch.empty_like(u), torch.empty_like(v)) for u, v in self.psi["H"]]
-        if mode == "fused" and E2 is None:
+        if mode in ("fused", "ahead") and E2 is None:
             E2 = torch.empty_like(self.E)
             pe2 = [(torch.empty_like(u), torch.empty_like(v)) for u, v in self.psi["E"]]
         self._scratch = (E2, H2, pe2, ph2)
@@ -476,14 +477,18 @@ class Simulation:
         values are rounded to the field dtype, as the host-side ``+=`` does.
 
         ``path`` picks the kernels, all giving identical fields and S:
-          'auto'   'hs' where it applies (Poynting on, no Bloch boundaries), else 'plain';
+          'auto'   the fastest of the next three for the simulation and the step count;
+          'ahead'  H and S of a step and E of the next in one launch, reading E, H and their CPML
+                   arrays from one copy and writing a second: 72 B per cell per step with
+                   Poynting on, 60 without (float32, no Bloch boundaries, no learned boundary;
+                   else, and where the device has no room for the copies, as 'hs' or 'plain');
           'hs'     update_E in place, then H and S in one launch reading H (and the H-side
                    CPML arrays) from one copy and writing a second: 96 B per cell per step;
           'plain'  the per-update kernels (E, H, S), optionally over L2-resident x slabs
                    (tune(slab=...));
           'fused'  E, sources, H and S in one kernel per step (no Bloch boundaries), reading
                    every field once and writing it once: 72 B per cell per step.
-        The 'hs' and 'fused' paths write oS on the last step only."""
+        The 'ahead', 'hs' and 'fused' paths write oS on the last step only."""
         nsteps = int(nsteps)
         if watchdog and int(watchdog) > 0:
             return self._run_watched(nsteps, int(watchdog), point_sources, wait_for, monitor, path)
@@ -511,20 +516,23 @@ class Simulation:
             idx_host = (ctypes.c_int64 * n)(*idx.tolist())
             keep = [val_t]
             src = _lib.FdtdPointSources(n, 0, ctypes.addressof(idx_host), val_t.data_ptr())
-        if path not in ("auto", "hs", "plain", "fused"):
-            raise ValueError("path must be 'auto', 'hs', 'plain' or 'fused'")
-        hs_ok = self.do_poynting and not self.bloch_boundaries
+        if path not in ("auto", "ahead", "hs", "plain", "fused"):
+            raise ValueError("path must be 'auto', 'ahead', 'hs', 'plain' or 'fused'")
         if path == "auto":
-            path = "hs" if hs_ok else "plain"
-        if path in ("hs", "fused") and self.bloch_boundaries:
+            path = self._auto_path(nsteps)
+        if path in ("ahead", "hs", "fused") and self.bloch_boundaries:
             raise ValueError("the '%s' path does not support Bloch boundaries" % path)
         if path == "hs" and not self.do_poynting:
             raise ValueError("the 'hs' path needs do_poynting=True")
         mode = None if path == "plain" else path
+        if mode == "ahead" and (self._np_dtype == numpy.float64 or getattr(self, "_lbc_keep", None) is not None
+                                or not self._try_scratch("ahead")):
+            mode = "hs" if self.do_poynting else None
         if mode:
             self._ensure_scratch(mode)
         bufs = self._buffers()
         self._attach_scratch(mode)
+        self._set_ahead(mode == "ahead")
         mon = monitor.struct(nsteps) if monitor is not None else None
         _lib.check(self._lib.fdtd_run(self._plan, ctypes.byref(bufs),
                                       ctypes.c_void_p(stream.cuda_stream), nsteps,
@@ -536,6 +544,37 @@ class Simulation:
             t.record_stream(stream)
         self.steps_run += nsteps
         return Event(stream)
+
+    def _set_ahead(self, on: bool):
+        if self._ahead != on:
+            _lib.check(self._lib.fdtd_plan_tune(self._plan, _lib.FDTD_TUNE_HS_AHEAD, int(on)))
+            self._ahead = on
+
+    def _auto_path(self, nsteps: int) -> str:
+        """The kernels run(path='auto') takes: 'ahead' where it applies and there is a next step, else
+        'hs' or 'plain'. Double precision is bound by its arithmetic units, where the per-update
+        kernels, which evaluate no cell twice, are the faster ones (0.44 ms a step of 197x173x73
+        cells against 0.57). Without Poynting 'ahead' saves only passes over memory (84 to 60 B per
+        cell), so it is taken where the fields exceed the L2: 0.142 against 0.165 ms a step of 200^3
+        cells, but 0.0326 against 0.0289 of 151x129x61."""
+        hs = "hs" if self.do_poynting else "plain"
+        if self.bloch_boundaries or self._np_dtype == numpy.float64:
+            return "plain"
+        if nsteps < 2 or getattr(self, "_lbc_keep", None) is not None:
+            return hs
+        if not self.do_poynting:
+            l2 = torch.cuda.get_device_properties(self.device).L2_cache_size
+            if 60 * self.N <= l2 or self.tuning("slab"):
+                return "plain"
+        return "ahead"
+
+    def _try_scratch(self, mode) -> bool:
+        """The second copies of a run path, or False when the device has no room for them."""
+        try:
+            self._ensure_scratch(mode)
+        except torch.cuda.OutOfMemoryError:
+            return False
+        return True
 
     def _run_watched(self, nsteps, every, point_sources, wait_for, monitor, path):
         if nsteps <= 0:
