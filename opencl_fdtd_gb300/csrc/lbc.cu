@@ -11,9 +11,9 @@
 // side-1 faces for the H update), which is what a wave leaving the grid needs from the CPML
 // layers that the learned layer replaces.
 //
-// Training runs in float32 with one thread per sample for the per-sample passes (weights in
-// shared memory, broadcast reads) and a split reduction over samples for the weight gradients
-// (deterministic: fixed partition, fixed folding order). Inference uses bfloat16 weights on
+// Training runs in float32 on the CUDA cores: blocks of 32 samples for the per-sample passes and a
+// split reduction over samples for the weight gradients (deterministic: fixed partition, fixed
+// folding order). Inference uses bfloat16 weights on
 // the tensor cores (mma.sync, float32 accumulation) or float32 weights on the CUDA cores.
 #include <cuda_bf16.h>
 
@@ -22,10 +22,6 @@
 namespace fdtd {
 
 namespace {
-
-constexpr int T_FWD = 128;
-constexpr int WG_ROWS = 32;      // rows staged per pass of the weight-gradient kernel
-constexpr int WG_THREADS = 256;
 
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 
@@ -105,159 +101,307 @@ __global__ void k_lbc_gather(const LGrid g, const float *E, const float *H, floa
     }
 }
 
-// ---- training: forward (float32), one thread per sample ---------------------------------------
-// Dynamic shared memory of the float32 MLP kernels: the parameters, then one column of 64
-// hidden activations per thread, stored k-major (hs[k * T + t]) so that the runtime loops over
-// k read them without bank conflicts and every register array keeps compile-time indices (a
-// hidden vector indexed by the runtime k would live in local memory).
-constexpr size_t MLP32_SMEM = ((size_t)LBC_NPARAM + (size_t)LBC_HID * 128) * sizeof(float);
-static_assert(T_FWD == 128, "MLP32_SMEM holds 128 hidden columns");
+// ---- training kernels (float32) -----------------------------------------------------------------
+// A batch of 4096 samples is 0.23 GFLOP and 9 MB: a few microseconds of the chip's float32 units, so
+// what costs time is how much of the chip works and how long the serial chain of a block is. One
+// thread per sample (32 blocks of 128 threads, 2.4% of the chip's threads) took 61 us forward and 46
+// us backward, and the weight gradients (16 blocks) 265 us. Now a block has 32 samples and 128
+// threads, each 4 samples x 4 units (16 independent sums; every value read from shared memory is
+// used four times), and the weight gradients are split by input row as well as by sample. The order of
+// every sum is the one of the per-sample form, so outputs and gradients are the same bits.
+constexpr int TR_ROWS = 32;      // samples of a block
+constexpr int TR_T = 128;        // threads: 8 row groups (4 samples each) x 16 unit lanes (4 units each)
+constexpr int TR_LD = LBC_HID + 4;   // row pitch of hidden values: the two row groups of a warp differ
+                                     // by 16 banks (as do input rows, 4 * 108 words apart)
+constexpr size_t FWD_SMEM = (size_t)(LBC_NPARAM + 2 + TR_ROWS * (LBC_IN + TR_LD)) * sizeof(float);
+static_assert((LBC_NPARAM + 2) % 4 == 0 && LBC_IN % 4 == 0 && TR_LD % 4 == 0, "16-byte rows in shared memory");
 
-__global__ void __launch_bounds__(T_FWD) k_mlp_fwd(const float *P, const float *X, int B, float *Y, float *A1,
-                                                    float *A2, float *H1, float *H2)
+// asynchronous 4-byte copy to shared memory (any float pointer is aligned for it); 0 when !in
+__device__ __forceinline__ void copy4(float *dst, const float *src, bool in)
 {
-    extern __shared__ float mlp_smem[];
-    float *const w = mlp_smem;
-    float *const hs = mlp_smem + LBC_NPARAM + threadIdx.x;   // hs[k * T_FWD]: this thread's column
-    for (int i = threadIdx.x; i < LBC_NPARAM; i += blockDim.x) w[i] = P[i];
-    __syncthreads();
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= B) return;
-    float a[LBC_HID];
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    const int n = in ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// acc[4 samples][4 units] += in[sample][k] w[k][unit], k ascending; the thread's units are u, u + 16, ...
+template <int K, int PITCH>
+__device__ __forceinline__ void dense(float (&acc)[4][4], const float *in, const float *w, int u)
+{
+#pragma unroll 3
+    for (int k = 0; k < K; k += 4) {
+        float x[4][4];
 #pragma unroll
-    for (int j = 0; j < LBC_HID; ++j) a[j] = w[LBC_B1 + j];
-    for (int k = 0; k < LBC_IN; ++k) {
-        const float xk = X[(uint64_t)r * LBC_IN + k];
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<float4 *>(x[i]) = *reinterpret_cast<const float4 *>(in + i * PITCH + k);
 #pragma unroll
-        for (int j = 0; j < LBC_HID; ++j) a[j] += xk * w[LBC_W1 + k * LBC_HID + j];
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float wj = w[(k + q) * LBC_HID + u + 16 * j];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i][j] += x[i][q] * wj;
+            }
     }
-#pragma unroll
-    for (int j = 0; j < LBC_HID; ++j) {
-        A1[(uint64_t)r * LBC_HID + j] = a[j];
-        const float hj = gelu(a[j]);
-        hs[j * T_FWD] = hj;
-        H1[(uint64_t)r * LBC_HID + j] = hj;
-    }
-#pragma unroll
-    for (int j = 0; j < LBC_HID; ++j) a[j] = w[LBC_B2 + j];
-    for (int k = 0; k < LBC_HID; ++k) {
-        const float hk = hs[k * T_FWD];
-#pragma unroll
-        for (int j = 0; j < LBC_HID; ++j) a[j] += hk * w[LBC_W2 + k * LBC_HID + j];
-    }
-#pragma unroll
-    for (int j = 0; j < LBC_HID; ++j) {
-        A2[(uint64_t)r * LBC_HID + j] = a[j];
-        const float hj = gelu(a[j]);
-        hs[j * T_FWD] = hj;
-        H2[(uint64_t)r * LBC_HID + j] = hj;
-    }
-    float y[LBC_OUT];
-#pragma unroll
-    for (int o = 0; o < LBC_OUT; ++o) y[o] = w[LBC_B3 + o];
-    for (int k = 0; k < LBC_HID; ++k) {
-        const float hk = hs[k * T_FWD];
-#pragma unroll
-        for (int o = 0; o < LBC_OUT; ++o) y[o] += hk * w[LBC_W3 + k * LBC_OUT + o];
-    }
-#pragma unroll
-    for (int o = 0; o < LBC_OUT; ++o) Y[(uint64_t)r * LBC_OUT + o] = y[o];
 }
 
-// ---- training: backward through the activations, one thread per sample ------------------------
+__global__ void __launch_bounds__(TR_T) k_mlp_fwd(const float *P, const float *X, int B, float *Y, float *A1,
+                                                  float *A2, float *H1, float *H2)
+{
+    extern __shared__ __align__(16) float mlp_smem[];
+    float *const w = mlp_smem;
+    float *const xs = w + LBC_NPARAM + 2;                    // [TR_ROWS][LBC_IN]
+    float *const hs = xs + TR_ROWS * LBC_IN;                 // [TR_ROWS][TR_LD]
+    const int t = threadIdx.x, u = t & 15, s0 = (t >> 4) * 4;
+    const int r0 = blockIdx.x * TR_ROWS, nr = min(TR_ROWS, B - r0);
+    // the first layer's operands first: the other layers' weights arrive behind its arithmetic
+    for (int i = t; i < TR_ROWS * LBC_IN; i += TR_T) {
+        const bool in = i < nr * LBC_IN;
+        copy4(xs + i, X + (uint64_t)r0 * LBC_IN + (in ? i : 0), in);
+    }
+    for (int i = t; i < LBC_W2; i += TR_T) copy4(w + i, P + i, true);
+    copy_commit();
+    for (int i = LBC_W2 + t; i < LBC_NPARAM; i += TR_T) copy4(w + i, P + i, true);
+    copy_commit();
+    copy_wait<1>();
+    __syncthreads();
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = w[LBC_B1 + u + 16 * j];
+    dense<LBC_IN, LBC_IN>(acc, xs + s0 * LBC_IN, w + LBC_W1, u);
+    // a layer's outputs: to the arrays and, activated, to shared memory for the next layer
+    const auto put = [&](float *A, float *Hh) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float hj = gelu(acc[i][j]);
+                hs[(s0 + i) * TR_LD + u + 16 * j] = hj;
+                if (s0 + i < nr) {
+                    const uint64_t o = (uint64_t)(r0 + s0 + i) * LBC_HID + u + 16 * j;
+                    A[o] = acc[i][j];
+                    Hh[o] = hj;
+                }
+            }
+    };
+    put(A1, H1);
+    copy_wait<0>();
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = w[LBC_B2 + u + 16 * j];
+    dense<LBC_HID, TR_LD>(acc, hs + s0 * TR_LD, w + LBC_W2, u);
+    __syncthreads();                                         // every thread has read the first layer's values
+    put(A2, H2);
+    __syncthreads();
+    for (int e = t; e < TR_ROWS * LBC_OUT; e += TR_T) {
+        const int r = e / LBC_OUT, o = e - r * LBC_OUT;
+        if (r >= nr) break;
+        float y = w[LBC_B3 + o];
+#pragma unroll 8
+        for (int k = 0; k < LBC_HID; ++k) y += hs[r * TR_LD + k] * w[LBC_W3 + k * LBC_OUT + o];
+        Y[(uint64_t)r0 * LBC_OUT + e] = y;
+    }
+}
+
+// ---- training: backward through the activations -------------------------------------------------
 // loss = scale * sum over the batch and the outputs of w_o (Y - T)^2 (scale = 1 / (B * 6) for the
 // mean, w_o = 1 without wout): DY, and the pre-activation gradients D2 (layer 2) and D1 (layer 1)
-__global__ void __launch_bounds__(T_FWD) k_mlp_bwd_rows(const float *P, const float *Y, const float *T,
-                                                         const float *wout, int B, float scale, const float *A1,
-                                                         const float *A2, float *DY, float *D2, float *D1)
+__global__ void __launch_bounds__(TR_T) k_mlp_bwd_rows(const float *P, const float *Y, const float *T,
+                                                       const float *wout, int B, float scale, const float *A1,
+                                                       const float *A2, float *DY, float *D2, float *D1)
 {
-    __shared__ float w[LBC_NPARAM];
-    for (int i = threadIdx.x; i < LBC_NPARAM; i += blockDim.x) w[i] = P[i];
+    __shared__ __align__(16) float w2[LBC_HID * TR_LD];      // pitch: 16 lanes' rows in different banks
+    __shared__ float w3[LBC_HID * LBC_OUT];
+    __shared__ float dy[TR_ROWS * LBC_OUT];
+    __shared__ __align__(16) float d2[TR_ROWS * TR_LD];
+    const int t = threadIdx.x, u = t & 15, s0 = (t >> 4) * 4;
+    const int r0 = blockIdx.x * TR_ROWS, nr = min(TR_ROWS, B - r0);
+    for (int i = t; i < LBC_HID * LBC_OUT; i += TR_T) copy4(w3 + i, P + LBC_W3 + i, true);
+    copy_commit();
+    for (int i = t; i < LBC_HID * LBC_HID; i += TR_T)
+        copy4(w2 + (i / LBC_HID) * TR_LD + i % LBC_HID, P + LBC_W2 + i, true);
+    copy_commit();
+    for (int e = t; e < TR_ROWS * LBC_OUT; e += TR_T) {
+        const int o = e % LBC_OUT;
+        float v = 0.f;
+        if (e < nr * LBC_OUT) {
+            const uint64_t g = (uint64_t)r0 * LBC_OUT + e;
+            const float wo = wout ? wout[o] : 1.0f;
+            v = 2.0f * scale * wo * (Y[g] - T[g]);
+            DY[g] = v;
+        }
+        dy[e] = v;
+    }
+    copy_wait<1>();
     __syncthreads();
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= B) return;
-    float dy[LBC_OUT];
 #pragma unroll
-    for (int o = 0; o < LBC_OUT; ++o) {
-        const float wo = wout ? wout[o] : 1.0f;
-        dy[o] = 2.0f * scale * wo * (Y[(uint64_t)r * LBC_OUT + o] - T[(uint64_t)r * LBC_OUT + o]);
-        DY[(uint64_t)r * LBC_OUT + o] = dy[o];
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = s0 + i, c = u + 16 * j;
+            float v = 0.f;
+            if (r < nr) {
+                float s = 0.f;
+#pragma unroll
+                for (int o = 0; o < LBC_OUT; ++o) s += dy[r * LBC_OUT + o] * w3[c * LBC_OUT + o];
+                const uint64_t g = (uint64_t)(r0 + r) * LBC_HID + c;
+                v = s * gelu_d(A2[g]);
+                D2[g] = v;
+            }
+            d2[r * TR_LD + c] = v;
+        }
+    copy_wait<0>();
+    __syncthreads();
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < LBC_HID; k += 4) {
+        float4 x[4], v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4 *>(d2 + (s0 + i) * TR_LD + k);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = *reinterpret_cast<const float4 *>(w2 + (u + 16 * j) * TR_LD + k);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[i][j] += x[i].x * v[j].x;
+                acc[i][j] += x[i].y * v[j].y;
+                acc[i][j] += x[i].z * v[j].z;
+                acc[i][j] += x[i].w * v[j].w;
+            }
     }
-    float d2[LBC_HID];
 #pragma unroll
-    for (int j = 0; j < LBC_HID; ++j) {
-        float s = 0.f;
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int o = 0; o < LBC_OUT; ++o) s += dy[o] * w[LBC_W3 + j * LBC_OUT + o];
-        d2[j] = s * gelu_d(A2[(uint64_t)r * LBC_HID + j]);
-        D2[(uint64_t)r * LBC_HID + j] = d2[j];
-    }
-    for (int i = 0; i < LBC_HID; ++i) {
-        float s = 0.f;
-#pragma unroll
-        for (int j = 0; j < LBC_HID; ++j) s += d2[j] * w[LBC_W2 + i * LBC_HID + j];
-        D1[(uint64_t)r * LBC_HID + i] = s * gelu_d(A1[(uint64_t)r * LBC_HID + i]);
-    }
+        for (int j = 0; j < 4; ++j)
+            if (s0 + i < nr) {
+                const uint64_t g = (uint64_t)(r0 + s0 + i) * LBC_HID + u + 16 * j;
+                D1[g] = acc[i][j] * gelu_d(A1[g]);
+            }
 }
 
 // ---- training: weight gradients dW[k][n] = sum_r In[r][k] D[r][n], bias row k = K ------------
-// Block b sums rows b*rpb .. (b+1)*rpb - 1 into partial[b][(K + 1) * N]; the fold kernel then
-// adds the partials in block order (same partition, same order: deterministic).
-__global__ void __launch_bounds__(WG_THREADS) k_mlp_wgrad(const float *In, const float *D, int B, int K, int N,
-                                                          int rpb, float *partial)
+// A block sums WG_RPB rows (blockIdx.y) of a tile of WG_KT input rows x NT columns into
+// partial[blockIdx.y][(K + 1) * N]; the fold kernel then adds the partials in block order (same
+// partition, same order: deterministic). All rows of the tile are requested at once and summed as
+// the groups arrive. The layers of the network are tiles of one launch (17 tiles x 16 row blocks for
+// 4096 samples), two blocks an SM by shared memory.
+constexpr int WG_RPB = 256;      // rows of a block: one float32 chain
+constexpr int WG_KT = 16;
+constexpr int WG_T = 128;
+constexpr int WG_GROUPS = 4;     // groups of rows waited for one after another
+constexpr size_t WG_SMEM = (size_t)WG_RPB * (WG_KT + 64) * sizeof(float);
+
+struct WLayer {
+    const float *in, *d;         // [rows][K], [rows][N]
+    int K, N;
+    int tile0;                   // first tile (blockIdx.x); tiles run over n within k
+    uint32_t part;               // offset of (k, n) = (0, 0) within a block's partials
+};
+struct WLayers {
+    WLayer l[3];
+    int n;
+    uint32_t stride;             // partials of a row block
+};
+
+// TN columns per thread, NT / TN lanes of columns, TK input rows per thread
+template <int NT, int TN>
+__device__ __forceinline__ void outer_tile(const WLayer &l, int tile, uint32_t stride, int rows, float *sh, float *partial)
 {
-    extern __shared__ float sh[];
-    float *si = sh;                       // [WG_ROWS][K]
-    float *sd = sh + WG_ROWS * K;         // [WG_ROWS][N]
-    const int KN = (K + 1) * N;
-    const int r0 = blockIdx.x * rpb, r1 = min(B, r0 + rpb);
-    float acc[28];
-#pragma unroll
-    for (int q = 0; q < 28; ++q) acc[q] = 0.f;
-    for (int rb = r0; rb < r1; rb += WG_ROWS) {
-        const int nr = min(WG_ROWS, r1 - rb);
-        __syncthreads();
-        for (int i = threadIdx.x; i < WG_ROWS * K; i += WG_THREADS) {
-            const int rr = i / K;
-            si[i] = rr < nr ? In[(uint64_t)(rb + rr) * K + (i - rr * K)] : 0.f;
-        }
-        for (int i = threadIdx.x; i < WG_ROWS * N; i += WG_THREADS) {
-            const int rr = i / N;
-            sd[i] = rr < nr ? D[(uint64_t)(rb + rr) * N + (i - rr * N)] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 28; ++q) {
-            const int e = threadIdx.x + q * WG_THREADS;
-            if (e >= KN) break;
-            const int k = e / N, n = e - k * N;
-            float s = acc[q];
-            if (k < K) {
-                for (int rr = 0; rr < WG_ROWS; ++rr) s += si[rr * K + k] * sd[rr * N + n];
-            } else {
-                for (int rr = 0; rr < WG_ROWS; ++rr) s += sd[rr * N + n];
+    constexpr int LANES = NT / TN, TK = WG_KT / (WG_T / LANES), GR = WG_RPB / WG_GROUPS;
+    static_assert(TK >= 1 && TN <= 4, "tile layout");
+    const int K = l.K, N = l.N, ntn = (N + NT - 1) / NT;
+    const int k0 = tile / ntn * WG_KT, n0 = tile % ntn * NT;
+    const int t = threadIdx.x;
+    const int r0 = blockIdx.y * WG_RPB, nr = min(WG_RPB, rows - r0);
+    float *const si = sh, *const sd = sh + WG_RPB * WG_KT;
+#pragma unroll 1
+    for (int g = 0; g < WG_GROUPS; ++g) {
+        for (int i = t; i < GR * WG_KT; i += WG_T) {
+            const int r = g * GR + i / WG_KT, k = k0 + i % WG_KT;
+            if (k == K) si[r * WG_KT + i % WG_KT] = r < nr ? 1.f : 0.f;      // the bias row
+            else {
+                const bool in = r < nr && k < K;
+                copy4(si + r * WG_KT + i % WG_KT, l.in + (in ? (uint64_t)(r0 + r) * K + k : 0), in);
             }
-            acc[q] = s;
         }
+        for (int i = t; i < GR * NT; i += WG_T) {
+            const int r = g * GR + i / NT, n = n0 + i % NT;
+            const bool in = r < nr && n < N;
+            copy4(sd + r * NT + i % NT, l.d + (in ? (uint64_t)(r0 + r) * N + n : 0), in);
+        }
+        copy_commit();
     }
+    const int nl = (t % LANES) * TN, kl = (t / LANES) * TK;
+    float acc[TK][TN];
 #pragma unroll
-    for (int q = 0; q < 28; ++q) {
-        const int e = threadIdx.x + q * WG_THREADS;
-        if (e < KN) partial[(uint64_t)blockIdx.x * KN + e] = acc[q];
-    }
+    for (int q = 0; q < TK; ++q)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[q][j] = 0.f;
+    const auto sum = [&](int g) {
+        __syncthreads();
+#pragma unroll 8
+        for (int r = g * GR; r < (g + 1) * GR; ++r) {
+            float d[TN], x[TK];
+            if (TN == 4) *reinterpret_cast<float4 *>(d) = *reinterpret_cast<const float4 *>(sd + r * NT + nl);
+            else
+#pragma unroll
+                for (int j = 0; j < TN; ++j) d[j] = sd[r * NT + nl + j];
+#pragma unroll
+            for (int q = 0; q < TK; ++q) x[q] = si[r * WG_KT + kl + q];
+#pragma unroll
+            for (int q = 0; q < TK; ++q)
+#pragma unroll
+                for (int j = 0; j < TN; ++j) acc[q][j] += x[q] * d[j];
+        }
+    };
+    static_assert(WG_GROUPS == 4, "one wait per group");
+    copy_wait<3>(); sum(0);
+    copy_wait<2>(); sum(1);
+    copy_wait<1>(); sum(2);
+    copy_wait<0>(); sum(3);
+#pragma unroll
+    for (int q = 0; q < TK; ++q)
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int k = k0 + kl + q, n = n0 + nl + j;
+            if (k <= K && n < N) partial[(uint64_t)blockIdx.y * stride + l.part + (uint32_t)k * N + n] = acc[q][j];
+        }
 }
 
-// grad[w_off + k*N + n] (k < K) and grad[b_off + n] (bias) from the partials, blocks in order
-__global__ void k_mlp_wgrad_fold(const float *partial, int G, int K, int N, float *grad, int w_off, int b_off)
+// narrow layers (N <= 8): one column a thread
+__device__ __host__ __forceinline__ int wg_nt(int N) { return N <= 8 ? 8 : 64; }
+
+__global__ void __launch_bounds__(WG_T) k_mlp_wgrad(const __grid_constant__ WLayers L, int rows, float *partial)
 {
-    const int KN = (K + 1) * N;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= KN) return;
+    extern __shared__ __align__(16) float wg_smem[];
+    int i = 0;
+    while (i + 1 < L.n && (int)blockIdx.x >= L.l[i + 1].tile0) ++i;
+    const WLayer &l = L.l[i];
+    const int tile = (int)blockIdx.x - l.tile0;
+    if (wg_nt(l.N) == 8) outer_tile<8, 1>(l, tile, L.stride, rows, wg_smem, partial);
+    else outer_tile<64, 4>(l, tile, L.stride, rows, wg_smem, partial);
+}
+
+// out[i] = the partials of entry i, row blocks in order
+__global__ void k_mlp_wgrad_fold(const float *partial, int G, uint32_t n, float *out)
+{
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
     float s = 0.f;
-    for (int b = 0; b < G; ++b) s += partial[(uint64_t)b * KN + e];
-    const int k = e / N, n = e - k * N;
-    if (k < K) grad[w_off + k * N + n] = s;
-    else grad[b_off + n] = s;
+#pragma unroll 16
+    for (int b = 0; b < G; ++b) s += partial[(uint64_t)b * n + e];
+    out[e] = s;
 }
 
 // ---- Adam (Kingma & Ba 2015) with bias correction ---------------------------------------------
@@ -281,6 +425,12 @@ __global__ void k_adam(float *P, const float *G, float *M, float *V, int n, floa
 // (k_lbc_fix). With memory = (1 - c dt) / (1 + c dt) the form contains Mur's first-order
 // absorbing condition written for the ghost (the rest of Mur's update is linear in the stencil).
 constexpr int T_APPLY = 128;
+
+// Dynamic shared memory of the float32 inference kernel: the parameters, then one column of 64
+// hidden activations per thread, stored k-major (hs[k * T + t]) so that the runtime loops over
+// k read them without bank conflicts and every register array keeps compile-time indices (a
+// hidden vector indexed by the runtime k would live in local memory).
+constexpr size_t MLP32_SMEM = ((size_t)LBC_NPARAM + (size_t)LBC_HID * 128) * sizeof(float);
 
 // float32 weights [6 faces][LBC_NPARAM] on the CUDA cores (the checker of the bfloat16 kernel)
 static_assert(T_APPLY == 128, "MLP32_SMEM holds 128 hidden columns");
@@ -887,7 +1037,7 @@ cudaError_t launch_lbc_gather(const LGrid &g, const float *E, const float *H, fl
 
 // The shared-memory opt-in above 48 KB is a per-device function attribute: set it once per device
 // and kernel slot (setting it twice from two threads is harmless).
-enum : int { SMEM_MLP_FWD = 0, SMEM_PREDICT32 = 1, SMEM_MMA = 2, SMEM_MMA_SPLIT = 3, SMEM_SLOTS = 4 };
+enum : int { SMEM_MLP_FWD = 0, SMEM_PREDICT32 = 1, SMEM_MMA = 2, SMEM_MMA_SPLIT = 3, SMEM_WGRAD = 4, SMEM_SLOTS = 5 };
 
 static cudaError_t smem_opt_in(const void *fn, int slot, size_t bytes)
 {
@@ -907,17 +1057,48 @@ cudaError_t launch_mlp_fwd(const float *P, const float *X, int B, float *Y, floa
                            float *H2, cudaStream_t st)
 {
     if (B <= 0) return cudaSuccess;
-    const cudaError_t e = smem_opt_in((const void *)k_mlp_fwd, SMEM_MLP_FWD, MLP32_SMEM);
+    const cudaError_t e = smem_opt_in((const void *)k_mlp_fwd, SMEM_MLP_FWD, FWD_SMEM);
     if (e != cudaSuccess) return e;
-    k_mlp_fwd<<<(B + T_FWD - 1) / T_FWD, T_FWD, MLP32_SMEM, st>>>(P, X, B, Y, A1, A2, H1, H2);
+    k_mlp_fwd<<<(B + TR_ROWS - 1) / TR_ROWS, TR_T, FWD_SMEM, st>>>(P, X, B, Y, A1, A2, H1, H2);
+    return cudaGetLastError();
+}
+
+// the tiles of the layers, one launch, then the fold into out (their (K + 1) * N entries in order)
+static cudaError_t launch_wgrad(WLayers L, int rows, float *ws, float *out, cudaStream_t st)
+{
+    cudaError_t e = smem_opt_in((const void *)k_mlp_wgrad, SMEM_WGRAD, WG_SMEM);
+    if (e != cudaSuccess) return e;
+    int tiles = 0;
+    uint32_t n = 0;
+    for (int i = 0; i < L.n; ++i) {
+        WLayer &l = L.l[i];
+        l.tile0 = tiles;
+        l.part = n;
+        tiles += (l.K + WG_KT) / WG_KT * ((l.N + wg_nt(l.N) - 1) / wg_nt(l.N));
+        n += (uint32_t)(l.K + 1) * l.N;
+    }
+    L.stride = n;
+    // row blocks beyond the y extent of a grid: further launches, partials side by side
+    const int G = (rows + WG_RPB - 1) / WG_RPB;
+    for (int g = 0; g < G; g += 65535) {
+        const int m = G - g < 65535 ? G - g : 65535, r0 = g * WG_RPB;
+        WLayers Lg = L;
+        for (int i = 0; i < L.n; ++i) {
+            Lg.l[i].in += (size_t)r0 * L.l[i].K;
+            Lg.l[i].d += (size_t)r0 * L.l[i].N;
+        }
+        k_mlp_wgrad<<<dim3(tiles, m), WG_T, WG_SMEM, st>>>(Lg, rows - r0, ws + (size_t)g * n);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    k_mlp_wgrad_fold<<<(n + 127) / 128, 128, 0, st>>>(ws, G, n, out);
     return cudaGetLastError();
 }
 
 // workspace floats needed by launch_mlp_bwd for a batch of B
 size_t mlp_bwd_workspace(int B)
 {
-    const int G = (B + 255) / 256;
-    return (size_t)B * (LBC_OUT + 2 * LBC_HID) + (size_t)G * (LBC_IN + 1) * LBC_HID;
+    const size_t G = ((size_t)B + WG_RPB - 1) / WG_RPB;
+    return (size_t)B * (LBC_OUT + 2 * LBC_HID) + G * LBC_NPARAM;
 }
 
 cudaError_t launch_mlp_bwd(const float *P, const float *X, const float *Y, const float *T, const float *wout,
@@ -927,39 +1108,29 @@ cudaError_t launch_mlp_bwd(const float *P, const float *X, const float *Y, const
     if (B <= 0) return cudaSuccess;
     float *DY = ws, *D2 = DY + (size_t)B * LBC_OUT, *D1 = D2 + (size_t)B * LBC_HID;
     float *part = D1 + (size_t)B * LBC_HID;
-    k_mlp_bwd_rows<<<(B + T_FWD - 1) / T_FWD, T_FWD, 0, st>>>(P, Y, T, wout, B, 1.0f / ((float)B * LBC_OUT),
-                                                              A1, A2, DY, D2, D1);
-    cudaError_t e = cudaGetLastError();
+    k_mlp_bwd_rows<<<(B + TR_ROWS - 1) / TR_ROWS, TR_T, 0, st>>>(P, Y, T, wout, B, 1.0f / ((float)B * LBC_OUT),
+                                                                 A1, A2, DY, D2, D1);
+    const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const int rpb = 256, G = (B + rpb - 1) / rpb;
-    struct L { const float *in; const float *d; int K, N, w, b; } layers[3] = {
-        {X, D1, LBC_IN, LBC_HID, LBC_W1, LBC_B1},
-        {H1, D2, LBC_HID, LBC_HID, LBC_W2, LBC_B2},
-        {H2, DY, LBC_HID, LBC_OUT, LBC_W3, LBC_B3}};
-    for (const L &l : layers) {
-        const size_t smem = (size_t)WG_ROWS * (l.K + l.N) * sizeof(float);
-        k_mlp_wgrad<<<G, WG_THREADS, smem, st>>>(l.in, l.d, B, l.K, l.N, rpb, part);
-        const int KN = (l.K + 1) * l.N;
-        k_mlp_wgrad_fold<<<(KN + 255) / 256, 256, 0, st>>>(part, G, l.K, l.N, grad, l.w, l.b);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    }
-    return cudaSuccess;
+    // the gradient's layout is the parameters': each layer's weights, then its bias row
+    static_assert(LBC_W1 == 0 && LBC_B1 == LBC_IN * LBC_HID && LBC_W2 == LBC_B1 + LBC_HID &&
+                      LBC_B2 == LBC_W2 + LBC_HID * LBC_HID && LBC_W3 == LBC_B2 + LBC_HID &&
+                      LBC_B3 == LBC_W3 + LBC_HID * LBC_OUT && LBC_NPARAM == LBC_B3 + LBC_OUT, "parameter layout");
+    const WLayers L = {{{X, D1, LBC_IN, LBC_HID, 0, 0}, {H1, D2, LBC_HID, LBC_HID, 0, 0}, {H2, DY, LBC_HID, LBC_OUT, 0, 0}},
+                       3, 0};
+    return launch_wgrad(L, B, part, grad, st);
 }
 
-// out[(K + 1) x N]: A^T B (rows k < K) and the column sums of B (row K), A [rows][K], B [rows][N]
-// (K, N with (K + 1) N <= 28 * WG_THREADS); ws: ceil(rows / 256) * (K + 1) * N floats
-size_t gram_workspace(int rows, int K, int N) { return (size_t)((rows + 255) / 256) * (K + 1) * N; }
+// out[(K + 1) x N]: A^T B (rows k < K) and the column sums of B (row K), A [rows][K], B [rows][N];
+// ws: ceil(rows / 256) * (K + 1) * N floats
+size_t gram_workspace(int rows, int K, int N) { return ((size_t)rows + WG_RPB - 1) / WG_RPB * (size_t)(K + 1) * N; }
 
 cudaError_t launch_gram(const float *A, int rows, int K, const float *B, int N, float *out, float *ws,
                         cudaStream_t st)
 {
     if (rows <= 0) return cudaSuccess;
-    const int rpb = 256, G = (rows + rpb - 1) / rpb;
-    const size_t smem = (size_t)WG_ROWS * (K + N) * sizeof(float);
-    k_mlp_wgrad<<<G, WG_THREADS, smem, st>>>(A, B, rows, K, N, rpb, ws);
-    const int KN = (K + 1) * N;
-    k_mlp_wgrad_fold<<<(KN + 255) / 256, 256, 0, st>>>(ws, G, K, N, out, 0, K * N);
-    return cudaGetLastError();
+    const WLayers L = {{{A, B, K, N, 0, 0}}, 1, 0};
+    return launch_wgrad(L, rows, ws, out, st);
 }
 
 cudaError_t launch_adam(float *P, const float *G, float *M, float *V, int n, float lr, float b1, float b2,
