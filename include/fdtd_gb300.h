@@ -413,6 +413,11 @@ int fdtd_mlp_backward_workspace(int32_t batch, int64_t *floats);
 int fdtd_mlp_backward(const float *params, const float *X, const float *Y, const float *T,
                       const float *out_weights, int32_t batch, const float *A1, const float *A2, const float *H1,
                       const float *H2, float *grad, float *workspace, int64_t workspace_floats, void *stream);
+/* The forward pass, that gradient and the loss (one device float) of a batch in one call; workspace
+ * floats from fdtd_mlp_gradient_workspace. The gradient has the bits of forward and backward. */
+int fdtd_mlp_gradient_workspace(int32_t batch, int64_t *floats);
+int fdtd_mlp_gradient(const float *params, const float *X, const float *T, const float *out_weights, int32_t batch,
+                      float *grad, float *loss, float *workspace, int64_t workspace_floats, void *stream);
 /* out [(K + 1) x N] float32: A^T B in rows 0..K-1 and the column sums of B in row K, for
  * A [rows][K], B [rows][N] (the least-squares normal equations of the linear start of
  * training); deterministic (fixed partition of the rows, fixed folding order). (K + 1) N <=

@@ -149,6 +149,8 @@ SIGNATURES = [
     ("fdtd_mlp_backward_workspace", c_i32, [c_i32, _P(c_i64)]),
     ("fdtd_mlp_backward", c_i32, [c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp,
                                   c_i64, c_vp]),
+    ("fdtd_mlp_gradient_workspace", c_i32, [c_i32, _P(c_i64)]),
+    ("fdtd_mlp_gradient", c_i32, [c_vp, c_vp, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_i64, c_vp]),
     ("fdtd_gram_workspace", c_i32, [c_i32, c_i32, c_i32, _P(c_i64)]),
     ("fdtd_gram", c_i32, [c_vp, c_i32, c_i32, c_vp, c_i32, c_vp, c_vp, c_i64, c_vp]),
     ("fdtd_adam", c_i32, [c_vp, c_vp, c_vp, c_vp, c_i32, ctypes.c_float, ctypes.c_float, ctypes.c_float,

@@ -72,6 +72,10 @@ size_t mlp_bwd_workspace(int B);
 cudaError_t launch_mlp_bwd(const float *P, const float *X, const float *Y, const float *T, const float *wout,
                            int B, const float *A1, const float *A2, const float *H1, const float *H2,
                            float *grad, float *ws, cudaStream_t st);
+// the forward pass, that gradient and the loss (one float) of a batch; nothing else is kept
+size_t mlp_grad_workspace(int B);
+cudaError_t launch_mlp_grad(const float *P, const float *X, const float *T, const float *wout, int B, float *grad,
+                            float *loss, float *ws, cudaStream_t st);
 size_t gram_workspace(int rows, int K, int N);
 cudaError_t launch_gram(const float *A, int rows, int K, const float *B, int N, float *out, float *ws,
                         cudaStream_t st);

@@ -130,6 +130,23 @@ int fdtd_mlp_backward(const float *params, const float *X, const float *Y, const
                       "mlp backward launch");
 }
 
+int fdtd_mlp_gradient_workspace(int32_t batch, int64_t *floats)
+{
+    if (batch < 0 || !floats) return bad("fdtd_mlp_gradient_workspace: bad argument");
+    *floats = (int64_t)mlp_grad_workspace(batch);
+    return FDTD_OK;
+}
+
+int fdtd_mlp_gradient(const float *params, const float *X, const float *T, const float *out_weights, int32_t batch,
+                      float *grad, float *loss, float *workspace, int64_t workspace_floats, void *stream)
+{
+    if (!params || !X || !T || !grad || !loss || !workspace) return bad("fdtd_mlp_gradient: NULL pointer");
+    if (batch < 1) return bad("fdtd_mlp_gradient: batch must be >= 1");
+    if (workspace_floats < (int64_t)mlp_grad_workspace(batch)) return bad("fdtd_mlp_gradient: workspace too small");
+    return check_cuda(launch_mlp_grad(params, X, T, out_weights, batch, grad, loss, workspace, (cudaStream_t)stream),
+                      "mlp gradient launch");
+}
+
 int fdtd_gram_workspace(int32_t rows, int32_t K, int32_t N, int64_t *floats)
 {
     if (rows < 0 || K < 1 || N < 1 || !floats) return bad("fdtd_gram_workspace: bad argument");

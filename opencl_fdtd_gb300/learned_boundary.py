@@ -204,6 +204,7 @@ class BoundaryNet:
         self.steps = [0] * 6
         self._packed = None
         self._bufs = {}
+        self._grad_bufs = {}
         self._wout = {}
         self.history = {}
         # the linear map of each face whose network is an exactly embedded linear map (None
@@ -215,14 +216,20 @@ class BoundaryNet:
     def _buffers(self, B):
         torch = _torch()
         if B not in self._bufs:
-            ws = ctypes.c_int64()
-            _lib.check(_lib.load().fdtd_mlp_backward_workspace(int(B), ctypes.byref(ws)))
             f32 = dict(dtype=torch.float32, device=self.device)
             self._bufs[B] = dict(Y=torch.empty((B, OUT), **f32), A1=torch.empty((B, HID), **f32),
                                  A2=torch.empty((B, HID), **f32), H1=torch.empty((B, HID), **f32),
-                                 H2=torch.empty((B, HID), **f32), ws=torch.empty(ws.value, **f32),
-                                 grad=torch.empty(NPARAM, **f32))
+                                 H2=torch.empty((B, HID), **f32))
         return self._bufs[B]
+
+    def _gradient_buffers(self, B):
+        torch = _torch()
+        if B not in self._grad_bufs:
+            ws = ctypes.c_int64()
+            _lib.check(_lib.load().fdtd_mlp_gradient_workspace(int(B), ctypes.byref(ws)))
+            f32 = dict(dtype=torch.float32, device=self.device)
+            self._grad_bufs[B] = torch.empty(ws.value, **f32), torch.empty(NPARAM, **f32)
+        return self._grad_bufs[B]
 
     def _stream(self):
         return ctypes.c_void_p(_torch().cuda.current_stream(self.device).cuda_stream)
@@ -255,16 +262,16 @@ class BoundaryNet:
         X = X.contiguous()
         T = T.contiguous()
         B = X.shape[0]
-        b = self._buffers(B)
-        Y = self.forward(face, X)
+        ws, grad = self._gradient_buffers(B)
         w = self.output_weights(face) if weighted else None
-        _lib.check(_lib.load().fdtd_mlp_backward(self.params[face].data_ptr(), X.data_ptr(), Y.data_ptr(),
-                                                 T.data_ptr(), w.data_ptr() if w is not None else None, B,
-                                                 b["A1"].data_ptr(), b["A2"].data_ptr(), b["H1"].data_ptr(),
-                                                 b["H2"].data_ptr(), b["grad"].data_ptr(), b["ws"].data_ptr(),
-                                                 b["ws"].numel(), self._stream()))
-        d = (Y - T) ** 2
-        return (d * w).mean() if w is not None else d.mean(), b["grad"]
+        loss = _torch().empty((), dtype=_torch().float32, device=self.device)
+        _lib.check(_lib.load().fdtd_mlp_gradient(self.params[face].data_ptr(), X.data_ptr(), T.data_ptr(),
+                                                 w.data_ptr() if w is not None else None, B, grad.data_ptr(),
+                                                 loss.data_ptr(), ws.data_ptr(), ws.numel(), self._stream()))
+        if T.requires_grad:                      # the loss as a function of the targets
+            d = (self.forward(face, X) - T) ** 2
+            loss = (d * w).mean() if w is not None else d.mean()
+        return loss, grad
 
     def adam_step(self, face: int, grad, lr: float, betas=(0.9, 0.999), eps: float = 1e-8):
         self.steps[face] += 1

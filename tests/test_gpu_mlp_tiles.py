@@ -2,6 +2,8 @@
 16 input rows x 64 or 8 columns a block of the weight gradients), against float64. Tolerances are
 forward error bounds: a float32 chain of n terms is off by at most n u times the sum of the terms'
 magnitudes (u = 2^-24), and a term carries the roundings of the chains that made it."""
+import ctypes
+
 import numpy
 import pytest
 
@@ -20,7 +22,7 @@ def _cuda(a):
 @pytest.mark.parametrize("B", SIZES)
 @pytest.mark.parametrize("weighted", [True, False])
 def test_gradient_at_tile_edges(B, weighted):
-    from opencl_fdtd_gb300 import learned_boundary as lb
+    from opencl_fdtd_gb300 import _lib, learned_boundary as lb
     rng = numpy.random.default_rng(B)
     net, face = lb.BoundaryNet(seed=B), 3
     flat = _cuda(rng.standard_normal(B * 108 + 1).astype(numpy.float32))
@@ -60,6 +62,16 @@ def test_gradient_at_tile_edges(B, weighted):
     assert abs(float(loss) - float((wo * (y - t) ** 2).mean())) <= (4 * n + 64) * U * float((wo * (my + t.abs()) ** 2).mean())
     again = net.gradient(face, X.clone(), T, weighted)[1].clone()
     assert torch.equal(net.gradient(face, X, T, weighted)[1], again)
+    # the same from the two separate calls
+    n = ctypes.c_int64()
+    _lib.check(_lib.load().fdtd_mlp_backward_workspace(B, ctypes.byref(n)))
+    ws, out = (torch.empty(k, dtype=torch.float32, device="cuda") for k in (n.value, lb.NPARAM))
+    b = net._buffers(B)
+    w = net.output_weights(face).data_ptr() if weighted else None
+    _lib.check(_lib.load().fdtd_mlp_backward(net.params[face].data_ptr(), X.data_ptr(), net.forward(face, X).data_ptr(),
+                                             T.data_ptr(), w, B, *(b[k].data_ptr() for k in ("A1", "A2", "H1", "H2")),
+                                             out.data_ptr(), ws.data_ptr(), ws.numel(), net._stream()))
+    assert torch.equal(out, again)
 
 
 @pytest.mark.parametrize("K,N", [(1, 1), (15, 8), (16, 9), (17, 64), (31, 65), (6, 130), (108, 6), (108, 64)])
