@@ -345,7 +345,8 @@ typedef struct FdtdBatchVariant {
 
 typedef struct FdtdBatch FdtdBatch;
 
-/* Validate n variants and build the tile list (x chunks of xchunk planes, default 8). rows:
+/* Validate n variants and build the tile list (x chunks of xchunk planes, default 8 or fewer
+ * where the batch is small). rows:
  * rows of every variant's src_values / series (steps past it add no source, record nothing). */
 int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, int64_t rows,
                       FdtdBatch **out);

@@ -2,11 +2,10 @@
 //
 // All variants' work is cut into tiles of BATCH_THREADS consecutive (y, z) cells times a chunk
 // of x planes. Two schedules run the same tile code:
-//   * persistent: a cooperative grid of two blocks per SM takes the tiles of every variant
+//   * persistent: a cooperative grid of resident blocks takes the tiles of every variant
 //     from a device work counter for the E half-step, synchronises the grid, does the same for
 //     the H half-step, synchronises again, and repeats -- one launch advances the whole sweep by
-//     nsteps steps (two blocks: the E and H tile bodies together need 128 registers without
-//     spilling; at three blocks per SM they spill and run slower);
+//     nsteps steps;
 //   * per half-step: one launch of one block per tile for E, one for H, per step (captured in
 //     a CUDA graph by the caller); the hardware scheduler then overlaps blocks.
 // Either way there is no per-variant launch or tail. Point sources are added and monitor
@@ -111,42 +110,38 @@ __device__ __forceinline__ void warp_exps(float a, float b, float c, int &ea, in
     ec = tile_exp(__uint_as_float(mc));
 }
 
-// CPML face of one axis fixed for the thread (y or z): depth, side, coefficients
+// CPML face of one axis fixed for the thread (y or z) of update H (0: E, 1: H): depth, coefficients,
+// thickness and psi. A store may alias the descriptor, so what is read through it is loaded again for
+// every plane: KEEP holds thickness and psi in registers instead.
+template <int H, bool KEEP>
 struct BFix {
+    const BAxis &a;
     int ir, side;
     float p0, p1, p2;
+    uint32_t T_;
+    float *u_, *v_;
+
+    __device__ __forceinline__ uint32_t T() const { return KEEP ? T_ : (uint32_t)(side ? a.Tp : a.Tn); }
+    __device__ __forceinline__ float *u() const { return KEEP ? u_ : a.psi[H][side][0]; }
+    __device__ __forceinline__ float *v() const { return KEEP ? v_ : a.psi[H][side][1]; }
 };
 
-__device__ __forceinline__ BFix bfix(const BAxis &a, int h, uint32_t s, uint32_t c, bool act)
+template <int h, bool KEEP>
+__device__ __forceinline__ BFix<h, KEEP> bfix(const BAxis &a, uint32_t s, uint32_t c, bool act)
 {
-    BFix f;
-    f.ir = -1;
-    f.side = 0;
-    f.p0 = f.p1 = f.p2 = 0.f;
-    if (!act) return f;
-    if (c < (uint32_t)a.Tn) {
-        f.ir = (int)c;
-    } else if (a.Tp && c >= s - (uint32_t)a.Tp) {
-        f.ir = (int)(s - 1u - c);
-        f.side = 1;
-    }
-    if (f.ir >= 0) {
-        f.p0 = ldg(a.tab[h][f.side][0] + f.ir);
-        f.p1 = ldg(a.tab[h][f.side][1] + f.ir);
-        f.p2 = ldg(a.tab[h][f.side][2] + f.ir);
+    BFix<h, KEEP> f = {a, -1, 0, 0.f, 0.f, 0.f, 0u, nullptr, nullptr};
+    const FaceAt at = face_at(a.Tn, a.Tp, s, c);
+    if (act && at.ir >= 0) {
+        f.ir = at.ir;
+        f.side = at.side;
+        f.T_ = (uint32_t)(at.side ? a.Tp : a.Tn);
+        f.p0 = ldg(a.tab[h][at.side][0] + at.ir);
+        f.p1 = ldg(a.tab[h][at.side][1] + at.ir);
+        f.p2 = ldg(a.tab[h][at.side][2] + at.ir);
+        f.u_ = a.psi[h][at.side][0];
+        f.v_ = a.psi[h][at.side][1];
     }
     return f;
-}
-
-__device__ __forceinline__ int bx_face(const BAxis &a, uint32_t sx, uint32_t x, int &side)
-{
-    side = 0;
-    if (x < (uint32_t)a.Tn) return (int)x;
-    if (a.Tp && x >= sx - (uint32_t)a.Tp) {
-        side = 1;
-        return (int)(sx - 1u - x);
-    }
-    return -1;
 }
 
 // decode of a stored value with its tile exponent (no scaling at all in float32 storage)
@@ -160,8 +155,7 @@ template <typename T>
 __device__ __forceinline__ T ldr(const T *p) { return __ldg(p); }
 
 // ---- E half-step of one tile (update_e.cl:39-107 per cell) ------------------------------------
-// Values one E plane reads (stored form and tile exponents), loaded one plane ahead as in the
-// per-update kernels.
+// Values one E plane reads (stored form and tile exponents).
 template <typename T>
 struct BELoad {
     T hx, hy, hz, nxy, nxz, nyz, nzy, ex, ey, ez, cx, cy, cz;
@@ -169,10 +163,7 @@ struct BELoad {
     float xu, xv, yu, yv, zu, zv;
 };
 
-// PF: the next plane's loads are issued before the current plane's arithmetic (latency hidden
-// by instruction-level parallelism, twice the registers for loaded values); without, latency
-// is hidden by more resident warps.
-template <int ST, bool PF = true>
+template <int ST, bool KEEP>
 __device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
 {
     using SS = Store<ST>;
@@ -184,30 +175,42 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
     const bool act = j < syz;
     const uint32_t y = act ? v.dsz.div(j) : 0u;
     const uint32_t z = act ? j - y * sz : 0u;
-    const T *Hx = (const T *)v.H, *Hy = Hx + N, *Hz = Hx + 2 * N;
-    T *Ex = (T *)v.E, *Ey = Ex + N, *Ez = Ex + 2 * N;
-    const T *C = (const T *)v.ce;
-    const int32_t *hexp = v.hexp;
-    int32_t *eexp = v.eexp;
+    const T *__restrict__ Hx = (const T *)v.H, *__restrict__ Hy = Hx + N, *__restrict__ Hz = Hx + 2 * N;
+    T *__restrict__ Ex = (T *)v.E, *__restrict__ Ey = Ex + N, *__restrict__ Ez = Ex + 2 * N;
+    const T *__restrict__ Cx = (const T *)v.ce, *__restrict__ Cy = Cx + N, *__restrict__ Cz = Cx + 2 * N;
+    const int32_t *__restrict__ hexp = v.hexp;
+    int32_t *__restrict__ eexp = v.eexp;
     // minus neighbours with periodic wrap (common.cl:75-81), 32-bit modular offsets
     const uint32_t dmy = y ? 0u - sz : (sy - 1u) * sz;
     const uint32_t dmz = z ? 0xffffffffu : sz - 1u;
     const uint32_t jt = j / BATCH_TILE;                          // own exponent tile
     const uint32_t jby = (j + dmy) / BATCH_TILE, jbz = (j + dmz) / BATCH_TILE;
-    const BFix fy = bfix(v.ax[1], 0, sy, y, act);
-    const BFix fz = bfix(v.ax[2], 0, sz, z, act);
+    const BFix<0, KEEP> fy = bfix<0, KEEP>(v.ax[1], sy, y, act);
+    const BFix<0, KEEP> fz = bfix<0, KEEP>(v.ax[2], sz, z, act);
+    // what the march needs of the descriptor in registers: a store may alias it, and a value read
+    // through it would be loaded again for every plane
     const float inv = v.inv_d;
-    const BAxis &ax0 = v.ax[0], &ax1 = v.ax[1], &ax2 = v.ax[2];
+    const bool scale = v.dxmode != 0;
+    const BAxis &ax0 = v.ax[0];
+    const int Tn = ax0.Tn, Tp = ax0.Tp;
+    const bool xf = xa < (uint32_t)Tn || (Tp && xb > sx - (uint32_t)Tp);   // an x face covers a plane of the tile
+    // a point source, a monitor point in this tile (block-uniform)
+    bool srcs = false, mons = false;
+    if (step < rows) {
+        for (int s = 0; s < v.nsrc; ++s)
+            srcs |= v.src_j[s] / BATCH_THREADS == jb && v.src_x[s] >= xa && v.src_x[s] < xb;
+        for (int m = 0; m < v.nmon; ++m)
+            mons |= v.mon_j[m] / BATCH_THREADS == jb && v.mon_x[m] >= xa && v.mon_x[m] < xb;
+    }
 
-    auto load = [&](uint32_t x) {
+    auto load = [&](uint32_t x, uint32_t i) {
         BELoad<T> q;
-        const uint32_t i = x * syz + j;
         const uint32_t imy = i + dmy, imz = i + dmz;   // 32-bit wrap arithmetic
         q.hx = ldr(Hx + i); q.hy = ldr(Hy + i); q.hz = ldr(Hz + i);
         q.nxy = ldr(Hx + imy); q.nzy = ldr(Hz + imy);
         q.nxz = ldr(Hx + imz); q.nyz = ldr(Hy + imz);
         q.ex = Ex[i]; q.ey = Ey[i]; q.ez = Ez[i];
-        q.cx = ldr(C + i); q.cy = ldr(C + N + i); q.cz = ldr(C + 2 * N + i);
+        q.cx = ldr(Cx + i); q.cy = ldr(Cy + i); q.cz = ldr(Cz + i);
         if (SS::scaled) {
             q.gh = hexp[texp_index(v, x, jt)];
             q.gy = hexp[texp_index(v, x, jby)];
@@ -215,85 +218,87 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
             q.ge = eexp[texp_index(v, x, jt)];
         }
         q.xu = q.xv = q.yu = q.yv = q.zu = q.zv = 0.f;
-        int side;
-        const int irx = bx_face(ax0, sx, x, side);
-        if (irx >= 0) {
-            const uint32_t ip = ((uint32_t)irx * sy + y) * sz + z;
-            q.xu = ax0.psi[0][side][0][ip]; q.xv = ax0.psi[0][side][1][ip];
+        if (xf) {
+            const FaceAt fx = face_at(Tn, Tp, sx, x);
+            if (fx.ir >= 0) {
+                const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                q.xu = ax0.psi[0][fx.side][0][ip]; q.xv = ax0.psi[0][fx.side][1][ip];
+            }
         }
         if (fy.ir >= 0) {
-            const uint32_t ip = (x * (uint32_t)(fy.side ? ax1.Tp : ax1.Tn) + (uint32_t)fy.ir) * sz + z;
-            q.yu = ax1.psi[0][fy.side][0][ip]; q.yv = ax1.psi[0][fy.side][1][ip];
+            const uint32_t ip = (x * fy.T() + (uint32_t)fy.ir) * sz + z;
+            q.yu = fy.u()[ip]; q.yv = fy.v()[ip];
         }
         if (fz.ir >= 0) {
-            const uint32_t ip = (x * sy + y) * (uint32_t)(fz.side ? ax2.Tp : ax2.Tn) + (uint32_t)fz.ir;
-            q.zu = ax2.psi[0][fz.side][0][ip]; q.zv = ax2.psi[0][fz.side][1][ip];
+            const uint32_t ip = (x * sy + y) * fz.T() + (uint32_t)fz.ir;
+            q.zu = fz.u()[ip]; q.zv = fz.v()[ip];
         }
         return q;
     };
 
     float hy_m = 0.f, hz_m = 0.f;
-    BELoad<T> cur;
     if (act) {
         const uint32_t xm = xa ? xa - 1u : sx - 1u;
         const uint32_t im = xm * syz + j;
         const int32_t wm = SS::scaled ? hexp[texp_index(v, xm, jt)] : 0;
         hy_m = dv<ST>(ldr(Hy + im), xe(wm, 1));
         hz_m = dv<ST>(ldr(Hz + im), xe(wm, 2));
-        if (PF) cur = load(xa);
     }
-    for (uint32_t x = xa; x < xb; ++x) {
-        const uint32_t i = x * syz + j;
-        BELoad<T> nxt;
+    uint32_t i = xa * syz + j;
+    for (uint32_t x = xa; x < xb; ++x, i += syz) {
         float nx = 0.f, ny = 0.f, nz = 0.f, hy = 0.f, hz = 0.f;
         if (act) {
-            if (!PF) cur = load(x);
-            else if (x + 1u < xb) nxt = load(x + 1u);
+            const BELoad<T> cur = load(x, i);
             const float hx = dv<ST>(cur.hx, xe(cur.gh, 0));
             hy = dv<ST>(cur.hy, xe(cur.gh, 1));
             hz = dv<ST>(cur.hz, xe(cur.gh, 2));
-            // backward differences (update_e.cl:39-46), times 1/dx (exact for dx = 1)
-            float d_xy = (hx - dv<ST>(cur.nxy, xe(cur.gy, 0))) * inv;
-            float d_xz = (hx - dv<ST>(cur.nxz, xe(cur.gz, 0))) * inv;
-            float d_yx = (hy - hy_m) * inv;
-            float d_yz = (hy - dv<ST>(cur.nyz, xe(cur.gz, 1))) * inv;
-            float d_zx = (hz - hz_m) * inv;
-            float d_zy = (hz - dv<ST>(cur.nzy, xe(cur.gy, 2))) * inv;
+            // backward differences (update_e.cl:39-46), times 1/dx
+            float d_xy = hx - dv<ST>(cur.nxy, xe(cur.gy, 0));
+            float d_xz = hx - dv<ST>(cur.nxz, xe(cur.gz, 0));
+            float d_yx = hy - hy_m;
+            float d_yz = hy - dv<ST>(cur.nyz, xe(cur.gz, 1));
+            float d_zx = hz - hz_m;
+            float d_zy = hz - dv<ST>(cur.nzy, xe(cur.gy, 2));
+            if (scale) {
+                d_xy = d_xy * inv; d_xz = d_xz * inv; d_yx = d_yx * inv;
+                d_yz = d_yz * inv; d_zx = d_zx * inv; d_zy = d_zy * inv;
+            }
             // CPML (update_e.cl:64-100): at most one face per axis
             float px = 0.f, py = 0.f, pz = 0.f;
-            int side;
-            const int irx = bx_face(ax0, sx, x, side);
-            if (irx >= 0) {
-                const uint32_t ip = ((uint32_t)irx * sy + y) * sz + z;
-                float su, sv;
-                face_update<float, true, 0>(ldg(ax0.tab[0][side][0] + irx), ldg(ax0.tab[0][side][1] + irx),
-                                            ldg(ax0.tab[0][side][2] + irx), cur.xu, cur.xv, su, sv,
-                                            d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-                ax0.psi[0][side][0][ip] = su;
-                ax0.psi[0][side][1][ip] = sv;
+            if (xf) {
+                const FaceAt fx = face_at(Tn, Tp, sx, x);
+                if (fx.ir >= 0) {
+                    float su, sv;
+                    face_update<float, true, 0>(ldg(ax0.tab[0][fx.side][0] + fx.ir), ldg(ax0.tab[0][fx.side][1] + fx.ir),
+                                              ldg(ax0.tab[0][fx.side][2] + fx.ir), cur.xu, cur.xv, su, sv,
+                                              d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                    const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                    ax0.psi[0][fx.side][0][ip] = su;
+                    ax0.psi[0][fx.side][1][ip] = sv;
+                }
             }
             if (fy.ir >= 0) {
-                const uint32_t ip = (x * (uint32_t)(fy.side ? ax1.Tp : ax1.Tn) + (uint32_t)fy.ir) * sz + z;
                 float su, sv;
                 face_update<float, true, 1>(fy.p0, fy.p1, fy.p2, cur.yu, cur.yv, su, sv,
-                                            d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-                ax1.psi[0][fy.side][0][ip] = su;
-                ax1.psi[0][fy.side][1][ip] = sv;
+                                          d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = (x * fy.T() + (uint32_t)fy.ir) * sz + z;
+                fy.u()[ip] = su;
+                fy.v()[ip] = sv;
             }
             if (fz.ir >= 0) {
-                const uint32_t ip = (x * sy + y) * (uint32_t)(fz.side ? ax2.Tp : ax2.Tn) + (uint32_t)fz.ir;
                 float su, sv;
                 face_update<float, true, 2>(fz.p0, fz.p1, fz.p2, cur.zu, cur.zv, su, sv,
-                                            d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-                ax2.psi[0][fz.side][0][ip] = su;
-                ax2.psi[0][fz.side][1][ip] = sv;
+                                          d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = (x * sy + y) * fz.T() + (uint32_t)fz.ir;
+                fz.u()[ip] = su;
+                fz.v()[ip] = sv;
             }
             // update_e.cl:105-107
             nx = dv<ST>(cur.ex, xe(cur.ge, 0)) + SS::dec(cur.cx) * ((d_zy - d_yz) + px);
             ny = dv<ST>(cur.ey, xe(cur.ge, 1)) + SS::dec(cur.cy) * ((d_xz - d_zx) + py);
             nz = dv<ST>(cur.ez, xe(cur.ge, 2)) + SS::dec(cur.cz) * ((d_yx - d_xy) + pz);
             // point sources after the update (fdtd.py:168-169: E[ind] += value)
-            if (v.nsrc > 0 && step < rows) {
+            if (srcs) {
                 for (int s = 0; s < v.nsrc; ++s) {
                     if (v.src_x[s] != x || v.src_j[s] != j) continue;
                     const float val = v.src_values[step * v.nsrc + s];
@@ -315,7 +320,7 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
             Ex[i] = wx;
             Ey[i] = wy;
             Ez[i] = wz;
-            if (v.nmon > 0 && step < rows) {
+            if (mons) {
                 for (int m = 0; m < v.nmon; ++m) {
                     if (v.mon_x[m] != x || v.mon_j[m] != j) continue;
                     const int c = v.mon_c[m];
@@ -325,7 +330,6 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
             }
             hy_m = hy;
             hz_m = hz;
-            if (PF) cur = nxt;
         }
     }
 }
@@ -338,7 +342,7 @@ struct BHLoad {
     float xu, xv, yu, yv, zu, zv;
 };
 
-template <int ST, bool PF = true>
+template <int ST, bool KEEP>
 __device__ void batch_h_tile(const BVar &v, int4 tl)
 {
     using SS = Store<ST>;
@@ -350,23 +354,25 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
     const bool act = j < syz;
     const uint32_t y = act ? v.dsz.div(j) : 0u;
     const uint32_t z = act ? j - y * sz : 0u;
-    const T *Ex = (const T *)v.E, *Ey = Ex + N, *Ez = Ex + 2 * N;
-    T *Hx = (T *)v.H, *Hy = Hx + N, *Hz = Hx + 2 * N;
-    int32_t *hexp = v.hexp;
-    const int32_t *eexp = v.eexp;
+    const T *__restrict__ Ex = (const T *)v.E, *__restrict__ Ey = Ex + N, *__restrict__ Ez = Ex + 2 * N;
+    T *__restrict__ Hx = (T *)v.H, *__restrict__ Hy = Hx + N, *__restrict__ Hz = Hx + 2 * N;
+    int32_t *__restrict__ hexp = v.hexp;
+    const int32_t *__restrict__ eexp = v.eexp;
     // plus neighbours with periodic wrap (common.cl:82-84)
     const uint32_t dpy = (y + 1u < sy) ? sz : 0u - (sy - 1u) * sz;
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
     const uint32_t jt = j / BATCH_TILE;
     const uint32_t jby = (j + dpy) / BATCH_TILE, jbz = (j + dpz) / BATCH_TILE;
-    const BFix fy = bfix(v.ax[1], 1, sy, y, act);
-    const BFix fz = bfix(v.ax[2], 1, sz, z, act);
+    const BFix<1, KEEP> fy = bfix<1, KEEP>(v.ax[1], sy, y, act);
+    const BFix<1, KEEP> fz = bfix<1, KEEP>(v.ax[2], sz, z, act);
     const float inv = v.inv_d, dt = v.dt;
-    const BAxis &ax0 = v.ax[0], &ax1 = v.ax[1], &ax2 = v.ax[2];
+    const bool scale = v.dxmode != 0;
+    const BAxis &ax0 = v.ax[0];
+    const int Tn = ax0.Tn, Tp = ax0.Tp;
+    const bool xf = xa < (uint32_t)Tn || (Tp && xb > sx - (uint32_t)Tp);
 
-    auto load = [&](uint32_t x) {
+    auto load = [&](uint32_t x, uint32_t i) {
         BHLoad<T> q;
-        const uint32_t i = x * syz + j;
         const uint32_t x1 = (x + 1u < sx) ? x + 1u : 0u;
         const uint32_t i1 = x1 * syz + j;
         const uint32_t ipy = i + dpy, ipz = i + dpz;   // 32-bit wrap arithmetic
@@ -381,77 +387,79 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
             q.gh = hexp[texp_index(v, x, jt)];
         }
         q.xu = q.xv = q.yu = q.yv = q.zu = q.zv = 0.f;
-        int side;
-        const int irx = bx_face(ax0, sx, x, side);
-        if (irx >= 0) {
-            const uint32_t ip = ((uint32_t)irx * sy + y) * sz + z;
-            q.xu = ax0.psi[1][side][0][ip]; q.xv = ax0.psi[1][side][1][ip];
+        if (xf) {
+            const FaceAt fx = face_at(Tn, Tp, sx, x);
+            if (fx.ir >= 0) {
+                const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                q.xu = ax0.psi[1][fx.side][0][ip]; q.xv = ax0.psi[1][fx.side][1][ip];
+            }
         }
         if (fy.ir >= 0) {
-            const uint32_t ip = (x * (uint32_t)(fy.side ? ax1.Tp : ax1.Tn) + (uint32_t)fy.ir) * sz + z;
-            q.yu = ax1.psi[1][fy.side][0][ip]; q.yv = ax1.psi[1][fy.side][1][ip];
+            const uint32_t ip = (x * fy.T() + (uint32_t)fy.ir) * sz + z;
+            q.yu = fy.u()[ip]; q.yv = fy.v()[ip];
         }
         if (fz.ir >= 0) {
-            const uint32_t ip = (x * sy + y) * (uint32_t)(fz.side ? ax2.Tp : ax2.Tn) + (uint32_t)fz.ir;
-            q.zu = ax2.psi[1][fz.side][0][ip]; q.zv = ax2.psi[1][fz.side][1][ip];
+            const uint32_t ip = (x * sy + y) * fz.T() + (uint32_t)fz.ir;
+            q.zu = fz.u()[ip]; q.zv = fz.v()[ip];
         }
         return q;
     };
 
     float ex = 0.f, ey = 0.f, ez = 0.f;
-    BHLoad<T> cur;
     if (act) {
         const uint32_t i = xa * syz + j;
         const int32_t wa = SS::scaled ? eexp[texp_index(v, xa, jt)] : 0;
         ex = dv<ST>(ldr(Ex + i), xe(wa, 0));
         ey = dv<ST>(ldr(Ey + i), xe(wa, 1));
         ez = dv<ST>(ldr(Ez + i), xe(wa, 2));
-        if (PF) cur = load(xa);
     }
-    for (uint32_t x = xa; x < xb; ++x) {
-        const uint32_t i = x * syz + j;
-        BHLoad<T> nxt;
+    uint32_t i = xa * syz + j;
+    for (uint32_t x = xa; x < xb; ++x, i += syz) {
         float nx = 0.f, ny = 0.f, nz = 0.f, ex1 = 0.f, ey1 = 0.f, ez1 = 0.f;
         if (act) {
-            if (!PF) cur = load(x);
-            else if (x + 1u < xb) nxt = load(x + 1u);
+            const BHLoad<T> cur = load(x, i);
             ex1 = dv<ST>(cur.ex1, xe(cur.ge, 0));
             ey1 = dv<ST>(cur.ey1, xe(cur.ge, 1));
             ez1 = dv<ST>(cur.ez1, xe(cur.ge, 2));
             // forward differences (update_h.cl:36-43), times 1/dx
-            float d_xy = (dv<ST>(cur.rxy, xe(cur.gy, 0)) - ex) * inv;
-            float d_xz = (dv<ST>(cur.rxz, xe(cur.gz, 0)) - ex) * inv;
-            float d_yx = (ey1 - ey) * inv;
-            float d_yz = (dv<ST>(cur.ryz, xe(cur.gz, 1)) - ey) * inv;
-            float d_zx = (ez1 - ez) * inv;
-            float d_zy = (dv<ST>(cur.rzy, xe(cur.gy, 2)) - ez) * inv;
+            float d_xy = dv<ST>(cur.rxy, xe(cur.gy, 0)) - ex;
+            float d_xz = dv<ST>(cur.rxz, xe(cur.gz, 0)) - ex;
+            float d_yx = ey1 - ey;
+            float d_yz = dv<ST>(cur.ryz, xe(cur.gz, 1)) - ey;
+            float d_zx = ez1 - ez;
+            float d_zy = dv<ST>(cur.rzy, xe(cur.gy, 2)) - ez;
+            if (scale) {
+                d_xy = d_xy * inv; d_xz = d_xz * inv; d_yx = d_yx * inv;
+                d_yz = d_yz * inv; d_zx = d_zx * inv; d_zy = d_zy * inv;
+            }
             float px = 0.f, py = 0.f, pz = 0.f;
-            int side;
-            const int irx = bx_face(ax0, sx, x, side);
-            if (irx >= 0) {
-                const uint32_t ip = ((uint32_t)irx * sy + y) * sz + z;
-                float su, sv;
-                face_update<float, false, 0>(ldg(ax0.tab[1][side][0] + irx), ldg(ax0.tab[1][side][1] + irx),
-                                             ldg(ax0.tab[1][side][2] + irx), cur.xu, cur.xv, su, sv,
-                                             d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-                ax0.psi[1][side][0][ip] = su;
-                ax0.psi[1][side][1][ip] = sv;
+            if (xf) {
+                const FaceAt fx = face_at(Tn, Tp, sx, x);
+                if (fx.ir >= 0) {
+                    float su, sv;
+                    face_update<float, false, 0>(ldg(ax0.tab[1][fx.side][0] + fx.ir), ldg(ax0.tab[1][fx.side][1] + fx.ir),
+                                              ldg(ax0.tab[1][fx.side][2] + fx.ir), cur.xu, cur.xv, su, sv,
+                                              d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                    const uint32_t ip = (uint32_t)fx.ir * syz + j;
+                    ax0.psi[1][fx.side][0][ip] = su;
+                    ax0.psi[1][fx.side][1][ip] = sv;
+                }
             }
             if (fy.ir >= 0) {
-                const uint32_t ip = (x * (uint32_t)(fy.side ? ax1.Tp : ax1.Tn) + (uint32_t)fy.ir) * sz + z;
                 float su, sv;
                 face_update<float, false, 1>(fy.p0, fy.p1, fy.p2, cur.yu, cur.yv, su, sv,
-                                             d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-                ax1.psi[1][fy.side][0][ip] = su;
-                ax1.psi[1][fy.side][1][ip] = sv;
+                                          d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = (x * fy.T() + (uint32_t)fy.ir) * sz + z;
+                fy.u()[ip] = su;
+                fy.v()[ip] = sv;
             }
             if (fz.ir >= 0) {
-                const uint32_t ip = (x * sy + y) * (uint32_t)(fz.side ? ax2.Tp : ax2.Tn) + (uint32_t)fz.ir;
                 float su, sv;
                 face_update<float, false, 2>(fz.p0, fz.p1, fz.p2, cur.zu, cur.zv, su, sv,
-                                             d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
-                ax2.psi[1][fz.side][0][ip] = su;
-                ax2.psi[1][fz.side][1][ip] = sv;
+                                          d_xy, d_xz, d_yx, d_yz, d_zx, d_zy, px, py, pz);
+                const uint32_t ip = (x * sy + y) * fz.T() + (uint32_t)fz.ir;
+                fz.u()[ip] = su;
+                fz.v()[ip] = sv;
             }
             // update_h.cl:129-131
             nx = dv<ST>(cur.hx, xe(cur.gh, 0)) - dt * ((d_zy - d_yz) - px);
@@ -470,23 +478,22 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
             ex = ex1;
             ey = ey1;
             ez = ez1;
-            if (PF) cur = nxt;
         }
     }
 }
 
-template <int ST, bool PF>
+template <int ST>
 __device__ __forceinline__ void batch_e_item(const BatchK &k, uint32_t ti, int64_t step)
 {
     const int4 tl = k.tiles[ti];
-    batch_e_tile<ST, PF>(k.vars[tl.x], tl, step, k.rows);
+    batch_e_tile<ST, false>(k.vars[tl.x], tl, step, k.rows);
 }
 
-template <int ST, bool PF>
+template <int ST>
 __device__ __forceinline__ void batch_h_item(const BatchK &k, uint32_t ti)
 {
     const int4 tl = k.tiles[ti];
-    batch_h_tile<ST, PF>(k.vars[tl.x], tl);
+    batch_h_tile<ST, false>(k.vars[tl.x], tl);
 }
 
 // next tile of the half-step whose counter is `ctr` (>= ntiles: none left)
@@ -498,9 +505,8 @@ __device__ __forceinline__ uint32_t next_tile(uint32_t *ctr, uint32_t *slot)
     return *slot;
 }
 
-// Persistent form: without the register prefetch (PF false) the E and H tile bodies together
-// fit BATCH_PERSIST_BLOCKS resident blocks per SM (64 registers), whose warps hide the load
-// latency; with it they need 128 registers and two blocks per SM, 1.3x slower.
+// Persistent form: the E and H tile bodies together at four resident blocks per SM (64 registers; the
+// descriptor is read again where it is used).
 constexpr int BATCH_PERSIST_BLOCKS = 4;
 
 template <int ST>
@@ -514,11 +520,11 @@ __global__ void __launch_bounds__(BATCH_THREADS, BATCH_PERSIST_BLOCKS) k_batch(c
         // half-step 2t uses counter 0, 2t + 1 counter 1; a counter is cleared right after the
         // grid barrier that ends its half-step, two barriers before its next use
         for (uint32_t ti = next_tile(&k.work[0], &item); ti < k.ntiles; ti = next_tile(&k.work[0], &item))
-            batch_e_item<ST, false>(k, ti, step);
+            batch_e_item<ST>(k, ti, step);
         grid.sync();
         if (blockIdx.x == 0 && threadIdx.x == 0) k.work[0] = 0u;
         for (uint32_t ti = next_tile(&k.work[1], &item); ti < k.ntiles; ti = next_tile(&k.work[1], &item))
-            batch_h_item<ST, false>(k, ti);
+            batch_h_item<ST>(k, ti);
         grid.sync();
         if (blockIdx.x == 0 && threadIdx.x == 0) k.work[1] = 0u;
     }
@@ -526,21 +532,29 @@ __global__ void __launch_bounds__(BATCH_THREADS, BATCH_PERSIST_BLOCKS) k_batch(c
     if (blockIdx.x == 0 && threadIdx.x == 0) *k.step = step0 + k.nsteps;
 }
 
-// One tile per block, all variants' tiles in one launch per half-step: three blocks per SM,
-// each warp with two planes of loads in flight (the register prefetch), about 1.5x the loads
-// in flight of the persistent form. The H launch advances the step counter.
+// One tile per block, all variants' tiles in one launch per half-step. Both bodies wait on memory, so
+// what counts is resident warps and a march without reloads: with the next plane loaded ahead (three
+// blocks per SM) and the descriptor's pointers, limits and source list read again for every plane, the
+// march was 261 (E) and 220 (H) instructions per warp and plane and a step of 8 variants (14.7 M cells)
+// took 0.389 ms in float32, 0.420 in bfloat16 without exponents and 0.619 with; now 184 and 163 and 0.337,
+// 0.304 and 0.417. E in float32 spills 56 bytes at five blocks and still gains (0.208 to 0.184 ms, four to
+// five); H loses there (0.146 to 0.163), and so does E with tile exponents. Six blocks: 0.211 and 0.174.
+// The H launch advances the step counter.
 template <int ST>
-__global__ void __launch_bounds__(BATCH_THREADS, 3) k_batch_e(const BatchK k)
+constexpr int batch_e_blocks() { return Store<ST>::scaled ? 4 : 5; }
+
+template <int ST>
+__global__ void __launch_bounds__(BATCH_THREADS, batch_e_blocks<ST>()) k_batch_e(const BatchK k)
 {
     const int4 tl = k.tiles[blockIdx.x];
-    batch_e_tile<ST>(k.vars[tl.x], tl, *k.step, k.rows);
+    batch_e_tile<ST, true>(k.vars[tl.x], tl, *k.step, k.rows);
 }
 
 template <int ST>
-__global__ void __launch_bounds__(BATCH_THREADS, 3) k_batch_h(const BatchK k)
+__global__ void __launch_bounds__(BATCH_THREADS, 4) k_batch_h(const BatchK k)
 {
     const int4 tl = k.tiles[blockIdx.x];
-    batch_h_tile<ST>(k.vars[tl.x], tl);
+    batch_h_tile<ST, true>(k.vars[tl.x], tl);
     // the E launch of this step, which reads the counter, has completed
     if (blockIdx.x == 0 && threadIdx.x == 0) *k.step += 1;
 }
