@@ -218,13 +218,16 @@ int fdtd_update_j(FdtdPlan *plan, const FdtdBuffers *buf, void *stream, double c
 /* Point sources for fdtd_run: after the E update of step t, E[index[k]] += values[t*n + k]
  * (the host-side `sim.E[ind] += field_source(t)` of opencl_fdtd's fdtd.py:168-169, moved on
  * the device; sources on one cell are added in list order). index holds flat indices into
- * the 3N E array in HOST memory (n <= 64); values is a DEVICE array of nsteps*n elements in
- * the plan's dtype. */
+ * the 3N E array in HOST memory (n <= 64); values is an array of nsteps*n elements in the plan's
+ * dtype, on the DEVICE, or with memory = FDTD_VALUES_HOST in host memory: each launch then carries
+ * its step's values (no copy), and the array is free when fdtd_run returns (a captured call keeps
+ * them); such sources are not taken by the one-pass step. */
+#define FDTD_VALUES_HOST 0x484f5354
 typedef struct FdtdPointSources {
     int32_t n;
-    int32_t _pad;
+    int32_t memory;          /* FDTD_VALUES_HOST; anything else: device */
     const int64_t *index;    /* host, n entries */
-    const void *values;      /* device, nsteps * n entries */
+    const void *values;      /* nsteps * n entries */
 } FdtdPointSources;
 
 /* FP64 DFT point monitor. After each step (E fully updated, point sources included) the

@@ -82,8 +82,11 @@ class FdtdBuffers(ctypes.Structure):
                 ("E2", c_vp), ("H2", c_vp), ("psi_e2", _PSI), ("psi_h2", _PSI)]
 
 
+FDTD_VALUES_HOST = 0x484f5354
+
+
 class FdtdPointSources(ctypes.Structure):
-    _fields_ = [("n", c_i32), ("_pad", c_i32), ("index", c_vp), ("values", c_vp)]
+    _fields_ = [("n", c_i32), ("memory", c_i32), ("index", c_vp), ("values", c_vp)]
 
 
 class FdtdDftMonitor(ctypes.Structure):

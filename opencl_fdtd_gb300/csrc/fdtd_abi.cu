@@ -144,6 +144,13 @@ YeeK<R> make_yee(const FdtdPlan *p, bool etype, bool imag, R *P, const R *Q, con
     return k;
 }
 
+// The values of step t, one per source, when they are in host memory (a launch carries them then), else NULL.
+template <typename R>
+const R *host_row(const FdtdPointSources *src, int t)
+{
+    return src->memory == FDTD_VALUES_HOST ? (const R *)src->values + (size_t)t * src->n : nullptr;
+}
+
 // The point sources of step t as arguments of a kernel that adds them itself (at most YEE_SRC).
 template <typename R, typename K>
 void kernel_sources(const FdtdPlan *p, K &k, const FdtdPointSources *src, int t)
@@ -151,8 +158,10 @@ void kernel_sources(const FdtdPlan *p, K &k, const FdtdPointSources *src, int t)
     k.nsrc = src->n;
     k.src_t = t;
     k.src_stride = src->n;
-    k.src_values = (const R *)src->values;
+    const R *const row = host_row<R>(src, t);
+    k.src_values = row ? nullptr : (const R *)src->values;
     for (int s = 0; s < src->n; ++s) {
+        if (row) k.src_val[s] = row[s];
         const uint64_t ind = (uint64_t)src->index[s], cell = ind % p->N;
         k.src_c[s] = (int32_t)(ind / p->N);
         k.src_x[s] = (uint32_t)(cell / p->syz);
@@ -301,7 +310,8 @@ PointK<R> source_args(FdtdPlan *p, const FdtdBuffers *b, const FdtdPointSources 
     PointK<R> k;
     std::memset(&k, 0, sizeof(k));
     k.E = (R *)b->E;
-    k.values = (const R *)src->values;
+    const R *const row = host_row<R>(src, t);
+    k.values = row ? nullptr : (const R *)src->values;
     k.t = t;
     k.stride = src->n;
     int n = 0;
@@ -310,6 +320,7 @@ PointK<R> source_args(FdtdPlan *p, const FdtdBuffers *b, const FdtdPointSources 
         if (plane < xbeg || plane >= xend) continue;
         k.index[n] = src->index[s];
         k.col[n] = s;
+        if (row) k.val[n] = row[s];
         ++n;
     }
     k.n = n;
@@ -955,7 +966,7 @@ bool fused_eligible(const FdtdPlan *p, const FdtdBuffers *b, const FdtdPointSour
         if (p->d.pml[f].thickness > 0 &&
             (!b->psi_e2[f][0] || !b->psi_e2[f][1] || !b->psi_h2[f][0] || !b->psi_h2[f][1]))
             return false;
-    if (src && src->n > STEP_MAX_SRC) return false;
+    if (src && (src->n > STEP_MAX_SRC || (src->n > 0 && src->memory == FDTD_VALUES_HOST))) return false;
     uint32_t threads = 0;
     size_t smem = 0;
     int fidx[3][2], shape = 0;

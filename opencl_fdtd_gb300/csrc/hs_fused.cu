@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
                     // point sources in list order (fdtd.py:168-169)
                     for (int s = 0; s < k.nsrc; ++s) {
                         if (k.src_x[s] != x || k.src_j[s] != j) continue;
-                        const R val = k.src_values[(int64_t)k.src_t * k.src_stride + k.src_col[s]];
+                        const R val = k.src_values ? k.src_values[(int64_t)k.src_t * k.src_stride + k.src_col[s]] : k.src_val[s];
                         if (k.src_c[s] == 0) nx = nx + val;
                         else if (k.src_c[s] == 1) ny = ny + val;
                         else nz = nz + val;

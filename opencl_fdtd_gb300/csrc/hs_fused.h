@@ -46,6 +46,7 @@ struct HSK {
     const R *src_values;
     uint32_t src_x[YEE_SRC], src_j[YEE_SRC];
     int32_t src_c[YEE_SRC], src_col[YEE_SRC];
+    R src_val[YEE_SRC];           // the step's values when src_values is NULL
     DftK<R> dft;
 };
 

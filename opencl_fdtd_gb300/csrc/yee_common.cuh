@@ -129,11 +129,13 @@ struct YeeK {
     int32_t bulk;               // 1: the bulk kernels apply
     uint32_t xbeg, xend;        // planes [xbeg, xend) this launch updates
     // point sources the bulk E kernel adds after the update, in list order (fdtd.py:168-169):
-    // E[c][x, j] += src_values[src_t * src_stride + src_col] for each of nsrc sources
+    // E[c][x, j] += src_values[src_t * src_stride + src_col] for each of nsrc sources; without
+    // src_values the step's values are src_val
     int32_t nsrc, src_t, src_stride, _pad2;
     const R *src_values;
     uint32_t src_x[YEE_SRC], src_j[YEE_SRC];
     int32_t src_c[YEE_SRC], src_col[YEE_SRC];
+    R src_val[YEE_SRC];
 };
 
 template <typename R>
@@ -164,10 +166,11 @@ constexpr int MAX_POINT_SOURCES = 64;
 template <typename R>
 struct PointK {
     R *E;
-    const R *values;            // [nsteps][stride]
+    const R *values;            // [nsteps][stride], or NULL: the step's values are val
     int32_t n, t, stride, _pad;
     int64_t index[MAX_POINT_SOURCES];
     int32_t col[MAX_POINT_SOURCES];   // column of each source in values
+    R val[MAX_POINT_SOURCES];
 };
 
 template <typename R>

@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
             // the same additions, in list order, as a separate launch after the update
             for (int s = 0; s < k.nsrc; ++s) {
                 if (k.src_x[s] != x || k.src_j[s] != j) continue;
-                const R val = k.src_values[(int64_t)k.src_t * k.src_stride + k.src_col[s]];
+                const R val = k.src_values ? k.src_values[(int64_t)k.src_t * k.src_stride + k.src_col[s]] : k.src_val[s];
                 if (k.src_c[s] == 0) ex = ex + val;
                 else if (k.src_c[s] == 1) ey = ey + val;
                 else ez = ez + val;
@@ -672,7 +672,7 @@ __global__ void k_point_sources(const PointK<R> k)
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     for (int s = 0; s < k.n; ++s) {
         const int64_t ind = k.index[s];
-        k.E[ind] = k.E[ind] + k.values[(int64_t)k.t * k.stride + k.col[s]];
+        k.E[ind] = k.E[ind] + (k.values ? k.values[(int64_t)k.t * k.stride + k.col[s]] : k.val[s]);
     }
 }
 
