@@ -67,11 +67,11 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
     constexpr uint32_t HS_THREADS = (uint32_t)hs_threads(AHEAD, MU, DX);
     __shared__ R sV[2][NV][HS_THREADS];
     __shared__ R sC[AHEAD ? 6 : 3][HS_THREADS];   // z-face coefficients of each thread: H, then E
-    grid_dependency_sync();
     const uint32_t t = threadIdx.x;
     const uint32_t chunk0 = blockIdx.x / k.ntile;
     if (chunk0 >= k.nchunk) {
         // the step's DFT sample: E is not written by this launch
+        grid_dependency_sync();
         const int nq = k.dft.npoint * (k.dft.nfreq > 0 ? k.dft.nfreq : 1);
         for (int q = (int)t; q < nq; q += (int)HS_THREADS) dft_sample(k.dft, q);
         return;
@@ -139,6 +139,7 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
         for (int s = 0; s < k.nsrc; ++s) srcs |= own && k.src_j[s] == j;
         srcs = __any_sync(0xffffffffu, srcs) != 0;
     }
+    grid_dependency_sync();
     const R *const E0 = k.E, *const E1 = k.E + N, *const E2 = k.E + 2 * N;
     const R *const H0 = k.HA, *const H1 = k.HA + N, *const H2 = k.HA + 2 * N;
 

@@ -229,6 +229,31 @@ __global__ void __launch_bounds__(BLOCK) k_generic_h(const YeeK<R> k)
 }
 
 // ---- bulk kernels ----------------------------------------------------------------------------
+// Cell t of a plane in the kernel's order (z_order on the host): row-major, or the cells outside the z
+// faces first, then those inside, so that a warp holds the one or the other.
+template <bool SPLIT, typename R>
+__device__ __forceinline__ void plane_cell(const YeeK<R> &k, uint32_t t, uint32_t &y, uint32_t &z)
+{
+    if (!SPLIT) {
+        y = k.dsz.div(t);
+        z = t - y * k.sz;
+    } else if (t < k.nin) {
+        y = k.dzi.div(t);
+        z = t - y * k.nzi + k.z0;
+    } else {
+        const uint32_t u = t - k.nin, nf = k.sz - k.nzi;
+        y = k.dzf.div(u);
+        z = u - y * nf;
+        if (z >= k.z0) z += k.nzi;
+    }
+}
+
+// Warps without absorbing cells leave out the terms of the CPML arrays (adding zero) in double precision,
+// which the FP64 units bound: with the z order a step of 197x173x73 cells went from 0.436 to 0.402 ms. In
+// float32 the test cost what it saved.
+template <typename R>
+constexpr bool skip_zero_psi() { return sizeof(R) == 8; }
+
 // Values one E-type iteration reads, loaded one iteration ahead.
 template <typename R>
 struct ELoad {
@@ -245,29 +270,33 @@ constexpr int EBLOCK = 256, EMINB = 3;
 
 // Forms of the bulk E kernel (FDTD_TUNE_E_FORM): 0 loads the next plane one iteration ahead
 // (80 registers, three blocks per SM); 1 (the default) loads each plane when it is updated, at
-// four blocks per SM (64 registers). Same arithmetic in both. On the 395x345x73 grid: 0.110
-// and 0.105 ms (a per-plane form at five blocks per SM spilled 80 B and took 0.131 ms).
-template <int FORM>
+// four blocks per SM (64 registers), in double precision at three (80: 0.128 ms against 0.130 on
+// 197x173x73). Same arithmetic in both. On the 395x345x73 grid in float32: 0.110 and 0.105 ms (a
+// per-plane form at five blocks per SM spilled 80 B and took 0.131 ms).
+template <int FORM, bool DBL>
 struct EForm {
     static constexpr bool prefetch = FORM == 0;
-    static constexpr int min_blocks = FORM == 0 ? EMINB : 4;
+    static constexpr int min_blocks = FORM == 0 || DBL ? EMINB : 4;
 };
 
 template <typename R, int DX, bool BLOCH, int FORM, bool AWAY>
-__global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(const YeeK<R> k)
+__global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_blocks) k_bulk_e(const YeeK<R> k)
 {
-    constexpr bool PF = EForm<FORM>::prefetch;
-    grid_dependency_sync();
-    const uint32_t j = blockIdx.x * EBLOCK + threadIdx.x;
-    const bool act = j < k.syz;
+    constexpr bool PF = EForm<FORM, sizeof(R) == 8>::prefetch, SKIP = skip_zero_psi<R>();
+    constexpr bool SPLIT = sizeof(R) == 8 || BLOCH;      // the other form keeps row order: 3 us of 105 faster there
+    const uint32_t t = blockIdx.x * EBLOCK + threadIdx.x;
+    const bool act = t < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
-    const uint32_t y = k.dsz.div(j);
-    const uint32_t z = j - y * sz;
+    uint32_t y, z;
+    plane_cell<SPLIT>(k, t, y, z);
+    const uint32_t j = SPLIT ? y * sz + z : t;
     const FixedFace<R, AWAY> fy = fixed_face<R, AWAY>(k.ax[1], sy, y, act);
     const FixedFace<R, AWAY> fz = fixed_face<R, AWAY>(k.ax[2], sz, z, act);
+    const bool wf = !SKIP || __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
     if (!act) return;
     const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
     const uint32_t xb = min(xa + k.xchunk, k.xend);
+    const bool wx = wf || x_faces(k.ax[0], sx, xa, xb);          // a cell of the warp's march is in a face
     const uint64_t N = k.N;
     const R *__restrict__ Qx = k.Q;
     const R *__restrict__ Qy = k.Q + N;
@@ -289,11 +318,13 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
     const bool bz = BLOCH && (k.bloch_mask & 4) && z == 0;
     R iy = k.inv_d, iz = k.inv_d;
     if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
-    // a point source in this block's cells and planes (block-uniform)
+    // a point source in this column and these planes
     bool srcs = false;
     for (int s = 0; s < k.nsrc; ++s)
-        srcs |= k.src_j[s] / (uint32_t)EBLOCK == blockIdx.x &&
+        srcs |= k.src_j[s] == j &&
+
                 (k.src_x[s] - k.xbeg) / k.xchunk == blockIdx.y;
+    grid_dependency_sync();
 
     auto load = [&](uint32_t x, uint32_t i) {
         ELoad<R> v;
@@ -381,9 +412,11 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM>::min_blocks) k_bulk_e(cons
             fz.pu[ip] = su; fz.pv[ip] = sv;
         }
         // update_e.cl:105-107
-        R ex = cur.ex + cur.cx * ((d_zy - d_yz) + px);
-        R ey = cur.ey + cur.cy * ((d_xz - d_zx) + py);
-        R ez = cur.ez + cur.cz * ((d_yx - d_xy) + pz);
+        R cu_x = d_zy - d_yz, cu_y = d_xz - d_zx, cu_z = d_yx - d_xy;
+        if (!SKIP || wx) { cu_x = cu_x + px; cu_y = cu_y + py; cu_z = cu_z + pz; }
+        R ex = cur.ex + cur.cx * cu_x;
+        R ey = cur.ey + cur.cy * cu_y;
+        R ez = cur.ez + cur.cz * cu_z;
         if (srcs) {
             // the same additions, in list order, as a separate launch after the update
             for (int s = 0; s < k.nsrc; ++s) {
@@ -417,27 +450,29 @@ struct HLoad {
 
 // Forms of the bulk H kernel, as those of E: with the next plane loaded one iteration ahead at three
 // blocks per SM (80 registers); with dt/mu or Bloch partners, whose values would spill there, with each
-// plane loaded when it is updated, at four (64 registers).
+// plane loaded when it is updated, at four (64 registers). In double precision, where values take two
+// registers and the FP64 units, not latency, are the bound, two blocks (0.211 to 0.199 ms on 197x173x73).
 constexpr bool h_prefetch(bool mu, bool bloch) { return !mu && !bloch; }
-constexpr int h_min_blocks(bool mu, bool bloch) { return h_prefetch(mu, bloch) ? 3 : 4; }
+constexpr int h_min_blocks(bool mu, bool bloch, bool dbl) { return dbl ? 2 : h_prefetch(mu, bloch) ? 3 : 4; }
 
 template <typename R, int DX, bool MU, bool POYNT, bool BLOCH, bool AWAY>
-__global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH)) k_bulk_h(const YeeK<R> k)
+__global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)) k_bulk_h(const YeeK<R> k)
 {
-    constexpr bool PF = h_prefetch(MU, BLOCH);
-    grid_dependency_sync();
-    const uint32_t j = blockIdx.x * BLOCK + threadIdx.x;
-    const bool act = j < k.syz;
+    constexpr bool PF = h_prefetch(MU, BLOCH), SKIP = skip_zero_psi<R>();
+    const uint32_t t = blockIdx.x * BLOCK + threadIdx.x;
+    const bool act = t < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
-    const uint32_t y = k.dsz.div(j);
-    const uint32_t z = j - y * sz;
+    uint32_t y, z;
+    plane_cell<true>(k, t, y, z);
+    const uint32_t j = y * sz + z;
     const FixedFace<R, AWAY> fy = fixed_face<R, AWAY>(k.ax[1], sy, y, act);
     const FixedFace<R, AWAY> fz = fixed_face<R, AWAY>(k.ax[2], sz, z, act);
-    const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
+        const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
     if (!act) return;
     const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
     const uint32_t xb = min(xa + k.xchunk, k.xend);
-    const bool xf = x_faces(k.ax[0], sx, xa, xb);
+        // asking once costs the form that also writes the products 2 us of 133 on 395x345x73 cells
+    const bool xf = (POYNT && sizeof(R) == 4) || x_faces(k.ax[0], sx, xa, xb);
     const uint64_t N = k.N;
     const R *__restrict__ Qx = k.Q;
     const R *__restrict__ Qy = k.Q + N;
@@ -446,9 +481,9 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH)) k_bulk_h(const
     const R *__restrict__ Px = k.P;
     const R *__restrict__ Py = k.P + N;
     const R *__restrict__ Pz = k.P + 2 * N;
-    R *__restrict__ Wx = k.W;
-    R *__restrict__ Wy = k.W + N;
-    R *__restrict__ Wz = k.W + 2 * N;
+    R *__restrict__ Wx = AWAY ? k.W : k.P;
+    R *__restrict__ Wy = AWAY ? k.W + N : k.P + N;
+    R *__restrict__ Wz = AWAY ? k.W + 2 * N : k.P + 2 * N;
     // y/z plus neighbours with periodic wrap (common.cl:82-84), fixed for the thread
     const uint32_t dpy = (y + 1u < sy) ? sz : 0u - (sy - 1u) * sz;
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
@@ -458,6 +493,7 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH)) k_bulk_h(const
     R iy = k.inv_d, iz = k.inv_d;
     if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
     const R dt = k.dt;
+    grid_dependency_sync();
 
     auto load = [&](uint32_t x, uint32_t i) {
         HLoad<R> v;
@@ -547,17 +583,12 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH)) k_bulk_h(const
                 fz.pu[ip] = su; fz.pv[ip] = sv;
             }
         }
-        R hx, hy, hz;
-        if (MU) {
-            hx = cur.hx - cur.cx * ((d_zy - d_yz) - px);
-            hy = cur.hy - cur.cy * ((d_xz - d_zx) - py);
-            hz = cur.hz - cur.cz * ((d_yx - d_xy) - pz);
-        } else {
-            // update_h.cl:129-131
-            hx = cur.hx - dt * ((d_zy - d_yz) - px);
-            hy = cur.hy - dt * ((d_xz - d_zx) - py);
-            hz = cur.hz - dt * ((d_yx - d_xy) - pz);
-        }
+        // update_h.cl:129-131
+        R cu_x = d_zy - d_yz, cu_y = d_xz - d_zx, cu_z = d_yx - d_xy;
+        if (!SKIP || wf || xf) { cu_x = cu_x - px; cu_y = cu_y - py; cu_z = cu_z - pz; }
+        const R hx = cur.hx - (MU ? cur.cx : dt) * cu_x;
+        const R hy = cur.hy - (MU ? cur.cy : dt) * cu_y;
+        const R hz = cur.hz - (MU ? cur.cz : dt) * cu_z;
         Wx[i] = hx;
         Wy[i] = hy;
         Wz[i] = hz;
@@ -618,6 +649,7 @@ __global__ void __launch_bounds__(BLOCK) k_bulk_s(const SK<R> k)
         v.yz_z = ldg(oyz + imz); v.zy_y = ldg(ozy + imy);
         return v;
     };
+    grid_dependency_sync();
     uint32_t i = xa * syz + j;
     const uint32_t im = xa ? i - syz : i + (sx - 1u) * syz;
     R yx_m = ldg(oyx + im), zx_m = ldg(ozx + im);
@@ -686,16 +718,18 @@ static uint32_t sm_count()
     return (uint32_t)n[dev];
 }
 
-// x planes a thread of a bulk kernel marches when none is set (xchunk 0): 8, or on grids too small to
-// fill the GPU that way the most that still gives every SM its resident blocks (1 at least), since
-// such a launch takes as long as one thread's march.
+// x planes a thread of a bulk kernel marches when none is set (xchunk 0): 8, or on small grids the fewest
+// with which every block is resident at once: a launch then takes one thread's march, and more blocks than
+// that cost a second wave (E and H of 64^3 cells 9.3 us a step with 1 plane, 1024 blocks, and 8.0 with 2;
+// 151x129x61: 25.8 with 7, 669 blocks for 608 places, and 22.5 with 8).
 template <typename K>
 static dim3 bulk_grid(K &k, uint32_t block, uint32_t resident)
 {
     const uint32_t nj = (k.syz + block - 1) / block, nx = k.xend - k.xbeg;
     if (!k.xchunk) {
-        const uint64_t slots = (uint64_t)sm_count() * resident, all = (uint64_t)nj * nx;
-        k.xchunk = all >= 8u * slots ? 8u : (uint32_t)(all / slots > 1u ? all / slots : 1u);
+        const uint64_t slots = (uint64_t)sm_count() * resident;
+        k.xchunk = 1u;
+        while (k.xchunk < 8u && (uint64_t)nj * ((nx + k.xchunk - 1) / k.xchunk) > slots) ++k.xchunk;
     }
     return dim3(nj, (nx + k.xchunk - 1) / k.xchunk, 1);
 }
@@ -705,11 +739,12 @@ static inline dim3 plane_grid(uint32_t syz, uint32_t nx)
     return dim3((syz + BLOCK - 1) / BLOCK, nx, 1);
 }
 
-// away: the result goes to other arrays (the first step of fdtd_run's E-ahead path; no Bloch there)
+// away: the result goes to other arrays (the first step of fdtd_run's E-ahead path: float32, no Bloch)
 template <typename R, bool BLOCH, int DX>
 static void (*bulk_e_form(int form, bool away))(YeeK<R>)
 {
-    if (!BLOCH && away) return k_bulk_e<R, DX, false, 1, true>;
+    if constexpr (!BLOCH && sizeof(R) == 4)
+        if (away) return k_bulk_e<R, DX, false, 1, true>;
     if (form == 1) return k_bulk_e<R, DX, BLOCH, 1, false>;
     return k_bulk_e<R, DX, BLOCH, 0, false>;
 }
@@ -731,7 +766,7 @@ cudaError_t launch_yee_e(const YeeK<R> &kk, cudaStream_t st, bool pdl)
         k_generic_e<R><<<plane_grid(k.syz, k.xend - k.xbeg), BLOCK, 0, st>>>(k);
         return cudaGetLastError();
     }
-    const dim3 g = bulk_grid(k, EBLOCK, 4u);
+    const dim3 g = bulk_grid(k, EBLOCK, sizeof(R) == 8 ? 3u : 4u);
     const int f = k.eform;
     const bool away = k.W != k.P;
     return launch_dependent(k.bloch_mask ? bulk_e_kernel<R, true>(k.dxmode, f, away) : bulk_e_kernel<R, false>(k.dxmode, f, away),
@@ -740,9 +775,10 @@ cudaError_t launch_yee_e(const YeeK<R> &kk, cudaStream_t st, bool pdl)
 
 // away: as above (the last step of that path; no Poynting or Bloch there)
 template <typename R, int DX, bool BLOCH>
-static void (*bulk_h_kernel(bool mu, bool poynting, bool away))(YeeK<R>)
+static void (*bulk_h_form(bool mu, bool poynting, bool away))(YeeK<R>)
 {
-    if (away) return mu ? k_bulk_h<R, DX, true, false, false, true> : k_bulk_h<R, DX, false, false, false, true>;
+    if constexpr (!BLOCH && sizeof(R) == 4)
+        if (away) return mu ? k_bulk_h<R, DX, true, false, false, true> : k_bulk_h<R, DX, false, false, false, true>;
     if (mu) return poynting ? k_bulk_h<R, DX, true, true, BLOCH, false> : k_bulk_h<R, DX, true, false, BLOCH, false>;
     return poynting ? k_bulk_h<R, DX, false, true, BLOCH, false> : k_bulk_h<R, DX, false, false, BLOCH, false>;
 }
@@ -750,8 +786,9 @@ static void (*bulk_h_kernel(bool mu, bool poynting, bool away))(YeeK<R>)
 template <typename R, bool BLOCH>
 static void (*bulk_h_kernel(int dxmode, bool mu, bool poynting, bool away))(YeeK<R>)
 {
-    return dxmode == 0 ? bulk_h_kernel<R, 0, BLOCH>(mu, poynting, away) : dxmode == 1 ? bulk_h_kernel<R, 1, BLOCH>(mu, poynting, away)
-                                                                                 : bulk_h_kernel<R, 2, BLOCH>(mu, poynting, away);
+    return dxmode == 0   ? bulk_h_form<R, 0, BLOCH>(mu, poynting, away)
+           : dxmode == 1 ? bulk_h_form<R, 1, BLOCH>(mu, poynting, away)
+                         : bulk_h_form<R, 2, BLOCH>(mu, poynting, away);
 }
 
 template <typename R>
@@ -771,19 +808,19 @@ cudaError_t launch_yee_h(const YeeK<R> &kk, bool mu, bool poynting, cudaStream_t
         return cudaGetLastError();
     }
     const bool away = k.W != k.P;
-    const dim3 g = bulk_grid(k, BLOCK, (uint32_t)h_min_blocks(mu, k.bloch_mask != 0));
-    return launch_dependent(k.bloch_mask ? bulk_h_kernel<R, true>(k.dxmode, mu, poynting, away) : bulk_h_kernel<R, false>(k.dxmode, mu, poynting, away),
+    const dim3 g = bulk_grid(k, BLOCK, (uint32_t)h_min_blocks(mu, k.bloch_mask != 0, sizeof(R) == 8));
+    return launch_dependent(k.bloch_mask ? bulk_h_kernel<R, true>(k.dxmode, mu, poynting, away)
+                                         : bulk_h_kernel<R, false>(k.dxmode, mu, poynting, away),
                             g, BLOCK, st, pdl, k);
 }
 
 template <typename R>
-cudaError_t launch_poynting(const SK<R> &kk, cudaStream_t st)
+cudaError_t launch_poynting(const SK<R> &kk, cudaStream_t st, bool pdl)
 {
     SK<R> k = kk;
     if (k.xend <= k.xbeg) return cudaSuccess;
     const dim3 g = bulk_grid(k, BLOCK, 5u);
-    k_bulk_s<R><<<g, BLOCK, 0, st>>>(k);
-    return cudaGetLastError();
+    return launch_dependent(k_bulk_s<R>, g, BLOCK, st, pdl, k);
 }
 
 template <typename R>
@@ -816,7 +853,7 @@ cudaError_t launch_point_sources(const PointK<R> &k, cudaStream_t st)
 #define FDTD_INSTANTIATE(R)                                                              \
     template cudaError_t launch_yee_e<R>(const YeeK<R> &, cudaStream_t, bool);         \
     template cudaError_t launch_yee_h<R>(const YeeK<R> &, bool, bool, cudaStream_t, bool); \
-    template cudaError_t launch_poynting<R>(const SK<R> &, cudaStream_t);              \
+    template cudaError_t launch_poynting<R>(const SK<R> &, cudaStream_t, bool);              \
     template cudaError_t launch_prepare<R>(const PrepK<R> &, cudaStream_t);            \
     template cudaError_t launch_fieldsrc<R>(const JK<R> &, cudaStream_t);              \
     template cudaError_t launch_point_sources<R>(const PointK<R> &, cudaStream_t);
