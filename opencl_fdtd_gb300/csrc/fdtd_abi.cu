@@ -553,7 +553,7 @@ int run_hs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
     // the step's DFT sample: in the H launch (one extra block) or on the side stream beside it
     const bool dft_in = mon && p->hs_dft;
     const bool dft_side = mon && !p->hs_dft;
-    const bool pdl = p->pdl != 0;
+    const bool pdl = p->pdl != 0, late = lbc_holds_source(p, src);
     if (dft_side && (rc = side_stream(p))) return rc;
     form.ahead = ahead && nsteps > 1;
     hs_layout<R>(p, k, form, dft_in ? 1u : 0u);
@@ -564,12 +564,12 @@ int run_hs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
         if (dft_side && t > 0 && (rc = check_cuda(cudaStreamWaitEvent(st, p->ev_join, 0), "join wait"))) return rc;
         if ((rc = timer.mark(t, 0))) return rc;
         if (t == 0 || !ahead) {
-            // without a learned boundary (whose E fix-up comes before the sources) the E kernel
-            // adds the point sources itself
+            // the E kernel adds the point sources itself, unless a learned boundary's E fix-up, which
+            // comes before them, changes one of their cells
             const bool away = ahead && ((nsteps - 1) & 1);
             bool added = false;
             if ((rc = lbc_before_e(p, b, H[ch], st))) return rc;
-            if ((rc = run_update_e<R>(p, &bb, st, false, 0, 0xffffffffu, p->lbc_mask ? nullptr : src, t, &added, pdl,
+            if ((rc = run_update_e<R>(p, &bb, st, false, 0, 0xffffffffu, late ? nullptr : src, t, &added, pdl,
                                       away ? E[1] : nullptr, away ? psi_e[1] : nullptr))) return rc;
             if (away) ce = 1;
             if ((rc = lbc_after_e(p, b, H[ch], st))) return rc;
@@ -656,14 +656,14 @@ int run_slabs(FdtdPlan *p, const FdtdBuffers *b, cudaStream_t st, int nsteps,
     const uint32_t sx = p->sx;
     // the learned boundary's E corrections must land before any H update reads them: whole grid
     const uint32_t W = p->slab && !p->lbc_mask ? p->slab : sx;
-    const bool bloch = p->d.n_bloch != 0, poynt = p->d.do_poynting != 0, pdl = p->pdl != 0;
+    const bool bloch = p->d.n_bloch != 0, poynt = p->d.do_poynting != 0, pdl = p->pdl != 0, late = lbc_holds_source(p, src);
     int rc;
     if (W >= sx) {
         // one slab: the plain whole-grid sequence
         for (int t = 0; t < nsteps; ++t) {
             bool added = false;
             if ((rc = lbc_before_e(p, b, b->H, st))) return rc;
-            if ((rc = run_update_e<R>(p, b, st, false, 0, 0xffffffffu, p->lbc_mask ? nullptr : src, t, &added, pdl))) return rc;
+            if ((rc = run_update_e<R>(p, b, st, false, 0, 0xffffffffu, late ? nullptr : src, t, &added, pdl))) return rc;
             if (bloch && (rc = run_update_e<R>(p, b, st, true, 0, 0xffffffffu, nullptr, 0, nullptr, pdl))) return rc;
             if ((rc = lbc_after_e(p, b, b->H, st))) return rc;
             if (!added && src && src->n > 0 && (rc = run_point_sources<R>(p, b, st, src, t))) return rc;

@@ -56,4 +56,6 @@ int check_cuda(cudaError_t e, const char *what);
 int lbc_before_e(const FdtdPlan *p, const FdtdBuffers *b, const void *H, cudaStream_t st);
 int lbc_after_e(const FdtdPlan *p, const FdtdBuffers *b, const void *H, cudaStream_t st);
 int lbc_after_h(const FdtdPlan *p, const FdtdBuffers *b, void *H, cudaStream_t st);
+// whether a point source lies on a cell that the E fix-up changes (its addition must then follow it)
+bool lbc_holds_source(const FdtdPlan *p, const FdtdPointSources *src);
 }  // namespace fdtd

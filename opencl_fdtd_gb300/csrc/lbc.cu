@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 
 #include "lbc.h"
+#include "yee_common.cuh"
 
 namespace fdtd {
 
@@ -722,8 +723,6 @@ constexpr int PK_B2 = PK_B1 + LBC_HID;            // float [64]
 constexpr int PK_B3 = PK_B2 + LBC_HID;            // float [8]
 static_assert(PK_B3 + 8 == LBC_PACK_WORDS, "packed layout size");
 
-constexpr int XS = 120;                           // float row stride of a warp's stencil tile
-
 // two floats rounded to bfloat16 in one conversion (lo in the low half)
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
@@ -840,100 +839,158 @@ __device__ __forceinline__ void act_to_a(const float acc[8][4], uint32_t ah[4][4
 }
 
 
-template <bool SPLIT>
-__global__ void __launch_bounds__(MMA_WARPS * 32) k_lbc_predict_mma(const LGrid g, int side, float memory,
-                                                                     const uint32_t *Wp, const float *E,
-                                                                     const float *H, float *pred)
+// A block holds its face's packed weights in shared memory and gives each warp a tile of MW_TU x 16
+// columns, whose stencil cells the warp stages as component pairs (two neighbouring inputs of the
+// network), plane (pair, depth) by plane. A lane then reads the A fragments of layer 1 straight from
+// the stage: inputs 2 m and 2 m + 1, m = 8 ks + tq (+ 4), of the columns gq and gq + 8.
+//
+// What bounds it: latency. One step's ghosts of a 203x177x61 grid are 118 k columns, 2.7 GFLOP: a few
+// microseconds of the tensor units and 15 of instruction issue. With the weights read through L1 (64%
+// hits beside the stages), inputs normalised into a second shared array, 4-row tiles (two uneven waves
+// of blocks, half of them empty) it took 55 us, now 36 (1-row tiles 38, 4-row 42; 8 warps a block 40).
+constexpr int MW_TU = 2, MW_WARPS = 4, MW_SU = MW_TU + 2, MW_SV = 18;
+// words of a plane; the three pairs' planes of a depth start 12 or 24 banks apart, so that the four inputs
+// that the lanes of a column read at once fall in different banks
+constexpr int mw_plane(int n)
 {
-    extern __shared__ __align__(16) float smem_f[];
-    const LFace &f = g.face[blockIdx.y];
-    if (side >= 0 && f.side != side) return;                             // block-uniform
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gq = lane >> 2, tq = lane & 3;
-    float *st = smem_f + warp * (MMA_STAGE + 16 * XS + 16);
-    float *xs = st + MMA_STAGE;                                           // [16][XS] network inputs
-    float *rr = xs + 16 * XS;                                             // [16] RMS of each row
-    // packed weights of the face (read through L1: every warp of the face reads the same 24 KB)
-    const uint32_t *w = Wp + (uint64_t)(f.axis * 2 + f.side) * LBC_PACK_WORDS;
-    const float *wb = reinterpret_cast<const float *>(w);
-    const uint2 *w1 = reinterpret_cast<const uint2 *>(w + PK_W1);
-    const uint2 *w2 = reinterpret_cast<const uint2 *>(w + PK_W2);
-    const uint2 *w3 = reinterpret_cast<const uint2 *>(w + PK_W3);
+    return (2 * n) % 32 == 24 || (2 * n) % 32 == 12 ? n : mw_plane(n + 2);
+}
+constexpr int MW_PL = mw_plane(MW_SU * MW_SV * 2);
+constexpr int MW_STAGE = 6 * MW_PL;                                       // words per warp
+constexpr size_t MW_SMEM = (size_t)(LBC_PACK_WORDS + MW_WARPS * MW_STAGE) * 4;
+static_assert(LBC_PACK_WORDS % 4 == 0 && MW_PL % 2 == 0, "16-byte weights, 8-byte pairs");
 
-    const uint32_t ntv = (f.nv + 15u) / 16u, ntu = (f.nu + MMA_TU - 1u) / MMA_TU;
-    const uint32_t job = blockIdx.x * MMA_WARPS + warp;
-    if (job >= ntu * ntv) return;                                         // warp-uniform; no block barrier below
-    const uint32_t tu = job / ntv, tv = job % ntv;
-    const uint32_t cu0 = tu * MMA_TU, cv0 = tv * 16u;                     // first column of the tile (face-local)
-    stage_tile(g, f, cu0, cv0, E, H, st, lane);
-    __syncwarp();
-    for (int tr = 0; tr < MMA_TU; ++tr) {
-        const uint32_t cu = cu0 + (uint32_t)tr;
-        if (cu >= f.nu) break;                                            // warp-uniform
-        // gather: lane pair (row = lane / 2) reads depth (lane & 1) of its column's stencil
-        {
-            const int row = lane >> 1, d = lane & 1;
-            const uint32_t cv = cv0 + (uint32_t)row;
-            const uint32_t u = f.u0 + cu, v = f.v0 + cv;
-            // columns outside the window read nothing: r = 0, no network term
-            const bool ok = cv < f.nv && in_window(g, blockIdx.y, u, v);
-            float x[54];
-            float ss = 0.f;
+struct MFirst {
+    uint32_t block[7];                                                    // first block of each face
+};
+
+// the cells of the tile whose first (face-local) column is (cu0, cv0), clamped to the grid like cell_of;
+// lanes take the positions (sv, d) in memory order, as in stage_tile
+__device__ __forceinline__ void stage_pairs(const LGrid &g, const LFace &f, uint32_t cu0, uint32_t cv0, const float *E,
+                                            const float *H, float *st, int lane)
+{
+    const int a = f.axis, ua = a == 0 ? 1 : 0, va = a == 2 ? 1 : 2;
+    const uint32_t syz = g.s[1] * g.s[2];
+    const uint32_t sd = a == 0 ? syz : a == 1 ? g.s[2] : 1u, sua = ua == 0 ? syz : g.s[2], sva = va == 1 ? g.s[2] : 1u;
 #pragma unroll
-            for (int du = -1; du <= 1; ++du)
+    for (int h = 0; h < 2; ++h) {
+        const int e = lane + 32 * h;
+        if (e >= 2 * MW_SV) break;
+        const int d = a == 2 ? (e & 1) : e / MW_SV, sv = a == 2 ? (e >> 1) : e % MW_SV;
+        const uint32_t cd = f.side ? g.s[a] - 1u - (uint32_t)d : (uint32_t)d;
+        const uint32_t off = cd * sd + clampu((int)(f.v0 + cv0) - 1 + sv, g.s[va]) * sva;
+        float *const dst = st + d * MW_PL + sv * 2;
+        float v[MW_SU][6];
 #pragma unroll
-                for (int dv = -1; dv <= 1; ++dv) {
-                    const int k0 = ((du + 1) * 3 + (dv + 1)) * 6;
-                    const float *sp = st + d * MMA_PL + (tr + 1 + du) * MMA_SV + (row + 1 + dv);
+        for (int su = 0; su < MW_SU; ++su) {
+            const uint32_t i = off + clampu((int)(f.u0 + cu0) - 1 + su, g.s[ua]) * sua;
 #pragma unroll
-                    for (int q = 0; q < 6; ++q) {
-                        const float xv = ok ? sp[q * 2 * MMA_PL] : 0.f;
-                        x[k0 + q] = xv;
-                        ss += xv * xv;
-                    }
-                }
-            ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-            const float r = sqrtf(ss * (1.0f / LBC_IN));
-            const float inv = r > 0.f ? 1.0f / r : 0.f;
-            float2 *xr = reinterpret_cast<float2 *>(xs + row * XS + d * 54);   // 8-byte aligned
-#pragma unroll
-            for (int k = 0; k < 27; ++k) xr[k] = make_float2(x[2 * k] * inv, x[2 * k + 1] * inv);
-            if (d == 1) {
-                xr[27] = make_float2(0.f, 0.f);                           // K padding 108..111
-                xr[28] = make_float2(0.f, 0.f);
-            } else {
-                rr[row] = r;
+            for (int q = 0; q < 3; ++q) {
+                v[su][q] = __ldg(E + q * g.N + i);
+                v[su][3 + q] = __ldg(H + q * g.N + i);
             }
         }
-        __syncwarp();
+#pragma unroll
+        for (int su = 0; su < MW_SU; ++su)
+#pragma unroll
+            for (int qp = 0; qp < 3; ++qp)
+                *reinterpret_cast<float2 *>(dst + qp * 2 * MW_PL + su * MW_SV * 2) = make_float2(v[su][2 * qp], v[su][2 * qp + 1]);
+    }
+}
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(MW_WARPS * 32, 4) k_lbc_predict_mma(const __grid_constant__ LGrid g, const __grid_constant__ MFirst first,
+                                                                      float memory, const uint32_t *Wp, const float *E,
+                                                                      const float *H, float *pred)
+{
+    extern __shared__ __align__(16) uint32_t smem_w[];
+    int fi = 0;
+    while (blockIdx.x >= first.block[fi + 1]) ++fi;
+    const LFace &f = g.face[fi];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gq = lane >> 2, tq = lane & 3;
+    float *const st = reinterpret_cast<float *>(smem_w + LBC_PACK_WORDS) + warp * MW_STAGE;
+    grid_dependency_sync();
+    {
+        const uint32_t *src = Wp + (uint64_t)(f.axis * 2 + f.side) * LBC_PACK_WORDS;
+        const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_w);
+        for (int i = threadIdx.x; i < LBC_PACK_WORDS / 4; i += MW_WARPS * 32)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * i), "l"(src + 4 * i) : "memory");
+        copy_commit();
+    }
+    const uint32_t ntv = (f.nv + 15u) / 16u, ntu = (f.nu + MW_TU - 1u) / MW_TU;
+    const uint32_t job = (blockIdx.x - first.block[fi]) * MW_WARPS + warp;
+    const bool work = job < ntu * ntv;                                    // warp-uniform
+    const uint32_t tu = job / ntv, tv = job - tu * ntv;
+    const uint32_t cu0 = tu * MW_TU, cv0 = tv * 16u;                      // first column of the tile (face-local)
+    if (work) stage_pairs(g, f, cu0, cv0, E, H, st, lane);
+    copy_wait<0>();
+    __syncthreads();
+    if (!work) return;
+    const float *const wb = reinterpret_cast<const float *>(smem_w);
+    const uint2 *const w1 = reinterpret_cast<const uint2 *>(smem_w + PK_W1);
+    const uint2 *const w2 = reinterpret_cast<const uint2 *>(smem_w + PK_W2);
+    const uint2 *const w3 = reinterpret_cast<const uint2 *>(smem_w + PK_W3);
+#pragma unroll 1
+    for (int tr = 0; tr < MW_TU; ++tr) {
+        const uint32_t cu = cu0 + (uint32_t)tr;
+        if (cu >= f.nu) break;                                            // warp-uniform
+        // RMS of column lane / 2, each lane of the pair one depth, in the order of the stencil
+        float rl;
+        {
+            const int row = lane >> 1;
+            const float *const sp = st + (lane & 1) * MW_PL + (tr * MW_SV + row) * 2;
+            float ss = 0.f;
+#pragma unroll
+            for (int du = 0; du < 3; ++du)
+#pragma unroll
+                for (int dv = 0; dv < 3; ++dv)
+#pragma unroll
+                    for (int qp = 0; qp < 3; ++qp) {
+                        const float2 v = *reinterpret_cast<const float2 *>(sp + qp * 2 * MW_PL + (du * MW_SV + dv) * 2);
+                        ss += v.x * v.x;
+                        ss += v.y * v.y;
+                    }
+            ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+            // columns outside the window: r = 0, no network term
+            const uint32_t cv = cv0 + (uint32_t)row;
+            rl = cv < f.nv && in_window(g, fi, f.u0 + cu, f.v0 + cv) ? sqrtf(ss * (1.0f / LBC_IN)) : 0.f;
+        }
+        // rows (columns of the face) gq and gq + 8
+        float r[2], inv[2];
+#pragma unroll
+        for (int hr = 0; hr < 2; ++hr) {
+            r[hr] = __shfl_sync(0xffffffffu, rl, 2 * (gq + 8 * hr));
+            inv[hr] = r[hr] > 0.f ? 1.0f / r[hr] : 0.f;
+        }
         // layer 1: [16 x 112] x [112 x 64]
         float acc[8][4];
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
-            const float b0 = __ldg(wb + PK_B1 + 8 * nt + 2 * tq), b1 = __ldg(wb + PK_B1 + 8 * nt + 2 * tq + 1);
+            const float b0 = wb[PK_B1 + 8 * nt + 2 * tq], b1 = wb[PK_B1 + 8 * nt + 2 * tq + 1];
             acc[nt][0] = b0; acc[nt][1] = b1; acc[nt][2] = b0; acc[nt][3] = b1;
         }
 #pragma unroll
         for (int ks = 0; ks < 7; ++ks) {
-            const float2 p0 = *reinterpret_cast<const float2 *>(xs + gq * XS + 16 * ks + 2 * tq);
-            const float2 p1 = *reinterpret_cast<const float2 *>(xs + (gq + 8) * XS + 16 * ks + 2 * tq);
-            const float2 p2 = *reinterpret_cast<const float2 *>(xs + gq * XS + 16 * ks + 8 + 2 * tq);
-            const float2 p3 = *reinterpret_cast<const float2 *>(xs + (gq + 8) * XS + 16 * ks + 8 + 2 * tq);
             uint32_t ah[4], al[4];
-            if (SPLIT) {
-                split_bf16(p0.x, p0.y, ah[0], al[0]);
-                split_bf16(p1.x, p1.y, ah[1], al[1]);
-                split_bf16(p2.x, p2.y, ah[2], al[2]);
-                split_bf16(p3.x, p3.y, ah[3], al[3]);
-            } else {
-                ah[0] = pack_bf16(p0.x, p0.y);
-                ah[1] = pack_bf16(p1.x, p1.y);
-                ah[2] = pack_bf16(p2.x, p2.y);
-                ah[3] = pack_bf16(p3.x, p3.y);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int m = 8 * ks + 4 * h + tq;
+                const int pos = m / 3, qp = m - 3 * pos, d = pos / 9, du = (pos - 9 * d) / 3, dv = pos - 9 * d - 3 * du;
+                const float *const sp = st + (qp * 2 + d) * MW_PL + ((tr + du) * MW_SV + gq + dv) * 2;
+#pragma unroll
+                for (int hr = 0; hr < 2; ++hr) {
+                    float2 v = make_float2(0.f, 0.f);                     // K padding 108..111
+                    if (8 * ks + 4 * h + 3 < 54 || m < 54) v = *reinterpret_cast<const float2 *>(sp + 16 * hr);
+                    v.x *= inv[hr];
+                    v.y *= inv[hr];
+                    if (SPLIT) split_bf16(v.x, v.y, ah[2 * h + hr], al[2 * h + hr]);
+                    else ah[2 * h + hr] = pack_bf16(v.x, v.y);
+                }
             }
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
-                const uint2 b = __ldg(w1 + (ks * 8 + nt) * 32 + lane);
+                const uint2 b = w1[(ks * 8 + nt) * 32 + lane];
                 mma_bf16(acc[nt], ah, b.x, b.y);
                 if (SPLIT) mma_bf16(acc[nt], al, b.x, b.y);
             }
@@ -943,14 +1000,14 @@ __global__ void __launch_bounds__(MMA_WARPS * 32) k_lbc_predict_mma(const LGrid 
         // layer 2: [16 x 64] x [64 x 64]
 #pragma unroll
         for (int nt = 0; nt < 8; ++nt) {
-            const float b0 = __ldg(wb + PK_B2 + 8 * nt + 2 * tq), b1 = __ldg(wb + PK_B2 + 8 * nt + 2 * tq + 1);
+            const float b0 = wb[PK_B2 + 8 * nt + 2 * tq], b1 = wb[PK_B2 + 8 * nt + 2 * tq + 1];
             acc[nt][0] = b0; acc[nt][1] = b1; acc[nt][2] = b0; acc[nt][3] = b1;
         }
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
 #pragma unroll
             for (int nt = 0; nt < 8; ++nt) {
-                const uint2 b = __ldg(w2 + (ks * 8 + nt) * 32 + lane);
+                const uint2 b = w2[(ks * 8 + nt) * 32 + lane];
                 mma_bf16(acc[nt], ah2[ks], b.x, b.y);
                 if (SPLIT) mma_bf16(acc[nt], al2[ks], b.x, b.y);
             }
@@ -958,12 +1015,12 @@ __global__ void __launch_bounds__(MMA_WARPS * 32) k_lbc_predict_mma(const LGrid 
         // layer 3: [16 x 64] x [64 x 8]
         float y[4];
         {
-            const float b0 = __ldg(wb + PK_B3 + 2 * tq), b1 = __ldg(wb + PK_B3 + 2 * tq + 1);
+            const float b0 = wb[PK_B3 + 2 * tq], b1 = wb[PK_B3 + 2 * tq + 1];
             y[0] = b0; y[1] = b1; y[2] = b0; y[3] = b1;
         }
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-            const uint2 b = __ldg(w3 + ks * 32 + lane);
+            const uint2 b = w3[ks * 32 + lane];
             mma_bf16(y, ah2[ks], b.x, b.y);
             if (SPLIT) mma_bf16(y, al2[ks], b.x, b.y);
         }
@@ -971,22 +1028,16 @@ __global__ void __launch_bounds__(MMA_WARPS * 32) k_lbc_predict_mma(const LGrid 
         if (tq < 3) {
 #pragma unroll
             for (int hr = 0; hr < 2; ++hr) {
-                const int row = gq + 8 * hr;
-                const uint32_t cv = cv0 + (uint32_t)row;
+                const uint32_t cv = cv0 + (uint32_t)(gq + 8 * hr);
                 if (cv < f.nv) {
-                    const uint32_t c = cu * f.nv + cv;
-                    const float r = rr[row];
-                    float *out = pred + (uint64_t)(f.col0 + c) * LBC_OUT + 2 * tq;
-                    out[0] = (r > 0.f ? y[2 * hr] * r : 0.f) + memory * out[0];
-                    out[1] = (r > 0.f ? y[2 * hr + 1] * r : 0.f) + memory * out[1];
+                    float *out = pred + (uint64_t)(f.col0 + cu * f.nv + cv) * LBC_OUT + 2 * tq;
+                    out[0] = (r[hr] > 0.f ? y[2 * hr] * r[hr] : 0.f) + memory * out[0];
+                    out[1] = (r[hr] > 0.f ? y[2 * hr + 1] * r[hr] : 0.f) + memory * out[1];
                 }
             }
         }
-        __syncwarp();
     }
 }
-
-constexpr size_t MMA_SMEM = (size_t)MMA_WARPS * (MMA_STAGE + 16 * XS + 16) * 4;
 
 // Levi-Civita sign of distinct (q, a, p): +1 for the cyclic orders of (0, 1, 2)
 __device__ __forceinline__ float lc(int q, int a) { return ((a - q + 3) % 3) == 1 ? 1.f : -1.f; }
@@ -998,44 +1049,60 @@ __device__ __forceinline__ int own_of(const LGrid &g, uint32_t col)
     return f;
 }
 
-// one thread per outer cell: every learned face through the cell adds its term, faces in order
-__global__ void k_lbc_fix(const LGrid g, int fields, const float *pred, float *E, float *H, const float *ce,
-                          const float *cm, float dt)
+// One thread per outer cell: every learned face of the side (E fix-up: side 0, H fix-up: side 1) through
+// the cell adds its term, faces in order. A cell lies on at most one such face per axis, so what its
+// terms need is requested at once (8.7 us a fix-up of a 203x177x61 grid when each face's values were
+// loaded after the one before, and the field after them).
+struct FixFaces {
+    uint32_t col0[3], nv[3];                                 // per axis: the face's first column and row length
+    int32_t on[3];
+};
+
+template <bool EFIX>
+__global__ void __launch_bounds__(128) k_lbc_fix(const __grid_constant__ LGrid g, const __grid_constant__ FixFaces ff,
+                                                 const float *pred, float *P, const float *Q, const float *coef, float dt)
 {
     const uint32_t col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= g.nown) return;
     const LFace &o = g.own[own_of(g, col)];
     const uint32_t k = col - o.col0;
-    uint32_t c[3];
-    {
-        const int a = o.axis, ua = a == 0 ? 1 : 0, va = a == 2 ? 1 : 2;
-        c[a] = o.side ? g.s[a] - 1u : 0u;
-        c[ua] = o.u0 + k / o.nv;
-        c[va] = o.v0 + k % o.nv;
-    }
+    const uint32_t cu = o.u0 + k / o.nv, cv = o.v0 + k % o.nv, cw = o.side ? g.s[o.axis] - 1u : 0u;
+    const uint32_t c[3] = {o.axis == 0 ? cw : cu, o.axis == 0 ? cu : o.axis == 1 ? cw : cv, o.axis == 2 ? cw : cv};
     const uint64_t st[3] = {(uint64_t)g.s[1] * g.s[2], g.s[2], 1};
     const uint64_t i = c[0] * st[0] + c[1] * st[1] + c[2];
-    float dE[3] = {0.f, 0.f, 0.f}, dH[3] = {0.f, 0.f, 0.f};
-    for (int fi = 0; fi < g.nface; ++fi) {
-        const LFace &f = g.face[fi];
-        const int a = f.axis, ua = a == 0 ? 1 : 0, va = a == 2 ? 1 : 2;
-        if (c[a] != (f.side ? g.s[a] - 1u : 0u)) continue;
-        const float *gp = pred + ((uint64_t)f.col0 + (uint64_t)c[ua] * f.nv + c[va]) * LBC_OUT;
+    bool on[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) on[a] = ff.on[a] && c[a] == (EFIX ? 0u : g.s[a] - 1u);
+    if (!(on[0] || on[1] || on[2])) return;
+    grid_dependency_sync();
+    float ghost[3][3], wrapped[3][3], co[3], p[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        co[q] = coef ? coef[q * g.N + i] : dt;
+        p[q] = P[q * g.N + i];
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (!on[a]) continue;
+        const float *gp = pred + ((uint64_t)ff.col0[a] + (uint64_t)c[a == 0 ? 1 : 0] * ff.nv[a] + c[a == 2 ? 1 : 2]) * LBC_OUT;
         // the wrapped neighbour: index s_a - 1 (side 0) or 0 (side 1) along a
-        const uint64_t j = f.side ? i - (uint64_t)(g.s[a] - 1u) * st[a] : i + (uint64_t)(g.s[a] - 1u) * st[a];
+        const uint64_t j = EFIX ? i + (uint64_t)(g.s[a] - 1u) * st[a] : i - (uint64_t)(g.s[a] - 1u) * st[a];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
             if (q == a) continue;
-            const int p = 3 - a - q;
-            if (f.side == 0 && (fields & LBC_FIX_E)) dE[q] -= lc(q, a) * (gp[3 + p] - H[p * g.N + j]);
-            if (f.side == 1 && (fields & LBC_FIX_H)) dH[q] -= lc(q, a) * (gp[p] - E[p * g.N + j]);
+            ghost[a][q] = gp[(EFIX ? 3 : 0) + q];
+            wrapped[a][q] = Q[q * g.N + j];
         }
     }
+    float d[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-        if ((fields & LBC_FIX_E) && dE[q] != 0.f) E[q * g.N + i] += ce[q * g.N + i] * dE[q];
-        if ((fields & LBC_FIX_H) && dH[q] != 0.f) H[q * g.N + i] += (cm ? cm[q * g.N + i] : dt) * dH[q];
-    }
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            if (q != a && on[a]) d[q] -= lc(q, a) * (ghost[a][3 - a - q] - wrapped[a][3 - a - q]);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        if (d[q] != 0.f) P[q * g.N + i] = p[q] + co[q] * d[q];
 }
 
 }  // namespace
@@ -1259,7 +1326,7 @@ cudaError_t launch_lbc_pack(const float *P, uint32_t *out, cudaStream_t st)
 }
 
 cudaError_t launch_lbc_predict(const LGrid &g, int side, int precision, float memory, const void *W, const float *E,
-                               const float *H, float *pred, cudaStream_t st)
+                               const float *H, float *pred, cudaStream_t st, bool pdl)
 {
     if (!g.ncol) return cudaSuccess;
     uint32_t maxc = 0;
@@ -1282,28 +1349,40 @@ cudaError_t launch_lbc_predict(const LGrid &g, int side, int precision, float me
         return cudaGetLastError();
     }
     const int split = precision == LBC_BF16X2 ? 1 : 0;
-    const cudaError_t e = split ? smem_opt_in((const void *)k_lbc_predict_mma<true>, SMEM_MMA_SPLIT, MMA_SMEM)
-                                : smem_opt_in((const void *)k_lbc_predict_mma<false>, SMEM_MMA, MMA_SMEM);
+    const cudaError_t e = split ? smem_opt_in((const void *)k_lbc_predict_mma<true>, SMEM_MMA_SPLIT, MW_SMEM)
+                                : smem_opt_in((const void *)k_lbc_predict_mma<false>, SMEM_MMA, MW_SMEM);
     if (e != cudaSuccess) return e;
-    uint32_t maxj = 0;
-    for (int f = 0; f < g.nface; ++f) {
-        const uint32_t nj = ((g.face[f].nu + MMA_TU - 1) / MMA_TU) * ((g.face[f].nv + 15) / 16);
-        maxj = nj > maxj ? nj : maxj;
+    // the blocks of every face that is asked for, side by side
+    MFirst first;
+    uint32_t blocks = 0;
+    for (int f = 0; f < 7; ++f) {
+        first.block[f] = blocks;
+        if (f < g.nface && (side < 0 || g.face[f].side == side))
+            blocks += ((g.face[f].nu + MW_TU - 1) / MW_TU * ((g.face[f].nv + 15) / 16) + MW_WARPS - 1) / MW_WARPS;
     }
-    const dim3 gi((maxj + MMA_WARPS - 1) / MMA_WARPS, (unsigned)g.nface, 1);
-    if (split)
-        k_lbc_predict_mma<true><<<gi, MMA_WARPS * 32, MMA_SMEM, st>>>(g, side, memory, (const uint32_t *)W, E, H, pred);
-    else
-        k_lbc_predict_mma<false><<<gi, MMA_WARPS * 32, MMA_SMEM, st>>>(g, side, memory, (const uint32_t *)W, E, H, pred);
-    return cudaGetLastError();
+    if (!blocks) return cudaSuccess;
+    return launch_dependent_smem(split ? k_lbc_predict_mma<true> : k_lbc_predict_mma<false>, dim3(blocks, 1, 1),
+                                 (unsigned)MW_WARPS * 32u, MW_SMEM, st, pdl, g, first, memory, (const uint32_t *)W, E, H, pred);
 }
 
 cudaError_t launch_lbc_fix(const LGrid &g, int fields, const float *pred, float *E, float *H, const float *ce,
-                           const float *cm, float dt, cudaStream_t st)
+                           const float *cm, float dt, cudaStream_t st, bool pdl)
 {
     if (!g.nown) return cudaSuccess;
-    k_lbc_fix<<<(g.nown + 127) / 128, 128, 0, st>>>(g, fields, pred, E, H, ce, cm, dt);
-    return cudaGetLastError();
+    const bool e = fields == LBC_FIX_E;
+    FixFaces ff = {};
+    for (int f = 0; f < g.nface; ++f) {
+        const LFace &lf = g.face[f];
+        if (lf.side != (e ? 0 : 1)) continue;
+        ff.on[lf.axis] = 1;
+        ff.col0[lf.axis] = lf.col0;
+        ff.nv[lf.axis] = lf.nv;
+    }
+    // nothing to do; and a launch without a thread that waits for the kernel before it could end first
+    if (!ff.on[0] && !ff.on[1] && !ff.on[2]) return cudaSuccess;
+    const dim3 grid((g.nown + 127) / 128, 1, 1);
+    return e ? launch_dependent_smem(k_lbc_fix<true>, grid, 128u, 0, st, pdl, g, ff, pred, E, (const float *)H, ce, dt)
+             : launch_dependent_smem(k_lbc_fix<false>, grid, 128u, 0, st, pdl, g, ff, pred, H, (const float *)E, cm, dt);
 }
 
 }  // namespace fdtd

@@ -87,7 +87,7 @@ cudaError_t launch_lbc_pack(const float *P, uint32_t *out, cudaStream_t st);
 // pred (the previous ghosts); W: float32 parameters [6][LBC_NPARAM] (LBC_F32) or packed words
 // [6][LBC_PACK_WORDS] (LBC_BF16, LBC_BF16X2), face = 2 * axis + side
 cudaError_t launch_lbc_predict(const LGrid &g, int side, int precision, float memory, const void *W, const float *E,
-                               const float *H, float *pred, cudaStream_t st);
+                               const float *H, float *pred, cudaStream_t st, bool pdl = false);
 // The plain update of a grid whose edges wrap reads, across a learned side-0 face of axis a,
 // H_p at index s_a - 1 for E_q at index 0 (q, a, p distinct), and across a learned side-1 face
 // E_p at index 0 for H_q at index s_a - 1. k_lbc_fix replaces those neighbours by the predicted
@@ -97,6 +97,6 @@ cudaError_t launch_lbc_predict(const LGrid &g, int side, int precision, float me
 constexpr int LBC_FIX_E = 1;
 constexpr int LBC_FIX_H = 2;
 cudaError_t launch_lbc_fix(const LGrid &g, int fields, const float *pred, float *E, float *H, const float *ce,
-                           const float *cm, float dt, cudaStream_t st);
+                           const float *cm, float dt, cudaStream_t st, bool pdl = false);
 
 }  // namespace fdtd

@@ -50,11 +50,23 @@ static LGrid plan_grid(const FdtdPlan *p)
     return lbc_grid_window(s, p->lbc_mask, lo, hi);
 }
 
+bool lbc_holds_source(const FdtdPlan *p, const FdtdPointSources *src)
+{
+    const uint32_t s[3] = {p->sx, p->sy, p->sz};
+    for (int k = 0; src && p->lbc_mask && k < src->n; ++k) {
+        const uint64_t cell = (uint64_t)src->index[k] % p->N;
+        const uint32_t c[3] = {(uint32_t)(cell / p->syz), (uint32_t)(cell % p->syz / p->sz), (uint32_t)(cell % p->sz)};
+        for (int f = 0; f < 6; ++f)
+            if (p->lbc_mask >> f & 1 && c[f / 2] == (f & 1 ? s[f / 2] - 1u : 0u)) return true;
+    }
+    return false;
+}
+
 int lbc_before_e(const FdtdPlan *p, const FdtdBuffers *b, const void *H, cudaStream_t st)
 {
     if (!p->lbc_mask) return FDTD_OK;
     return check_cuda(launch_lbc_predict(plan_grid(p), -1, p->lbc_precision, p->lbc_memory, p->lbc_w,
-                                         (const float *)b->E, (const float *)H, p->lbc_pred, st),
+                                         (const float *)b->E, (const float *)H, p->lbc_pred, st, p->pdl != 0),
                       "lbc predict launch");
 }
 
@@ -62,14 +74,14 @@ int lbc_after_e(const FdtdPlan *p, const FdtdBuffers *b, const void *H, cudaStre
 {
     if (!p->lbc_mask) return FDTD_OK;
     return check_cuda(launch_lbc_fix(plan_grid(p), LBC_FIX_E, p->lbc_pred, (float *)b->E, (float *)H,
-                                     (const float *)b->ce, nullptr, (float)p->d.dt, st), "lbc fix launch");
+                                     (const float *)b->ce, nullptr, (float)p->d.dt, st, p->pdl != 0), "lbc fix launch");
 }
 
 int lbc_after_h(const FdtdPlan *p, const FdtdBuffers *b, void *H, cudaStream_t st)
 {
     if (!p->lbc_mask) return FDTD_OK;
     return check_cuda(launch_lbc_fix(plan_grid(p), LBC_FIX_H, p->lbc_pred, (float *)b->E, (float *)H, nullptr,
-                                     p->d.has_mu ? (const float *)b->cm : nullptr, (float)p->d.dt, st),
+                                     p->d.has_mu ? (const float *)b->cm : nullptr, (float)p->d.dt, st, p->pdl != 0),
                       "lbc fix launch");
 }
 

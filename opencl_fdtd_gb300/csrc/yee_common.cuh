@@ -50,13 +50,13 @@ __device__ __forceinline__ void grid_dependency_sync()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// Launches kern<<<g, block, smem, st>>>(arg), with programmatic stream serialization when pdl.
-template <typename K>
-inline cudaError_t launch_dependent(void (*kern)(K), dim3 g, unsigned block, cudaStream_t st,
-                                    bool pdl, const K &arg, size_t smem = 0)
+// Launches kern<<<g, block, smem, st>>>(args...), with programmatic stream serialization when pdl.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent_smem(void (*kern)(P...), dim3 g, unsigned block, size_t smem, cudaStream_t st, bool pdl,
+                                         const A &...args)
 {
     if (!pdl) {
-        kern<<<g, block, smem, st>>>(arg);
+        kern<<<g, block, smem, st>>>(args...);
         return cudaGetLastError();
     }
     cudaLaunchConfig_t cfg = {};
@@ -69,7 +69,13 @@ inline cudaError_t launch_dependent(void (*kern)(K), dim3 g, unsigned block, cud
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, arg);
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+template <typename K>
+inline cudaError_t launch_dependent(void (*kern)(K), dim3 g, unsigned block, cudaStream_t st, bool pdl, const K &arg)
+{
+    return launch_dependent_smem(kern, g, block, 0, st, pdl, arg);
 }
 
 // The CPML faces of one axis for one update: coefficient tables [n/p][p0,p1,p2], the auxiliary
