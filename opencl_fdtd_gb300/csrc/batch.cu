@@ -536,8 +536,8 @@ __global__ void __launch_bounds__(BATCH_THREADS, BATCH_PERSIST_BLOCKS) k_batch(c
 // what counts is resident warps and a march without reloads: with the next plane loaded ahead (three
 // blocks per SM) and the descriptor's pointers, limits and source list read again for every plane, the
 // march was 261 (E) and 220 (H) instructions per warp and plane and a step of 8 variants (14.7 M cells)
-// took 0.389 ms in float32, 0.420 in bfloat16 without exponents and 0.619 with; now 184 and 163 and 0.337,
-// 0.304 and 0.417. E in float32 spills 56 bytes at five blocks and still gains (0.208 to 0.184 ms, four to
+// took 0.389 ms in float32, 0.420 in bfloat16 without exponents and 0.619 with; now 184 and 163 and 0.331,
+// 0.298 and 0.407. E in float32 spills 56 bytes at five blocks and still gains (0.208 to 0.184 ms, four to
 // five); H loses there (0.146 to 0.163), and so does E with tile exponents. Six blocks: 0.211 and 0.174.
 // The H launch advances the step counter.
 template <int ST>
@@ -547,6 +547,7 @@ template <int ST>
 __global__ void __launch_bounds__(BATCH_THREADS, batch_e_blocks<ST>()) k_batch_e(const BatchK k)
 {
     const int4 tl = k.tiles[blockIdx.x];
+    grid_dependency_sync();
     batch_e_tile<ST, true>(k.vars[tl.x], tl, *k.step, k.rows);
 }
 
@@ -554,6 +555,7 @@ template <int ST>
 __global__ void __launch_bounds__(BATCH_THREADS, 4) k_batch_h(const BatchK k)
 {
     const int4 tl = k.tiles[blockIdx.x];
+    grid_dependency_sync();
     batch_h_tile<ST, true>(k.vars[tl.x], tl);
     // the E launch of this step, which reads the counter, has completed
     if (blockIdx.x == 0 && threadIdx.x == 0) *k.step += 1;
@@ -630,10 +632,13 @@ template <int ST>
 cudaError_t launch_batch_steps(const BatchK &k, cudaStream_t st)
 {
     for (int t = 0; t < k.nsteps; ++t) {
-        k_batch_e<ST><<<k.ntiles, BATCH_THREADS, 0, st>>>(k);
-        k_batch_h<ST><<<k.ntiles, BATCH_THREADS, 0, st>>>(k);
+        // a block's launch overlaps the tail of the launch before: 8 variants of 1.8 M cells 0.337 to 0.331 ms
+        // a step, two of 0.1 M 19 to 14 us (the set-up before the wait as well: 0.355 ms and 12 us)
+        cudaError_t e = launch_dependent(k_batch_e<ST>, dim3(k.ntiles, 1, 1), BATCH_THREADS, st, true, k);
+        if (e == cudaSuccess) e = launch_dependent(k_batch_h<ST>, dim3(k.ntiles, 1, 1), BATCH_THREADS, st, true, k);
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_batch_encode(int store, const BVar &v, int field, const float *src, cudaStream_t st)
