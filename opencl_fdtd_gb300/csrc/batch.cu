@@ -163,8 +163,8 @@ struct BELoad {
     float xu, xv, yu, yv, zu, zv;
 };
 
-template <int ST, bool KEEP>
-__device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
+template <int ST, bool KEEP, bool LATE = false>
+__device__ void batch_e_tile(const BVar &v, int4 tl, const int64_t *counter, int t, int64_t rows)
 {
     using SS = Store<ST>;
     using T = typename SS::T;
@@ -196,6 +196,8 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, int64_t step, int64_t rows)
     const bool xf = xa < (uint32_t)Tn || (Tp && xb > sx - (uint32_t)Tp);   // an x face covers a plane of the tile
     // a point source, a monitor point in this tile (block-uniform)
     bool srcs = false, mons = false;
+    if (LATE) grid_dependency_sync();
+    const int64_t step = *counter + t;
     if (step < rows) {
         for (int s = 0; s < v.nsrc; ++s)
             srcs |= v.src_j[s] / BATCH_THREADS == jb && v.src_x[s] >= xa && v.src_x[s] < xb;
@@ -342,7 +344,7 @@ struct BHLoad {
     float xu, xv, yu, yv, zu, zv;
 };
 
-template <int ST, bool KEEP>
+template <int ST, bool KEEP, bool LATE = false>
 __device__ void batch_h_tile(const BVar &v, int4 tl)
 {
     using SS = Store<ST>;
@@ -370,6 +372,7 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
     const BAxis &ax0 = v.ax[0];
     const int Tn = ax0.Tn, Tp = ax0.Tp;
     const bool xf = xa < (uint32_t)Tn || (Tp && xb > sx - (uint32_t)Tp);
+    if (LATE) grid_dependency_sync();
 
     auto load = [&](uint32_t x, uint32_t i) {
         BHLoad<T> q;
@@ -483,10 +486,10 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
 }
 
 template <int ST>
-__device__ __forceinline__ void batch_e_item(const BatchK &k, uint32_t ti, int64_t step)
+__device__ __forceinline__ void batch_e_item(const BatchK &k, uint32_t ti, int t)
 {
     const int4 tl = k.tiles[ti];
-    batch_e_tile<ST, false>(k.vars[tl.x], tl, step, k.rows);
+    batch_e_tile<ST, false>(k.vars[tl.x], tl, k.step, t, k.rows);
 }
 
 template <int ST>
@@ -516,11 +519,10 @@ __global__ void __launch_bounds__(BATCH_THREADS, BATCH_PERSIST_BLOCKS) k_batch(c
     cg::grid_group grid = cg::this_grid();
     const int64_t step0 = *k.step;
     for (int t = 0; t < k.nsteps; ++t) {
-        const int64_t step = step0 + t;
         // half-step 2t uses counter 0, 2t + 1 counter 1; a counter is cleared right after the
         // grid barrier that ends its half-step, two barriers before its next use
         for (uint32_t ti = next_tile(&k.work[0], &item); ti < k.ntiles; ti = next_tile(&k.work[0], &item))
-            batch_e_item<ST>(k, ti, step);
+            batch_e_item<ST>(k, ti, t);
         grid.sync();
         if (blockIdx.x == 0 && threadIdx.x == 0) k.work[0] = 0u;
         for (uint32_t ti = next_tile(&k.work[1], &item); ti < k.ntiles; ti = next_tile(&k.work[1], &item))
@@ -539,7 +541,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, BATCH_PERSIST_BLOCKS) k_batch(c
 // took 0.389 ms in float32, 0.420 in bfloat16 without exponents and 0.619 with; now 184 and 163 and 0.331,
 // 0.298 and 0.407. E in float32 spills 56 bytes at five blocks and still gains (0.208 to 0.184 ms, four to
 // five); H loses there (0.146 to 0.163), and so does E with tile exponents. Six blocks: 0.211 and 0.174.
-// The H launch advances the step counter.
+// A call's last H launch advances the step counter.
 template <int ST>
 constexpr int batch_e_blocks() { return Store<ST>::scaled ? 4 : 5; }
 
@@ -548,7 +550,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, batch_e_blocks<ST>()) k_batch_e
 {
     const int4 tl = k.tiles[blockIdx.x];
     grid_dependency_sync();
-    batch_e_tile<ST, true>(k.vars[tl.x], tl, *k.step, k.rows);
+    batch_e_tile<ST, true>(k.vars[tl.x], tl, k.step, k.t, k.rows);
 }
 
 template <int ST>
@@ -557,8 +559,27 @@ __global__ void __launch_bounds__(BATCH_THREADS, 4) k_batch_h(const BatchK k)
     const int4 tl = k.tiles[blockIdx.x];
     grid_dependency_sync();
     batch_h_tile<ST, true>(k.vars[tl.x], tl);
-    // the E launch of this step, which reads the counter, has completed
-    if (blockIdx.x == 0 && threadIdx.x == 0) *k.step += 1;
+    // the last launch of a call: the E launches, which read the counter, have completed
+    if (k.advance && blockIdx.x == 0 && threadIdx.x == 0) *k.step += k.advance;
+}
+
+// One variant per launch, its descriptor among the kernel's arguments (five blocks per SM: 0.317 ms a step
+// instead of 0.306); the set-up stands before the wait (0.297).
+constexpr int BATCH_ONE_BLOCKS = 4;
+
+__global__ void __launch_bounds__(BATCH_THREADS, BATCH_ONE_BLOCKS) k_batch_e1(const __grid_constant__ BatchOne k)
+{
+    const uint32_t xa = blockIdx.y * k.xchunk;
+    const int4 tl = make_int4(0, (int)xa, (int)min(xa + k.xchunk, k.v.sx), (int)blockIdx.x);
+    batch_e_tile<BATCH_F32, true, true>(k.v, tl, k.step, k.t, k.rows);
+}
+
+__global__ void __launch_bounds__(BATCH_THREADS, BATCH_ONE_BLOCKS) k_batch_h1(const __grid_constant__ BatchOne k)
+{
+    const uint32_t xa = blockIdx.y * k.xchunk;
+    const int4 tl = make_int4(0, (int)xa, (int)min(xa + k.xchunk, k.v.sx), (int)blockIdx.x);
+    batch_h_tile<BATCH_F32, true, true>(k.v, tl);
+    if (k.advance && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *k.step += k.advance;
 }
 
 // one block per (column jb of BATCH_THREADS cells, plane x): float32 <-> storage, all three
@@ -629,16 +650,45 @@ cudaError_t launch_batch(const BatchK &k, int blocks, cudaStream_t st)
 }
 
 template <int ST>
-cudaError_t launch_batch_steps(const BatchK &k, cudaStream_t st)
+cudaError_t launch_batch_steps(const BatchK &kk, const BatchGroup *groups, int n, cudaStream_t st)
 {
-    for (int t = 0; t < k.nsteps; ++t) {
-        // a block's launch overlaps the tail of the launch before: 8 variants of 1.8 M cells 0.337 to 0.331 ms
-        // a step, two of 0.1 M 19 to 14 us (the set-up before the wait as well: 0.355 ms and 12 us)
-        cudaError_t e = launch_dependent(k_batch_e<ST>, dim3(k.ntiles, 1, 1), BATCH_THREADS, st, true, k);
-        if (e == cudaSuccess) e = launch_dependent(k_batch_h<ST>, dim3(k.ntiles, 1, 1), BATCH_THREADS, st, true, k);
-        if (e != cudaSuccess) return e;
+    BatchK k = kk;
+    BatchOne o;
+    o.step = k.step;
+    o.rows = k.rows;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    for (int g = 0; g < n; ++g) {
+        const BVar *const one = groups[g].one;
+        dim3 grid(k.ntiles, 1, 1);
+        if (one) {
+            // as the per-update kernels: 8 planes, or the fewest with which all blocks are resident
+            o.v = *one;
+            o.xchunk = groups[g].xchunk ? groups[g].xchunk : 1u;
+            while (!groups[g].xchunk && o.xchunk < 8u &&
+                   (uint64_t)one->njb * ((one->sx + o.xchunk - 1) / o.xchunk) > (uint64_t)sms * BATCH_ONE_BLOCKS)
+                ++o.xchunk;
+            grid = dim3(one->njb, (one->sx + o.xchunk - 1) / o.xchunk, 1);
+        }
+        for (int t = 0; t < kk.nsteps && e == cudaSuccess; ++t) {
+            const int advance = g == n - 1 && t == kk.nsteps - 1 ? kk.nsteps : 0;
+            k.t = o.t = t;
+            k.advance = o.advance = advance;
+            // a block's launch overlaps the tail of the launch before: 8 variants of 1.8 M cells 0.337 to 0.331
+            // ms a step, two of 0.1 M 19 to 14 us (the set-up before the wait as well: 0.355 ms and 12 us)
+            if (one) {
+                if constexpr (ST == BATCH_F32) {             // launched_alone
+                    e = launch_dependent(k_batch_e1, grid, BATCH_THREADS, st, true, o);
+                    if (e == cudaSuccess) e = launch_dependent(k_batch_h1, grid, BATCH_THREADS, st, true, o);
+                }
+            } else {
+                e = launch_dependent(k_batch_e<ST>, grid, BATCH_THREADS, st, true, k);
+                if (e == cudaSuccess) e = launch_dependent(k_batch_h<ST>, grid, BATCH_THREADS, st, true, k);
+            }
+        }
     }
-    return cudaSuccess;
+    return e;
 }
 
 cudaError_t launch_batch_encode(int store, const BVar &v, int field, const float *src, cudaStream_t st)
@@ -664,14 +714,14 @@ cudaError_t launch_batch_decode(int store, const BVar &v, int field, float *dst,
 template cudaError_t launch_batch<BATCH_F32>(const BatchK &, int, cudaStream_t);
 template cudaError_t launch_batch<BATCH_BF16>(const BatchK &, int, cudaStream_t);
 template cudaError_t launch_batch<BATCH_F16>(const BatchK &, int, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_F32>(const BatchK &, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_BF16>(const BatchK &, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_F16>(const BatchK &, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_F32>(const BatchK &, const BatchGroup *, int, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_BF16>(const BatchK &, const BatchGroup *, int, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_F16>(const BatchK &, const BatchGroup *, int, cudaStream_t);
 template int batch_max_blocks_per_sm<BATCH_F32>();
 template int batch_max_blocks_per_sm<BATCH_BF16>();
 template int batch_max_blocks_per_sm<BATCH_F16>();
 template cudaError_t launch_batch<BATCH_BF16U>(const BatchK &, int, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_BF16U>(const BatchK &, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_BF16U>(const BatchK &, const BatchGroup *, int, cudaStream_t);
 template int batch_max_blocks_per_sm<BATCH_BF16U>();
 
 }  // namespace fdtd

@@ -57,6 +57,7 @@ struct BatchK {
     int32_t nsteps;
     int64_t *step;              // device step counter: read at start, advanced by nsteps at end
     int64_t rows;               // rows of the source and series arrays
+    int32_t t, advance;         // launches: the step within the call, what the launch adds to the step counter
     uint32_t *work;             // persistent schedule: tiles handed out so far in the current
                                 // half-step, two counters used alternately (zero between launches)
 };
@@ -65,9 +66,23 @@ template <int ST>
 cudaError_t launch_batch(const BatchK &k, int blocks, cudaStream_t st);
 template <int ST>
 int batch_max_blocks_per_sm();
-// nsteps x (one launch of every tile's E update, one of every tile's H update)
+// The launches of a half-step: a variant of its own (one; planes per thread, 0: chosen by the launcher), or
+// the tiles of every variant that has none.
+struct BatchGroup {
+    const BVar *one;
+    uint32_t xchunk;
+};
+struct BatchOne {
+    BVar v;
+    int64_t *step;
+    int64_t rows;
+    uint32_t xchunk;
+    int32_t t, advance;
+};
+
+// For each group of variants: nsteps x (one launch of its E update, one of its H update)
 template <int ST>
-cudaError_t launch_batch_steps(const BatchK &k, cudaStream_t st);
+cudaError_t launch_batch_steps(const BatchK &k, const BatchGroup *groups, int n, cudaStream_t st);
 
 // f32 <-> storage of one field of one variant, choosing the tile exponents (encode)
 cudaError_t launch_batch_encode(int store, const BVar &v, int field, const float *src, cudaStream_t st);

@@ -25,6 +25,9 @@ struct FdtdBatch {
     BVar *vars = nullptr;        // device copy
     int4 *tiles = nullptr;       // device tile list
     uint32_t ntiles = 0;
+    std::vector<BatchGroup> groups;    // the launches of a half-step (build_tiles)
+    uint32_t shared = 0;               // tiles of the variants that share launches
+    bool tuned = false;
     int64_t *step = nullptr;     // device step counter
     uint32_t *work = nullptr;    // persistent schedule's two tile counters
 };
@@ -46,15 +49,27 @@ uint32_t default_xchunk(const FdtdBatch *b)
     return planes >= 8 * slots ? 8u : (uint32_t)(planes / slots > 1 ? planes / slots : 1);
 }
 
+// Whether a variant's updates are launches of their own in the launches schedule: the descriptor is then
+// among the kernel's arguments, which spares the march's registers and reloads, at the price of a tail per
+// launch. Float32: 8 variants of 1.8 M cells 0.331 to 0.297 ms a step, 3 of 0.95 M 87 to 64 us, 6 of 0.5 M 86
+// to 82, but 6 of 0.2 M 36 to 55. With 16-bit storage the tiles spill less and it lost (0.298 to 0.303 ms).
+bool launched_alone(const BVar &h, int storage) { return storage == BATCH_F32 && h.N >= 500000; }
+
 int build_tiles(FdtdBatch *b)
 {
     std::vector<int4> t;
-    for (size_t v = 0; v < b->host.size(); ++v) {
-        const BVar &h = b->host[v];
-        for (uint32_t x0 = 0; x0 < h.sx; x0 += b->xchunk)
-            for (uint32_t jb = 0; jb < h.njb; ++jb)
-                t.push_back(make_int4((int)v, (int)x0, (int)(x0 + b->xchunk < h.sx ? x0 + b->xchunk : h.sx), (int)jb));
-    }
+    b->groups.clear();
+    // the variants that share launches first
+    for (int alone = 0; alone < 2; ++alone)
+        for (size_t v = 0; v < b->host.size(); ++v) {
+            const BVar &h = b->host[v];
+            if (launched_alone(h, b->storage) != (alone != 0)) continue;
+            if (alone || b->groups.empty()) b->groups.push_back({alone ? &h : nullptr, b->tuned ? b->xchunk : 0u});
+            for (uint32_t x0 = 0; x0 < h.sx; x0 += b->xchunk)
+                for (uint32_t jb = 0; jb < h.njb; ++jb)
+                    t.push_back(make_int4((int)v, (int)x0, (int)(x0 + b->xchunk < h.sx ? x0 + b->xchunk : h.sx), (int)jb));
+            if (!alone) b->shared = (uint32_t)t.size();
+        }
     if (b->tiles) cudaFree(b->tiles);
     b->tiles = nullptr;
     int rc = check_cuda(cudaMalloc(&b->tiles, t.size() * sizeof(int4)), "cudaMalloc(batch tiles)");
@@ -222,8 +237,9 @@ int fdtd_batch_tune(FdtdBatch *b, int32_t xchunk, int32_t blocks_per_sm)
     if (xchunk < 1 || xchunk > 4096) return fail(FDTD_ERR_INVALID, "xchunk must be in [1, 4096]");
     if (blocks_per_sm < 0 || blocks_per_sm > 32) return fail(FDTD_ERR_INVALID, "blocks_per_sm must be in [0, 32]");
     b->blocks_per_sm = blocks_per_sm;
-    if ((uint32_t)xchunk != b->xchunk) {
+    if ((uint32_t)xchunk != b->xchunk || !b->tuned) {
         b->xchunk = (uint32_t)xchunk;
+        b->tuned = true;
         return build_tiles(b);
     }
     return FDTD_OK;
@@ -248,13 +264,17 @@ int fdtd_batch_run(FdtdBatch *b, void *stream, int32_t nsteps)
     k.step = b->step;
     k.rows = b->rows;
     k.work = b->work;
+    k.t = k.advance = 0;
     cudaStream_t st = (cudaStream_t)stream;
     cudaError_t e;
     if (b->schedule == FDTD_BATCH_LAUNCHES) {
-        if (b->storage == BATCH_BF16) e = launch_batch_steps<BATCH_BF16>(k, st);
-        else if (b->storage == BATCH_F16) e = launch_batch_steps<BATCH_F16>(k, st);
-        else if (b->storage == BATCH_BF16U) e = launch_batch_steps<BATCH_BF16U>(k, st);
-        else e = launch_batch_steps<BATCH_F32>(k, st);
+        k.ntiles = b->shared;
+        const BatchGroup *const groups = b->groups.data();
+        const int ng = (int)b->groups.size();
+        if (b->storage == BATCH_BF16) e = launch_batch_steps<BATCH_BF16>(k, groups, ng, st);
+        else if (b->storage == BATCH_F16) e = launch_batch_steps<BATCH_F16>(k, groups, ng, st);
+        else if (b->storage == BATCH_BF16U) e = launch_batch_steps<BATCH_BF16U>(k, groups, ng, st);
+        else e = launch_batch_steps<BATCH_F32>(k, groups, ng, st);
         return check_cuda(e, "batch launch");
     }
     if (b->storage == BATCH_BF16) e = launch_batch<BATCH_BF16>(k, per * nsm, st);

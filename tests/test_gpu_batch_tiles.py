@@ -62,3 +62,33 @@ def test_tiles_equal_single_variants(storage, dx, schedule):
             assert torch.equal(ref.E, alone.E) and torch.equal(ref.H, alone.H)
         assert torch.equal(together[i].E, alone.E) and torch.equal(together[i].H, alone.H)
         assert numpy.array_equal(series[i], one)
+
+
+@pytest.mark.parametrize("dx,chunk", [(1.0, None), (0.5, 3), (1.0, 64)])
+def test_large_variants_launched_alone(dx, chunk):
+    """From half a million cells on a float32 variant has launches of its own; beside smaller ones, which
+    share theirs."""
+    from opencl_fdtd_gb300 import Simulation
+    from opencl_fdtd_gb300.batch import BatchSimulation
+    cases = [((12, 10, 9), (2, 0, 3)), ((84, 77, 79), (5, 4, 8)), ((7, 85, 3), (1, 5, 1)), ((65, 64, 125), (0, 8, 1))]
+    kws = [_kw(s, t, 20 + i, dx) for i, (s, t) in enumerate(cases)]
+    pts = [_points(s) for s, _ in cases]
+    n = 5
+    src = [[(p, [math.sin(0.3 * t + k) for t in range(n)]) for k, p in enumerate(ps)] for ps in pts]
+    sims = [Simulation(**copy.deepcopy(kw)) for kw in kws]
+    b = BatchSimulation(sims, storage="f32", sources=src, monitors=pts, steps=n)
+    if chunk:
+        b.tune(xchunk=chunk)
+    b.run(2)
+    b.run(3)
+    torch.cuda.synchronize()
+    assert b.step_counter() == n
+    for kw, sim, ps, ss, ser in zip(kws, sims, pts, src, b.series):
+        ref = Simulation(**copy.deepcopy(kw))
+        m = ref.dft_monitor([(i // ref.N, numpy.unravel_index(i % ref.N, ref.shape)) for i in ps], ())
+        ref.run(n, point_sources=ss, monitor=m, path="plain")
+        assert torch.equal(ref.E, sim.E) and torch.equal(ref.H, sim.H)
+        for f in "EH":
+            for (u, v), (p, q) in zip(ref.psi[f], sim.psi[f]):
+                assert torch.equal(u, p) and torch.equal(v, q)
+        assert numpy.array_equal(m.series(), ser.cpu().numpy())
