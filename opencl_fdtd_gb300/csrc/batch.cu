@@ -185,6 +185,7 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, const int64_t *counter, int
     const uint32_t dmz = z ? 0xffffffffu : sz - 1u;
     const uint32_t jt = j / BATCH_TILE;                          // own exponent tile
     const uint32_t jby = (j + dmy) / BATCH_TILE, jbz = (j + dmz) / BATCH_TILE;
+    if (LATE) grid_dependency_sync();                            // the tables are the caller's
     const BFix<0, KEEP> fy = bfix<0, KEEP>(v.ax[1], sy, y, act);
     const BFix<0, KEEP> fz = bfix<0, KEEP>(v.ax[2], sz, z, act);
     // what the march needs of the descriptor in registers: a store may alias it, and a value read
@@ -196,7 +197,6 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, const int64_t *counter, int
     const bool xf = xa < (uint32_t)Tn || (Tp && xb > sx - (uint32_t)Tp);   // an x face covers a plane of the tile
     // a point source, a monitor point in this tile (block-uniform)
     bool srcs = false, mons = false;
-    if (LATE) grid_dependency_sync();
     const int64_t step = *counter + t;
     if (step < rows) {
         for (int s = 0; s < v.nsrc; ++s)
@@ -365,6 +365,7 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
     const uint32_t jt = j / BATCH_TILE;
     const uint32_t jby = (j + dpy) / BATCH_TILE, jbz = (j + dpz) / BATCH_TILE;
+    if (LATE) grid_dependency_sync();                            // the tables are the caller's
     const BFix<1, KEEP> fy = bfix<1, KEEP>(v.ax[1], sy, y, act);
     const BFix<1, KEEP> fz = bfix<1, KEEP>(v.ax[2], sz, z, act);
     const float inv = v.inv_d, dt = v.dt;
@@ -372,7 +373,6 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
     const BAxis &ax0 = v.ax[0];
     const int Tn = ax0.Tn, Tp = ax0.Tp;
     const bool xf = xa < (uint32_t)Tn || (Tp && xb > sx - (uint32_t)Tp);
-    if (LATE) grid_dependency_sync();
 
     auto load = [&](uint32_t x, uint32_t i) {
         BHLoad<T> q;
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 4) k_batch_h(const BatchK k)
 }
 
 // One variant per launch, its descriptor among the kernel's arguments (five blocks per SM: 0.317 ms a step
-// instead of 0.306); the set-up stands before the wait (0.297).
+// instead of 0.306); index arithmetic stands before the wait (0.304).
 constexpr int BATCH_ONE_BLOCKS = 4;
 
 __global__ void __launch_bounds__(BATCH_THREADS, BATCH_ONE_BLOCKS) k_batch_e1(const __grid_constant__ BatchOne k)

@@ -128,18 +128,18 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
             if (AHEAD) sC[3 + q][t] = face_tab(k.ax[2].e, fz, q);
         }
     }
-    R iy = k.inv_d, iz = k.inv_d, iyh = k.inv_d, izh = k.inv_d;
-    if (DX == 2) {
-        iy = ldg(k.inv_de[1] + y);
-        iz = ldg(k.inv_de[2] + z);
-        if (AHEAD) { iyh = ldg(k.inv_dh[1] + y); izh = ldg(k.inv_dh[2] + z); }
-    }
     bool srcs = false;                                           // a point source of the next step in the tile
     if (AHEAD) {
         for (int s = 0; s < k.nsrc; ++s) srcs |= own && k.src_j[s] == j;
         srcs = __any_sync(0xffffffffu, srcs) != 0;
     }
     grid_dependency_sync();
+    R iy = k.inv_d, iz = k.inv_d, iyh = k.inv_d, izh = k.inv_d;
+    if (DX == 2) {
+        iy = ldg(k.inv_de[1] + y);
+        iz = ldg(k.inv_de[2] + z);
+        if (AHEAD) { iyh = ldg(k.inv_dh[1] + y); izh = ldg(k.inv_dh[2] + z); }
+    }
     const R *const E0 = k.E, *const E1 = k.E + N, *const E2 = k.E + 2 * N;
     const R *const H0 = k.HA, *const H1 = k.HA + N, *const H2 = k.HA + 2 * N;
 

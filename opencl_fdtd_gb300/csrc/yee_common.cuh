@@ -40,7 +40,7 @@ struct FastDiv {
 // programmatic stream serialization may be scheduled while the kernel before it in the stream
 // still runs; it waits here until that kernel has completed and its writes are visible, and then
 // lets the next kernel of the stream be scheduled. Before it stand only index arithmetic and reads
-// of what no kernel writes (coefficient tables, spacings): a thread's set-up then overlaps the
+// of the plan's own coefficient tables, which no kernel writes: a thread's set-up then overlaps the
 // kernel before, which is most of what a small grid's step costs (E and H of 24^3 cells 5.6 to
 // 4.3 us, of 40^3 7.5 to 4.9, of 64^3 11.9 to 10.2; letting the next kernel in before the wait:
 // 4.6, 5.0, 10.6). Without the launch attribute both instructions have no effect.

@@ -317,7 +317,6 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
     const bool by = BLOCH && (k.bloch_mask & 2) && y == 0;
     const bool bz = BLOCH && (k.bloch_mask & 4) && z == 0;
     R iy = k.inv_d, iz = k.inv_d;
-    if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
     // a point source in this column and these planes
     bool srcs = false;
     for (int s = 0; s < k.nsrc; ++s)
@@ -325,6 +324,7 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
 
                 (k.src_x[s] - k.xbeg) / k.xchunk == blockIdx.y;
     grid_dependency_sync();
+    if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
 
     auto load = [&](uint32_t x, uint32_t i) {
         ELoad<R> v;
@@ -491,9 +491,9 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
     const bool by = BLOCH && (k.bloch_mask & 2) && y + 1u == sy;
     const bool bz = BLOCH && (k.bloch_mask & 4) && z + 1u == sz;
     R iy = k.inv_d, iz = k.inv_d;
-    if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
     const R dt = k.dt;
     grid_dependency_sync();
+    if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
 
     auto load = [&](uint32_t x, uint32_t i) {
         HLoad<R> v;

@@ -560,18 +560,21 @@ class Simulation:
         'hs' or 'plain'. Double precision is bound by its arithmetic units, where the per-update
         kernels, which evaluate no cell twice, are the faster ones (0.44 ms a step of 197x173x73
         cells against 0.57). Without Poynting 'ahead' saves only passes over memory (84 to 60 B per
-        cell), so it is taken where the fields exceed the L2: 0.142 against 0.165 ms a step of 200^3
-        cells, but 0.0326 against 0.0289 of 151x129x61."""
+        cell), so it is taken where the fields exceed the L2: 0.147 against 0.157 ms a step of 200^3
+        cells, but 0.0326 against 0.0224 of 151x129x61. With Poynting it also saves a launch: it is the
+        fastest below 1e5 cells, where launches are the cost (24^3 5.3 us a step against 6.1 of 'hs'),
+        and where the fields exceed the L2 (170x175x65 48.8 against 54.4, 200^3 148 against 185); in
+        between 'hs', which evaluates fewer values twice (64^3 12.0 against 13.0, 128x100x50 20.6
+        against 22.4, 151x129x61 31.4 against 34.1)."""
         hs = "hs" if self.do_poynting else "plain"
         if self.bloch_boundaries or self._np_dtype == numpy.float64:
             return "plain"
         if nsteps < 2 or getattr(self, "_lbc_keep", None) is not None:
             return hs
+        l2 = torch.cuda.get_device_properties(self.device).L2_cache_size
         if not self.do_poynting:
-            l2 = torch.cuda.get_device_properties(self.device).L2_cache_size
-            if 60 * self.N <= l2 or self.tuning("slab"):
-                return "plain"
-        return "ahead"
+            return "plain" if 60 * self.N <= l2 or self.tuning("slab") else "ahead"
+        return "hs" if self.N > 100000 and 84 * self.N <= l2 else "ahead"
 
     def _try_scratch(self, mode) -> bool:
         """The second copies of a run path, or False when the device has no room for them."""

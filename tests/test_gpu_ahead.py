@@ -103,12 +103,16 @@ def test_ahead_point_sources(count):
 
 
 def test_auto_path_choice():
-    """Poynting on: 'ahead' from two steps on; off: per-update kernels while the fields fit the L2;
-    double precision and Bloch boundaries: per-update kernels."""
+    """Poynting on: 'ahead' from two steps on, but 'hs' where launches no longer count and the fields fit
+    the L2; off: per-update kernels while they fit; double precision and Bloch boundaries: per-update."""
     from opencl_fdtd_gb300 import Simulation
     kw = _kwargs((8, 8, 8), _six(2), 1)
     s = Simulation(**copy.deepcopy(kw))
     assert (s._auto_path(1), s._auto_path(2)) == ("hs", "ahead")
+    mid = Simulation(**_kwargs((60, 50, 40), _six(2), 1))
+    assert mid._auto_path(2) == "hs"
+    mid.run(3)
+    assert mid.tuning("last_run_path") == 2
     kw["do_poynting"] = False
     assert Simulation(**copy.deepcopy(kw))._auto_path(5) == "plain"
     kw["float_type"] = numpy.float64
