@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(TR_T) k_mlp_rows(const __grid_constant__ RowsK
     const float *const P = g.P;
     const int t = threadIdx.x, u = t & 15, s0 = (t >> 4) * 4;
     const int r0 = blockIdx.x * TR_ROWS, nr = min(TR_ROWS, g.B - r0);
+    grid_dependency_sync();
     // the first layer's operands first: the other layers' weights arrive behind its arithmetic
     for (int i = t; i < TR_ROWS * LBC_IN; i += TR_T) {
         const bool in = i < nr * LBC_IN;
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(TR_T) k_mlp_bwd_rows(const float *P, const flo
     __shared__ __align__(16) float d2[TR_ROWS * TR_LD];
     const int t = threadIdx.x, u = t & 15, s0 = (t >> 4) * 4;
     const int r0 = blockIdx.x * TR_ROWS, nr = min(TR_ROWS, B - r0);
+    grid_dependency_sync();
     for (int i = t; i < LBC_HID * LBC_OUT; i += TR_T) copy4(w3 + i, P + LBC_W3 + i, true);
     copy_commit();
     for (int i = t; i < LBC_HID * LBC_HID; i += TR_T) copy4(w2 + i / LBC_HID * TR_LD + i % LBC_HID, P + LBC_W2 + i, true);
@@ -390,6 +392,7 @@ __device__ __forceinline__ void outer_tile(const WLayer &l, int tile, uint32_t s
     const int t = threadIdx.x;
     const int r0 = blockIdx.y * WG_RPB, nr = min(WG_RPB, rows - r0);
     float *const si = sh, *const sd = sh + WG_RPB * WG_KT;
+    grid_dependency_sync();
 #pragma unroll 1
     for (int g = 0; g < WG_GROUPS; ++g) {
         for (int i = t; i < GR * WG_KT; i += WG_T) {
@@ -465,6 +468,7 @@ constexpr int FOLD_T = 128;
 __global__ void __launch_bounds__(FOLD_T) k_mlp_wgrad_fold(const float *partial, int G, uint32_t n, float *out,
                                                            const float *lpart, int nl, float count, float *loss)
 {
+    grid_dependency_sync();
     if (loss && blockIdx.x == gridDim.x - 1) {
         __shared__ float part[FOLD_T / 32];
         float s = 0.f;
@@ -490,6 +494,7 @@ __global__ void k_adam(float *P, const float *G, float *M, float *V, int n, floa
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    grid_dependency_sync();
     const float g = G[i];
     const float m = b1 * M[i] + (1.f - b1) * g;
     const float v = b2 * V[i] + (1.f - b2) * g * g;
@@ -1235,12 +1240,11 @@ static cudaError_t launch_wgrad(WLayers L, int rows, float *ws, float *out, cons
             Lg.l[i].in += (size_t)r0 * L.l[i].K;
             Lg.l[i].d += (size_t)r0 * L.l[i].N;
         }
-        k_mlp_wgrad<<<dim3(tiles, m), WG_T, WG_SMEM, st>>>(Lg, rows - r0, ws + (size_t)g * n);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        e = launch_dependent_smem(k_mlp_wgrad, dim3(tiles, m, 1), WG_T, WG_SMEM, st, true, Lg, rows - r0, ws + (size_t)g * n);
+        if (e != cudaSuccess) return e;
     }
-    k_mlp_wgrad_fold<<<(n + FOLD_T - 1) / FOLD_T + (loss ? 1 : 0), FOLD_T, 0, st>>>(
-        ws, G, n, out, lpart, (rows + TR_ROWS - 1) / TR_ROWS, (float)rows * LBC_OUT, loss);
-    return cudaGetLastError();
+    return launch_dependent_smem(k_mlp_wgrad_fold, dim3((n + FOLD_T - 1) / FOLD_T + (loss ? 1 : 0), 1, 1), FOLD_T, 0, st, true,
+                                 (const float *)ws, G, n, out, lpart, (rows + TR_ROWS - 1) / TR_ROWS, (float)rows * LBC_OUT, loss);
 }
 
 // the weight gradients of the network's layers from their inputs and pre-activation gradients
@@ -1293,8 +1297,8 @@ cudaError_t launch_mlp_grad(const float *P, const float *X, const float *T, cons
     float *DY = ws, *D2 = DY + (size_t)B * LBC_OUT, *D1 = D2 + nh, *H1 = D1 + nh, *H2 = H1 + nh, *lpart = H2 + nh;
     const int blocks = (B + TR_ROWS - 1) / TR_ROWS;
     const RowsK k = {P, X, B, nullptr, nullptr, nullptr, H1, H2, T, wout, 1.0f / ((float)B * LBC_OUT), DY, D2, D1, lpart};
-    k_mlp_rows<true><<<blocks, TR_T, ROWS_SMEM, st>>>(k);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    // the launches of a training step depend on each other: each is set up while the one before drains
+    if ((e = launch_dependent_smem(k_mlp_rows<true>, dim3(blocks, 1, 1), TR_T, ROWS_SMEM, st, true, k)) != cudaSuccess) return e;
     return launch_layers(X, H1, H2, D1, D2, DY, B, lpart + blocks, grad, lpart, loss, st);
 }
 
@@ -1315,8 +1319,7 @@ cudaError_t launch_adam(float *P, const float *G, float *M, float *V, int n, flo
 {
     if (n <= 0) return cudaSuccess;
     const float c1 = 1.f - powf(b1, (float)step), c2 = 1.f - powf(b2, (float)step);
-    k_adam<<<(n + 255) / 256, 256, 0, st>>>(P, G, M, V, n, lr, b1, b2, eps, c1, c2);
-    return cudaGetLastError();
+    return launch_dependent_smem(k_adam, dim3((n + 255) / 256, 1, 1), 256, 0, st, true, P, G, M, V, n, lr, b1, b2, eps, c1, c2);
 }
 
 cudaError_t launch_lbc_pack(const float *P, uint32_t *out, cudaStream_t st)
