@@ -287,7 +287,7 @@ int fdtd_count_nonfinite(FdtdPlan *plan, const FdtdBuffers *buf, uint32_t *count
  * place, then H and S) or one (E2, H2 and every psi copy: FDTD_TUNE_HS_AHEAD, or the one-pass step
  * with at most 8 sources); oS is then written on the last step only. The path taken is read back
  * with fdtd_plan_get(FDTD_GET_LAST_RUN_PATH). The kernel that updates E adds up to 8 point sources
- * itself (without a learned boundary); on the H path the monitor sample of each step is taken by
+ * itself (unless a learned boundary's fix-up changes one of their cells); on the H path the monitor sample of each step is taken by
  * one extra block of the H launch (FDTD_TUNE_HS_DFT; 0: by the monitor kernel on a stream of the
  * plan beside the H launch, joined back into `stream` before the call returns). The E and H kernels
  * of a run use programmatic dependent launch (FDTD_TUNE_PDL). */

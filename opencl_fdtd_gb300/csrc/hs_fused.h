@@ -33,10 +33,8 @@ struct HSK {
     R dt, inv_d, sf;
     const R *inv_de[3], *inv_dh[3];
     HSAxis<R> ax[3];
-    // tiles of a plane: rows own rows by seglen own columns (a z row is nseg segments), and the
-    // division by the extended segment length, seglen + 1
+    // tiles of a plane: rows own rows by seglen own columns (a z row is nseg segments)
     uint32_t rows, seglen, nseg, ntile;
-    FastDiv dext;
     uint32_t xchunk, nchunk;   // x planes per block, x chunks (ceil(sx / xchunk))
     int32_t write_oS;
     int32_t reverse;       // 1: the x chunks in descending order

@@ -558,7 +558,7 @@ class Simulation:
     def _auto_path(self, nsteps: int) -> str:
         """The kernels run(path='auto') takes: 'ahead' where it applies and there is a next step, else
         'hs' or 'plain'. Double precision is bound by its arithmetic units, where the per-update
-        kernels, which evaluate no cell twice, are the faster ones (0.44 ms a step of 197x173x73
+        kernels, which evaluate no cell twice, are the faster ones (0.36 ms a step of 197x173x73
         cells against 0.57). Without Poynting 'ahead' saves only passes over memory (84 to 60 B per
         cell), so it is taken where the fields exceed the L2: 0.147 against 0.157 ms a step of 200^3
         cells, but 0.0326 against 0.0224 of 151x129x61. With Poynting it also saves a launch: it is the
