@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 4) k_batch_h(const BatchK k)
 }
 
 // One variant per launch, its descriptor among the kernel's arguments (five blocks per SM: 0.317 ms a step
-// instead of 0.306); index arithmetic stands before the wait (0.304).
+// instead of 0.306); index arithmetic stands before the wait (0.304), chunks by fit_xchunk (0.286).
 constexpr int BATCH_ONE_BLOCKS = 4;
 
 __global__ void __launch_bounds__(BATCH_THREADS, BATCH_ONE_BLOCKS) k_batch_e1(const __grid_constant__ BatchOne k)
@@ -663,12 +663,8 @@ cudaError_t launch_batch_steps(const BatchK &kk, const BatchGroup *groups, int n
         const BVar *const one = groups[g].one;
         dim3 grid(k.ntiles, 1, 1);
         if (one) {
-            // as the per-update kernels: 8 planes, or the fewest with which all blocks are resident
             o.v = *one;
-            o.xchunk = groups[g].xchunk ? groups[g].xchunk : 1u;
-            while (!groups[g].xchunk && o.xchunk < 8u &&
-                   (uint64_t)one->njb * ((one->sx + o.xchunk - 1) / o.xchunk) > (uint64_t)sms * BATCH_ONE_BLOCKS)
-                ++o.xchunk;
+            o.xchunk = groups[g].xchunk ? groups[g].xchunk : fit_xchunk(one->njb, one->sx, (uint64_t)sms * BATCH_ONE_BLOCKS);
             grid = dim3(one->njb, (one->sx + o.xchunk - 1) / o.xchunk, 1);
         }
         for (int t = 0; t < kk.nsteps && e == cudaSuccess; ++t) {

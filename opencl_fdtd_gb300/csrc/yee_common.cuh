@@ -50,6 +50,28 @@ __device__ __forceinline__ void grid_dependency_sync()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// x planes per thread of a launch with nj blocks across a plane, for nx planes and `slots` resident blocks.
+// 8 where the launch is many waves of blocks. Below six waves the shortest estimate of waves, rounded up,
+// times a march (its planes and one for the set-up): on small grids that is one wave with the
+// fewest planes (E and H of 64^3 cells 8.0 us a step with 2 planes, 9.3 with 1 and 1024 blocks), in between
+// a whole number of waves (208x202x71: 10 planes, 1.97 waves, E 33 us, against 36 with 8 and 2.44;
+// 128x128x256 Bloch 172 us a step with 7, 4.0 waves, against 180 with 8 and 3.4).
+inline uint32_t fit_xchunk(uint64_t nj, uint64_t nx, uint64_t slots)
+{
+    if (!slots || nj * ((nx + 7u) / 8u) >= 6u * slots) return 8u;
+    uint32_t best = 8u;
+    uint64_t least = 0;
+    for (uint32_t c = 1; c <= 12u; ++c) {
+        const uint64_t blocks = nj * ((nx + c - 1u) / c), waves = (blocks + slots - 1u) / slots;
+        const uint64_t t = waves * (c + 1u);
+        if (!least || t <= least) {
+            least = t;
+            best = c;
+        }
+    }
+    return best;
+}
+
 // Launches kern<<<g, block, smem, st>>>(args...), with programmatic stream serialization when pdl.
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent_smem(void (*kern)(P...), dim3 g, unsigned block, size_t smem, cudaStream_t st, bool pdl,

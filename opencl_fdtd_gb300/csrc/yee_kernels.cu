@@ -718,22 +718,15 @@ static uint32_t sm_count()
     return (uint32_t)n[dev];
 }
 
-// x planes a thread of a bulk kernel marches when none is set (xchunk 0): 8, or on small grids the fewest
-// with which every block is resident at once: a launch then takes one thread's march, and more blocks than
-// that cost a second wave (E and H of 64^3 cells 9.3 us a step with 1 plane, 1024 blocks, and 8.0 with 2;
-// 151x129x61: 25.8 with 7, 669 blocks for 608 places, and 22.5 with 8). In double precision 1: the FP64
-// units are the bound, so what counts is that every SM has work to the end, not the loads that a longer
-// march saves (197x173x73 0.389 ms a step with 8 planes, 0.374 with 4, 0.360 with 1; 151x129x61 0.223 and
-// 0.186; 128x128x64 0.216 and 0.165).
+// x planes a thread of a bulk kernel marches when none is set (xchunk 0): fit_xchunk. In double precision
+// 1: the FP64 units are the bound, so what counts is that every SM has work to the end, not the loads that
+// a longer march saves (197x173x73 0.389 ms a step with 8 planes, 0.374 with 4, 0.360 with 1; 151x129x61
+// 0.223 and 0.186; 128x128x64 0.216 and 0.165).
 template <template <typename> class K, typename R>
 static dim3 bulk_grid(K<R> &k, uint32_t block, uint32_t resident)
 {
     const uint32_t nj = (k.syz + block - 1) / block, nx = k.xend - k.xbeg;
-    if (!k.xchunk) {
-        const uint64_t slots = (uint64_t)sm_count() * resident;
-        k.xchunk = 1u;
-        while (sizeof(R) == 4 && k.xchunk < 8u && (uint64_t)nj * ((nx + k.xchunk - 1) / k.xchunk) > slots) ++k.xchunk;
-    }
+    if (!k.xchunk) k.xchunk = sizeof(R) == 8 ? 1u : fit_xchunk(nj, nx, (uint64_t)sm_count() * resident);
     return dim3(nj, (nx + k.xchunk - 1) / k.xchunk, 1);
 }
 
