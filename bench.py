@@ -715,7 +715,7 @@ def run_e2e(sim, wl, steps: int, world: int, run_api: bool = False, path: str = 
         N = int(numpy.prod(wl["shape"]))
         return {"value": round(world * N * n / el / 1e6, 2), "unit": UNIT,
                 "h2d_bytes_per_step": 4, "d2h_bytes_per_step": round(4 / chunk, 2), "steps": n,
-                "api": "Simulation.run(10 steps, point_sources from host, DFT monitor) + field sample read back",
+                "api": "Simulation.run(10 steps, point_sources from host memory, carried by the launches; DFT monitor) + field sample read back",
                 "monitor": monitor is not None}
     ind = wl["source_index"]
     poynting = wl["kwargs"].get("do_poynting", True)
