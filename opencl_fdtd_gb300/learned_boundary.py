@@ -256,19 +256,35 @@ class BoundaryNet:
             self._wout[face] = torch.tensor(w, dtype=torch.float32, device=self.device)
         return self._wout[face]
 
+    @staticmethod
+    def _targets(T, B):
+        """Targets of another type or shape as the kernel reads them: float32, broadcast to [B][6], and
+        those with further dimensions as their mean over these, which has the same gradient."""
+        torch = _torch()
+        T = T.detach().to(torch.float32)
+        shape = torch.broadcast_shapes((B, OUT), T.shape)
+        T = T.expand(shape)
+        if shape != (B, OUT):
+            T = T.sum_to_size(B, OUT) * (B * OUT / math.prod(shape))
+        return T.contiguous()
+
     def gradient(self, face: int, X, T, weighted: bool = True):
         """(loss tensor, gradient [NPARAM]) of mean(w (net(X) - T)^2) for face ``face``, w the
         output weights (all 1 when ``weighted`` is False)."""
+        torch = _torch()
         X = X.contiguous()
-        T = T.contiguous()
         B = X.shape[0]
+        # the kernel reads the targets as [B][6] float32; others are brought to that
+        plain = T.dtype == torch.float32 and T.shape == (B, OUT)
+        Tk = T.contiguous() if plain else self._targets(T, B)
         ws, grad = self._gradient_buffers(B)
         w = self.output_weights(face) if weighted else None
-        loss = _torch().empty((), dtype=_torch().float32, device=self.device)
-        _lib.check(_lib.load().fdtd_mlp_gradient(self.params[face].data_ptr(), X.data_ptr(), T.data_ptr(),
+        loss = torch.empty((), dtype=torch.float32, device=self.device)
+        _lib.check(_lib.load().fdtd_mlp_gradient(self.params[face].data_ptr(), X.data_ptr(), Tk.data_ptr(),
                                                  w.data_ptr() if w is not None else None, B, grad.data_ptr(),
                                                  loss.data_ptr(), ws.data_ptr(), ws.numel(), self._stream()))
-        if T.requires_grad:                      # the loss as a function of the targets
+        # the loss as a function of the targets (reverse or forward mode), in their type, over all of them
+        if T.requires_grad or not plain or torch.autograd.forward_ad.unpack_dual(T).tangent is not None:
             d = (self.forward(face, X) - T) ** 2
             loss = (d * w).mean() if w is not None else d.mean()
         return loss, grad
