@@ -304,13 +304,10 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
     const R *__restrict__ Cx = k.coef;
     const R *__restrict__ Cy = k.coef + N;
     const R *__restrict__ Cz = k.coef + 2 * N;
-    // W may be P itself: a thread reads its own cells of P only, each before it writes it
-    R *__restrict__ Px = k.P;
-    R *__restrict__ Py = k.P + N;
-    R *__restrict__ Pz = k.P + 2 * N;
-    R *__restrict__ Wx = AWAY ? k.W : k.P;
-    R *__restrict__ Wy = AWAY ? k.W + N : Py;
-    R *__restrict__ Wz = AWAY ? k.W + 2 * N : Pz;
+    // W may be P itself (a thread reads its own cells of P only, each before it writes it), so neither is
+    // restrict
+    const R *const Px = k.P, *const Py = k.P + N, *const Pz = k.P + 2 * N;
+    R *const Wx = AWAY ? k.W : k.P, *const Wy = Wx + N, *const Wz = Wx + 2 * N;
     // y/z minus neighbours with periodic wrap (common.cl:75-81), fixed for the thread
     const uint32_t dmy = y ? 0u - sz : (sy - 1u) * sz;
     const uint32_t dmz = z ? 0xffffffffu : sz - 1u;
@@ -427,9 +424,9 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
                 else ez = ez + val;
             }
         }
-        (AWAY ? Wx : Px)[i] = ex;
-        (AWAY ? Wy : Py)[i] = ey;
-        (AWAY ? Wz : Pz)[i] = ez;
+        Wx[i] = ex;
+        Wy[i] = ey;
+        Wz[i] = ez;
         hy_m = cur.hy;
         hz_m = cur.hz;
         if (PF) cur = nxt;
@@ -477,13 +474,10 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
     const R *__restrict__ Qx = k.Q;
     const R *__restrict__ Qy = k.Q + N;
     const R *__restrict__ Qz = k.Q + 2 * N;
-    // W may be P itself: a thread reads its own cells of P only, each before it writes it
-    const R *__restrict__ Px = k.P;
-    const R *__restrict__ Py = k.P + N;
-    const R *__restrict__ Pz = k.P + 2 * N;
-    R *__restrict__ Wx = AWAY ? k.W : k.P;
-    R *__restrict__ Wy = AWAY ? k.W + N : k.P + N;
-    R *__restrict__ Wz = AWAY ? k.W + 2 * N : k.P + 2 * N;
+    // W may be P itself (a thread reads its own cells of P only, each before it writes it), so neither is
+    // restrict
+    const R *const Px = k.P, *const Py = k.P + N, *const Pz = k.P + 2 * N;
+    R *const Wx = AWAY ? k.W : k.P, *const Wy = Wx + N, *const Wz = Wx + 2 * N;
     // y/z plus neighbours with periodic wrap (common.cl:82-84), fixed for the thread
     const uint32_t dpy = (y + 1u < sy) ? sz : 0u - (sy - 1u) * sz;
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
