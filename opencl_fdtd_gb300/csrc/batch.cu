@@ -151,9 +151,6 @@ __device__ __forceinline__ float dv(typename Store<ST>::T v, int e)
     return Store<ST>::scaled ? Store<ST>::dec(v) * pow2(e) : Store<ST>::dec(v);
 }
 
-template <typename T>
-__device__ __forceinline__ T ldr(const T *p) { return __ldg(p); }
-
 // ---- E half-step of one tile (update_e.cl:39-107 per cell) ------------------------------------
 // Values one E plane reads (stored form and tile exponents).
 template <typename T>
@@ -175,11 +172,11 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, const int64_t *counter, int
     const bool act = j < syz;
     const uint32_t y = act ? v.dsz.div(j) : 0u;
     const uint32_t z = act ? j - y * sz : 0u;
-    const T *__restrict__ Hx = (const T *)v.H, *__restrict__ Hy = Hx + N, *__restrict__ Hz = Hx + 2 * N;
-    T *__restrict__ Ex = (T *)v.E, *__restrict__ Ey = Ex + N, *__restrict__ Ez = Ex + 2 * N;
-    const T *__restrict__ Cx = (const T *)v.ce, *__restrict__ Cy = Cx + N, *__restrict__ Cz = Cx + 2 * N;
-    const int32_t *__restrict__ hexp = v.hexp;
-    int32_t *__restrict__ eexp = v.eexp;
+    const T *const Hx = (const T *)v.H, *const Hy = Hx + N, *const Hz = Hx + 2 * N;
+    T *const Ex = (T *)v.E, *const Ey = Ex + N, *const Ez = Ex + 2 * N;
+    const T *const Cx = (const T *)v.ce, *const Cy = Cx + N, *const Cz = Cx + 2 * N;
+    const int32_t *const hexp = v.hexp;
+    int32_t *const eexp = v.eexp;
     // minus neighbours with periodic wrap (common.cl:75-81), 32-bit modular offsets
     const uint32_t dmy = y ? 0u - sz : (sy - 1u) * sz;
     const uint32_t dmz = z ? 0xffffffffu : sz - 1u;
@@ -208,11 +205,11 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, const int64_t *counter, int
     auto load = [&](uint32_t x, uint32_t i) {
         BELoad<T> q;
         const uint32_t imy = i + dmy, imz = i + dmz;   // 32-bit wrap arithmetic
-        q.hx = ldr(Hx + i); q.hy = ldr(Hy + i); q.hz = ldr(Hz + i);
-        q.nxy = ldr(Hx + imy); q.nzy = ldr(Hz + imy);
-        q.nxz = ldr(Hx + imz); q.nyz = ldr(Hy + imz);
+        q.hx = Hx[i]; q.hy = Hy[i]; q.hz = Hz[i];
+        q.nxy = Hx[imy]; q.nzy = Hz[imy];
+        q.nxz = Hx[imz]; q.nyz = Hy[imz];
         q.ex = Ex[i]; q.ey = Ey[i]; q.ez = Ez[i];
-        q.cx = ldr(Cx + i); q.cy = ldr(Cy + i); q.cz = ldr(Cz + i);
+        q.cx = Cx[i]; q.cy = Cy[i]; q.cz = Cz[i];
         if (SS::scaled) {
             q.gh = hexp[texp_index(v, x, jt)];
             q.gy = hexp[texp_index(v, x, jby)];
@@ -243,8 +240,8 @@ __device__ void batch_e_tile(const BVar &v, int4 tl, const int64_t *counter, int
         const uint32_t xm = xa ? xa - 1u : sx - 1u;
         const uint32_t im = xm * syz + j;
         const int32_t wm = SS::scaled ? hexp[texp_index(v, xm, jt)] : 0;
-        hy_m = dv<ST>(ldr(Hy + im), xe(wm, 1));
-        hz_m = dv<ST>(ldr(Hz + im), xe(wm, 2));
+        hy_m = dv<ST>(Hy[im], xe(wm, 1));
+        hz_m = dv<ST>(Hz[im], xe(wm, 2));
     }
     uint32_t i = xa * syz + j;
     for (uint32_t x = xa; x < xb; ++x, i += syz) {
@@ -356,10 +353,10 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
     const bool act = j < syz;
     const uint32_t y = act ? v.dsz.div(j) : 0u;
     const uint32_t z = act ? j - y * sz : 0u;
-    const T *__restrict__ Ex = (const T *)v.E, *__restrict__ Ey = Ex + N, *__restrict__ Ez = Ex + 2 * N;
-    T *__restrict__ Hx = (T *)v.H, *__restrict__ Hy = Hx + N, *__restrict__ Hz = Hx + 2 * N;
-    int32_t *__restrict__ hexp = v.hexp;
-    const int32_t *__restrict__ eexp = v.eexp;
+    const T *const Ex = (const T *)v.E, *const Ey = Ex + N, *const Ez = Ex + 2 * N;
+    T *const Hx = (T *)v.H, *const Hy = Hx + N, *const Hz = Hx + 2 * N;
+    int32_t *const hexp = v.hexp;
+    const int32_t *const eexp = v.eexp;
     // plus neighbours with periodic wrap (common.cl:82-84)
     const uint32_t dpy = (y + 1u < sy) ? sz : 0u - (sy - 1u) * sz;
     const uint32_t dpz = (z + 1u < sz) ? 1u : 0u - (sz - 1u);
@@ -379,9 +376,9 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
         const uint32_t x1 = (x + 1u < sx) ? x + 1u : 0u;
         const uint32_t i1 = x1 * syz + j;
         const uint32_t ipy = i + dpy, ipz = i + dpz;   // 32-bit wrap arithmetic
-        q.ex1 = ldr(Ex + i1); q.ey1 = ldr(Ey + i1); q.ez1 = ldr(Ez + i1);
-        q.rxy = ldr(Ex + ipy); q.rzy = ldr(Ez + ipy);
-        q.rxz = ldr(Ex + ipz); q.ryz = ldr(Ey + ipz);
+        q.ex1 = Ex[i1]; q.ey1 = Ey[i1]; q.ez1 = Ez[i1];
+        q.rxy = Ex[ipy]; q.rzy = Ez[ipy];
+        q.rxz = Ex[ipz]; q.ryz = Ey[ipz];
         q.hx = Hx[i]; q.hy = Hy[i]; q.hz = Hz[i];
         if (SS::scaled) {
             q.ge = eexp[texp_index(v, x1, jt)];
@@ -412,9 +409,9 @@ __device__ void batch_h_tile(const BVar &v, int4 tl)
     if (act) {
         const uint32_t i = xa * syz + j;
         const int32_t wa = SS::scaled ? eexp[texp_index(v, xa, jt)] : 0;
-        ex = dv<ST>(ldr(Ex + i), xe(wa, 0));
-        ey = dv<ST>(ldr(Ey + i), xe(wa, 1));
-        ez = dv<ST>(ldr(Ez + i), xe(wa, 2));
+        ex = dv<ST>(Ex[i], xe(wa, 0));
+        ey = dv<ST>(Ey[i], xe(wa, 1));
+        ez = dv<ST>(Ez[i], xe(wa, 2));
     }
     uint32_t i = xa * syz + j;
     for (uint32_t x = xa; x < xb; ++x, i += syz) {

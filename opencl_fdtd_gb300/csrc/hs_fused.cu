@@ -136,9 +136,9 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
     grid_dependency_sync();
     R iy = k.inv_d, iz = k.inv_d, iyh = k.inv_d, izh = k.inv_d;
     if (DX == 2) {
-        iy = ldg(k.inv_de[1] + y);
-        iz = ldg(k.inv_de[2] + z);
-        if (AHEAD) { iyh = ldg(k.inv_dh[1] + y); izh = ldg(k.inv_dh[2] + z); }
+        iy = ldf(k.inv_de[1] + y);
+        iz = ldf(k.inv_de[2] + z);
+        if (AHEAD) { iyh = ldf(k.inv_dh[1] + y); izh = ldf(k.inv_dh[2] + z); }
     }
     const R *const E0 = k.E, *const E1 = k.E + N, *const E2 = k.E + 2 * N;
     const R *const H0 = k.HA, *const H1 = k.HA + N, *const H2 = k.HA + 2 * N;
@@ -146,18 +146,18 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
     const bool xf = xa < (uint32_t)k.ax[0].Tn + 1u || (k.ax[0].Tp && (xa == 0u || xb > sx - (uint32_t)k.ax[0].Tp));
     auto load = [&](uint32_t x, uint32_t i, uint32_t i1, HLoads<R> &v) {
         const uint32_t ipy = i + dpy, ipz = i + dpz;             // 32-bit wrap arithmetic
-        v.ex1 = ldg(E0 + i1); v.ey1 = ldg(E1 + i1); v.ez1 = ldg(E2 + i1);
-        v.rxy = ldg(E0 + ipy); v.rzy = ldg(E2 + ipy);
-        v.rxz = ldg(E0 + ipz); v.ryz = ldg(E1 + ipz);
-        v.hx = ldg(H0 + i); v.hy = ldg(H1 + i); v.hz = ldg(H2 + i);
-        if (MU) { v.cx = ldg(k.cm + i); v.cy = ldg(k.cm + N + i); v.cz = ldg(k.cm + 2 * N + i); }
+        v.ex1 = ldf(E0 + i1); v.ey1 = ldf(E1 + i1); v.ez1 = ldf(E2 + i1);
+        v.rxy = ldf(E0 + ipy); v.rzy = ldf(E2 + ipy);
+        v.rxz = ldf(E0 + ipz); v.ryz = ldf(E1 + ipz);
+        v.hx = ldf(H0 + i); v.hy = ldf(H1 + i); v.hz = ldf(H2 + i);
+        if (MU) { v.cx = ldf(k.cm + i); v.cy = ldf(k.cm + N + i); v.cz = ldf(k.cm + 2 * N + i); }
         if (wf && fz.ir >= 0) {
             const uint32_t ip = psi_at<2>(fz, k.ax[2].Tn, k.ax[2].Tp, x, y, z, sy, sz);
-            v.zu = ldg(face_A(k.ax[2].h, fz, 0) + ip); v.zv = ldg(face_A(k.ax[2].h, fz, 1) + ip);
+            v.zu = ldf(face_A(k.ax[2].h, fz, 0) + ip); v.zv = ldf(face_A(k.ax[2].h, fz, 1) + ip);
         }
         if (wf && fy.ir >= 0) {
             const uint32_t ip = psi_at<1>(fy, k.ax[1].Tn, k.ax[1].Tp, x, y, z, sy, sz);
-            v.yu = ldg(face_A(k.ax[1].h, fy, 0) + ip); v.yv = ldg(face_A(k.ax[1].h, fy, 1) + ip);
+            v.yu = ldf(face_A(k.ax[1].h, fy, 0) + ip); v.yv = ldf(face_A(k.ax[1].h, fy, 1) + ip);
         }
         FaceAt fx;
         fx.ir = -1;
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
         if (xf) fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
         if (fx.ir >= 0) {
             const uint32_t ip = (uint32_t)fx.ir * syz + j;
-            v.xu = ldg(face_A(k.ax[0].h, fx, 0) + ip); v.xv = ldg(face_A(k.ax[0].h, fx, 1) + ip);
+            v.xu = ldf(face_A(k.ax[0].h, fx, 0) + ip); v.xv = ldf(face_A(k.ax[0].h, fx, 1) + ip);
         }
     };
 
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
     // neighbours of the chunk's first plane.
     uint32_t x = xa ? xa - 1u : sx - 1u;
     uint32_t i = x * syz + j;
-    R ex = ldg(E0 + i), ey = ldg(E1 + i), ez = ldg(E2 + i);
+    R ex = ldf(E0 + i), ey = ldf(E1 + i), ez = ldf(E2 + i);
     R p_yx = R(0), p_zx = R(0), p_hy = R(0), p_hz = R(0);
     HLoads<R> v;
     uint32_t i1 = xa * syz + j;
@@ -188,18 +188,18 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
         // what the E update after the barrier reads
         R c0, c1, c2, exu, exv, eyu, eyv, ezu, ezv;
         if (AHEAD) {
-            c0 = ldg(k.ce + i); c1 = ldg(k.ce + N + i); c2 = ldg(k.ce + 2 * N + i);
+            c0 = ldf(k.ce + i); c1 = ldf(k.ce + N + i); c2 = ldf(k.ce + 2 * N + i);
             if (wf && fz.ir >= 0) {
                 const uint32_t ip = psi_at<2>(fz, k.ax[2].Tn, k.ax[2].Tp, x, y, z, sy, sz);
-                ezu = ldg(face_A(k.ax[2].e, fz, 0) + ip); ezv = ldg(face_A(k.ax[2].e, fz, 1) + ip);
+                ezu = ldf(face_A(k.ax[2].e, fz, 0) + ip); ezv = ldf(face_A(k.ax[2].e, fz, 1) + ip);
             }
             if (wf && fy.ir >= 0) {
                 const uint32_t ip = psi_at<1>(fy, k.ax[1].Tn, k.ax[1].Tp, x, y, z, sy, sz);
-                eyu = ldg(face_A(k.ax[1].e, fy, 0) + ip); eyv = ldg(face_A(k.ax[1].e, fy, 1) + ip);
+                eyu = ldf(face_A(k.ax[1].e, fy, 0) + ip); eyv = ldf(face_A(k.ax[1].e, fy, 1) + ip);
             }
             if (fx.ir >= 0) {
                 const uint32_t ip = (uint32_t)fx.ir * syz + j;
-                exu = ldg(face_A(k.ax[0].e, fx, 0) + ip); exv = ldg(face_A(k.ax[0].e, fx, 1) + ip);
+                exu = ldf(face_A(k.ax[0].e, fx, 0) + ip); exv = ldf(face_A(k.ax[0].e, fx, 1) + ip);
             }
         }
         // ---- H (update_h.cl): forward differences (36-43)
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
         R d_zx = v.ez1 - ez;
         R d_zy = v.rzy - ez;
         if (DX != 0) {
-            const R ix = DX == 2 ? ldg(k.inv_de[0] + x) : k.inv_d;
+            const R ix = DX == 2 ? ldf(k.inv_de[0] + x) : k.inv_d;
             d_xy = d_xy * iy; d_xz = d_xz * iz; d_yx = d_yx * ix;
             d_yz = d_yz * iz; d_zx = d_zx * ix; d_zy = d_zy * iy;
         }
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(hs_threads(AHEAD, MU, DX), 2) k_tile_h(const _
                 R e_zx = hz - p_hz;
                 R e_zy = hz - sv[HZ][p - ext];
                 if (DX != 0) {
-                    const R ix = DX == 2 ? ldg(k.inv_dh[0] + x) : k.inv_d;
+                    const R ix = DX == 2 ? ldf(k.inv_dh[0] + x) : k.inv_d;
                     e_xy = e_xy * iyh; e_xz = e_xz * izh; e_yx = e_yx * ix;
                     e_yz = e_yz * izh; e_zx = e_zx * ix; e_zy = e_zy * iyh;
                 }

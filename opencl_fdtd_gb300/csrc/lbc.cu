@@ -891,8 +891,8 @@ __device__ __forceinline__ void stage_pairs(const LGrid &g, const LFace &f, uint
             const uint32_t i = off + clampu((int)(f.u0 + cu0) - 1 + su, g.s[ua]) * sua;
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-                v[su][q] = __ldg(E + q * g.N + i);
-                v[su][3 + q] = __ldg(H + q * g.N + i);
+                v[su][q] = E[q * g.N + i];
+                v[su][3 + q] = H[q * g.N + i];
             }
         }
 #pragma unroll

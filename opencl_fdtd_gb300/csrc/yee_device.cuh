@@ -6,8 +6,29 @@
 
 namespace fdtd {
 
+// Coefficient tables, which no launch writes.
 template <typename T>
 __device__ __forceinline__ T ldg(const T *p) { return __ldg(p); }
+
+// Fields, psi and what else the launch before may write, where the kernel itself does not write it: a
+// coherent load that stays behind the wait of a dependent launch (grid_dependency_sync). Such a launch runs
+// beside the one that writes them, while ld.global.nc, which __ldg and const restrict pointers become, is for
+// data that stays as it is as long as the kernel lives. As an instruction that stays where it is written the
+// load costs nothing (a step of 395x345x73 cells 0.196 ms either way); left to the compiler as *p the next
+// plane's loads came too late (0.340 ms).
+__device__ __forceinline__ float ldf(const float *p)
+{
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+
+__device__ __forceinline__ double ldf(const double *p)
+{
+    double v;
+    asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 
 // Depth index of the cell inside the face's slab, or -1 (update_e.cl:81-90). A 'p' face
 // thicker than its axis never applies (the reference's unsigned s - T wraps).

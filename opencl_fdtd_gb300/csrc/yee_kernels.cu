@@ -298,12 +298,12 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
     const uint32_t xb = min(xa + k.xchunk, k.xend);
     const bool wx = wf || x_faces(k.ax[0], sx, xa, xb);          // a cell of the warp's march is in a face
     const uint64_t N = k.N;
-    const R *__restrict__ Qx = k.Q;
-    const R *__restrict__ Qy = k.Q + N;
-    const R *__restrict__ Qz = k.Q + 2 * N;
-    const R *__restrict__ Cx = k.coef;
-    const R *__restrict__ Cy = k.coef + N;
-    const R *__restrict__ Cz = k.coef + 2 * N;
+    const R *const Qx = k.Q;
+    const R *const Qy = k.Q + N;
+    const R *const Qz = k.Q + 2 * N;
+    const R *const Cx = k.coef;
+    const R *const Cy = k.coef + N;
+    const R *const Cz = k.coef + 2 * N;
     // W may be P itself (a thread reads its own cells of P only, each before it writes it), so neither is
     // restrict
     const R *const Px = k.P, *const Py = k.P + N, *const Pz = k.P + 2 * N;
@@ -321,20 +321,20 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
 
                 (k.src_x[s] - k.xbeg) / k.xchunk == blockIdx.y;
     grid_dependency_sync();
-    if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
+    if (DX == 2) { iy = ldf(k.inv_tab[1] + y); iz = ldf(k.inv_tab[2] + z); }
 
     auto load = [&](uint32_t x, uint32_t i) {
         ELoad<R> v;
-        v.hx = ldg(Qx + i); v.hy = ldg(Qy + i); v.hz = ldg(Qz + i);
+        v.hx = ldf(Qx + i); v.hy = ldf(Qy + i); v.hz = ldf(Qz + i);
         // neighbour indices in 32-bit arithmetic (dmy / dmz may be wrapped negatives)
         const uint32_t imy = i + dmy, imz = i + dmz;
-        v.nxy = ldg(Qx + imy); v.nxz = ldg(Qx + imz);
-        v.nyz = ldg(Qy + imz); v.nzy = ldg(Qz + imy);
+        v.nxy = ldf(Qx + imy); v.nxz = ldf(Qx + imz);
+        v.nyz = ldf(Qy + imz); v.nzy = ldf(Qz + imy);
         v.bxy = v.bzy = v.bxz = v.byz = R(0);
-        if (by) { v.bxy = ldg(k.Rp + imy); v.bzy = ldg(k.Rp + 2 * N + imy); }
-        if (bz) { v.bxz = ldg(k.Rp + imz); v.byz = ldg(k.Rp + N + imz); }
+        if (by) { v.bxy = ldf(k.Rp + imy); v.bzy = ldf(k.Rp + 2 * N + imy); }
+        if (bz) { v.bxz = ldf(k.Rp + imz); v.byz = ldf(k.Rp + N + imz); }
         v.ex = Px[i]; v.ey = Py[i]; v.ez = Pz[i];
-        v.cx = ldg(Cx + i); v.cy = ldg(Cy + i); v.cz = ldg(Cz + i);
+        v.cx = ldf(Cx + i); v.cy = ldf(Cy + i); v.cz = ldf(Cz + i);
         v.xu = v.xv = v.yu = v.yv = v.zu = v.zv = R(0);
         const FaceAt fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
         if (fx.ir >= 0) {
@@ -355,10 +355,10 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
     uint32_t i = xa * syz + j;
     // x-1 plane of the first iteration, wrapped and Bloch-coupled at x = 0
     const uint32_t im = xa ? i - syz : i + (sx - 1u) * syz;
-    R hy_m = ldg(Qy + im), hz_m = ldg(Qz + im);
+    R hy_m = ldf(Qy + im), hz_m = ldf(Qz + im);
     if (BLOCH && xa == 0 && (k.bloch_mask & 1)) {
-        hy_m = hy_m * k.br[0] + ldg(k.Rp + N + im) * k.bi[0];
-        hz_m = hz_m * k.br[0] + ldg(k.Rp + 2 * N + im) * k.bi[0];
+        hy_m = hy_m * k.br[0] + ldf(k.Rp + N + im) * k.bi[0];
+        hz_m = hz_m * k.br[0] + ldf(k.Rp + 2 * N + im) * k.bi[0];
     }
     ELoad<R> cur;
     if (PF) cur = load(xa, i);
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
         R d_zx = cur.hz - hz_m;
         R d_zy = cur.hz - n_zy;
         if (DX != 0) {
-            const R ix = (DX == 2) ? ldg(k.inv_tab[0] + x) : k.inv_d;
+            const R ix = (DX == 2) ? ldf(k.inv_tab[0] + x) : k.inv_d;
             d_xy = d_xy * iy; d_xz = d_xz * iz; d_yx = d_yx * ix;
             d_yz = d_yz * iz; d_zx = d_zx * ix; d_zy = d_zy * iy;
         }
@@ -471,9 +471,9 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
         // asking once costs the form that also writes the products 2 us of 133 on 395x345x73 cells
     const bool xf = (POYNT && sizeof(R) == 4) || x_faces(k.ax[0], sx, xa, xb);
     const uint64_t N = k.N;
-    const R *__restrict__ Qx = k.Q;
-    const R *__restrict__ Qy = k.Q + N;
-    const R *__restrict__ Qz = k.Q + 2 * N;
+    const R *const Qx = k.Q;
+    const R *const Qy = k.Q + N;
+    const R *const Qz = k.Q + 2 * N;
     // W may be P itself (a thread reads its own cells of P only, each before it writes it), so neither is
     // restrict
     const R *const Px = k.P, *const Py = k.P + N, *const Pz = k.P + 2 * N;
@@ -487,23 +487,23 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
     R iy = k.inv_d, iz = k.inv_d;
     const R dt = k.dt;
     grid_dependency_sync();
-    if (DX == 2) { iy = ldg(k.inv_tab[1] + y); iz = ldg(k.inv_tab[2] + z); }
+    if (DX == 2) { iy = ldf(k.inv_tab[1] + y); iz = ldf(k.inv_tab[2] + z); }
 
     auto load = [&](uint32_t x, uint32_t i) {
         HLoad<R> v;
         const uint32_t i1 = (x + 1u < sx) ? i + syz : i - (sx - 1u) * syz;
-        v.ex1 = ldg(Qx + i1); v.ey1 = ldg(Qy + i1); v.ez1 = ldg(Qz + i1);
+        v.ex1 = ldf(Qx + i1); v.ey1 = ldf(Qy + i1); v.ez1 = ldf(Qz + i1);
         // neighbour indices in 32-bit arithmetic (dpy / dpz may be wrapped negatives)
         const uint32_t ipy = i + dpy, ipz = i + dpz;
-        v.rxy = ldg(Qx + ipy); v.rxz = ldg(Qx + ipz);
-        v.ryz = ldg(Qy + ipz); v.rzy = ldg(Qz + ipy);
+        v.rxy = ldf(Qx + ipy); v.rxz = ldf(Qx + ipz);
+        v.ryz = ldf(Qy + ipz); v.rzy = ldf(Qz + ipy);
         v.bxy = v.bzy = v.bxz = v.byz = v.byx = v.bzx = R(0);
-        if (bx && x + 1u == sx) { v.byx = ldg(k.Rp + N + i1); v.bzx = ldg(k.Rp + 2 * N + i1); }
-        if (by) { v.bxy = ldg(k.Rp + ipy); v.bzy = ldg(k.Rp + 2 * N + ipy); }
-        if (bz) { v.bxz = ldg(k.Rp + ipz); v.byz = ldg(k.Rp + N + ipz); }
+        if (bx && x + 1u == sx) { v.byx = ldf(k.Rp + N + i1); v.bzx = ldf(k.Rp + 2 * N + i1); }
+        if (by) { v.bxy = ldf(k.Rp + ipy); v.bzy = ldf(k.Rp + 2 * N + ipy); }
+        if (bz) { v.bxz = ldf(k.Rp + ipz); v.byz = ldf(k.Rp + N + ipz); }
         v.hx = Px[i]; v.hy = Py[i]; v.hz = Pz[i];
         v.cx = v.cy = v.cz = R(0);
-        if (MU) { v.cx = ldg(k.coef + i); v.cy = ldg(k.coef + N + i); v.cz = ldg(k.coef + 2 * N + i); }
+        if (MU) { v.cx = ldf(k.coef + i); v.cy = ldf(k.coef + N + i); v.cz = ldf(k.coef + 2 * N + i); }
         v.xu = v.xv = v.yu = v.yv = v.zu = v.zv = R(0);
         if (xf) {
             const FaceAt fx = face_at(k.ax[0].Tn, k.ax[0].Tp, sx, x);
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
     };
 
     uint32_t i = xa * syz + j;
-    R ex = ldg(Qx + i), ey = ldg(Qy + i), ez = ldg(Qz + i);
+    R ex = ldf(Qx + i), ey = ldf(Qy + i), ez = ldf(Qz + i);
     HLoad<R> cur;
     if (PF) cur = load(xa, i);
     for (uint32_t x = xa; x < xb; ++x, i += syz) {
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
         R d_zx = n_zx - ez;
         R d_zy = n_zy - ez;
         if (DX != 0) {
-            const R ix = (DX == 2) ? ldg(k.inv_tab[0] + x) : k.inv_d;
+            const R ix = (DX == 2) ? ldf(k.inv_tab[0] + x) : k.inv_d;
             d_xy = d_xy * iy; d_xz = d_xz * iz; d_yx = d_yx * ix;
             d_yz = d_yz * iz; d_zx = d_zx * ix; d_zy = d_zy * iy;
         }
@@ -623,30 +623,30 @@ __global__ void __launch_bounds__(BLOCK) k_bulk_s(const SK<R> k)
     const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
     const uint32_t xb = min(xa + k.xchunk, k.xend);
     const uint64_t N = k.N;
-    const R *__restrict__ oxy = k.oS;
-    const R *__restrict__ oyz = k.oS + N;
-    const R *__restrict__ ozx = k.oS + 2 * N;
-    const R *__restrict__ oxz = k.oS + 3 * N;
-    const R *__restrict__ oyx = k.oS + 4 * N;
-    const R *__restrict__ ozy = k.oS + 5 * N;
-    R *__restrict__ Sx = k.S;
-    R *__restrict__ Sy = k.S + N;
-    R *__restrict__ Sz = k.S + 2 * N;
+    const R *const oxy = k.oS;
+    const R *const oyz = k.oS + N;
+    const R *const ozx = k.oS + 2 * N;
+    const R *const oxz = k.oS + 3 * N;
+    const R *const oyx = k.oS + 4 * N;
+    const R *const ozy = k.oS + 5 * N;
+    R *const Sx = k.S;
+    R *const Sy = k.S + N;
+    R *const Sz = k.S + 2 * N;
     const uint32_t dmy = y ? 0u - sz : (sy - 1u) * sz;
     const uint32_t dmz = z ? 0xffffffffu : sz - 1u;
     auto load = [&](uint32_t i) {
         SLoad<R> v;
-        v.xy = ldg(oxy + i); v.yz = ldg(oyz + i); v.zx = ldg(ozx + i);
-        v.xz = ldg(oxz + i); v.yx = ldg(oyx + i); v.zy = ldg(ozy + i);
+        v.xy = ldf(oxy + i); v.yz = ldf(oyz + i); v.zx = ldf(ozx + i);
+        v.xz = ldf(oxz + i); v.yx = ldf(oyx + i); v.zy = ldf(ozy + i);
         const uint32_t imy = i + dmy, imz = i + dmz;   // 32-bit wrap arithmetic
-        v.xy_y = ldg(oxy + imy); v.xz_z = ldg(oxz + imz);
-        v.yz_z = ldg(oyz + imz); v.zy_y = ldg(ozy + imy);
+        v.xy_y = ldf(oxy + imy); v.xz_z = ldf(oxz + imz);
+        v.yz_z = ldf(oyz + imz); v.zy_y = ldf(ozy + imy);
         return v;
     };
     grid_dependency_sync();
     uint32_t i = xa * syz + j;
     const uint32_t im = xa ? i - syz : i + (sx - 1u) * syz;
-    R yx_m = ldg(oyx + im), zx_m = ldg(ozx + im);
+    R yx_m = ldf(oyx + im), zx_m = ldf(ozx + im);
     const R sf = k.sf;
     SLoad<R> cur = load(i);
     for (uint32_t x = xa; x < xb; ++x, i += syz) {

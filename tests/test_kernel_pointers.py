@@ -28,3 +28,19 @@ def test_pointers_to_the_updated_field_are_not_restrict():
     assert len(declared) >= 4                                # P and W of the E and of the H kernel
     for d in declared:
         assert "__restrict__" not in d, d
+
+
+def test_dependent_kernels_read_fields_coherently():
+    """Kernels launched dependently run beside the one that writes what they read, and the persistent
+    batch kernel writes the fields it reads: non-coherent loads (__ldg, const restrict pointers) are left
+    to the coefficient tables, which no launch writes."""
+    yee = _source("yee_kernels.cu")
+    bodies = {"yee_kernels.cu": yee[yee.index("k_bulk_e(const YeeK"):yee.index("k_prepare(const PrepK")]}
+    for name in ("hs_fused.cu", "batch.cu", "lbc.cu", "yee_device.cuh"):
+        bodies[name] = _source(name)
+    for name, text in bodies.items():
+        assert "__restrict__" not in text, name
+        assert text.count("__ldg") == (1 if name == "yee_device.cuh" else 0), name
+        for arg in re.findall(r"(?<!_)\bldg\(([^;]*?)[,;]", text):
+            assert "tab[" in arg or arg.startswith("const T *p"), (name, arg)
+    assert set(bodies) < set(_files())
