@@ -417,15 +417,18 @@ class Simulation:
                 b.psi_e2[f][0], b.psi_e2[f][1] = u.data_ptr(), v.data_ptr()
 
     def _ensure_scratch(self, mode):
-        """Second copies of H and the H-side CPML arrays (the default run path) and, for the
-        fused path, of E and the E-side arrays; allocated on first use and kept."""
+        """Second copies of H and the H-side CPML arrays ('hs') and, for 'ahead' and 'fused', of E and
+        the E-side arrays; allocated on first use and kept. They belong to the queue, whose launches
+        alone use them: a block that the caching allocator takes back from another stream may still be
+        in use there, and one that it gives back may still be written here."""
         E2, H2, pe2, ph2 = self._scratch if self._scratch is not None else (None, None, None, None)
-        if H2 is None:
-            H2 = torch.empty_like(self.H)
-            ph2 = [(torch.empty_like(u), torch.empty_like(v)) for u, v in self.psi["H"]]
-        if mode in ("fused", "ahead") and E2 is None:
-            E2 = torch.empty_like(self.E)
-            pe2 = [(torch.empty_like(u), torch.empty_like(v)) for u, v in self.psi["E"]]
+        with torch.cuda.stream(self.queue):
+            if H2 is None:
+                H2 = torch.empty_like(self.H)
+                ph2 = [(torch.empty_like(u), torch.empty_like(v)) for u, v in self.psi["H"]]
+            if mode in ("fused", "ahead") and E2 is None:
+                E2 = torch.empty_like(self.E)
+                pe2 = [(torch.empty_like(u), torch.empty_like(v)) for u, v in self.psi["E"]]
         self._scratch = (E2, H2, pe2, ph2)
 
     def _prepare(self, mat_key):
