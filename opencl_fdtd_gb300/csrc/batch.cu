@@ -662,6 +662,9 @@ cudaError_t launch_batch_steps(const BatchK &kk, const BatchGroup *groups, int n
         if (one) {
             o.v = *one;
             o.xchunk = groups[g].xchunk ? groups[g].xchunk : fit_xchunk(one->njb, one->sx, (uint64_t)sms * BATCH_ONE_BLOCKS);
+            // the chunks are the grid's y extent, at most 65535
+            const uint32_t least = (one->sx + 65534u) / 65535u;
+            if (o.xchunk < least) o.xchunk = least;
             grid = dim3(one->njb, (one->sx + o.xchunk - 1) / o.xchunk, 1);
         }
         for (int t = 0; t < kk.nsteps && e == cudaSuccess; ++t) {
