@@ -354,8 +354,9 @@ typedef struct FdtdBatch FdtdBatch;
 int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, int64_t rows,
                       FdtdBatch **out);
 int fdtd_batch_destroy(FdtdBatch *batch);
-/* Tile shape and grid: x planes per tile (>= 1) and resident blocks per SM (0: the most that
- * fit). Rebuilds the tile list. */
+/* Tile shape and grid: x planes per tile (0: automatic, as after fdtd_batch_create) and resident
+ * blocks per SM (0: the most that fit). A change of the tiles rebuilds their list, after which a
+ * run captured before must not be replayed. */
 int fdtd_batch_tune(FdtdBatch *batch, int32_t xchunk, int32_t blocks_per_sm);
 /* Advance every variant by nsteps steps (E, sources, H per step) on the stream: with the
  * FDTD_BATCH_LAUNCHES schedule (default) as two launches per step, each covering the tiles of

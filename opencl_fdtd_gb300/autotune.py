@@ -15,7 +15,7 @@ from __future__ import annotations
 import json
 import os
 
-XCHUNKS = (2, 4, 8, 16, 32)
+XCHUNKS = (0, 2, 4, 8, 16, 32)          # 0: the automatic choice
 BLOCKS_PER_SM = (1, 2)
 SCHEDULES = ("launches", "persistent")
 

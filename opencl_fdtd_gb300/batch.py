@@ -131,6 +131,7 @@ class BatchSimulation:
         _lib.check(self._lib.fdtd_batch_create(arr, n, _STORE[storage], self.steps, ctypes.byref(self._batch)))
         self._arr = arr
         self.schedule = "launches"
+        self.xchunk = 0
         if half is not None:
             self.load()
         self._graph = None
@@ -155,11 +156,14 @@ class BatchSimulation:
             _lib.check(self._lib.fdtd_batch_decode(self._batch, v, 1, ctypes.c_void_p(sim.H.data_ptr()), st))
 
     # ---- stepping ---------------------------------------------------------------------------
-    def tune(self, xchunk: int = 8, blocks_per_sm: int = 0, schedule: str = None):
-        """Tile shape (x planes per tile), resident blocks per SM of the persistent schedule
+    def tune(self, xchunk: int = None, blocks_per_sm: int = 0, schedule: str = None):
+        """Tile shape (x planes per tile; 0: automatic, None: as it is), resident blocks per SM of the persistent schedule
         (0: as many as fit) and the schedule: 'launches' (two launches per step, each over the
         tiles of every variant; default) or 'persistent' (one cooperative launch per run)."""
+        if xchunk is None:
+            xchunk = self.xchunk
         _lib.check(self._lib.fdtd_batch_tune(self._batch, int(xchunk), int(blocks_per_sm)))
+        self.xchunk = int(xchunk)
         if schedule is not None:
             if schedule not in ("launches", "persistent"):
                 raise ValueError("schedule must be 'launches' or 'persistent'")

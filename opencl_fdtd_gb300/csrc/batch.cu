@@ -647,7 +647,7 @@ cudaError_t launch_batch(const BatchK &k, int blocks, cudaStream_t st)
 }
 
 template <int ST>
-cudaError_t launch_batch_steps(const BatchK &kk, const BatchGroup *groups, int n, cudaStream_t st)
+cudaError_t launch_batch_steps(const BatchK &kk, const BVar *const *groups, int n, uint32_t xchunk, cudaStream_t st)
 {
     BatchK k = kk;
     BatchOne o;
@@ -657,11 +657,11 @@ cudaError_t launch_batch_steps(const BatchK &kk, const BatchGroup *groups, int n
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     for (int g = 0; g < n; ++g) {
-        const BVar *const one = groups[g].one;
+        const BVar *const one = groups[g];
         dim3 grid(k.ntiles, 1, 1);
         if (one) {
             o.v = *one;
-            o.xchunk = groups[g].xchunk ? groups[g].xchunk : fit_xchunk(one->njb, one->sx, (uint64_t)sms * BATCH_ONE_BLOCKS);
+            o.xchunk = xchunk ? xchunk : fit_xchunk(one->njb, one->sx, (uint64_t)sms * BATCH_ONE_BLOCKS);
             // the chunks are the grid's y extent, at most 65535
             const uint32_t least = (one->sx + 65534u) / 65535u;
             if (o.xchunk < least) o.xchunk = least;
@@ -710,14 +710,14 @@ cudaError_t launch_batch_decode(int store, const BVar &v, int field, float *dst,
 template cudaError_t launch_batch<BATCH_F32>(const BatchK &, int, cudaStream_t);
 template cudaError_t launch_batch<BATCH_BF16>(const BatchK &, int, cudaStream_t);
 template cudaError_t launch_batch<BATCH_F16>(const BatchK &, int, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_F32>(const BatchK &, const BatchGroup *, int, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_BF16>(const BatchK &, const BatchGroup *, int, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_F16>(const BatchK &, const BatchGroup *, int, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_F32>(const BatchK &, const BVar *const *, int, uint32_t, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_BF16>(const BatchK &, const BVar *const *, int, uint32_t, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_F16>(const BatchK &, const BVar *const *, int, uint32_t, cudaStream_t);
 template int batch_max_blocks_per_sm<BATCH_F32>();
 template int batch_max_blocks_per_sm<BATCH_BF16>();
 template int batch_max_blocks_per_sm<BATCH_F16>();
 template cudaError_t launch_batch<BATCH_BF16U>(const BatchK &, int, cudaStream_t);
-template cudaError_t launch_batch_steps<BATCH_BF16U>(const BatchK &, const BatchGroup *, int, cudaStream_t);
+template cudaError_t launch_batch_steps<BATCH_BF16U>(const BatchK &, const BVar *const *, int, uint32_t, cudaStream_t);
 template int batch_max_blocks_per_sm<BATCH_BF16U>();
 
 }  // namespace fdtd

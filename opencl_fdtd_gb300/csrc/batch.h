@@ -66,12 +66,6 @@ template <int ST>
 cudaError_t launch_batch(const BatchK &k, int blocks, cudaStream_t st);
 template <int ST>
 int batch_max_blocks_per_sm();
-// The launches of a half-step: a variant of its own (one; planes per thread, 0: chosen by the launcher), or
-// the tiles of every variant that has none.
-struct BatchGroup {
-    const BVar *one;
-    uint32_t xchunk;
-};
 struct BatchOne {
     BVar v;
     int64_t *step;
@@ -80,9 +74,10 @@ struct BatchOne {
     int32_t t, advance;
 };
 
-// For each group of variants: nsteps x (one launch of its E update, one of its H update)
+// For each group of variants (one of its own, or NULL: the tiles of those that share a launch): nsteps x (one
+// launch of its E update, one of its H update). xchunk: planes per thread of the former, 0: fit_xchunk.
 template <int ST>
-cudaError_t launch_batch_steps(const BatchK &k, const BatchGroup *groups, int n, cudaStream_t st);
+cudaError_t launch_batch_steps(const BatchK &k, const BVar *const *groups, int n, uint32_t xchunk, cudaStream_t st);
 
 // f32 <-> storage of one field of one variant, choosing the tile exponents (encode)
 cudaError_t launch_batch_encode(int store, const BVar &v, int field, const float *src, cudaStream_t st);

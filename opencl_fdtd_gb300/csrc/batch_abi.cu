@@ -18,16 +18,16 @@ struct FdtdBatch {
     int storage;
     int device;
     int64_t rows;
-    uint32_t xchunk;
+    uint32_t xchunk;             // planes per tile asked for (0: automatic)
+    uint32_t tile_xchunk;        // planes per tile of the tile list
     int blocks_per_sm;
     int schedule;                // FDTD_BATCH_PERSISTENT or FDTD_BATCH_LAUNCHES
     std::vector<BVar> host;      // descriptors as uploaded
     BVar *vars = nullptr;        // device copy
     int4 *tiles = nullptr;       // device tile list
     uint32_t ntiles = 0;
-    std::vector<BatchGroup> groups;    // the launches of a half-step (build_tiles)
+    std::vector<const BVar *> groups;  // the launches of a half-step (build_tiles): a variant, or NULL for those that share one
     uint32_t shared = 0;               // tiles of the variants that share launches
-    bool tuned = false;
     int64_t *step = nullptr;     // device step counter
     uint32_t *work = nullptr;    // persistent schedule's two tile counters
 };
@@ -36,7 +36,7 @@ namespace {
 
 int fail(int code, const std::string &msg) { return set_error(code, msg.c_str()); }
 
-// Planes per tile until fdtd_batch_tune sets them: 8 (12: 1% faster on 8 variants of 1.8 M cells, 4: 6%
+// Planes per tile unless fdtd_batch_tune sets them: 8 (12: 1% faster on 8 variants of 1.8 M cells, 4: 6%
 // slower), fewer where that would leave resident blocks without a tile: two variants of 0.1 M cells took
 // 25 us a step at 8 and 19 at 4.
 uint32_t default_xchunk(const FdtdBatch *b)
@@ -64,10 +64,11 @@ int build_tiles(FdtdBatch *b)
         for (size_t v = 0; v < b->host.size(); ++v) {
             const BVar &h = b->host[v];
             if (launched_alone(h, b->storage) != (alone != 0)) continue;
-            if (alone || b->groups.empty()) b->groups.push_back({alone ? &h : nullptr, b->tuned ? b->xchunk : 0u});
-            for (uint32_t x0 = 0; x0 < h.sx; x0 += b->xchunk)
+            if (alone || b->groups.empty()) b->groups.push_back(alone ? &h : nullptr);
+            const uint32_t xc = b->tile_xchunk;
+            for (uint32_t x0 = 0; x0 < h.sx; x0 += xc)
                 for (uint32_t jb = 0; jb < h.njb; ++jb)
-                    t.push_back(make_int4((int)v, (int)x0, (int)(x0 + b->xchunk < h.sx ? x0 + b->xchunk : h.sx), (int)jb));
+                    t.push_back(make_int4((int)v, (int)x0, (int)(x0 + xc < h.sx ? x0 + xc : h.sx), (int)jb));
             if (!alone) b->shared = (uint32_t)t.size();
         }
     if (b->tiles) cudaFree(b->tiles);
@@ -193,7 +194,7 @@ int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, 
     FdtdBatch *b = new FdtdBatch();
     b->storage = storage;
     b->rows = rows;
-    b->xchunk = 8;              // see default_xchunk
+    b->xchunk = 0;
     b->blocks_per_sm = 0;
     b->schedule = FDTD_BATCH_LAUNCHES;
     cudaGetDevice(&b->device);
@@ -209,7 +210,7 @@ int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, 
     if (!rc) rc = check_cuda(cudaMalloc(&b->work, 2 * sizeof(uint32_t)), "cudaMalloc(batch work counters)");
     if (!rc) rc = check_cuda(cudaMemset(b->work, 0, 2 * sizeof(uint32_t)), "clear batch work counters");
     if (!rc) {
-        b->xchunk = default_xchunk(b);
+        b->tile_xchunk = default_xchunk(b);
         rc = build_tiles(b);
     }
     if (rc) {
@@ -234,15 +235,15 @@ int fdtd_batch_destroy(FdtdBatch *b)
 int fdtd_batch_tune(FdtdBatch *b, int32_t xchunk, int32_t blocks_per_sm)
 {
     if (!b) return fail(FDTD_ERR_INVALID, "batch is NULL");
-    if (xchunk < 1 || xchunk > 4096) return fail(FDTD_ERR_INVALID, "xchunk must be in [1, 4096]");
+    if (xchunk < 0 || xchunk > 4096) return fail(FDTD_ERR_INVALID, "xchunk must be in [0, 4096] (0: automatic)");
     if (blocks_per_sm < 0 || blocks_per_sm > 32) return fail(FDTD_ERR_INVALID, "blocks_per_sm must be in [0, 32]");
     b->blocks_per_sm = blocks_per_sm;
-    if ((uint32_t)xchunk != b->xchunk || !b->tuned) {
-        b->xchunk = (uint32_t)xchunk;
-        b->tuned = true;
-        return build_tiles(b);
-    }
-    return FDTD_OK;
+    b->xchunk = (uint32_t)xchunk;
+    // the tile list stays where it is unless it changes: a captured run refers to it
+    const uint32_t tile = b->xchunk ? b->xchunk : default_xchunk(b);
+    if (tile == b->tile_xchunk) return FDTD_OK;
+    b->tile_xchunk = tile;
+    return build_tiles(b);
 }
 
 int fdtd_batch_run(FdtdBatch *b, void *stream, int32_t nsteps)
@@ -269,12 +270,12 @@ int fdtd_batch_run(FdtdBatch *b, void *stream, int32_t nsteps)
     cudaError_t e;
     if (b->schedule == FDTD_BATCH_LAUNCHES) {
         k.ntiles = b->shared;
-        const BatchGroup *const groups = b->groups.data();
+        const BVar *const *const groups = b->groups.data();
         const int ng = (int)b->groups.size();
-        if (b->storage == BATCH_BF16) e = launch_batch_steps<BATCH_BF16>(k, groups, ng, st);
-        else if (b->storage == BATCH_F16) e = launch_batch_steps<BATCH_F16>(k, groups, ng, st);
-        else if (b->storage == BATCH_BF16U) e = launch_batch_steps<BATCH_BF16U>(k, groups, ng, st);
-        else e = launch_batch_steps<BATCH_F32>(k, groups, ng, st);
+        if (b->storage == BATCH_BF16) e = launch_batch_steps<BATCH_BF16>(k, groups, ng, b->xchunk, st);
+        else if (b->storage == BATCH_F16) e = launch_batch_steps<BATCH_F16>(k, groups, ng, b->xchunk, st);
+        else if (b->storage == BATCH_BF16U) e = launch_batch_steps<BATCH_BF16U>(k, groups, ng, b->xchunk, st);
+        else e = launch_batch_steps<BATCH_F32>(k, groups, ng, b->xchunk, st);
         return check_cuda(e, "batch launch");
     }
     if (b->storage == BATCH_BF16) e = launch_batch<BATCH_BF16>(k, per * nsm, st);

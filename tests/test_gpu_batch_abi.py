@@ -70,3 +70,87 @@ def test_more_planes_than_a_grid_has_rows(shape, xchunk):
     persistent schedule has no such limit."""
     for a, b in zip(_result([shape], (2, 1), xchunk=xchunk), _result([shape], (2, 1), persistent=True)):
         assert torch.equal(a, b)
+
+
+def test_automatic_tiles_can_be_asked_for_again():
+    """A tile length of 0 is the automatic one: the same launches, and the same tile list, which a
+    captured run refers to, as before the batch was tuned to what it had chosen."""
+    shapes, steps = [(128, 72, 64), (64, 64, 37), (80, 80, 80)], (1, 2)
+    ref = _result(shapes, steps)
+    for chunks in ((0,), (3, 0), (8, 0)):
+        b = _Batch(shapes, sum(steps))
+        for c in chunks:
+            b.check(b.lib.fdtd_batch_tune(b.handle, c, 0))
+        for n in steps:
+            b.run(n)
+        out = b.state()
+        b.close()
+        for x, y in zip(ref, out):
+            assert torch.equal(x, y)
+    # 25 blocks a plane and 238 planes that share launches, far more than the GPU holds: 8 planes a tile
+    shapes = [(80, 79, 79), (79, 80, 79), (79, 79, 80)]
+    ref = _result(shapes, steps)
+    b = _Batch(shapes, sum(steps))
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        b.run(1, stream)
+    b.check(b.lib.fdtd_batch_tune(b.handle, 8, 0))
+    b.check(b.lib.fdtd_batch_tune(b.handle, 0, 0))
+    for _ in range(sum(steps)):
+        graph.replay()
+    for x, y in zip(ref, b.state()):
+        assert torch.equal(x, y)
+    del graph
+    b.close()
+
+
+def _simulations():
+    from opencl_fdtd_gb300 import Simulation
+    sims = []
+    for shape in ((84, 77, 79), (12, 10, 9)):
+        rng = numpy.random.default_rng(shape[0])
+        sims.append(Simulation([rng.uniform(1, 4, shape).astype(numpy.float32) for _ in range(3)], [], do_poynting=False,
+                               initial_fields={k: [rng.standard_normal(shape).astype(numpy.float32) for _ in range(3)]
+                                               for k in "EH"}))
+    return sims
+
+
+def test_tune_keeps_the_automatic_tiles():
+    from opencl_fdtd_gb300.batch import BatchSimulation
+    b = BatchSimulation(_simulations())
+    assert b.xchunk == 0
+    b.tune(schedule="persistent")
+    b.tune(schedule="launches")
+    assert b.xchunk == 0
+    b.tune(xchunk=5)
+    b.tune(blocks_per_sm=1)
+    assert b.xchunk == 5
+    b.tune(xchunk=0)
+    assert b.xchunk == 0
+
+
+def test_autotune_times_the_automatic_tiles(monkeypatch):
+    from opencl_fdtd_gb300 import autotune
+    from opencl_fdtd_gb300.batch import BatchSimulation
+    b = BatchSimulation(_simulations())
+    monkeypatch.setattr(autotune, "_MEMO", {})
+    monkeypatch.setattr(autotune, "time_config",
+                        lambda batch, xc, blocks, steps, sched: 1.0 if (xc, sched) == (0, "launches") else 2.0)
+    choice = b.autotune(steps=1)
+    assert (choice["xchunk"], choice["schedule"]) == (0, "launches") and b.xchunk == 0
+    assert b.autotune(steps=1)["cached"] and b.xchunk == 0
+
+
+def test_captured_run_with_a_variant_launched_alone():
+    """The descriptor of such a variant is in the captured launches themselves."""
+    from opencl_fdtd_gb300.batch import BatchSimulation
+    ref, sims = _simulations(), _simulations()
+    BatchSimulation(ref).run(6)
+    b = BatchSimulation(sims)
+    b.capture(2)
+    for _ in range(3):
+        b.replay()
+    torch.cuda.synchronize()
+    assert b.step_counter() == 6
+    for x, y in zip(ref, sims):
+        assert torch.equal(x.E, y.E) and torch.equal(x.H, y.H)
