@@ -121,8 +121,9 @@ int fdtd_plan_create(const FdtdDesc *desc, FdtdPlan **out);
 int fdtd_plan_destroy(FdtdPlan *plan);
 
 /* Tuning keys of fdtd_plan_tune. Any values give the same results.
- *   XCHUNK        consecutive x planes one thread of the update kernels advances (default 8, fewer
- *                 on grids too small to fill the GPU with that many)
+ *   XCHUNK        consecutive x planes one thread of the update kernels advances; 0 (default):
+ *                 chosen per launch (1 in double precision; else 8, or on grids of a few waves of
+ *                 blocks the number up to 12 with the shortest whole waves)
  *   SLAB          x planes per L2-resident slab of fdtd_run's per-update schedule
  *                 (default 0 = whole grid)
  *   FUSED_ROWS    own y rows of a tile of the one-pass step (default 0: the most that fit a

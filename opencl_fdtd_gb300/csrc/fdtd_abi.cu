@@ -1143,7 +1143,7 @@ int fdtd_plan_tune(FdtdPlan *p, int32_t key, int32_t value)
     if (!p) return fail(FDTD_ERR_INVALID, "plan is NULL");
     switch (key) {
     case FDTD_TUNE_XCHUNK:
-        if (value < 1 || value > 4096) return fail(FDTD_ERR_INVALID, "xchunk must be in [1, 4096]");
+        if (value < 0 || value > 4096) return fail(FDTD_ERR_INVALID, "xchunk must be in [0, 4096] (0: automatic)");
         p->xchunk = value;
         return FDTD_OK;
     case FDTD_TUNE_SLAB:
@@ -1212,7 +1212,7 @@ int fdtd_plan_get(const FdtdPlan *p, int32_t key, int32_t *value)
 {
     if (!p || !value) return fail(FDTD_ERR_INVALID, "plan or value is NULL");
     switch (key) {
-    case FDTD_TUNE_XCHUNK: *value = p->xchunk ? p->xchunk : 8; return FDTD_OK;
+    case FDTD_TUNE_XCHUNK: *value = (int32_t)p->xchunk; return FDTD_OK;
     case FDTD_TUNE_SLAB: *value = (int32_t)p->slab; return FDTD_OK;
     case FDTD_TUNE_FUSED_ROWS: *value = (int32_t)p->fused_rows; return FDTD_OK;
     case FDTD_TUNE_FUSED_XCHUNK: *value = (int32_t)p->fused_xchunk; return FDTD_OK;

@@ -676,6 +676,7 @@ class Simulation:
              e_form: int = None):
         """Kernel tiling and launch options (None keeps a value); results do not depend on them.
 
+        xchunk: x planes per thread of the per-update kernels (0, the default: automatic);
         fused_rows / fused_xchunk / fused_stages: own y rows of a one-pass step tile, x planes
         of a block, planes in its shared-memory ring (0: automatic); fused_tma: stage the rows
         of non-wrapping tiles with bulk asynchronous copies (default) or per element;
