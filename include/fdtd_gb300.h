@@ -368,6 +368,13 @@ int fdtd_batch_tune(FdtdBatch *batch, int32_t xchunk, int32_t blocks_per_sm);
 #define FDTD_BATCH_LAUNCHES 1
 int fdtd_batch_schedule(FdtdBatch *batch, int32_t schedule);
 int fdtd_batch_run(FdtdBatch *batch, void *stream, int32_t nsteps);
+/* Tiling of the batch: the planes per tile asked for (0: automatic), those of the launches that
+ * variants share, and the launches per step (0 with the persistent schedule, which has one per
+ * run). */
+#define FDTD_BATCH_GET_XCHUNK 0
+#define FDTD_BATCH_GET_TILE_XCHUNK 1
+#define FDTD_BATCH_GET_STEP_LAUNCHES 2
+int fdtd_batch_get(const FdtdBatch *batch, int32_t key, int32_t *value);
 /* Read / set the batch's device step counter (waits for the device). */
 int fdtd_batch_get_step(FdtdBatch *batch, int64_t *step);
 int fdtd_batch_set_step(FdtdBatch *batch, int64_t step);

@@ -97,6 +97,7 @@ class FdtdDftMonitor(ctypes.Structure):
 FDTD_STORE_F32, FDTD_STORE_BF16, FDTD_STORE_F16, FDTD_STORE_BF16U = 0, 1, 2, 3
 FDTD_BATCH_MAX_SRC, FDTD_BATCH_MAX_MON = 4, 8
 FDTD_BATCH_PERSISTENT, FDTD_BATCH_LAUNCHES = 0, 1
+FDTD_BATCH_GET_XCHUNK, FDTD_BATCH_GET_TILE_XCHUNK, FDTD_BATCH_GET_STEP_LAUNCHES = 0, 1, 2
 
 
 class FdtdBatchFace(ctypes.Structure):
@@ -142,6 +143,7 @@ SIGNATURES = [
     ("fdtd_batch_tune", c_i32, [c_vp, c_i32, c_i32]),
     ("fdtd_batch_schedule", c_i32, [c_vp, c_i32]),
     ("fdtd_batch_run", c_i32, [c_vp, c_vp, c_i32]),
+    ("fdtd_batch_get", c_i32, [c_vp, c_i32, _P(c_i32)]),
     ("fdtd_batch_get_step", c_i32, [c_vp, _P(c_i64)]),
     ("fdtd_batch_set_step", c_i32, [c_vp, c_i64]),
     ("fdtd_batch_encode", c_i32, [c_vp, c_i32, c_i32, c_vp, c_vp]),

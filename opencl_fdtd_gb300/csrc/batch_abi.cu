@@ -19,7 +19,7 @@ struct FdtdBatch {
     int device;
     int64_t rows;
     uint32_t xchunk;             // planes per tile asked for (0: automatic)
-    uint32_t tile_xchunk;        // planes per tile of the tile list
+    uint32_t tile_xchunk[2];     // planes per tile: of the shared launches, of the persistent schedule
     int blocks_per_sm;
     int schedule;                // FDTD_BATCH_PERSISTENT or FDTD_BATCH_LAUNCHES
     std::vector<BVar> host;      // descriptors as uploaded
@@ -27,7 +27,7 @@ struct FdtdBatch {
     int4 *tiles = nullptr;       // device tile list
     uint32_t ntiles = 0;
     std::vector<const BVar *> groups;  // the launches of a half-step (build_tiles): a variant, or NULL for those that share one
-    uint32_t shared = 0;               // tiles of the variants that share launches
+    uint32_t shared = 0;               // tiles of the shared launches, at the head of the list
     int64_t *step = nullptr;     // device step counter
     uint32_t *work = nullptr;    // persistent schedule's two tile counters
 };
@@ -36,40 +36,54 @@ namespace {
 
 int fail(int code, const std::string &msg) { return set_error(code, msg.c_str()); }
 
-// Planes per tile unless fdtd_batch_tune sets them: 8 (12: 1% faster on 8 variants of 1.8 M cells, 4: 6%
-// slower), fewer where that would leave resident blocks without a tile: two variants of 0.1 M cells took
-// 25 us a step at 8 and 19 at 4.
-uint32_t default_xchunk(const FdtdBatch *b)
-{
-    int nsm = 0;
-    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || nsm < 1) return 8;
-    uint64_t planes = 0;
-    for (const BVar &h : b->host) planes += (uint64_t)h.njb * h.sx;
-    const uint64_t slots = 4ull * (uint64_t)nsm;
-    return planes >= 8 * slots ? 8u : (uint32_t)(planes / slots > 1 ? planes / slots : 1);
-}
-
 // Whether a variant's updates are launches of their own in the launches schedule: the descriptor is then
 // among the kernel's arguments, which spares the march's registers and reloads, at the price of a tail per
 // launch. Float32: 8 variants of 1.8 M cells 0.331 to 0.286 ms a step, 3 of 0.95 M 87 to 64 us, 6 of 0.5 M 86
 // to 82, but 6 of 0.2 M 36 to 55. With 16-bit storage the tiles spill less and it lost (0.298 to 0.303 ms).
 bool launched_alone(const BVar &h, int storage) { return storage == BATCH_F32 && h.N >= 500000; }
 
+// Planes per tile of the shared launches and of the persistent schedule, unless fdtd_batch_tune sets them:
+// 8 (12: 1% faster on 8 variants of 1.8 M cells, 4: 6% slower), fewer where that would leave resident blocks
+// without a tile: two variants of 0.1 M cells took 25 us a step at 8 and 19 at 4. The shared launches hold
+// nothing but their own variants (one of 0.1 M cells beside one of 1.8 M: 34.6 us a step with 8 planes,
+// 28.3 with 1); the persistent schedule hands out all tiles (the same batch 30.3 and 33.1).
+void tile_lengths(const FdtdBatch *b, uint32_t xc[2])
+{
+    xc[0] = xc[1] = b->xchunk ? b->xchunk : 8u;
+    int nsm = 0;
+    if (b->xchunk || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || nsm < 1) return;
+    uint64_t planes[2] = {0, 0};
+    for (const BVar &h : b->host) {
+        const uint64_t n = (uint64_t)h.njb * h.sx;
+        if (!launched_alone(h, b->storage)) planes[0] += n;
+        planes[1] += n;
+    }
+    const uint64_t slots = 4ull * (uint64_t)nsm;
+    for (int g = 0; g < 2; ++g)
+        if (planes[g] < 8 * slots) xc[g] = (uint32_t)(planes[g] / slots > 1 ? planes[g] / slots : 1);
+}
+
+// The tile list: the tiles of the shared launches, then all variants' as the persistent schedule hands them out.
 int build_tiles(FdtdBatch *b)
 {
     std::vector<int4> t;
+    const auto add = [&](size_t v, uint32_t xc) {
+        const BVar &h = b->host[v];
+        for (uint32_t x0 = 0; x0 < h.sx; x0 += xc)
+            for (uint32_t jb = 0; jb < h.njb; ++jb)
+                t.push_back(make_int4((int)v, (int)x0, (int)(x0 + xc < h.sx ? x0 + xc : h.sx), (int)jb));
+    };
     b->groups.clear();
-    // the variants that share launches first
+    for (size_t v = 0; v < b->host.size(); ++v)
+        if (!launched_alone(b->host[v], b->storage)) add(v, b->tile_xchunk[0]);
+    b->shared = (uint32_t)t.size();
+    if (b->shared) b->groups.push_back(nullptr);
     for (int alone = 0; alone < 2; ++alone)
         for (size_t v = 0; v < b->host.size(); ++v) {
             const BVar &h = b->host[v];
             if (launched_alone(h, b->storage) != (alone != 0)) continue;
-            if (alone || b->groups.empty()) b->groups.push_back(alone ? &h : nullptr);
-            const uint32_t xc = b->tile_xchunk;
-            for (uint32_t x0 = 0; x0 < h.sx; x0 += xc)
-                for (uint32_t jb = 0; jb < h.njb; ++jb)
-                    t.push_back(make_int4((int)v, (int)x0, (int)(x0 + xc < h.sx ? x0 + xc : h.sx), (int)jb));
-            if (!alone) b->shared = (uint32_t)t.size();
+            if (alone) b->groups.push_back(&h);
+            add(v, b->tile_xchunk[1]);
         }
     if (b->tiles) cudaFree(b->tiles);
     b->tiles = nullptr;
@@ -210,7 +224,7 @@ int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, 
     if (!rc) rc = check_cuda(cudaMalloc(&b->work, 2 * sizeof(uint32_t)), "cudaMalloc(batch work counters)");
     if (!rc) rc = check_cuda(cudaMemset(b->work, 0, 2 * sizeof(uint32_t)), "clear batch work counters");
     if (!rc) {
-        b->tile_xchunk = default_xchunk(b);
+        tile_lengths(b, b->tile_xchunk);
         rc = build_tiles(b);
     }
     if (rc) {
@@ -240,9 +254,11 @@ int fdtd_batch_tune(FdtdBatch *b, int32_t xchunk, int32_t blocks_per_sm)
     b->blocks_per_sm = blocks_per_sm;
     b->xchunk = (uint32_t)xchunk;
     // the tile list stays where it is unless it changes: a captured run refers to it
-    const uint32_t tile = b->xchunk ? b->xchunk : default_xchunk(b);
-    if (tile == b->tile_xchunk) return FDTD_OK;
-    b->tile_xchunk = tile;
+    uint32_t xc[2];
+    tile_lengths(b, xc);
+    if (xc[0] == b->tile_xchunk[0] && xc[1] == b->tile_xchunk[1]) return FDTD_OK;
+    b->tile_xchunk[0] = xc[0];
+    b->tile_xchunk[1] = xc[1];
     return build_tiles(b);
 }
 
@@ -278,6 +294,8 @@ int fdtd_batch_run(FdtdBatch *b, void *stream, int32_t nsteps)
         else e = launch_batch_steps<BATCH_F32>(k, groups, ng, b->xchunk, st);
         return check_cuda(e, "batch launch");
     }
+    k.tiles = b->tiles + b->shared;
+    k.ntiles = b->ntiles - b->shared;
     if (b->storage == BATCH_BF16) e = launch_batch<BATCH_BF16>(k, per * nsm, st);
     else if (b->storage == BATCH_F16) e = launch_batch<BATCH_F16>(k, per * nsm, st);
     else if (b->storage == BATCH_BF16U) e = launch_batch<BATCH_BF16U>(k, per * nsm, st);
@@ -292,6 +310,17 @@ int fdtd_batch_schedule(FdtdBatch *b, int32_t schedule)
         return fail(FDTD_ERR_INVALID, "schedule must be FDTD_BATCH_PERSISTENT or FDTD_BATCH_LAUNCHES");
     b->schedule = schedule;
     return FDTD_OK;
+}
+
+int fdtd_batch_get(const FdtdBatch *b, int32_t key, int32_t *value)
+{
+    if (!b || !value) return fail(FDTD_ERR_INVALID, "fdtd_batch_get: NULL pointer");
+    switch (key) {
+    case FDTD_BATCH_GET_XCHUNK: *value = (int32_t)b->xchunk; return FDTD_OK;
+    case FDTD_BATCH_GET_TILE_XCHUNK: *value = (int32_t)b->tile_xchunk[0]; return FDTD_OK;
+    case FDTD_BATCH_GET_STEP_LAUNCHES: *value = b->schedule == FDTD_BATCH_LAUNCHES ? 2 * (int32_t)b->groups.size() : 0; return FDTD_OK;
+    default: return fail(FDTD_ERR_INVALID, "fdtd_batch_get: unknown key");
+    }
 }
 
 int fdtd_batch_get_step(FdtdBatch *b, int64_t *step)

@@ -154,3 +154,22 @@ def test_captured_run_with_a_variant_launched_alone():
     assert b.step_counter() == 6
     for x, y in zip(ref, sims):
         assert torch.equal(x.E, y.E) and torch.equal(x.H, y.H)
+
+
+@pytest.mark.parametrize("shapes,length,launches", [
+    ([(48, 47, 45)], 1, 2),                                  # 432 blocks for the GPU's 608 places
+    ([(48, 47, 45), (165, 150, 73)], 1, 4),                  # beside a variant launched alone: the same
+    ([(48, 47, 45)] * 4, 2, 2),
+    ([(80, 79, 79), (79, 80, 79), (79, 79, 80)], 8, 2),
+])
+def test_shared_launches_hold_their_own_variants(shapes, length, launches):
+    from opencl_fdtd_gb300 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count != 152:
+        pytest.skip("the lengths are those of 152 SMs")
+    b = _Batch(shapes, 1)
+    v = ctypes.c_int32()
+    for key, want in ((_lib.FDTD_BATCH_GET_XCHUNK, 0), (_lib.FDTD_BATCH_GET_TILE_XCHUNK, length),
+                      (_lib.FDTD_BATCH_GET_STEP_LAUNCHES, launches)):
+        b.check(b.lib.fdtd_batch_get(b.handle, key, ctypes.byref(v)))
+        assert v.value == want, key
+    b.close()
