@@ -533,6 +533,8 @@ class Simulation:
         if path == "hs" and not self.do_poynting:
             raise ValueError("the 'hs' path needs do_poynting=True")
         mode = None if path == "plain" else path
+        if mode == "ahead" and self._faces_overlap():
+            mode = None
         if mode == "ahead" and (self._np_dtype == numpy.float64 or getattr(self, "_lbc_keep", None) is not None
                                 or not self._try_scratch("ahead")):
             mode = "hs" if self.do_poynting else None
@@ -568,9 +570,10 @@ class Simulation:
         fastest below 1e5 cells, where launches are the cost (24^3 5.3 us a step against 6.1 of 'hs'),
         and where the fields exceed the L2 (170x175x65 48.8 against 54.4, 200^3 148 against 185); in
         between 'hs', which evaluates fewer values twice (64^3 12.0 against 13.0, 128x100x50 20.6
-        against 22.4, 151x129x61 31.4 against 34.1)."""
+        against 22.4, 151x129x61 31.4 against 34.1). Where two faces of one axis overlap, every path
+        is the per-update one, and the others' copies would be memory for nothing."""
         hs = "hs" if self.do_poynting else "plain"
-        if self.bloch_boundaries or self._np_dtype == numpy.float64:
+        if self.bloch_boundaries or self._np_dtype == numpy.float64 or self._faces_overlap():
             return "plain"
         if nsteps < 2 or getattr(self, "_lbc_keep", None) is not None:
             return hs
@@ -578,6 +581,14 @@ class Simulation:
         if not self.do_poynting:
             return "plain" if 60 * self.N <= l2 or self.tuning("slab") else "ahead"
         return "hs" if self.N > 100000 and 84 * self.N <= l2 else "ahead"
+
+    def _faces_overlap(self) -> bool:
+        """Whether two CPML faces of one axis share cells (a 'p' face thicker than its axis never applies)."""
+        thick = [0, 0, 0]
+        for a, pol, T, _, _ in self._pml_tables:
+            if pol == 0 or T <= self.shape[a]:
+                thick[a] += T
+        return any(t > s for t, s in zip(thick, self.shape))
 
     def _try_scratch(self, mode) -> bool:
         """The second copies of a run path, or False when the device has no room for them."""
