@@ -204,6 +204,7 @@ class Simulation:
         self._buf = _lib.FdtdBuffers()
         self._scratch = None
         self._ahead = False
+        self._refused = False
         self.steps_run = 0
 
         self.update_E = self._create_operation(self._lib.fdtd_update_e)
@@ -591,10 +592,19 @@ class Simulation:
         return any(t > s for t, s in zip(thick, self.shape))
 
     def _try_scratch(self, mode) -> bool:
-        """The second copies of a run path, or False when the device has no room for them."""
+        """The second copies of a run path, or False when the device has no room for them. A refused
+        allocation flushes the allocator's cache, so after one the next try waits for room."""
+        have = self._scratch if self._scratch is not None else (None, None)
+        if self._refused and (have[0] is None or have[1] is None):
+            need = sum(t.numel() * t.element_size() for k, f in (("E", have[0]), ("H", have[1])) if f is None
+                       for t in [getattr(self, k)] + [t for pair in self.psi[k] for t in pair])
+            cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+            if torch.cuda.mem_get_info(self.device)[0] + cached < need:
+                return False
         try:
             self._ensure_scratch(mode)
         except torch.cuda.OutOfMemoryError:
+            self._refused = True
             return False
         return True
 

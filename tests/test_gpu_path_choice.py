@@ -48,3 +48,25 @@ def test_overlapping_faces_need_no_copies(faces, overlap, path, poynting):
     _same(a, b)
     if overlap:
         assert b._scratch is None and b.tuning("last_run_path") == 1
+
+
+@pytest.mark.parametrize("poynting", [True, False])
+def test_no_room_for_the_copies(poynting, monkeypatch):
+    """A refused copy of E sends 'ahead' to the path that needs none, with the same results."""
+    from opencl_fdtd_gb300 import Simulation
+    a, b = _sim(poynting=poynting), _sim(poynting=poynting)
+    ensure = Simulation._ensure_scratch
+
+    def refuse(self, mode):
+        if mode == "ahead":
+            raise torch.cuda.OutOfMemoryError("no room")
+        ensure(self, mode)
+    monkeypatch.setattr(Simulation, "_ensure_scratch", refuse)
+    _loop(a, 7)
+    for n in (4, 3):
+        b.run(n, path="ahead")
+        assert b.tuning("last_run_path") == (2 if poynting else 1)
+    _same(a, b)
+    assert (b._scratch is None) == (not poynting)
+    if poynting:
+        assert b._scratch[0] is None and b._scratch[1] is not None
