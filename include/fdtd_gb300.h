@@ -179,7 +179,8 @@ int fdtd_plan_destroy(FdtdPlan *plan);
 #define FDTD_TUNE_HS_AHEAD 16
 /* Read-only keys of fdtd_plan_get: the path of the last fdtd_run (FDTD_PATH_*), the tiling
  * of its last one-pass launch (own rows per tile, x chunk, stages, threads per block, shape)
- * and the x chunk of its last H+S launch. */
+ * the x chunk of its last H+S launch, and whether the H launches of the last fdtd_run also made
+ * the next step's E (FDTD_TUNE_HS_AHEAD). */
 #define FDTD_GET_LAST_RUN_PATH 100
 #define FDTD_GET_STEP_ROWS 101
 #define FDTD_GET_STEP_XCHUNK 102
@@ -187,6 +188,7 @@ int fdtd_plan_destroy(FdtdPlan *plan);
 #define FDTD_GET_STEP_THREADS 104
 #define FDTD_GET_STEP_SHAPE 105
 #define FDTD_GET_HS_XCHUNK_USED 106
+#define FDTD_GET_LAST_RUN_AHEAD 107
 #define FDTD_PATH_NONE 0
 #define FDTD_PATH_PER_UPDATE 1     /* update_E, sources, update_H, update_S launches */
 #define FDTD_PATH_HS 2             /* H and S in one launch, after update_E or (HS_AHEAD) with the next step's E */

@@ -45,6 +45,7 @@ FDTD_GET_STEP_STAGES = 103
 FDTD_GET_STEP_THREADS = 104
 FDTD_GET_STEP_SHAPE = 105
 FDTD_GET_HS_XCHUNK_USED = 106
+FDTD_GET_LAST_RUN_AHEAD = 107
 FDTD_PATH_NONE = 0
 FDTD_PATH_PER_UPDATE = 1
 FDTD_PATH_HS = 2

@@ -1076,6 +1076,7 @@ int fdtd_plan_create(const FdtdDesc *desc, FdtdPlan **out)
     p->hs_xchunk_used = 0;
     p->hs_dft = 1;
     p->hs_ahead = 0;
+    p->ran_ahead = 0;
     p->pdl = 1;
     p->timing = 0;
     p->kernel_ms[0] = p->kernel_ms[1] = 0.0;
@@ -1229,6 +1230,7 @@ int fdtd_plan_get(const FdtdPlan *p, int32_t key, int32_t *value)
     case FDTD_TUNE_HS_XCHUNK: *value = (int32_t)p->hs_xchunk; return FDTD_OK;
     case FDTD_TUNE_HS_PREFETCH: *value = p->hs_prefetch; return FDTD_OK;
     case FDTD_GET_HS_XCHUNK_USED: *value = p->hs_xchunk_used; return FDTD_OK;
+    case FDTD_GET_LAST_RUN_AHEAD: *value = p->ran_ahead; return FDTD_OK;
     case FDTD_TUNE_HS_DFT: *value = p->hs_dft; return FDTD_OK;
     case FDTD_TUNE_PDL: *value = p->pdl; return FDTD_OK;
     case FDTD_TUNE_E_FORM: *value = p->eform; return FDTD_OK;
@@ -1474,10 +1476,12 @@ int fdtd_run(FdtdPlan *p, const FdtdBuffers *b, void *stream, int32_t nsteps,
     if ((rc = check_monitor(p, mon))) return rc;
     const bool f64 = p->d.dtype == FDTD_F64;
     const bool ahead = p->hs_ahead && hs_eligible(p, b, true);
+    p->ran_ahead = 0;
     if (ahead || (!b->E2 && hs_eligible(p, b, false))) {
         if ((rc = check_run_buffers(p, b))) return rc;
         cudaStream_t st = (cudaStream_t)stream;
         p->last_run_path = FDTD_PATH_HS;
+        p->ran_ahead = ahead && nsteps > 1;
         rc = f64 ? run_hs<double>(p, b, st, nsteps, src, mon, ahead) : run_hs<float>(p, b, st, nsteps, src, mon, ahead);
         if (!rc && mon) { mon->step += nsteps; mon->series_row += nsteps; }
         return rc;

@@ -27,6 +27,7 @@ struct FdtdPlan {
     int32_t hs_reverse;         // H+S kernel takes its x chunks in descending order
     int32_t hs_xchunk_used;     // x chunk of the last H+S launch (hs_xchunk or the automatic one)
     int32_t hs_ahead;           // H path: with second copies of E, make the next step's E in the H launch
+    int32_t ran_ahead;          // the last fdtd_run did so
     int32_t hs_dft;             // H+S path: the DFT sample in the H+S launch, not a side stream
     int32_t pdl;                // fdtd_run: programmatic dependent launches of E and H
     int32_t timing;             // fdtd_run's H+S path records per-kernel CUDA events

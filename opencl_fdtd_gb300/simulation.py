@@ -726,7 +726,8 @@ class Simulation:
         """Current value of a tuning key ('fused_rows', 'hs_xchunk', ...) or of a read-only key:
         'last_run_path' (0 none, 1 per-update, 2 H+S, 3 one-pass), 'step_rows',
         'step_xchunk', 'step_stages', 'step_threads', 'step_shape' (tiling of the last one-pass
-        launch) and 'hs_xchunk_used' (x chunk of the last H+S launch)."""
+        launch), 'hs_xchunk_used' (x chunk of the last H+S launch) and 'last_run_ahead' (1 when the
+        H launches of the last run also made the next step's E)."""
         name = key.upper()
         const = getattr(_lib, "FDTD_GET_" + name, None)
         if const is None:

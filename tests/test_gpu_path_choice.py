@@ -65,8 +65,50 @@ def test_no_room_for_the_copies(poynting, monkeypatch):
     _loop(a, 7)
     for n in (4, 3):
         b.run(n, path="ahead")
+        assert b.tuning("last_run_ahead") == 0
         assert b.tuning("last_run_path") == (2 if poynting else 1)
     _same(a, b)
     assert (b._scratch is None) == (not poynting)
     if poynting:
         assert b._scratch[0] is None and b._scratch[1] is not None
+
+
+def _graded(shape, rng=numpy.random.default_rng(2)):
+    return [[rng.uniform(0.8, 1.25, n) for n in shape] for _ in range(2)]
+
+
+@pytest.mark.parametrize("dx", ["unit", "half", "table"])
+@pytest.mark.parametrize("mu", [False, True])
+@pytest.mark.parametrize("poynting", [True, False])
+def test_ahead_is_the_path_that_runs(dx, mu, poynting):
+    """'ahead' and 'hs' share their path code: the launches that make the next step's E are told apart."""
+    shape, kw = (14, 11, 300), {}
+    if dx != "unit":
+        kw["dxes"] = 0.5 if dx == "half" else _graded(shape)
+    if mu:
+        kw["mu"] = [numpy.full(shape, 1.5, numpy.float32)] * 3
+    faces = [(a, p, 3) for a in "xyz" for p in "np"]
+    a, b = _sim(shape, faces, poynting, **kw), _sim(shape, faces, poynting, **kw)
+    _loop(a, 6)
+    b.run(5, path="ahead")
+    assert b.tuning("last_run_ahead") == 1 and b.tuning("last_run_path") == 2
+    b.run(1, path="ahead")
+    assert b.tuning("last_run_ahead") == 0
+    _same(a, b)
+
+
+@pytest.mark.parametrize("shape,poynting,path,ahead", [
+    ((24, 24, 24), True, 2, 1), ((24, 24, 24), False, 1, 0), ((64, 64, 64), True, 2, 0), ((64, 64, 64), False, 1, 0),
+    ((180, 150, 90), True, 2, 1), ((180, 150, 90), False, 2, 1),
+])
+def test_automatic_path(shape, poynting, path, ahead):
+    """By cells and L2: the lines of Simulation._auto_path for an L2 of about 130 MB."""
+    l2 = torch.cuda.get_device_properties(0).L2_cache_size
+    if not 115e6 < l2 < 144e6:
+        pytest.skip("the lines are those of another L2")
+    sim = _sim(shape, [(a, p, 4) for a in "xyz" for p in "np"], poynting)
+    sim.run(3)
+    assert (sim.tuning("last_run_path"), sim.tuning("last_run_ahead")) == (path, ahead)
+    double = _sim((24, 24, 24), (("x", "n", 4),), poynting, float_type=numpy.float64)
+    double.run(3)
+    assert (double.tuning("last_run_path"), double.tuning("last_run_ahead")) == (1, 0)
