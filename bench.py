@@ -15,8 +15,8 @@ Printed as one JSON line:
               sample copied host->device from pinned memory and one field sample read back
   roofline    the dominant kernel's algorithmic bytes per launch / its mean event-timed
               duration, against the measured HBM copy bandwidth
-  step_roofline  the whole step's algorithmic bytes (84 B/cell for E+H, +12 B/cell S,
-              +32 B per CPML face-cell) per step time
+  step_roofline  the bytes that the path's launches of a step read and write (one launch for a
+              step: 72 B/cell, +32 B per CPML face-cell) per step time
   cpu_baseline   the reference's own kernels (oracle/_ref replay; else the C restatement)
               timed on the host cores on a bounded number of full-grid steps
 
@@ -154,20 +154,21 @@ class ClockSampler:
 
 
 def algorithmic_bytes(N: int, face_cells: int, elem: int, poynting: bool):
-    """Per-launch compulsory bytes (each input read once, each output written once)."""
+    """Compulsory bytes (each input read once, each output written once): per launch, and of a step by
+    the path that makes it, the sum over its launches."""
     e = N * 12 * elem + face_cells * 4 * elem           # E r/w, H r, eps r; psi_E r/w
     h = N * 9 * elem + face_cells * 4 * elem             # H r/w, E r; psi_H r/w
     s = 0
     if poynting:
         h += N * 6 * elem                                 # oS w
         s = N * 9 * elem                                  # oS r, S w
-    step = N * 21 * elem + face_cells * 8 * elem + (N * 3 * elem if poynting else 0)
     # run()'s H+S kernel: H read (one copy) and written (the other), E read, S written;
     # psi_H read / written
-    hs = N * 12 * elem + face_cells * 4 * elem
+    hs = N * (12 if poynting else 9) * elem + face_cells * 4 * elem
     # the same launch with the next step's E in it: dt/eps read and E written too, psi_E read / written
-    ahead = N * 18 * elem + face_cells * 8 * elem
-    return {"k_bulk_e": e, "k_bulk_h": h, "k_bulk_s": s, "k_tile_h": hs, "k_tile_h (E ahead)": ahead}, step
+    ahead = hs + N * 6 * elem + face_cells * 4 * elem
+    return ({"k_bulk_e": e, "k_bulk_h": h, "k_bulk_s": s, "k_tile_h": hs, "k_tile_h (E ahead)": ahead},
+            {"dropin": e + h + s, "slab": e + h + s, "hs": e + hs, "ahead": ahead, "fused": ahead})
 
 
 # FP64 DFT monitor of the c2 ringdown (the north star's "FP64 DFT monitor at 5 interior points"):
@@ -401,7 +402,8 @@ def c2_parity(wl, steps: int):
     vals = [wl["wave"](t) for t in range(steps)]
     g = Simulation(**copy.deepcopy(wl["kwargs"]))
     g.run(steps, point_sources=[(wl["source_index"], vals)])
-    path = {1: "per-update", 2: "H+S", 3: "one-pass"}.get(g.tuning("last_run_path"), "?")
+    path = {1: "per-update", 2: "H, S and the next E" if g.tuning("last_run_ahead") else "H+S",
+            3: "one-pass"}.get(g.tuning("last_run_path"), "?")
     got = {k: g.get(k).astype(numpy.float64) for k in ("E", "H", "S")}
     del g
     kw = copy.deepcopy(wl["kwargs"])
@@ -562,13 +564,12 @@ def main():
                          "traffic": traffic.get(dom), "algorithmic_bytes_per_launch": per_launch[dom],
                          "mean_launch_ms": round(per[dom], 5),
                          "per_kernel_ms": {k: round(v, 5) for k, v in per.items()}}}
-    compulsory = N * (18 if poynting else 15) * elem + fc * 8 * elem
     for name in ("fused", "slab", "hs", "ahead"):
         if name not in res:
             continue
         total = allmax(res[name])
         ms = total / K
-        ach = step_bytes / (ms * 1e-3) / 1e9
+        ach = step_bytes[name] / (ms * 1e-3) / 1e9
         nslab = (wl["shape"][0] + sim.slab_planes() - 1) // sim.slab_planes()
         # per step: the path's kernels (the workload's one point source is added inside k_step
         # on the fused path and inside the kernel that updates E on the hs and ahead paths) and the
@@ -588,10 +589,8 @@ def main():
                          "achieved": round(ach, 1),
                          "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4),
                          "peak_source": peak_kind, "traffic": traffic.get(name),
-                         "algorithmic_bytes_per_launch" if name == "fused" else "algorithmic_bytes_per_step": step_bytes,
-                         "accounting": "84 B/cell E+H, +12 B/cell S, +32 B per CPML face-cell (f32)",
-                         "compulsory_bytes_per_step": compulsory,
-                         "compulsory_frac": round(compulsory / (ms * 1e-3) / 1e9 / peak, 4),
+                         "algorithmic_bytes_per_launch" if name == "fused" else "algorithmic_bytes_per_step": step_bytes[name],
+                         "accounting": "the arrays that the path's launches read and write, each once a launch",
                          "mean_step_ms": round(ms, 5)}}
     for name in ("hs", "ahead"):
         if name not in out_paths:
@@ -609,7 +608,7 @@ def main():
     cands = [n for n in ("fused", "slab", "hs", "ahead") if n in out_paths]
     head = min(cands, key=lambda n: out_paths[n]["ms_per_step"]) if cands else "dropin"
     hp = out_paths[head]
-    step_gbs = step_bytes / (hp["ms_per_step"] * 1e-3) / 1e9
+    step_gbs = step_bytes[head] / (hp["ms_per_step"] * 1e-3) / 1e9
     # launch options of the H+S path as the timed run used them
     launch = ({"hs_xchunk": sim.tuning("hs_xchunk_used"), "pdl": sim.tuning("pdl"),
                "dft_in_hs_launch": sim.tuning("hs_dft"), "e_xchunk": sim.tuning("xchunk"),
@@ -664,17 +663,15 @@ def main():
                          out_paths["dropin"]["roofline"] if head != "fused" and "dropin" in out_paths
                          else hp["roofline"]),
             "step_roofline": {"achieved": round(step_gbs, 1), "peak": peak, "unit": "GB/s",
-                              "frac": round(step_gbs / peak, 4), "bytes_per_step": step_bytes},
+                              "frac": round(step_gbs / peak, 4), "bytes_per_step": step_bytes[head]},
             "clocks": clock, "e2e": e2e, "gpu_launches": hp["gpu_launches"],
             "cpu_baseline": cpu,
             "dropin_roofline": out_paths["dropin"]["roofline"] if "dropin" in out_paths else None,
             # roofline_frac: the path's own kernel (dropin: its dominant kernel per launch);
-            # step_roofline_frac: the whole step against the step's algorithmic bytes, the same
-            # basis for every path (the per-call loop moves more than those bytes: it writes
-            # and re-reads the six Poynting products)
+            # step_roofline_frac: the whole step against the bytes that the path's launches move
             "paths": {k: {"value": round(v["value"], 2), "ms_per_step": round(v["ms_per_step"], 5),
                           "roofline_frac": v["roofline"]["frac"], "kernel": v["roofline"]["kernel"],
-                          "step_roofline_frac": round(step_bytes / (v["ms_per_step"] * 1e-3) / 1e9 / peak, 4)}
+                          "step_roofline_frac": round(step_bytes[k] / (v["ms_per_step"] * 1e-3) / 1e9 / peak, 4)}
                       for k, v in out_paths.items()},
         }
         out.update(extras)
@@ -843,7 +840,7 @@ def c4_measure(n_variants: int, steps: int, chunk: int, storages=("f32", "bf16",
             "interior_value": round(interior * steps / (ms * 1e-3) / 1e6, 2),
             "tiles": {"schedule": tune["schedule"], "xchunk": tune["xchunk"],
                       "blocks_per_sm": tune["blocks_per_sm"], "autotune_ms_per_step": tune.get("timings")},
-            "launches": steps // chunk if tune["schedule"] == "persistent" else 2 * steps,
+            "launches": steps // chunk if tune["schedule"] == "persistent" else b.step_launches() * steps,
             "steps_per_graph": chunk, "graph_replays": steps // chunk}
         b.close()
         del b

@@ -207,6 +207,13 @@ class BatchSimulation:
         for sim in self.sims:
             sim.steps_run += n
 
+    def step_launches(self) -> int:
+        """Launches per step of the 'launches' schedule: E and H of the variants that share theirs, and of
+        each with launches of its own (0 with 'persistent', which has one launch per run)."""
+        v = ctypes.c_int32()
+        _lib.check(self._lib.fdtd_batch_get(self._batch, _lib.FDTD_BATCH_GET_STEP_LAUNCHES, ctypes.byref(v)))
+        return int(v.value)
+
     def step_counter(self) -> int:
         """The device step counter: the source / monitor row of the next step."""
         v = ctypes.c_int64()

@@ -154,6 +154,9 @@ def test_captured_run_with_a_variant_launched_alone():
     assert b.step_counter() == 6
     for x, y in zip(ref, sims):
         assert torch.equal(x.E, y.E) and torch.equal(x.H, y.H)
+    assert b.step_launches() == 4
+    b.tune(schedule="persistent")
+    assert b.step_launches() == 0
 
 
 @pytest.mark.parametrize("shapes,length,launches", [
