@@ -25,7 +25,7 @@ What differs:
   * an unstable dt warns and is then used (the reference warns and leaves dt unset), and
     malformed initial fields raise (the reference builds the exceptions but never raises);
   * ``run(nsteps, point_sources)`` advances many canonical steps in one call with the
-    per-step source values already on the device, and ``state_dict()`` /
+    per-step source values carried by the launches, and ``state_dict()`` /
     ``load_state_dict()`` checkpoint every field and CPML auxiliary array.
 """
 from __future__ import annotations
@@ -292,6 +292,12 @@ class Simulation:
             for k in fields:
                 self.psi[k].append((torch.zeros(shp, dtype=self._dtype, device=self.device),
                                     torch.zeros(shp, dtype=self._dtype, device=self.device)))
+        # whether two faces of one axis share cells (a 'p' face thicker than its axis never applies)
+        thick = [0, 0, 0]
+        for a, pol, T, _, _ in self._pml_tables:
+            if pol == 0 or T <= self.shape[a]:
+                thick[a] += T
+        self._overlap = any(t > s for t, s in zip(thick, self.shape))
 
     def _create_plan(self, uniform_dx):
         d = _lib.FdtdDesc()
@@ -534,7 +540,7 @@ class Simulation:
         if path == "hs" and not self.do_poynting:
             raise ValueError("the 'hs' path needs do_poynting=True")
         mode = None if path == "plain" else path
-        if mode == "ahead" and self._faces_overlap():
+        if mode == "ahead" and self._overlap:
             mode = None
         if mode == "ahead" and (self._np_dtype == numpy.float64 or getattr(self, "_lbc_keep", None) is not None
                                 or not self._try_scratch("ahead")):
@@ -574,7 +580,7 @@ class Simulation:
         against 22.4, 151x129x61 31.4 against 34.1). Where two faces of one axis overlap, every path
         is the per-update one, and the others' copies would be memory for nothing."""
         hs = "hs" if self.do_poynting else "plain"
-        if self.bloch_boundaries or self._np_dtype == numpy.float64 or self._faces_overlap():
+        if self.bloch_boundaries or self._np_dtype == numpy.float64 or self._overlap:
             return "plain"
         if nsteps < 2 or getattr(self, "_lbc_keep", None) is not None:
             return hs
@@ -582,14 +588,6 @@ class Simulation:
         if not self.do_poynting:
             return "plain" if 60 * self.N <= l2 or self.tuning("slab") else "ahead"
         return "hs" if self.N > 100000 and 84 * self.N <= l2 else "ahead"
-
-    def _faces_overlap(self) -> bool:
-        """Whether two CPML faces of one axis share cells (a 'p' face thicker than its axis never applies)."""
-        thick = [0, 0, 0]
-        for a, pol, T, _, _ in self._pml_tables:
-            if pol == 0 or T <= self.shape[a]:
-                thick[a] += T
-        return any(t > s for t, s in zip(thick, self.shape))
 
     def _try_scratch(self, mode) -> bool:
         """The second copies of a run path, or False when the device has no room for them. A refused

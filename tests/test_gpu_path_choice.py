@@ -42,7 +42,7 @@ def _same(a, b):
 def test_overlapping_faces_need_no_copies(faces, overlap, path, poynting):
     shape = (16, 20, 24)
     a, b = _sim(shape, faces, poynting), _sim(shape, faces, poynting)
-    assert a._faces_overlap() == overlap
+    assert a._overlap == overlap
     _loop(a, 4)
     b.run(4, path=path)
     _same(a, b)
