@@ -1,12 +1,12 @@
-"""Many independent cavity variants stepped together in one persistent launch.
+"""Many independent cavity variants stepped together.
 
 ``BatchSimulation`` takes ordinary ``Simulation`` objects (float32, diagonal eps, no mu, no
-Bloch boundaries, Poynting off, uniform dx) and advances all of them with one cooperative
-kernel launch per call of ``run`` (``fdtd_batch_run``): the grid of a few blocks per SM works
-through the tiles of every variant for the E half-step, synchronises, does the H half-step,
-and repeats. There is no per-variant launch, no per-variant tail and no host round trip; a
-call can also be captured once in a CUDA graph and replayed (``capture``), since the step
-counter lives on the device.
+Bloch boundaries, Poynting off, uniform dx) and advances all of them with one call of ``run``
+(``fdtd_batch_run``). A step is one launch for E and one for H over the tiles of every variant that
+shares launches, and the same for each large float32 variant by itself (the 'launches' schedule), or
+one cooperative launch takes all variants' tiles for all steps of the call ('persistent'). There is
+no host round trip; a call can also be captured once in a CUDA graph and replayed (``capture``),
+since the step counter lives on the device.
 
 Storage: ``'f32'`` updates the simulations' own tensors in place (results are bit-identical
 to ``Simulation.run`` of each variant). ``'bf16'`` / ``'fp16'`` keep E, H and dt/eps in 16-bit
@@ -158,8 +158,9 @@ class BatchSimulation:
     # ---- stepping ---------------------------------------------------------------------------
     def tune(self, xchunk: int = None, blocks_per_sm: int = 0, schedule: str = None):
         """Tile shape (x planes per tile; 0: automatic, None: as it is), resident blocks per SM of the persistent schedule
-        (0: as many as fit) and the schedule: 'launches' (two launches per step, each over the
-        tiles of every variant; default) or 'persistent' (one cooperative launch per run)."""
+        (0: as many as fit) and the schedule: 'launches' (two launches per step for the variants that
+        share them and for each that does not; default) or 'persistent' (one cooperative launch per run).
+        A run captured before must be captured again."""
         if xchunk is None:
             xchunk = self.xchunk
         _lib.check(self._lib.fdtd_batch_tune(self._batch, int(xchunk), int(blocks_per_sm)))
@@ -179,7 +180,7 @@ class BatchSimulation:
         return tune_batch(self, steps=steps, cache_path=cache_path, **kw)
 
     def run(self, nsteps: int):
-        """Advance every variant by nsteps steps in one launch on the simulations' stream."""
+        """Advance every variant by nsteps steps on the simulations' stream."""
         _lib.check(self._lib.fdtd_batch_run(self._batch, ctypes.c_void_p(self.queue.cuda_stream), int(nsteps)))
         self.steps_run += int(nsteps)
         for sim in self.sims:

@@ -1,15 +1,15 @@
-// Batched stepping of many independent cavity variants in one persistent launch.
+// Batched stepping of many independent cavity variants.
 //
 // All variants' work is cut into tiles of BATCH_THREADS consecutive (y, z) cells times a chunk
 // of x planes. Two schedules run the same tile code:
+//   * per half-step: launches of one block per tile, one for E and one for H per step: of the tiles of all
+//     variants that share launches, or of one variant, whose descriptor is then among the arguments
+//     (k_batch_e1 / h1; large float32 variants). A launch starts while the one before drains;
 //   * persistent: a cooperative grid of resident blocks takes the tiles of every variant
 //     from a device work counter for the E half-step, synchronises the grid, does the same for
 //     the H half-step, synchronises again, and repeats -- one launch advances the whole sweep by
-//     nsteps steps;
-//   * per half-step: one launch of one block per tile for E, one for H, per step (captured in
-//     a CUDA graph by the caller); the hardware scheduler then overlaps blocks.
-// Either way there is no per-variant launch or tail. Point sources are added and monitor
-// points recorded by the thread that updates the cell.
+//     nsteps steps.
+// Point sources are added and monitor points recorded by the thread that updates the cell.
 //
 // Storage: E, H and dt/eps in float32, or in bfloat16 / float16 with float32 arithmetic. In
 // 16-bit storage every tile (one component of the BATCH_TILE cells one warp updates in one x
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, BATCH_PERSIST_BLOCKS) k_batch(c
 // blocks per SM) and the descriptor's pointers, limits and source list read again for every plane, the
 // march was 261 (E) and 220 (H) instructions per warp and plane and a step of 8 variants (14.7 M cells)
 // took 0.389 ms in float32, 0.420 in bfloat16 without exponents and 0.619 with; now 184 and 163 and 0.331,
-// 0.298 and 0.407. E in float32 spills 56 bytes at five blocks and still gains (0.208 to 0.184 ms, four to
+// 0.297 and 0.406. E in float32 spills 56 bytes at five blocks and still gains (0.208 to 0.184 ms, four to
 // five); H loses there (0.146 to 0.163), and so does E with tile exponents. Six blocks: 0.211 and 0.174.
 // A call's last H launch advances the step counter.
 template <int ST>
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 4) k_batch_h(const BatchK k)
 }
 
 // One variant per launch, its descriptor among the kernel's arguments (five blocks per SM: 0.317 ms a step
-// instead of 0.306); index arithmetic stands before the wait (0.304), chunks by fit_xchunk (0.286).
+// instead of 0.306); index arithmetic stands before the wait (0.304), chunks by fit_xchunk (0.279).
 constexpr int BATCH_ONE_BLOCKS = 4;
 
 __global__ void __launch_bounds__(BATCH_THREADS, BATCH_ONE_BLOCKS) k_batch_e1(const __grid_constant__ BatchOne k)

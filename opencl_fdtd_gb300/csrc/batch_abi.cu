@@ -38,7 +38,7 @@ int fail(int code, const std::string &msg) { return set_error(code, msg.c_str())
 
 // Whether a variant's updates are launches of their own in the launches schedule: the descriptor is then
 // among the kernel's arguments, which spares the march's registers and reloads, at the price of a tail per
-// launch. Float32: 8 variants of 1.8 M cells 0.331 to 0.286 ms a step, 3 of 0.95 M 87 to 64 us, 6 of 0.5 M 86
+// launch. Float32: 8 variants of 1.8 M cells 0.331 to 0.279 ms a step, 3 of 0.95 M 87 to 64 us, 6 of 0.5 M 86
 // to 82, but 6 of 0.2 M 36 to 55. With 16-bit storage the tiles spill less and it lost (0.298 to 0.303 ms).
 bool launched_alone(const BVar &h, int storage) { return storage == BATCH_F32 && h.N >= 500000; }
 

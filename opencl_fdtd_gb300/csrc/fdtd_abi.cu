@@ -445,8 +445,11 @@ static void hs_layout(const FdtdPlan *p, HSK<R> &k, const HSForm &f, uint32_t ex
     const bool ahead = f.ahead;
     const uint32_t threads = (uint32_t)hs_threads(f.ahead, f.mu, f.dxmode);
     uint64_t best = 0;
-    for (uint32_t n = (p->sz + threads / 2u - 2u) / (threads / 2u - 1u); n <= p->sz; ++n) {
-        const uint32_t len = (p->sz + n - 1u) / n;
+    // from one segment length that a row divides into to the next, some 200 at most: a row of 2e7 cells has half a
+    // million counts of segments, most of the same lengths, and trying each took milliseconds of every call
+    uint32_t n = (p->sz + threads / 2u - 2u) / (threads / 2u - 1u), len;
+    for (; n <= p->sz; n = len > 1u ? (p->sz + len - 2u) / (len - 1u) : p->sz + 1u) {
+        len = (p->sz + n - 1u) / n;
         if (best && len < 37u) break;
         uint32_t r = threads / (len + 1u) - 1u;                  // at least one own row
         if (r > p->sy) r = p->sy;

@@ -43,7 +43,8 @@ struct FastDiv {
 // of the plan's own coefficient tables, which no kernel writes: a thread's set-up then overlaps the
 // kernel before, which is most of what a small grid's step costs (E and H of 24^3 cells 5.6 to
 // 4.3 us, of 40^3 7.5 to 4.9, of 64^3 11.9 to 10.2; letting the next kernel in before the wait:
-// 4.6, 5.0, 10.6). Without the launch attribute both instructions have no effect.
+// 4.6, 5.0, 10.6). What other launches write is read behind it with coherent loads (ldf, yee_device.cuh).
+// Without the launch attribute both instructions have no effect.
 __device__ __forceinline__ void grid_dependency_sync()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");

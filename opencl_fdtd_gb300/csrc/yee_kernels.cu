@@ -2,9 +2,10 @@
 //
 // Bulk kernels (the normal path): thread (y, z) of the plane marches a chunk of consecutive
 // x planes. The x-neighbour plane is carried in registers (the E update's x-1 values are the
-// previous iteration's own loads; the H update's x+1 loads become the next iteration's own),
-// and every load of iteration x+1 (fields, neighbours, dt/eps, CPML psi) is issued before
-// iteration x computes and stores, so each warp keeps a full iteration of loads in flight.
+// previous iteration's own loads; the H update's x+1 loads become the next iteration's own).
+// A plane's values (fields, neighbours, dt/eps, CPML psi) are loaded when it is updated, at as many
+// blocks per SM as the registers allow, or, where the form says so, one iteration ahead (EForm,
+// h_prefetch).
 // Consecutive threads walk consecutive z, so a warp's loads are contiguous runs. CPML faces
 // are handled per axis: x-faces are uniform for a whole iteration, y- and z-face membership
 // is fixed for a thread, so the depth index and the coefficients of y/z faces are looked up
@@ -22,8 +23,6 @@
 #include "yee_launch.h"
 
 namespace fdtd {
-
-
 
 // ---- CPML contribution of one face ---------------------------------------------------------
 template <typename R, bool ETYPE, int AX>
@@ -250,11 +249,11 @@ __device__ __forceinline__ void plane_cell(const YeeK<R> &k, uint32_t t, uint32_
 
 // Warps without absorbing cells leave out the terms of the CPML arrays (adding zero) in double precision,
 // which the FP64 units bound: with the z order a step of 197x173x73 cells went from 0.436 to 0.402 ms. In
-// float32 the test cost what it saved.
+// float32 the test cost what it saved. (A sum that is -0 stays -0 instead of becoming +0: equal values.)
 template <typename R>
 constexpr bool skip_zero_psi() { return sizeof(R) == 8; }
 
-// Values one E-type iteration reads, loaded one iteration ahead.
+// Values one E-type iteration reads.
 template <typename R>
 struct ELoad {
     R hx, hy, hz;                 // Q at x
@@ -317,9 +316,7 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
     // a point source in this column and these planes
     bool srcs = false;
     for (int s = 0; s < k.nsrc; ++s)
-        srcs |= k.src_j[s] == j &&
-
-                (k.src_x[s] - k.xbeg) / k.xchunk == blockIdx.y;
+        srcs |= k.src_j[s] == j && (k.src_x[s] - k.xbeg) / k.xchunk == blockIdx.y;
     grid_dependency_sync();
     if (DX == 2) { iy = ldf(k.inv_tab[1] + y); iz = ldf(k.inv_tab[2] + z); }
 
@@ -433,7 +430,7 @@ __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_block
     }
 }
 
-// Values one H-type iteration reads, loaded one iteration ahead.
+// Values one H-type iteration reads.
 template <typename R>
 struct HLoad {
     R ex1, ey1, ez1;              // Q at x+1 (wrapped)
@@ -464,11 +461,11 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
     const uint32_t j = y * sz + z;
     const FixedFace<R, AWAY> fy = fixed_face<R, AWAY>(k.ax[1], sy, y, act);
     const FixedFace<R, AWAY> fz = fixed_face<R, AWAY>(k.ax[2], sz, z, act);
-        const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
+    const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
     if (!act) return;
     const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
     const uint32_t xb = min(xa + k.xchunk, k.xend);
-        // asking once costs the form that also writes the products 2 us of 133 on 395x345x73 cells
+    // asking once costs the form that also writes the products 2 us of 133 on 395x345x73 cells
     const bool xf = (POYNT && sizeof(R) == 4) || x_faces(k.ax[0], sx, xa, xb);
     const uint64_t N = k.N;
     const R *const Qx = k.Q;

@@ -112,3 +112,33 @@ def test_automatic_path(shape, poynting, path, ahead):
     double = _sim((24, 24, 24), (("x", "n", 4),), poynting, float_type=numpy.float64)
     double.run(3)
     assert (double.tuning("last_run_path"), double.tuning("last_run_ahead")) == (1, 0)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 1, 2), (3, 1, 1), (1, 5, 37), (2, 3, 511), (1, 1, 4096), (2, 1, 10007)])
+@pytest.mark.parametrize("mu", [False, True])
+def test_rows_of_any_length(shape, mu):
+    """Tiles of whole and of divided rows, down to one cell."""
+    kw = {"mu": [numpy.full(shape, 1.5, numpy.float32)] * 3} if mu else {}
+    faces = [("z", p, 8) for p in "np"] if shape[2] > 100 else []
+    a, b = _sim(shape, faces, **kw), _sim(shape, faces, **kw)
+    _loop(a, 5)
+    b.run(5, path="ahead")
+    assert b.tuning("last_run_ahead") == 1
+    _same(a, b)
+
+
+def test_a_long_row_costs_the_host_no_time():
+    """20 million cells in a row: finding the tiles takes microseconds, not a try of every division."""
+    import time
+    one = numpy.ones((1, 1, 20_000_000), numpy.float32)
+    from opencl_fdtd_gb300 import Simulation
+    sim = Simulation([one] * 3, [], do_poynting=False)
+    sim.run(2, path="ahead")
+    took = []
+    for _ in range(10):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        sim.run(2, path="ahead")
+        took.append(time.perf_counter() - t)
+    assert sim.tuning("last_run_ahead") == 1
+    assert min(took) < 1e-3
