@@ -12,7 +12,7 @@ steps.
 Printed as one JSON line:
   value       Mcell-updates/s with every buffer resident in HBM (device-timed, CUDA events)
   e2e         the same metric through the public Simulation API, with the per-step source
-              sample copied host->device from pinned memory and one field sample read back
+              sample taken from host memory and one field sample read back
   roofline    the dominant kernel's algorithmic bytes per launch / its mean event-timed
               duration, against the measured HBM copy bandwidth
   step_roofline  the bytes that the path's launches of a step read and write (one launch for a
@@ -684,8 +684,7 @@ def run_e2e(sim, wl, steps: int, world: int, run_api: bool = False, path: str = 
     """End to end through the public API with host buffers.
 
     API: Simulation.run() in calls of 10 steps, each given its 10 source samples from host
-    memory (copied to the device inside the call, from pinned staging, without blocking the
-    host) and followed by a device-to-host copy of the driven field sample into pinned host
+    memory (every launch carries its step's) and followed by a device-to-host copy of the driven field sample into pinned host
     memory on the simulation's stream; the host synchronizes once at the end and the samples
     are checked; `monitor` (the workload's DFT monitor) is sampled every step as in the
     device-timed run. Otherwise the per-call loop of fdtd.py:162-175 with the source sample copied

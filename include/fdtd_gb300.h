@@ -310,7 +310,7 @@ int fdtd_run_kernel_ms(const FdtdPlan *plan, double ms[2], int32_t *samples);
  * counterpart in the reference. */
 int fdtd_device_status(FdtdPlan *plan, void *stream, int32_t *bits);
 
-/* ---- batched stepping of many independent variants (one persistent launch) ---------------
+/* ---- batched stepping of many independent variants ---------------------------------------
  * No counterpart in the reference, which steps one grid per Simulation. Each variant is a
  * grid with diagonal eps (no mu, no Bloch boundaries, no Poynting, uniform dx) whose E, H and
  * dt/eps arrays are stored in float32, bfloat16 or float16 (arithmetic is float32 in every
@@ -351,9 +351,8 @@ typedef struct FdtdBatchVariant {
 
 typedef struct FdtdBatch FdtdBatch;
 
-/* Validate n variants and build the tile list (x chunks of xchunk planes, default 8 or fewer
- * where the batch is small). rows:
- * rows of every variant's src_values / series (steps past it add no source, record nothing). */
+/* Validate n variants and build the tile list (x chunks of 8 planes, fewer where the batch is
+ * small, until fdtd_batch_tune sets them). rows: rows of every variant's src_values / series (steps past it add no source, record nothing). */
 int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, int64_t rows,
                       FdtdBatch **out);
 int fdtd_batch_destroy(FdtdBatch *batch);
@@ -362,8 +361,9 @@ int fdtd_batch_destroy(FdtdBatch *batch);
  * run captured before must not be replayed. */
 int fdtd_batch_tune(FdtdBatch *batch, int32_t xchunk, int32_t blocks_per_sm);
 /* Advance every variant by nsteps steps (E, sources, H per step) on the stream: with the
- * FDTD_BATCH_LAUNCHES schedule (default) as two launches per step, each covering the tiles of
- * every variant; with FDTD_BATCH_PERSISTENT as one cooperative launch for all nsteps steps.
+ * FDTD_BATCH_LAUNCHES schedule (default) as two launches per step for the variants that share
+ * them and two for each float32 variant of at least half a million cells, whose steps of the call
+ * follow each other; with FDTD_BATCH_PERSISTENT as one cooperative launch for all nsteps steps.
  * The step counter lives on the device (read and advanced by the launches), so captured
  * launches keep counting when a CUDA graph replays them. */
 #define FDTD_BATCH_PERSISTENT 0

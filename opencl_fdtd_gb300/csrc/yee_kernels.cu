@@ -443,16 +443,17 @@ struct HLoad {
 };
 
 // Forms of the bulk H kernel, as those of E: with the next plane loaded one iteration ahead at three
-// blocks per SM (80 registers); with dt/mu or Bloch partners, whose values would spill there, with each
-// plane loaded when it is updated, at four (64 registers). In double precision, where values take two
-// registers and the FP64 units, not latency, are the bound, two blocks (0.211 to 0.199 ms on 197x173x73).
-constexpr bool h_prefetch(bool mu, bool bloch) { return !mu && !bloch; }
-constexpr int h_min_blocks(bool mu, bool bloch, bool dbl) { return dbl ? 2 : h_prefetch(mu, bloch) ? 3 : 4; }
+// blocks per SM (80 registers); with Bloch partners, whose values would spill there, with each
+// plane loaded when it is updated, at four (64 registers; with dt/mu that takes 0.121 ms without and 0.160
+// with the products on 395x345x73 cells, the other form 0.106 and 0.146). In double precision, where values
+// take two registers and the FP64 units, not latency, are the bound, two blocks (0.211 to 0.199 ms on 197x173x73).
+constexpr bool h_prefetch(bool bloch) { return !bloch; }
+constexpr int h_min_blocks(bool bloch, bool dbl) { return dbl ? 2 : h_prefetch(bloch) ? 3 : 4; }
 
 template <typename R, int DX, bool MU, bool POYNT, bool BLOCH, bool AWAY>
-__global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)) k_bulk_h(const YeeK<R> k)
+__global__ void __launch_bounds__(BLOCK, h_min_blocks(BLOCH, sizeof(R) == 8)) k_bulk_h(const YeeK<R> k)
 {
-    constexpr bool PF = h_prefetch(MU, BLOCH), SKIP = skip_zero_psi<R>();
+    constexpr bool PF = h_prefetch(BLOCH), SKIP = skip_zero_psi<R>();
     const uint32_t t = blockIdx.x * BLOCK + threadIdx.x;
     const bool act = t < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
@@ -461,12 +462,14 @@ __global__ void __launch_bounds__(BLOCK, h_min_blocks(MU, BLOCH, sizeof(R) == 8)
     const uint32_t j = y * sz + z;
     const FixedFace<R, AWAY> fy = fixed_face<R, AWAY>(k.ax[1], sy, y, act);
     const FixedFace<R, AWAY> fz = fixed_face<R, AWAY>(k.ax[2], sz, z, act);
-    const bool wf = __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
+    // asking once for the warp costs the form that also writes the products: 395x345x73 cells 2 us of 133 for the x
+    // faces, with dt/mu 22 of 168 for the others
+    constexpr bool ASK = !POYNT || sizeof(R) == 8;
+    const bool wf = !ASK || __any_sync(0xffffffffu, fy.ir >= 0 || fz.ir >= 0) != 0;
     if (!act) return;
     const uint32_t xa = k.xbeg + blockIdx.y * k.xchunk;
     const uint32_t xb = min(xa + k.xchunk, k.xend);
-    // asking once costs the form that also writes the products 2 us of 133 on 395x345x73 cells
-    const bool xf = (POYNT && sizeof(R) == 4) || x_faces(k.ax[0], sx, xa, xb);
+    const bool xf = !ASK || x_faces(k.ax[0], sx, xa, xb);
     const uint64_t N = k.N;
     const R *const Qx = k.Q;
     const R *const Qy = k.Q + N;
@@ -795,7 +798,7 @@ cudaError_t launch_yee_h(const YeeK<R> &kk, bool mu, bool poynting, cudaStream_t
         return cudaGetLastError();
     }
     const bool away = k.W != k.P;
-    const dim3 g = bulk_grid(k, BLOCK, (uint32_t)h_min_blocks(mu, k.bloch_mask != 0, sizeof(R) == 8));
+    const dim3 g = bulk_grid(k, BLOCK, (uint32_t)h_min_blocks(k.bloch_mask != 0, sizeof(R) == 8));
     return launch_dependent(k.bloch_mask ? bulk_h_kernel<R, true>(k.dxmode, mu, poynting, away)
                                          : bulk_h_kernel<R, false>(k.dxmode, mu, poynting, away),
                             g, BLOCK, st, pdl, k);
