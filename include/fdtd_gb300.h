@@ -122,8 +122,9 @@ int fdtd_plan_destroy(FdtdPlan *plan);
 
 /* Tuning keys of fdtd_plan_tune. Any values give the same results.
  *   XCHUNK        consecutive x planes one thread of the update kernels advances; 0 (default):
- *                 chosen per launch (1 in double precision; else 8, or on grids of a few waves of
- *                 blocks the number up to 12 with the shortest whole waves)
+ *                 chosen per launch (in double precision 1, in H without the products up to 4; else
+ *                 8, or on grids of a few waves of blocks the number up to 12 with the shortest
+ *                 whole waves)
  *   SLAB          x planes per L2-resident slab of fdtd_run's per-update schedule
  *                 (default 0 = whole grid)
  *   FUSED_ROWS    own y rows of a tile of the one-pass step (default 0: the most that fit a

@@ -446,14 +446,16 @@ struct HLoad {
 // blocks per SM (80 registers); with Bloch partners, whose values would spill there, with each
 // plane loaded when it is updated, at four (64 registers; with dt/mu that takes 0.121 ms without and 0.160
 // with the products on 395x345x73 cells, the other form 0.106 and 0.146). In double precision, where values
-// take two registers and the FP64 units, not latency, are the bound, two blocks (0.211 to 0.199 ms on 197x173x73).
-constexpr bool h_prefetch(bool bloch) { return !bloch; }
-constexpr int h_min_blocks(bool bloch, bool dbl) { return dbl ? 2 : h_prefetch(bloch) ? 3 : 4; }
+// take two registers and the FP64 units, not latency, are the bound, two blocks (0.211 to 0.199 ms on 197x173x73);
+// with dt/mu there each plane when it is updated (200^3 cells 0.358 ms against 0.378, with the products 0.582
+// against 0.598).
+constexpr bool h_prefetch(bool mu, bool bloch, bool dbl) { return !bloch && !(mu && dbl); }
+constexpr int h_min_blocks(bool bloch, bool dbl) { return dbl ? 2 : bloch ? 4 : 3; }
 
 template <typename R, int DX, bool MU, bool POYNT, bool BLOCH, bool AWAY>
 __global__ void __launch_bounds__(BLOCK, h_min_blocks(BLOCH, sizeof(R) == 8)) k_bulk_h(const YeeK<R> k)
 {
-    constexpr bool PF = h_prefetch(BLOCH), SKIP = skip_zero_psi<R>();
+    constexpr bool PF = h_prefetch(MU, BLOCH, sizeof(R) == 8), SKIP = skip_zero_psi<R>();
     const uint32_t t = blockIdx.x * BLOCK + threadIdx.x;
     const bool act = t < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
@@ -715,7 +717,14 @@ static uint32_t sm_count()
 // x planes a thread of a bulk kernel marches when none is set (xchunk 0): fit_xchunk. In double precision
 // 1: the FP64 units are the bound, so what counts is that every SM has work to the end, not the loads that
 // a longer march saves (197x173x73 0.389 ms a step with 8 planes, 0.374 with 4, 0.360 with 1; 151x129x61
-// 0.223 and 0.186; 128x128x64 0.216 and 0.165).
+// 0.223 and 0.186; 128x128x64 0.216 and 0.165). Not so H without the products and Bloch partners, whose march
+// saves it a third of its loads and is over sooner: from ten waves of single planes on 2, from 24 on 4 (H of
+// 200^3 cells 0.329 ms, 0.412 with 1; 197x173x73 0.123 and 0.137; 128x128x64 with 2 58 us, 60 with 1 and 63 with 4).
+inline uint32_t h_xchunk_double(uint64_t nj, uint64_t nx, uint64_t slots)
+{
+    return nj * nx < 10u * slots ? 1u : nj * nx < 24u * slots ? 2u : 4u;
+}
+
 template <template <typename> class K, typename R>
 static dim3 bulk_grid(K<R> &k, uint32_t block, uint32_t resident)
 {
@@ -798,6 +807,8 @@ cudaError_t launch_yee_h(const YeeK<R> &kk, bool mu, bool poynting, cudaStream_t
         return cudaGetLastError();
     }
     const bool away = k.W != k.P;
+    if (sizeof(R) == 8 && !poynting && !k.bloch_mask && !k.xchunk)
+        k.xchunk = h_xchunk_double((k.syz + BLOCK - 1) / BLOCK, k.xend - k.xbeg, 2ull * sm_count());
     const dim3 g = bulk_grid(k, BLOCK, (uint32_t)h_min_blocks(k.bloch_mask != 0, sizeof(R) == 8));
     return launch_dependent(k.bloch_mask ? bulk_h_kernel<R, true>(k.dxmode, mu, poynting, away)
                                          : bulk_h_kernel<R, false>(k.dxmode, mu, poynting, away),
