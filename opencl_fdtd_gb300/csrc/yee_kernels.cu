@@ -282,7 +282,9 @@ template <typename R, int DX, bool BLOCH, int FORM, bool AWAY>
 __global__ void __launch_bounds__(EBLOCK, EForm<FORM, sizeof(R) == 8>::min_blocks) k_bulk_e(const YeeK<R> k)
 {
     constexpr bool PF = EForm<FORM, sizeof(R) == 8>::prefetch, SKIP = skip_zero_psi<R>();
-    constexpr bool SPLIT = sizeof(R) == 8 || BLOCH;      // the other form keeps row order: 3 us of 105 faster there
+    // the others keep row order: 3 us of 105 faster in float32, and Bloch pairs on graded cells 70 us instead of 78
+    // on 33x700x300
+    constexpr bool SPLIT = sizeof(R) == 8 || (BLOCH && DX != 2);
     const uint32_t t = blockIdx.x * EBLOCK + threadIdx.x;
     const bool act = t < k.syz;
     const uint32_t sx = k.sx, sy = k.sy, sz = k.sz, syz = k.syz;
