@@ -56,10 +56,11 @@ __device__ __forceinline__ void grid_dependency_sync()
 // times a march (its planes and one for the set-up): on small grids that is one wave with the
 // fewest planes (E and H of 64^3 cells 8.0 us a step with 2 planes, 9.3 with 1 and 1024 blocks), in between
 // a whole number of waves (208x202x71: 10 planes, 1.97 waves, E 33 us, against 36 with 8 and 2.44;
-// 128x128x256 Bloch 172 us a step with 7, 4.0 waves, against 180 with 8 and 3.4).
-inline uint32_t fit_xchunk(uint64_t nj, uint64_t nx, uint64_t slots)
+// 128x128x256 Bloch 172 us a step with 7, 4.0 waves, against 180 with 8 and 3.4). `many`: the waves from which
+// on it is 8.
+inline uint32_t fit_xchunk(uint64_t nj, uint64_t nx, uint64_t slots, uint32_t many = 6u)
 {
-    if (!slots || nj * ((nx + 7u) / 8u) >= 6u * slots) return 8u;
+    if (!slots || nj * ((nx + 7u) / 8u) >= many * slots) return 8u;
     uint32_t best = 8u;
     uint64_t least = 0;
     for (uint32_t c = 1; c <= 12u; ++c) {
