@@ -19,7 +19,7 @@ struct FdtdBatch {
     int device;
     int64_t rows;
     uint32_t xchunk;             // planes per tile asked for (0: automatic)
-    uint32_t tile_xchunk[2];     // planes per tile: of the shared launches, of the persistent schedule
+    uint32_t tile_xchunk[2] = {0, 0};   // planes per tile: of the shared launches, of the persistent schedule
     int blocks_per_sm;
     int schedule;                // FDTD_BATCH_PERSISTENT or FDTD_BATCH_LAUNCHES
     std::vector<BVar> host;      // descriptors as uploaded
@@ -47,11 +47,11 @@ bool launched_alone(const BVar &h, int storage) { return storage == BATCH_F32 &&
 // without a tile: two variants of 0.1 M cells took 25 us a step at 8 and 19 at 4. The shared launches hold
 // nothing but their own variants (one of 0.1 M cells beside one of 1.8 M: 34.6 us a step with 8 planes,
 // 28.3 with 1); the persistent schedule hands out all tiles (the same batch 30.3 and 33.1).
-void tile_lengths(const FdtdBatch *b, uint32_t xc[2])
+void tile_lengths(const FdtdBatch *b, uint32_t asked, uint32_t xc[2])
 {
-    xc[0] = xc[1] = b->xchunk ? b->xchunk : 8u;
+    xc[0] = xc[1] = asked ? asked : 8u;
     int nsm = 0;
-    if (b->xchunk || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || nsm < 1) return;
+    if (asked || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || nsm < 1) return;
     uint64_t planes[2] = {0, 0};
     for (const BVar &h : b->host) {
         const uint64_t n = (uint64_t)h.njb * h.sx;
@@ -63,35 +63,44 @@ void tile_lengths(const FdtdBatch *b, uint32_t xc[2])
         if (planes[g] < 8 * slots) xc[g] = (uint32_t)(planes[g] / slots > 1 ? planes[g] / slots : 1);
 }
 
-// The tile list: the tiles of the shared launches, then all variants' as the persistent schedule hands them out.
-int build_tiles(FdtdBatch *b)
+// The tile list: the tiles of the shared launches, then all variants' as the persistent schedule hands them
+// out, of xc[0] and xc[1] planes. The batch keeps its old list until the new one is on the device.
+int build_tiles(FdtdBatch *b, const uint32_t xc[2])
 {
     std::vector<int4> t;
-    const auto add = [&](size_t v, uint32_t xc) {
+    const auto add = [&](size_t v, uint32_t c) {
         const BVar &h = b->host[v];
-        for (uint32_t x0 = 0; x0 < h.sx; x0 += xc)
+        for (uint32_t x0 = 0; x0 < h.sx; x0 += c)
             for (uint32_t jb = 0; jb < h.njb; ++jb)
-                t.push_back(make_int4((int)v, (int)x0, (int)(x0 + xc < h.sx ? x0 + xc : h.sx), (int)jb));
+                t.push_back(make_int4((int)v, (int)x0, (int)(x0 + c < h.sx ? x0 + c : h.sx), (int)jb));
     };
-    b->groups.clear();
+    std::vector<const BVar *> groups;
     for (size_t v = 0; v < b->host.size(); ++v)
-        if (!launched_alone(b->host[v], b->storage)) add(v, b->tile_xchunk[0]);
-    b->shared = (uint32_t)t.size();
-    if (b->shared) b->groups.push_back(nullptr);
+        if (!launched_alone(b->host[v], b->storage)) add(v, xc[0]);
+    const size_t shared = t.size();
+    if (shared) groups.push_back(nullptr);
     for (int alone = 0; alone < 2; ++alone)
         for (size_t v = 0; v < b->host.size(); ++v) {
             const BVar &h = b->host[v];
             if (launched_alone(h, b->storage) != (alone != 0)) continue;
-            if (alone) b->groups.push_back(&h);
-            add(v, b->tile_xchunk[1]);
+            if (alone) groups.push_back(&h);
+            add(v, xc[1]);
         }
+    int4 *tiles = nullptr;
+    int rc = check_cuda(cudaMalloc(&tiles, t.size() * sizeof(int4)), "cudaMalloc(batch tiles)");
+    if (rc) return rc;
+    rc = check_cuda(cudaMemcpy(tiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice), "copy batch tiles");
+    if (rc) {
+        cudaFree(tiles);
+        return rc;
+    }
     if (b->tiles) cudaFree(b->tiles);
-    b->tiles = nullptr;
-    int rc = check_cuda(cudaMalloc(&b->tiles, t.size() * sizeof(int4)), "cudaMalloc(batch tiles)");
-    if (rc) return rc;
-    rc = check_cuda(cudaMemcpy(b->tiles, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice), "copy batch tiles");
-    if (rc) return rc;
+    b->tiles = tiles;
     b->ntiles = (uint32_t)t.size();
+    b->shared = (uint32_t)shared;
+    b->groups.swap(groups);
+    b->tile_xchunk[0] = xc[0];
+    b->tile_xchunk[1] = xc[1];
     return FDTD_OK;
 }
 
@@ -224,8 +233,9 @@ int fdtd_batch_create(const FdtdBatchVariant *vars, int32_t n, int32_t storage, 
     if (!rc) rc = check_cuda(cudaMalloc(&b->work, 2 * sizeof(uint32_t)), "cudaMalloc(batch work counters)");
     if (!rc) rc = check_cuda(cudaMemset(b->work, 0, 2 * sizeof(uint32_t)), "clear batch work counters");
     if (!rc) {
-        tile_lengths(b, b->tile_xchunk);
-        rc = build_tiles(b);
+        uint32_t xc[2];
+        tile_lengths(b, 0, xc);
+        rc = build_tiles(b, xc);
     }
     if (rc) {
         fdtd_batch_destroy(b);
@@ -251,15 +261,16 @@ int fdtd_batch_tune(FdtdBatch *b, int32_t xchunk, int32_t blocks_per_sm)
     if (!b) return fail(FDTD_ERR_INVALID, "batch is NULL");
     if (xchunk < 0 || xchunk > 4096) return fail(FDTD_ERR_INVALID, "xchunk must be in [0, 4096] (0: automatic)");
     if (blocks_per_sm < 0 || blocks_per_sm > 32) return fail(FDTD_ERR_INVALID, "blocks_per_sm must be in [0, 32]");
-    b->blocks_per_sm = blocks_per_sm;
-    b->xchunk = (uint32_t)xchunk;
     // the tile list stays where it is unless it changes: a captured run refers to it
     uint32_t xc[2];
-    tile_lengths(b, xc);
-    if (xc[0] == b->tile_xchunk[0] && xc[1] == b->tile_xchunk[1]) return FDTD_OK;
-    b->tile_xchunk[0] = xc[0];
-    b->tile_xchunk[1] = xc[1];
-    return build_tiles(b);
+    tile_lengths(b, (uint32_t)xchunk, xc);
+    if (xc[0] != b->tile_xchunk[0] || xc[1] != b->tile_xchunk[1]) {
+        const int rc = build_tiles(b, xc);
+        if (rc) return rc;
+    }
+    b->blocks_per_sm = blocks_per_sm;
+    b->xchunk = (uint32_t)xchunk;
+    return FDTD_OK;
 }
 
 int fdtd_batch_run(FdtdBatch *b, void *stream, int32_t nsteps)

@@ -44,3 +44,17 @@ def test_dependent_kernels_read_fields_coherently():
         for arg in re.findall(r"(?<!_)\bldg\(([^;]*?)[,;]", text):
             assert "tab[" in arg or arg.startswith("const T *p"), (name, arg)
     assert set(bodies) < set(_files())
+
+
+def test_a_batch_keeps_its_tiles_until_it_has_new_ones():
+    """A refused allocation must leave a batch that can run: a launch without a tile list would read
+    address zero. What a batch has is therefore touched after the last step that can fail only."""
+    text = _source("batch_abi.cu")
+    body = text[text.index("int build_tiles("):text.index("int make_var(")]
+    fails = body.index("cudaMemcpyHostToDevice")
+    changes = re.findall(r"cudaFree\(b->tiles\)|b->\w+(?:\[\d\])?\s*=[^=]|b->groups\.(?:clear|push_back|swap)", body)
+    assert len(changes) >= 6
+    for m in re.finditer(r"cudaFree\(b->tiles\)|b->\w+(?:\[\d\])?\s*=[^=]|b->groups\.(?:clear|push_back|swap)", body):
+        assert m.start() > fails, m.group()
+    tune = text[text.index("int fdtd_batch_tune("):text.index("int fdtd_batch_run(")]
+    assert tune.index("b->xchunk =") > tune.index("build_tiles(")
